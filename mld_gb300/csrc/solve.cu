@@ -329,7 +329,8 @@ __global__ void __launch_bounds__(1024) k_pcg_alpha(int D, const double* __restr
   }
 }
 
-// p = z + beta p with beta = (r.z)_new / (r.z)_old; first: p = z
+// p = z + beta p with beta = (r.z)_new / (r.z)_old; first: p = z, without reading p (its buffer
+// still holds what the memory held before, possibly NaN)
 __global__ void __launch_bounds__(1024) k_pcg_beta(int D, const double* __restrict__ z, const double* __restrict__ r,
                                                    double* __restrict__ p, double* __restrict__ scal, int first) {
   __shared__ double red[32];
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(1024) k_pcg_beta(int D, const double* __restri
   for (int i = threadIdx.x; i < D; i += blockDim.x) s = fma(r[i], z[i], s);
   const double rz = block_sum(s, red);
   const double beta = (first || !(scal[0] > 0.0)) ? 0.0 : rz / scal[0];
-  for (int i = threadIdx.x; i < D; i += blockDim.x) p[i] = fma(beta, p[i], z[i]);
+  for (int i = threadIdx.x; i < D; i += blockDim.x) p[i] = first ? z[i] : fma(beta, p[i], z[i]);
   __syncthreads();
   if (threadIdx.x == 0) {
     scal[0] = rz;
