@@ -346,14 +346,14 @@ int y_scratch(mld_gpu_handle* h, void** p, size_t* bytes) {
 constexpr int kTuneMinAtoms = 64;
 
 template <typename T>
-int tuned_launch(mld_gpu_handle* h, int mode, T* Bout, T* dB, const DevEval<T>* ev, void* ys, size_t ysb) {
+int tuned_launch(mld_gpu_handle* h, int mode, T* Bout, T* dB, void* ys, size_t ysb) {
   auto& tn = h->tune[mode];
   const int* order = bp_<int>(h, mld_gpu_handle::B_ORDER);
   int* counter = bp_<int>(h, mld_gpu_handle::B_QCNT);
   // only the design-row stage of a fit is tuned: it is repeated on the same batch, while
   // evaluation batches (serving) and descriptor dumps change from call to call
   if (tn.done || mode != 0 || h->A < kTuneMinAtoms * std::max(1, h->nsm)) {
-    CK(launch_bso4<T>(h->dt, h->b, h->bp, Bout, dB, ev, order, counter, h->st, ys, ysb, &tn.best));
+    CK(launch_bso4<T>(h->dt, h->b, h->bp, Bout, dB, order, counter, h->st, ys, ysb, &tn.best));
     return MLD_OK;
   }
   tn.cand.clear();
@@ -367,7 +367,7 @@ int tuned_launch(mld_gpu_handle* h, int mode, T* Bout, T* dB, const DevEval<T>* 
   float best = 0.f;
   for (const Bso4Launch& c : tn.cand) {
     CK(cudaEventRecord(ev0, h->st));
-    CK(launch_bso4<T>(h->dt, h->b, h->bp, Bout, dB, ev, order, counter, h->st, ys, ysb, &c));
+    CK(launch_bso4<T>(h->dt, h->b, h->bp, Bout, dB, order, counter, h->st, ys, ysb, &c));
     CK(cudaEventRecord(ev1, h->st));
     CK(cudaEventSynchronize(ev1));
     float ms = 0.f;
@@ -396,14 +396,13 @@ int prepare_descriptors(mld_gpu_handle* h, bool want_dB, void** ys, size_t* ysb)
 // B and w_ch * dB of the staged batch into B_BOUT / B_DBOUT (dB optional) through the
 // descriptor kernel's queue
 template <typename T>
-int run_descriptors(mld_gpu_handle* h, bool want_dB, const DevEval<T>* ev, T* Bout) {
+int run_descriptors(mld_gpu_handle* h, bool want_dB, T* Bout) {
   void* ys = nullptr;
   size_t ysb = 0;
   int rcy = prepare_descriptors<T>(h, want_dB, &ys, &ysb);
   if (rcy) return rcy;
   T* dB = want_dB ? bp_<T>(h, mld_gpu_handle::B_DBOUT) : nullptr;
-  const int mode = ev ? 1 : (want_dB ? 0 : 2);
-  int rc = tuned_launch<T>(h, mode, Bout, dB, ev, ys, ysb);
+  int rc = tuned_launch<T>(h, want_dB ? 0 : 2, Bout, dB, ys, ysb);
   if (rc) return rc;
   nl(h, 1);
   return MLD_OK;
@@ -469,7 +468,7 @@ int run_rows(mld_gpu_handle* h, const RowLayout& L, bool with_labels, T** Xout) 
     T* dBq = bp_<T>(h, mld_gpu_handle::B_DBOUT);
     // the stage of this batch: descriptor kernel, reverse pairs, linear (and quadratic) rows
     auto stage = [&]() -> int {
-      int rc = run_descriptors<T>(h, true, nullptr, Bq);
+      int rc = run_descriptors<T>(h, true, Bq);
       if (rc) return rc;
       CK(launch_reverse_pairs(h->b, bp_<int>(h, mld_gpu_handle::B_REV), h->st));
       CK(launch_lin_rows<T>(h->b, rows, h->bp, h->KK, bp_<int>(h, mld_gpu_handle::B_REV), Bq, dBq,
@@ -1122,7 +1121,9 @@ int mld_gpu_create(const mld_gpu_config* cfg, mld_gpu_handle** out) {
   h->Dfull = h->DL + (h->quad ? h->KK * h->KK : 0);           // reference layout (dim_design_line)
   h->ldx = round_up4(h->D);
   // device tables
-  e = fill_dev_tables(t, &h->dt, [h](const auto& vec, auto** dst) { return dev_alloc_copy(h, dst, vec.data(), vec.size()); });
+  auto put = [h](const auto& vec, auto** dst) { return dev_alloc_copy(h, dst, vec.data(), vec.size()); };
+  e = fill_dev_tables(t, &h->dt, put);
+  if (e == cudaSuccess) e = fill_deriv_tables(t, &h->dt, put);
   if (e != cudaSuccess) {
     int code = cuda_fail(h, e, "table upload");
     mld_gpu_destroy(h);
@@ -1331,7 +1332,7 @@ int mld_gpu_descriptors(mld_gpu_handle* h, double* B_out, int* n_neigh_out) {
   const size_t nB = (size_t)h->A * h->KK;
   if (h->mixed) {
     CK(ensure(h, mld_gpu_handle::B_BOUT, sizeof(float) * std::max<size_t>(nB, 1)));
-    rc = run_descriptors<float>(h, true, nullptr, bp_<float>(h, mld_gpu_handle::B_BOUT));
+    rc = run_descriptors<float>(h, true, bp_<float>(h, mld_gpu_handle::B_BOUT));
     if (rc) return rc;
     if (B_out) {
       std::vector<float> tmp(nB);
@@ -1342,7 +1343,7 @@ int mld_gpu_descriptors(mld_gpu_handle* h, double* B_out, int* n_neigh_out) {
     }
   } else {
     CK(ensure(h, mld_gpu_handle::B_BOUT, sizeof(double) * std::max<size_t>(nB, 1)));
-    rc = run_descriptors<double>(h, true, nullptr, bp_<double>(h, mld_gpu_handle::B_BOUT));
+    rc = run_descriptors<double>(h, true, bp_<double>(h, mld_gpu_handle::B_BOUT));
     if (rc) return rc;
     if (B_out)
       CK(cudaMemcpyAsync(B_out, bp_<double>(h, mld_gpu_handle::B_BOUT), sizeof(double) * nB, cudaMemcpyDeviceToHost,
@@ -1632,7 +1633,7 @@ int upload_weights(mld_gpu_handle* h, const double* w_full, double** w_dev) {
 
 // ---- evaluation with fitted weights, without design rows (bispectrum.cu eval mode, eval.cu) ----
 // Weights of the reference's full layout [w0, w_lin (KK), W (KK x KK, quadratic)] are kept on
-// the device as w_lin (FP64), w_lin in the descriptor precision, and Wsym = W + W^T (FP64).
+// the device as w_lin and Wsym = W + W^T (FP64) and, for the linear model, the Z-block weights.
 int eval_weights_upload(mld_gpu_handle* h, const double* w_full) {
   if (h->krr) return fail(h, MLD_ERR_UNSUPPORTED, "evaluation without design rows covers ml_type 0 only");
   const int KK = h->KK;
@@ -1645,18 +1646,15 @@ int eval_weights_upload(mld_gpu_handle* h, const double* w_full) {
       for (int j = 0; j < KK; ++j) hw[KK + (size_t)i * KK + j] = W[(size_t)i * KK + j] + W[(size_t)j * KK + i];
   }
   const size_t eb = h->mixed ? sizeof(float) : sizeof(double);
-  CK(ensure(h, mld_gpu_handle::B_EW, sizeof(double) * hw.size() + eb * KK + 256));
+  CK(ensure(h, mld_gpu_handle::B_EW, sizeof(double) * hw.size() + eb * h->nch * h->dt.NBLK + 256));
   double* dw = bp_<double>(h, mld_gpu_handle::B_EW);
   CK(cudaMemcpyAsync(dw, hw.data(), sizeof(double) * hw.size(), cudaMemcpyHostToDevice, h->st));
-  void* wt = dw + hw.size();
-  if (h->mixed) {
-    std::vector<float> f(w_full + 1, w_full + 1 + KK);
-    CK(cudaMemcpyAsync(wt, f.data(), sizeof(float) * KK, cudaMemcpyHostToDevice, h->st));
-    CK(cudaStreamSynchronize(h->st));
-  } else {
-    CK(cudaMemcpyAsync(wt, w_full + 1, sizeof(double) * KK, cudaMemcpyHostToDevice, h->st));
-    CK(cudaStreamSynchronize(h->st));
+  if (!h->quad) {
+    void* g = dw + hw.size();
+    if (h->mixed) CK(launch_eval_gamma<float>(h->dt, nullptr, 1, h->nch, dw, nullptr, 0.0, (float*)g, nullptr, h->st));
+    else CK(launch_eval_gamma<double>(h->dt, nullptr, 1, h->nch, dw, nullptr, 0.0, (double*)g, nullptr, h->st));
   }
+  CK(cudaStreamSynchronize(h->st));
   h->ew0 = w_full[0];
   h->ew_ready = true;
   return MLD_OK;
@@ -1670,39 +1668,37 @@ static int eval_run(mld_gpu_handle* h, double* out) {
   double* S = F + 3 * (size_t)h->A;
   const double* wlin = bp_<double>(h, mld_gpu_handle::B_EW);
   const double* wsym = wlin + KK;
-  const T* wlinT = reinterpret_cast<const T*>(wlin + KK + (h->quad ? (size_t)KK * KK : 0));
-  CK(ensure(h, mld_gpu_handle::B_EPAIR, sizeof(double) * 9 * (size_t)std::max<long long>(1, h->b.P)));
-  CK(ensure(h, mld_gpu_handle::B_EATOM, sizeof(double) * (size_t)std::max(1, h->A)));
+  const T* gammaT = reinterpret_cast<const T*>(wlin + KK + (h->quad ? (size_t)KK * KK : 0));
+  CK(ensure(h, mld_gpu_handle::B_EPAIR, sizeof(T) * 3 * (size_t)std::max<long long>(1, h->b.P)));
+  CK(ensure(h, mld_gpu_handle::B_EATOM, sizeof(double) * 7 * (size_t)std::max(1, h->A)));
   CK(ensure(h, mld_gpu_handle::B_REV, sizeof(int) * (size_t)std::max<long long>(1, h->b.P)));
-  double* Eatom = bp_<double>(h, mld_gpu_handle::B_EATOM);
   DevEval<T> ev;
-  ev.pair = bp_<double>(h, mld_gpu_handle::B_EPAIR);
+  ev.pair = bp_<T>(h, mld_gpu_handle::B_EPAIR);
+  ev.Eatom = bp_<double>(h, mld_gpu_handle::B_EATOM);
+  ev.Satom = ev.Eatom + std::max(1, h->A);
   ev.w0 = h->ew0;
   if (h->quad) {
-    // pass 1: B of every atom; beta_a and the atom energies; pass 2: per-pair forces and stress
-    CK(ensure(h, mld_gpu_handle::B_EB, sizeof(T) * std::max<size_t>(1, (size_t)h->A * KK)));
-    CK(ensure(h, mld_gpu_handle::B_EBETA, sizeof(T) * std::max<size_t>(1, (size_t)h->A * KK)));
+    // B of every atom; its weights and energy; then the evaluation kernel
+    const size_t na = (size_t)std::max(1, h->A);
+    CK(ensure(h, mld_gpu_handle::B_EB, sizeof(T) * na * KK));
+    CK(ensure(h, mld_gpu_handle::B_EBETA, sizeof(T) * na * h->nch * h->dt.NBLK));
     T* B = bp_<T>(h, mld_gpu_handle::B_EB);
-    T* beta = bp_<T>(h, mld_gpu_handle::B_EBETA);
-    int rc = run_descriptors<T>(h, false, nullptr, B);
+    T* gamma = bp_<T>(h, mld_gpu_handle::B_EBETA);
+    int rc = run_descriptors<T>(h, false, B);
     if (rc) return rc;
-    CK(launch_eval_beta<T>(B, h->A, KK, wlin, wsym, h->ew0, beta, Eatom, h->st));
-    ev.beta = beta;
-    ev.beta_per_atom = 1;
-    rc = run_descriptors<T>(h, false, &ev, (T*)nullptr);
-    if (rc) return rc;
+    CK(launch_eval_gamma<T>(h->dt, B, h->A, h->nch, wlin, wsym, h->ew0, gamma, ev.Eatom, h->st));
+    ev.gamma = gamma;
+    ev.per_atom = 1;
     nl(h, 1);
   } else {
-    ev.beta = wlinT;
-    ev.beta_per_atom = 0;
+    ev.gamma = gammaT;
     ev.wlin = wlin;
-    ev.Eatom = Eatom;
-    int rc = run_descriptors<T>(h, false, &ev, (T*)nullptr);
-    if (rc) return rc;
   }
+  CK(launch_bso4_eval<T>(h->dt, h->b, h->bp, ev, bp_<int>(h, mld_gpu_handle::B_ORDER), bp_<int>(h, mld_gpu_handle::B_QCNT),
+                         h->st));
   CK(launch_reverse_pairs(h->b, bp_<int>(h, mld_gpu_handle::B_REV), h->st));
-  CK(launch_eval_gather(h->b, h->bp, bp_<int>(h, mld_gpu_handle::B_REV), ev.pair, Eatom, E, F, S, h->st));
-  nl(h, 3);
+  CK(launch_eval_gather<T>(h->b, h->bp, bp_<int>(h, mld_gpu_handle::B_REV), ev, E, F, S, h->st));
+  nl(h, 4);
   return MLD_OK;
 }
 

@@ -6,8 +6,8 @@
 //            B_k = Re sum conj(c^l) ZA_k                                               (:1014-1143, :469-560)
 //   phase 3  per chunk of neighbours: U/dU recursion -> vecall V = conj(d(f_c U)/du)  (angular_functions.f90:41-273),
 //            dB_k/du_n = w_ch(type_n) Re sum Y V (register-tiled per layer)           (:469-717, descriptors.F90:298-302)
-// Outputs: B per atom and w_ch * dB per pair (the design rows are gathered from them by
-// rows.cu), or, for evaluation with fitted weights, per-pair force and stress contributions.
+// Outputs: B per atom and w_ch * dB per pair (the design rows are gathered from them by rows.cu).
+// Evaluation with fitted weights has a kernel of its own (bispectrum_eval.cu).
 // Only half of every layer is computed (X(-p,-q) = (-1)^((p-q)/2) conj X(p,q) for U, c, Z, V);
 // full-layer sums fold into weighted sums over the half.  The recursions run on lane groups:
 // in phase 1 of 16, 8, 6 or 4 lanes per neighbour (the widest that covers the atom's neighbours
@@ -313,10 +313,9 @@ struct KernelArgs {
   void* yglobal;
   int g1;  // narrowest lane groups per neighbour in phase 1 (4, 6, 8 or 16) the U store allows
   int geo_cap;  // neighbours whose phase-1 geometry records are kept for phase 3 (the rest recompute)
-  // outputs: B (A x nch*K) and w_ch * dB (P x 3 x nch*K); or evaluation (ev.pair != nullptr)
+  // outputs: B (A x nch*K) and w_ch * dB (P x 3 x nch*K)
   T* Bout;
   T* dBout;
-  DevEval<T> ev;
 };
 
 constexpr int kNW = 8;                  // warps per CTA (== kZWarps)
@@ -335,11 +334,11 @@ static_assert(kNW == kZWarps, "phase-2 schedule is built for the CTA's warps");
 //   term buffer; phase 3: vecall of a chunk)
 //   W region (phase 2: CG coefficients; phase 3: recursion buffers, then the chunk's dB by rank:
 //   rank 0 [cols][K], rank 1 [cols][nrank1], rank 2 [cols][nrank2])
-//   Bk[nch*K]  nwt[nch*NB]  nuu[NB*4]  nidx[NB]  pacc[NB*9] (FP64)  next atom
+//   Bk[nch*K]  nwt[nch*NB]  nuu[NB*4]  nidx[NB]  next atom
 //   sc[256] (Y-slot scales)  expand[NU]  half_diag[HU]  bk_off[K+1] (tables staged once per CTA)
 //   geo[geo_cap*kGeo] (geometry records of the atom's first geo_cap neighbours)
 struct SmemPlan {
-  size_t rec, hoff, rowk, tiles, rslot, cfull, Y, V, W, Bk, nwt, nuu, nidx, pacc, next, sc, exp, hd, bko, geo, total;
+  size_t rec, hoff, rowk, tiles, rslot, cfull, Y, V, W, Bk, nwt, nuu, nidx, next, sc, exp, hd, bko, geo, total;
 };
 
 __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~(size_t)15; }
@@ -377,7 +376,6 @@ __host__ __device__ inline SmemPlan smem_plan(const DevTables& tb, int nch, int 
   s.nwt = o;   o = al16(o + (size_t)eb * nch * kNB);
   s.nuu = o;   o = al16(o + (size_t)eb * kNB * 4);
   s.nidx = o;  o = al16(o + sizeof(int) * kNB);
-  s.pacc = o;  o = al16(o + sizeof(double) * kNB * 9);
   s.next = o;  o = al16(o + sizeof(int) * (4 + 3 * kMaxJ + 4 + kRounds));
   s.sc = o;    o = al16(o + (size_t)eb * 256);
   s.exp = o;   o = al16(o + sizeof(int16_t) * tb.NU);
@@ -532,7 +530,6 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
   T* nwt = reinterpret_cast<T*>(smem_raw + sp.nwt);
   T* nuu = reinterpret_cast<T*>(smem_raw + sp.nuu);
   int* nidx = reinterpret_cast<int*>(smem_raw + sp.nidx);
-  double* pacc = reinterpret_cast<double*>(smem_raw + sp.pacc);
   int* snext = reinterpret_cast<int*>(smem_raw + sp.next);
   T* sgeo = reinterpret_cast<T*>(smem_raw + sp.geo);
   T* ssc = reinterpret_cast<T*>(smem_raw + sp.sc);  // ssc[16 n + d] = n / d, the Y-slot scales
@@ -561,8 +558,7 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
   const int zr0 = tb.zitem_off[warp], zr1 = tb.zitem_off[warp + 1];  // this warp's Z rounds
 
   const T rcut = (T)args.p.rcut, inv_r0 = (T)args.p.inv_r0;
-  const bool eval = args.ev.pair != nullptr;
-  const bool need_d = eval || args.dBout != nullptr;
+  const bool need_d = args.dBout != nullptr;
 
   // thread 0 takes the next queue position while the current atom runs; it publishes it at the
   // top of the loop, after at least one barrier that follows every thread's read of the last one
@@ -710,14 +706,6 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
     }
     if (args.Bout)
       for (int e = tid; e < nchK; e += nth) args.Bout[(size_t)atom * nchK + e] = Bk[e];
-    if (args.ev.Eatom && warp == 0) {
-      // linear model: energy of the atom, w0 + w_lin . B_a (FP64, fixed lane order)
-      double e = 0.0;
-      if (nn > 0)
-        for (int k = lane; k < nchK; k += 32) e += args.ev.wlin[k] * (double)Bk[k];
-      for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-      if (lane == 0) args.ev.Eatom[atom] = e + args.ev.w0;
-    }
     if (!need_d || nn == 0) continue;
 
     // ---------------- phase 3: dB per neighbour chunk (kNB neighbours, the last one the rest) -
@@ -766,7 +754,6 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
             nuu[n * 4 + 3] = rinv;
           }
         }
-        if (eval && sl < 9) pacc[min(n, kNB - 1) * 9 + sl] = 0.0;
         if (wide)
           group_recursion<T, 32>(g, srec, J, shoff, ubuf3 + (size_t)grp * 2 * LH, LH,
                                  V + (size_t)min(n, kNB - 1) * 3 * HU, HU, sl, active);
@@ -840,50 +827,7 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
         // element (col, k): lanes take the components k, warps the columns, so each lane looks
         // up its k's rank slots once and a warp's stores are contiguous
         const int nr1 = tb.nrank[1], nr2 = tb.nrank[2];
-        if (eval) {
-          for (int k = lane; k < K; k += 32) {
-            const int s1 = srslot[k * (kRounds - 1)], s2 = srslot[k * (kRounds - 1) + 1];
-            for (int col = warp; col < ncols; col += kNW) {
-              T v = dBs[col * K + k];
-              if (s1 >= 0) v += dB1[col * nr1 + s1];
-              if (s2 >= 0) v += dB2[col * nr2 + s2];
-              dBs[col * K + k] = v;  // in place: own element
-            }
-          }
-          __syncthreads();
-          // forces and stress with the effective weights: the centre's for the forces, the
-          // neighbour's for the stress (the neighbour's B in the quadratic stress rows,
-          // mld_stress.F90:580-603); sums per (neighbour, component) in T, per-pair totals in
-          // FP64 accumulated over the channels in channel order
-          const T* bc = args.ev.beta + (args.ev.beta_per_atom ? (size_t)atom * nchK : 0) + ch * K;
-          for (int it = tid; it < 3 * nb_here; it += nth) {
-            const int n = it / 3, a = it - 3 * n;
-            const T* d = dBs + (size_t)(n * 3 + a) * K;
-            T f = T(0);
-            for (int k = 0; k < K; ++k) f = fma(d[k], bc[k], f);
-            const T wn = nwt[ch * kNB + n];
-            double* pa = pacc + n * 9;
-            pa[a] += (double)(f * wn);
-            T gsum = f;
-            if (args.ev.beta_per_atom) {
-              const T* bn = args.ev.beta + (size_t)nidx[n] * nchK + ch * K;
-              gsum = T(0);
-              for (int k = 0; k < K; ++k) gsum = fma(d[k], bn[k], gsum);
-            }
-            const double gv = (double)(gsum * wn) * (double)nuu[n * 4 + 3];
-            const double ux = nuu[n * 4 + 0], uy = nuu[n * 4 + 1], uz = nuu[n * 4 + 2];
-            if (a == 0) {  // xx, xz, xy
-              pa[3] += gv * ux;
-              pa[7] += gv * uz;
-              pa[8] += gv * uy;
-            } else if (a == 1) {  // yy, yz
-              pa[4] += gv * uy;
-              pa[6] += gv * uz;
-            } else {  // zz
-              pa[5] += gv * uz;
-            }
-          }
-        } else {
+        {
           // w_ch * dB of every pair of the chunk; one channel's columns per pass
           T* out = args.dBout + (size_t)(p0 + base) * 3 * nchK + ch * K;
           for (int k = lane; k < K; k += 32) {
@@ -896,10 +840,6 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
             }
           }
         }
-        __syncthreads();
-      }
-      if (eval) {
-        for (int e = tid; e < nb_here * 9; e += nth) args.ev.pair[(size_t)(p0 + base) * 9 + e] = pacc[e];
         __syncthreads();
       }
     }
@@ -931,8 +871,8 @@ size_t bso4_y_scratch_bytes(const DevTables& tb, int nch, int eb, int max_ctas, 
 
 template <typename T>
 cudaError_t launch_bso4(const DevTables& tb, const DevBatch& b, const BsoParams& p, T* Bout, T* dBout,
-                        const DevEval<T>* ev, const int* order, int* counter, cudaStream_t st, void* yscratch,
-                        size_t yscratch_bytes, const Bso4Launch* shape) {
+                        const int* order, int* counter, cudaStream_t st, void* yscratch, size_t yscratch_bytes,
+                        const Bso4Launch* shape) {
   const Bso4Launch sh = shape ? *shape : Bso4Launch{};
   if (b.A == 0) return cudaSuccess;
   if (!counter) return cudaErrorInvalidValue;
@@ -960,8 +900,6 @@ cudaError_t launch_bso4(const DevTables& tb, const DevBatch& b, const BsoParams&
   a.p = p;
   a.Bout = Bout;
   a.dBout = dBout;
-  if (ev) a.ev = *ev;
-  if (a.ev.pair && dBout) return cudaErrorInvalidValue;
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -1026,10 +964,8 @@ cudaError_t launch_bso4(const DevTables& tb, const DevBatch& b, const BsoParams&
 }
 
 template cudaError_t launch_bso4<double>(const DevTables&, const DevBatch&, const BsoParams&, double*, double*,
-                                         const DevEval<double>*, const int*, int*, cudaStream_t, void*, size_t,
-                                         const Bso4Launch*);
+                                         const int*, int*, cudaStream_t, void*, size_t, const Bso4Launch*);
 template cudaError_t launch_bso4<float>(const DevTables&, const DevBatch&, const BsoParams&, float*, float*,
-                                        const DevEval<float>*, const int*, int*, cudaStream_t, void*, size_t,
-                                        const Bso4Launch*);
+                                        const int*, int*, cudaStream_t, void*, size_t, const Bso4Launch*);
 
 }  // namespace mld

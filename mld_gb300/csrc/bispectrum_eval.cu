@@ -1,0 +1,538 @@
+// Evaluation with fitted weights: per-pair forces, per-atom stress and energy, without dB.
+//
+// With beta = dE/dB_i the force of pair (i, n) is f_c' and U' contracted with the effective
+// y = dE/dc, a sum of the distinct Z blocks with weights gamma (eval.cu), so the K contractions of dB
+// collapse into one per direction.  The directions are the three generators of SU(2)
+// (bispectrum.cuh): dU = U sum_b xi_b rho(T_b), and the generators move to the y side, once per atom:
+//   S_b = Re sum y conj(U rho(T_b)) = sum_e y_b[e] . U[e],   y_0 = y, y_1 = i q y,
+//   y_2 = -i (c- y[q-2] + c+ y[q+2]),  y_3 = c+ y[q+2] - c- y[q-2]
+//   force_a = f_c sum_b xi[a][b] S_b + f_c' e_a S_0.
+// A pair then costs its U (computed once, kept in shared memory from the sum for c) and four dot
+// products of HU complex entries.
+//
+// Persistent CTAs take atoms from a queue.  Per atom: geometry and U of the neighbours (column
+// chains), c, the Z terms, y, the energy (linear model: B from the Z terms), the generators' y_b,
+// the pairs.  An atom with more neighbours than the U store holds is done in passes, whose U is
+// computed again for the pairs.
+//
+// The quadratic model's stress takes the neighbour's beta (the neighbour's B in the quadratic stress
+// rows, mld_stress.F90:580-603): y is formed per neighbour from the Z terms of all channels (one
+// real by complex product per term, a third of a dB contraction), and its dot products are taken
+// with the generators applied to U.
+//
+// Bound: FP32 arithmetic and shared memory; most of an atom's time is its Z terms.  Every sum has a
+// fixed order that does not depend on the batch.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "bispectrum.cuh"
+#include "ds.cuh"
+
+namespace mld {
+
+namespace {
+
+constexpr int kChunk = 16;  // neighbours whose own y is formed at a time (quadratic stress)
+// row stride of the chunk's gamma: 16-byte aligned, few store conflicts
+template <typename T>
+constexpr int kGrow = sizeof(T) == 4 ? 20 : 18;
+
+// A stress sum: FP64, or a double-FP32 pair (the products and sums of FP32 forces and lever arms are
+// then as exact as FP64 ones without its 64 times slower issue).
+template <typename T>
+struct StressSum;
+template <>
+struct StressSum<double> {
+  double v = 0.0;
+  __device__ __forceinline__ void add(double f, double u, double rinv) { v += f * rinv * u; }
+  __device__ __forceinline__ void add(const StressSum& o) { v += o.v; }
+  __device__ __forceinline__ StressSum down(int d) const { return {__shfl_down_sync(0xffffffffu, v, d)}; }
+  __device__ __forceinline__ double value() const { return v; }
+};
+template <>
+struct StressSum<float> {
+  float h = 0.f, l = 0.f;
+  __device__ __forceinline__ void add(float f, float u, float rinv) {
+    const float p = f * rinv, pe = fmaf(f, rinv, -p);
+    ds_fma(h, l, u, p, pe);
+  }
+  __device__ __forceinline__ void add(const StressSum& o) { ds_add(h, l, o.h, o.l); }
+  __device__ __forceinline__ StressSum down(int d) const {
+    return {__shfl_down_sync(0xffffffffu, h, d), __shfl_down_sync(0xffffffffu, l, d)};
+  }
+  __device__ __forceinline__ double value() const { return (double)h + (double)l; }
+};
+
+template <typename T>
+struct EvalArgs {
+  DevTables tb;
+  const GenEntry<T>* gen;
+  const T* cg;
+  PairSource<T> src;
+  const int* atom_struct;
+  const int* small;
+  const int* nbr_off;
+  T chw[kMaxCh * kMaxTypes];
+  T rin[kMaxTypes * kMaxTypes];
+  T sign_big;
+  int nch;
+  const int* order;
+  int* counter;
+  unsigned long long chains;
+  int slots;  // neighbours of the U store
+  DevEval<T> ev;
+};
+
+struct EvalPlan {
+  size_t hoff, exp, hd, sj, cfull, chalf, gamma, bk, cg, tbuf, yb, yt, geo, fcw, red, grow, next, U, total;
+};
+
+__host__ __device__ inline size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
+
+__host__ __device__ inline EvalPlan eval_plan(const DevTables& tb, int nch, int eb, int slots, bool quad) {
+  const size_t cxb = 2 * (size_t)eb;
+  EvalPlan s;
+  size_t o = 0;
+  s.hoff = o;  o = up16(o + sizeof(int) * (kMaxJ + 2));
+  s.exp = o;   o = up16(o + sizeof(int16_t) * tb.NU);
+  s.hd = o;    o = up16(o + tb.HU);
+  s.sj = o;    o = up16(o + tb.HU);
+  s.cfull = o; o = up16(o + cxb * nch * tb.NU);
+  s.chalf = o; o = up16(o + cxb * nch * tb.HU);
+  s.gamma = o; o = up16(o + (size_t)eb * nch * tb.NBLK);
+  s.bk = o;    o = up16(o + (size_t)eb * nch * tb.K);
+  s.cg = o;    o = up16(o + up16((size_t)eb * tb.NCG));
+  // Z terms (of every channel for the quadratic stress) and the generators' y_b (4 * nch * HU complex),
+  // which take the place of the Z terms in the linear model
+  const size_t ny = (size_t)4 * nch * tb.HU, nz = quad ? (size_t)nch * tb.NZT : (tb.NZT > (int)ny ? (size_t)tb.NZT : ny);
+  s.tbuf = o;  o = up16(o + cxb * nz);
+  s.yb = quad ? o : s.tbuf;
+  o = up16(o + (quad ? cxb * ny : 0));
+  s.yt = o;    o = up16(o + cxb * nch * tb.HU);
+  s.geo = o;   o = up16(o + (size_t)eb * kGeo * slots);
+  s.fcw = o;   o = up16(o + (size_t)eb * nch * slots);
+  s.red = o;   o = up16(o + (size_t)eb * (kNW * kChunk * 4));
+  s.grow = o;  o = up16(o + (quad ? (size_t)eb * tb.NBLK * (eb == 4 ? 20 : 18) : 0));
+  s.next = o;  o = up16(o + 16);
+  s.U = o;     o = up16(o + cxb * u_stride(tb.HU) * slots);
+  s.total = o;
+  return s;
+}
+
+// (aa, bb) of the stress components xx yy zz yz xz xy
+__device__ __forceinline__ int stress_a(int c) { return c < 3 ? c : (c == 3 ? 1 : 0); }
+__device__ __forceinline__ int stress_b(int c) { return c < 3 ? c : (c == 5 ? 1 : 2); }
+
+template <typename T, bool kQuad>
+__global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(EvalArgs<T> args, int A) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const DevTables& tb = args.tb;
+  const int J = tb.J, NU = tb.NU, HU = tb.HU, K = tb.K;
+  const int nch = args.nch, nchK = nch * K, nchG = nch * tb.NBLK;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int nth = kNW * 32;
+  const EvalPlan sp = eval_plan(tb, nch, (int)sizeof(T), args.slots, kQuad);
+  int* shoff = reinterpret_cast<int*>(smem_raw + sp.hoff);
+  int16_t* sexp = reinterpret_cast<int16_t*>(smem_raw + sp.exp);
+  int8_t* shd = reinterpret_cast<int8_t*>(smem_raw + sp.hd);
+  int8_t* sj = reinterpret_cast<int8_t*>(smem_raw + sp.sj);  // layer of each half entry
+  cx<T>* cfull = reinterpret_cast<cx<T>*>(smem_raw + sp.cfull);
+  cx<T>* chalf = reinterpret_cast<cx<T>*>(smem_raw + sp.chalf);
+  T* sgam = reinterpret_cast<T*>(smem_raw + sp.gamma);
+  T* Bk = reinterpret_cast<T*>(smem_raw + sp.bk);
+  T* scg = reinterpret_cast<T*>(smem_raw + sp.cg);
+  cx<T>* tbuf = reinterpret_cast<cx<T>*>(smem_raw + sp.tbuf);
+  cx<T>* yb = reinterpret_cast<cx<T>*>(smem_raw + sp.yb);  // [nch][HU][4]
+  cx<T>* yt = reinterpret_cast<cx<T>*>(smem_raw + sp.yt);
+  T* sgeo = reinterpret_cast<T*>(smem_raw + sp.geo);
+  T* fcw = reinterpret_cast<T*>(smem_raw + sp.fcw);
+  T* red = reinterpret_cast<T*>(smem_raw + sp.red);
+  T* grow = reinterpret_cast<T*>(smem_raw + sp.grow);
+  int* snext = reinterpret_cast<int*>(smem_raw + sp.next);
+  cx<T>* Us = reinterpret_cast<cx<T>*>(smem_raw + sp.U);
+  const int HS = u_stride(HU);
+  auto geo = [&](int n) { return sgeo + (size_t)n * kGeo; };
+
+  // tables, once per CTA
+  for (int e = tid; e < kMaxJ + 2; e += nth) shoff[e] = tb.hoff[e];
+  for (int e = tid; e < NU; e += nth) sexp[e] = tb.expand[e];
+  for (int e = tid; e < HU; e += nth) {
+    shd[e] = tb.half_diag[e];
+    int j = 0;
+    while (j < J && tb.hoff[j + 1] <= e) ++j;
+    sj[e] = (int8_t)j;
+  }
+  for (int e = tid; e < tb.NCG; e += nth) scg[e] = args.cg[e];
+  if constexpr (!kQuad) {
+    for (int e = tid; e < nchG; e += nth) sgam[e] = args.ev.gamma[e];
+  }
+  const int zr0 = tb.zitem_off[warp], zr1 = tb.zitem_off[warp + 1];
+
+  int nxt = 0;
+  if (tid == 0) nxt = atomicAdd(args.counter, 1);
+  for (;;) {
+    if (tid == 0) snext[0] = nxt;
+    __syncthreads();  // also orders the table staging and the previous atom's last reads
+    const int qi = snext[0];
+    if (qi >= A) break;
+    if (tid == 0) nxt = atomicAdd(args.counter, 1);
+    const int atom = args.order ? args.order[qi] : qi;
+    const int ti = args.src.types[atom];
+    const int p0 = args.nbr_off[atom];
+    const int nn = args.nbr_off[atom + 1] - p0;
+    if constexpr (kQuad) {
+      for (int e = tid; e < nchG; e += nth) sgam[e] = args.ev.gamma[(size_t)atom * nchG + e];
+    }
+    const int npass = (nn + args.slots - 1) / args.slots;
+    // geometry and U of the neighbours of one pass
+    auto load_pass = [&](int base, int count) {
+      for (int n = tid; n < count; n += nth) {
+        T* g = geo(n);
+        pair_geometry<T>(args.src, args.rin, (size_t)(p0 + base + n), ti, g);
+        const int tn = reinterpret_cast<int*>(g + kGeoIdx)[1];
+        for (int ch = 0; ch < nch; ++ch) fcw[n * nch + ch] = g[kGeoFc] * args.chw[ch * args.src.ntypes + tn];
+        Us[(size_t)n * HS] = {T(1), T(0)};
+      }
+      __syncthreads();
+      u_store<T>(Us, HS, count, J, args.chains, warp, lane, geo);
+      __syncthreads();
+    };
+    // ---- c -----------------------------------------------------------------------------------
+    for (int ps = 0; ps < npass; ++ps) {
+      const int base = ps * args.slots, count = min(args.slots, nn - base);
+      load_pass(base, count);
+      c_sum<T>(chalf, Us, HS, fcw, shd, count, nch, HU, ps == 0, ps == npass - 1, tid);
+      __syncthreads();
+    }
+    if (npass == 0) {  // no neighbours: c is the identity
+      for (int e = tid; e < nch * HU; e += nth) chalf[e] = {shd[e % HU] ? T(1) : T(0), T(0)};
+      __syncthreads();
+    }
+    for (int e = tid; e < nch * NU; e += nth) {
+      const int ch = e / NU, f = e - ch * NU;
+      cfull[e] = fetch(chalf + ch * HU, sexp[f]);
+    }
+    __syncthreads();
+    // ---- Z terms, y, and B (linear model) ------------------------------------------------------
+    for (int ch = 0; ch < nch; ++ch) {
+      cx<T>* zt = tbuf + (kQuad ? (size_t)ch * tb.NZT : 0);
+      z_rounds<T>(tb.zitems, zr0, zr1, cfull + ch * NU, scg, zt, lane);
+      __syncthreads();
+      // y of each half entry: the blocks of its layer with their weights, in order
+      const T* gc = sgam + ch * tb.NBLK;
+      for (int h = tid; h < HU; h += nth) {
+        const int j = sj[h], H = shoff[j + 1] - shoff[j];
+        const cx<T>* z = zt + tb.zoff[j] + (h - shoff[j]);
+        const T* g = gc + tb.blk_off[j];
+        const int nb = tb.blk_off[j + 1] - tb.blk_off[j];
+        cx<T> v = {T(0), T(0)};
+#pragma unroll 4
+        for (int r = 0; r < nb; ++r) {
+          const cx<T> zr = z[r * H];
+          v.x = fma(g[r], zr.x, v.x);
+          v.y = fma(g[r], zr.y, v.y);
+        }
+        yt[ch * HU + h] = v;
+      }
+      if constexpr (!kQuad) {
+        b_sums<T>(tb.trz, K, shoff, chalf + ch * HU, zt, warp, lane, Bk + ch * K);
+        __syncthreads();
+      }
+    }
+    if constexpr (kQuad) __syncthreads();
+    if constexpr (!kQuad) {
+      if (warp == 0) {  // energy of the atom, w0 + w_lin . B_a (FP64, fixed lane order)
+        double e = 0.0;
+        if (nn > 0)
+          for (int k = lane; k < nchK; k += 32) e += args.ev.wlin[k] * (double)Bk[k];
+        for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+        if (lane == 0) args.ev.Eatom[atom] = e + args.ev.w0;
+      }
+    }
+    if (nn == 0) {
+      if (tid < 6) args.ev.Satom[(size_t)atom * 6 + tid] = 0.0;
+      continue;
+    }
+    // ---- the generators' y_b, weighted for sums over the half layers ---------------------------
+    for (int e = tid; e < nch * HU; e += nth) {
+      const int ch = e / HU, h = e - ch * HU;
+      const GenEntry<T> g = args.gen[h];
+      const cx<T>* y = yt + ch * HU;
+      const cx<T> y0 = y[h], ym = y[max(h - 1, 0)];
+      cx<T> yp = y[min(h + 1, HU - 1)];
+      if (g.w == T(1)) yp = {-ym.x, ym.y};  // centre of an even layer: y(0, 2) = -conj y(0, -2)
+      const cx<T> a = {g.cm * ym.x, g.cm * ym.y}, b = {g.cp * yp.x, g.cp * yp.y};
+      const T w = g.w, qw = g.q * g.w;
+      cx<T>* o = yb + (size_t)e * 4;
+      o[0] = {w * y0.x, w * y0.y};
+      o[1] = {-qw * y0.y, qw * y0.x};
+      o[2] = {w * (a.y + b.y), -w * (a.x + b.x)};
+      o[3] = {w * (b.x - a.x), w * (b.y - a.y)};
+    }
+    __syncthreads();
+    // ---- pairs: forces (and, linear model, stress) ---------------------------------------------
+    const T lev = args.small[args.atom_struct[atom]] ? T(1) : -args.sign_big;  // stress lever arm: sign * u
+    StressSum<T> sacc;  // of this thread's (pair slot, component)
+    for (int ps = npass - 1; ps >= 0; --ps) {
+      const int base = ps * args.slots, count = min(args.slots, nn - base);
+      if (ps != npass - 1) load_pass(base, count);  // (the last pass is still in shared memory)
+      for (int g4 = warp * 4; g4 < count; g4 += kNW * 4) {
+        // a warp takes four pairs, its lanes the half entries
+        T tot[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) tot[i] = T(0);
+        const cx<T>* up[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) up[i] = Us + (size_t)min(g4 + i, count - 1) * HS;
+        for (int ch = 0; ch < nch; ++ch) {
+          cx<T> acc[4][4];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) acc[i >> 2][i & 3] = {T(0), T(0)};
+          const cx<T>* yc = yb + (size_t)ch * HU * 4;
+          for (int e = lane; e < HU; e += 32) {
+            cx<T> y[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) y[b] = yc[e * 4 + b];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const cx<T> u = up[i][e];
+#pragma unroll
+              for (int b = 0; b < 4; ++b) acc[i][b] = fma2(y[b], u, acc[i][b]);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int tn = reinterpret_cast<const int*>(geo(min(g4 + i, count - 1)) + kGeoIdx)[1];
+            const T w = args.chw[ch * args.src.ntypes + tn];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) tot[i * 4 + b] = fma(w, acc[i][b].x + acc[i][b].y, tot[i * 4 + b]);
+          }
+        }
+        // sums over the lanes: lane l ends with value l / 2 (pair l / 8, direction (l / 2) % 4)
+#pragma unroll
+        for (int s = 8; s > 0; s >>= 1) {
+          const bool hi = lane & (2 * s);
+#pragma unroll
+          for (int i = 0; i < s; ++i) {
+            const T keep = hi ? tot[i + s] : tot[i], send = hi ? tot[i] : tot[i + s];
+            tot[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * s);
+          }
+        }
+        const T v = tot[0] + __shfl_xor_sync(0xffffffffu, tot[0], 1);
+        // forces on lanes (pair, component) = (l / 3, l % 3) < 12
+        const int fi = min(lane / 3, 3), fa = lane % 3;
+        T S[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) S[b] = __shfl_sync(0xffffffffu, v, (fi * 4 + b) * 2);
+        const T* g = geo(min(g4 + fi, count - 1));
+        const T* xi = g + kGeoXi + 3 * fa;
+        const T f = fma(g[kGeoFc], fma(xi[0], S[1], fma(xi[1], S[2], xi[2] * S[3])), g[kGeoDfr + fa] * S[0]);
+        if (lane < 12 && g4 + fi < count) args.ev.pair[(size_t)(p0 + base + g4 + fi) * 3 + fa] = f;
+        if constexpr (!kQuad) {
+          // stress on lanes (pair, component) = (l / 6, l % 6) < 24
+          const int si = min(lane / 6, 3), sc = lane % 6;
+          const T fs = __shfl_sync(0xffffffffu, f, si * 3 + stress_a(sc));
+          const T* gs = geo(min(g4 + si, count - 1));
+          if (lane < 24 && g4 + si < count)
+            sacc.add(fs, lev * gs[kGeoU + stress_b(sc)], gs[kGeoU + 3]);
+        }
+      }
+      if constexpr (kQuad) {
+        // stress with the neighbours' beta, kChunk neighbours at a time: thread (4 neighbours, entry)
+        const int nt = tid & 3;
+        for (int c0 = 0; c0 < count; c0 += kChunk) {
+          T tot[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) tot[i] = T(0);
+          const cx<T>* up[4];
+          T wn[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) up[i] = Us + (size_t)min(c0 + nt * 4 + i, count - 1) * HS;
+          for (int ch = 0; ch < nch; ++ch) {
+            __syncthreads();  // the previous weights have been read
+            for (int e = tid; e < kChunk * tb.NBLK; e += nth) {
+              const int n = e / tb.NBLK, r = e - n * tb.NBLK;
+              T g = T(0);
+              if (c0 + n < count) {
+                const int nb = reinterpret_cast<const int*>(geo(c0 + n) + kGeoIdx)[0];
+                g = args.ev.gamma[(size_t)nb * nchG + ch * tb.NBLK + r];
+              }
+              grow[r * kGrow<T> + n] = g;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int tn = reinterpret_cast<const int*>(geo(min(c0 + nt * 4 + i, count - 1)) + kGeoIdx)[1];
+              wn[i] = args.chw[ch * args.src.ntypes + tn];
+            }
+            const cx<T>* zc = tbuf + (size_t)ch * tb.NZT;
+            for (int e = tid >> 2; e < HU; e += nth / 4) {
+              const int j = sj[e], H = shoff[j + 1] - shoff[j], nb = tb.blk_off[j + 1] - tb.blk_off[j];
+              const cx<T>* z = zc + tb.zoff[j] + (e - shoff[j]);
+              const T* gr = grow + (size_t)tb.blk_off[j] * kGrow<T> + nt * 4;
+              cx<T> y[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) y[i] = {T(0), T(0)};
+#pragma unroll 4
+              for (int r = 0; r < nb; ++r) {
+                const cx<T> zr = z[r * H];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const T b = gr[r * kGrow<T> + i];
+                  y[i].x = fma(b, zr.x, y[i].x);
+                  y[i].y = fma(b, zr.y, y[i].y);
+                }
+              }
+              const GenEntry<T> g = args.gen[e];
+              const int em = max(e - 1, 0), ep = min(e + 1, HU - 1);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                // w y . (U, T1 U, T2 U, T3 U)
+                const cx<T> u = up[i][e], um = up[i][em];
+                cx<T> uq = up[i][ep];
+                if (g.w == T(1)) uq = {-um.x, um.y};
+                const cx<T> a = {g.cm * um.x, g.cm * um.y}, b = {g.cp * uq.x, g.cp * uq.y};
+                const cx<T> s = {a.x + b.x, a.y + b.y}, d = {a.x - b.x, a.y - b.y};
+                const T wg = g.w * wn[i];
+                const cx<T> yw = {wg * y[i].x, wg * y[i].y};
+                tot[i * 4 + 0] = fma(yw.x, u.x, fma(yw.y, u.y, tot[i * 4 + 0]));
+                tot[i * 4 + 1] = fma(g.q, fma(yw.x, u.y, -(yw.y * u.x)), tot[i * 4 + 1]);
+                tot[i * 4 + 2] = fma(-yw.x, s.y, fma(yw.y, s.x, tot[i * 4 + 2]));
+                tot[i * 4 + 3] = fma(yw.x, d.x, fma(yw.y, d.y, tot[i * 4 + 3]));
+              }
+            }
+          }
+          // sums over the lanes of equal nt: a lane ends with two of its 16 values
+#pragma unroll
+          for (int s = 8; s > 1; s >>= 1) {
+            const bool hi = lane & (2 * s);
+#pragma unroll
+            for (int i = 0; i < s; ++i) {
+              const T keep = hi ? tot[i + s] : tot[i], send = hi ? tot[i] : tot[i + s];
+              tot[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * s);
+            }
+          }
+          const int vi = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2;
+          __syncthreads();  // red is free
+          red[(warp * kChunk + nt * 4 + (vi >> 2)) * 4 + (vi & 3)] = tot[0];
+          red[(warp * kChunk + nt * 4 + (vi >> 2)) * 4 + (vi & 3) + 1] = tot[1];
+          __syncthreads();
+          if (tid < kChunk * 6 && c0 + tid / 6 < count) {
+            const int n = tid / 6, sc = tid - n * 6, aa = stress_a(sc);
+            T S[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+              S[b] = T(0);
+              for (int w = 0; w < kNW; ++w) S[b] += red[(w * kChunk + n) * 4 + b];
+            }
+            const T* g = geo(c0 + n);
+            const T* xi = g + kGeoXi + 3 * aa;
+            const T f = fma(g[kGeoFc], fma(xi[0], S[1], fma(xi[1], S[2], xi[2] * S[3])), g[kGeoDfr + aa] * S[0]);
+            sacc.add(f, lev * g[kGeoU + stress_b(sc)], g[kGeoU + 3]);
+          }
+        }
+      }
+      if (ps > 0) __syncthreads();  // the pass's U and geometry have been read
+    }
+    // stress of the atom: the partial sums of (slot, component), slots in order
+    StressSum<T>* sred = reinterpret_cast<StressSum<T>*>(red);
+    if constexpr (kQuad) {
+      __syncthreads();
+      if (tid < kChunk * 6) sred[tid] = sacc;
+      __syncthreads();
+      if (tid < 6) {
+        StressSum<T> v;
+        for (int n = 0; n < kChunk; ++n) v.add(sred[n * 6 + tid]);
+        args.ev.Satom[(size_t)atom * 6 + tid] = v.value();
+      }
+    } else {
+      if (lane < 24) sred[warp * 24 + lane] = sacc;
+      __syncthreads();
+      if (warp == 0) {
+        StressSum<T> v;
+        if (lane < 24)
+          for (int w = 0; w < kNW; ++w) v.add(sred[w * 24 + lane]);
+        v.add(v.down(12));  // slots (0 + 2) and (1 + 3), then both
+        v.add(v.down(6));
+        if (lane < 6) args.ev.Satom[(size_t)atom * 6 + lane] = v.value();
+      }
+    }
+  }
+}
+
+int max_optin() {
+  static int v = 0;
+  if (!v) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  }
+  return v;
+}
+
+}  // namespace
+
+template <typename T>
+cudaError_t launch_bso4_eval(const DevTables& tb, const DevBatch& b, const BsoParams& p, const DevEval<T>& ev,
+                             const int* order, int* counter, cudaStream_t st) {
+  if (b.A == 0) return cudaSuccess;
+  if (!counter || !ev.pair || !ev.Satom || !tb.gen32) return cudaErrorInvalidValue;
+  const bool quad = ev.per_atom != 0;
+  EvalArgs<T> a{};
+  a.tb = tb;
+  if constexpr (sizeof(T) == 8) {
+    a.gen = reinterpret_cast<const GenEntry<T>*>(tb.gen64);
+    a.cg = reinterpret_cast<const T*>(tb.cg64);
+  } else {
+    a.gen = reinterpret_cast<const GenEntry<T>*>(tb.gen32);
+    a.cg = reinterpret_cast<const T*>(tb.cg32);
+  }
+  a.src = {b.types, b.nbr_idx, b.nbr_u, sizeof(T) == 4 ? b.nbr_u32 : nullptr, (T)p.rcut, (T)p.inv_r0,
+           (T)p.rin_width, p.ntypes, p.has_rin};
+  a.atom_struct = b.atom_struct;
+  a.small = b.small;
+  a.nbr_off = b.nbr_off;
+  for (int e = 0; e < kMaxCh * kMaxTypes; ++e) a.chw[e] = (T)p.chw[e];
+  for (int e = 0; e < kMaxTypes * kMaxTypes; ++e) a.rin[e] = (T)p.rin[e];
+  a.sign_big = (T)p.sign_big;
+  a.nch = p.nch;
+  a.order = order;
+  a.counter = counter;
+  a.chains = chain_order(tb.J);
+  a.ev = ev;
+  // the largest U store (up to 64 neighbours) that keeps the CTAs per SM of a 32-neighbour one (at
+  // most two: registers); it depends on the configuration only, not on the batch
+  const size_t per_sm = 228 * 1024;
+  auto bytes = [&](int slots) { return eval_plan(tb, p.nch, (int)sizeof(T), slots, quad).total; };
+  const size_t want = std::min<size_t>(sizeof(T) == 4 ? 2 : 1, per_sm / (bytes(32) + 1024));
+  a.slots = 8;
+  for (int s = 64; s > 8; s -= 4)
+    if (bytes(s) <= (size_t)max_optin() && per_sm / (bytes(s) + 1024) >= std::max<size_t>(want, 1)) {
+      a.slots = s;
+      break;
+    }
+  const size_t smem = bytes(a.slots);
+  if (smem > (size_t)max_optin()) return cudaErrorInvalidConfiguration;
+  auto kern = quad ? k_bso4_eval<T, true> : k_bso4_eval<T, false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int dev = 0, nsm = 0, occ = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kNW * 32, smem);
+  if (e != cudaSuccess) return e;
+  if (occ < 1) return cudaErrorInvalidConfiguration;
+  const long long grid = std::min<long long>((long long)b.A, (long long)nsm * occ);
+  e = cudaMemsetAsync(counter, 0, sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  kern<<<(unsigned)grid, kNW * 32, smem, st>>>(a, b.A);
+  return cudaGetLastError();
+}
+
+template cudaError_t launch_bso4_eval<double>(const DevTables&, const DevBatch&, const BsoParams&,
+                                              const DevEval<double>&, const int*, int*, cudaStream_t);
+template cudaError_t launch_bso4_eval<float>(const DevTables&, const DevBatch&, const BsoParams&,
+                                             const DevEval<float>&, const int*, int*, cudaStream_t);
+
+}  // namespace mld

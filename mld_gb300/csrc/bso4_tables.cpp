@@ -202,26 +202,48 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
     *err = "contraction tables exceed 16-bit offsets";
     return false;
   }
-  // Z outputs with identical operands (the same c entries, CG lists and extents, e.g. the ZA
-  // block of one triple and the ZB block of another) are one computation: each is evaluated
-  // once, into the term buffer at its computation index, and every slot reads it there with its
-  // own scale
+  // Z blocks with identical operands (e.g. the ZA block of one triple and the ZB block of another)
+  // are one computation: each is evaluated once, into the term buffer, and every slot reads it
+  // there with its own scale.  The term buffer is ordered by output layer, block and half entry.
   std::vector<int> zu(t->zterms.size());
   std::vector<int> zrep;  // representative output of each computation
+  std::map<std::tuple<int, int, int>, int> blkid;  // (jA, jB, jO) -> block within the layer jO
   {
-    std::map<std::tuple<int, int, int, int, int, int, int, int>, int> ids;
-    for (size_t zi = 0; zi < t->zterms.size(); ++zi) {
-      const ZTerm& z = t->zterms[zi];
-      const auto key = std::make_tuple((int)z.i1, (int)z.i2, (int)z.cg1, (int)z.cg2, (int)z.na, (int)z.nb, (int)z.s1,
-                                       (int)z.s2);
-      auto it = ids.find(key);
-      if (it == ids.end()) {
-        it = ids.emplace(key, (int)zrep.size()).first;
-        zrep.push_back((int)zi);
-      }
-      zu[zi] = it->second;
+    std::vector<int> nb(J + 1, 0);
+    for (int k = 0; k < t->K; ++k)
+      for (const Block& B : kblocks[k])
+        if (blkid.emplace(std::make_tuple(B.jA, B.jB, B.jO), nb[B.jO]).second) ++nb[B.jO];
+    int z = 0;
+    for (int j = 0; j <= J; ++j) {
+      t->blk_off[j] = t->nblk;
+      t->zoff[j] = z;
+      t->nblk += nb[j];
+      z += nb[j] * H(j);
     }
-    t->nzu = (int)zrep.size();
+    t->blk_off[J + 1] = t->nblk;
+    t->nzu = z;
+    zrep.assign(z, -1);
+    for (int k = 0; k < t->K; ++k)
+      for (const Block& B : kblocks[k]) {
+        const int u0 = t->zoff[B.jO] + blkid[std::make_tuple(B.jA, B.jB, B.jO)] * H(B.jO);
+        for (int e = 0; e < H(B.jO); ++e) {
+          zu[B.first + e] = u0 + e;
+          if (zrep[u0 + e] < 0) zrep[u0 + e] = B.first + e;
+        }
+      }
+    std::vector<std::vector<GammaItem>> gam(t->nblk);
+    for (int k = 0; k < t->K; ++k)
+      for (int b = 0; b < 3; ++b) {
+        const Block& B = kblocks[k][b];
+        const int r = blkid[std::make_tuple(B.jA, B.jB, B.jO)];
+        gam[t->blk_off[B.jO] + r].push_back(GammaItem{(uint16_t)k, (uint8_t)B.snum, (uint8_t)B.sden});
+        if (b == 0) t->trz.push_back(TripleZ{(uint16_t)(t->zoff[B.jO] + r * H(B.jO)), (uint16_t)B.jO});
+      }
+    for (const auto& v : gam) {
+      t->gam_off.push_back((int)t->gam.size());
+      t->gam.insert(t->gam.end(), v.begin(), v.end());
+    }
+    t->gam_off.push_back((int)t->gam.size());
   }
 
   // layer-blocked Y: rows of layer j are the triples using layer j (any of l, l1, l2).  A
@@ -289,6 +311,31 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
   // row tiles of the dB contraction, heaviest layers first
   for (int j = J; j >= 0; --j)
     for (int rt = 0; rt < t->Mp[j] / kRowTile; ++rt) t->tiles.push_back((j << 8) | rt);
+
+  // generators on the half layers; the Z blocks of every contraction row
+  t->gen.assign(4 * (size_t)HU, 0.0);
+  for (int j = 0; j <= J; ++j)
+    for (int e = 0; e < H(j); ++e) {
+      const int p = -j + 2 * (e / (j + 1)), q = -j + 2 * (e % (j + 1));
+      double* g = &t->gen[4 * (size_t)(t->hoff[j] + e)];
+      g[0] = std::sqrt((double)((j + q) / 2) * (double)((j - q) / 2 + 1));
+      g[1] = std::sqrt((double)((j - q) / 2) * (double)((j + q) / 2 + 1));
+      g[2] = (double)q;
+      g[3] = (p == 0 && q == 0) ? 1.0 : 2.0;
+    }
+  for (int j = 0; j <= J; ++j)
+    for (int k : rows[j]) {
+      RowSource rs{};
+      if (k >= 0)
+        for (const Block& B : kblocks[k]) {
+          if (B.jO != j) continue;
+          rs.z[rs.nterm] = (uint16_t)(t->zoff[j] + blkid[std::make_tuple(B.jA, B.jB, B.jO)] * H(j));
+          rs.snum[rs.nterm] = (uint8_t)B.snum;
+          rs.sden[rs.nterm] = (uint8_t)B.sden;
+          ++rs.nterm;
+        }
+      t->rowsrc.push_back(rs);
+    }
 
   // folded slots; the kernel's slot entries; the ZA entries of every triple for B
   std::vector<std::vector<BkItem>> bk(t->K);

@@ -85,6 +85,25 @@ struct BkItem {
 static_assert(sizeof(BkItem) == 8, "B items are 8 bytes");
 static_assert(offsetof(BkItem, ufull) == 2 && offsetof(BkItem, wgt) == 4, "BkItem layout (decoded by the descriptor kernel)");
 
+// Layer l of a triple and the first term of its ZA block: B_k = sum_e w_e Re(conj(c^l[e]) Z[za + e]).
+struct TripleZ {
+  uint16_t za;
+  uint16_t l;
+};
+// A contribution of triple k to the weight of a Z block.
+struct GammaItem {
+  uint16_t k;
+  uint8_t snum, sden;
+};
+// A contraction row (triple, layer): Y[e] = w_e sum_t (snum_t / sden_t) Z[z_t + e], nterm <= 3 (0: padding).
+struct alignas(16) RowSource {
+  uint16_t z[3];
+  uint16_t nterm;
+  uint8_t snum[3], sden[3];
+  uint16_t pad;
+};
+static_assert(sizeof(RowSource) == 16, "row sources are 16 bytes");
+
 // Packed per-entry recursion record of the half layers (one 16-byte load per entry).  tz and tx
 // (>= 0 in the tables) are stored with the sign that selects the entry's Z / conj(Z) and X
 // (+ for qneg != 0), so the kernel takes their magnitudes with fabs.
@@ -133,6 +152,22 @@ struct Bso4Tables {
   std::vector<int16_t> rec_sz, rec_sx;
   std::vector<int8_t> rec_qneg;
   std::vector<int16_t> expand;  // full index -> encoded half source
+  // generators on the half layers (4 values per entry (j, p, q)): c- = sqrt((j+q)/2 ((j-q)/2 + 1)) and
+  // c+ = sqrt((j-q)/2 ((j+q)/2 + 1)), the weights of the entries at q - 2 and q + 2; q; the entry's
+  // weight in a sum over full layers (2; 1 on the centre (0, 0) of an even layer, whose entry at
+  // q + 2 is -conj of the one at q - 2)
+  std::vector<double> gen;
+  // the distinct Z blocks (jA, jB -> jO), grouped by output layer: block r of layer j holds the terms
+  // zoff[j] + r * H_j + e of its half entries e, so sums over blocks or entries need no index lists
+  int nblk = 0;
+  int blk_off[kMaxJ + 2] = {0};
+  int zoff[kMaxJ + 1] = {0};
+  // dE/dB_k = beta_k weighs block b with gamma_b = sum over [gam_off[b], gam_off[b + 1]) of
+  // (snum / sden) beta_k
+  std::vector<int> gam_off;
+  std::vector<GammaItem> gam;
+  std::vector<TripleZ> trz;       // the ZA block and layer of each triple
+  std::vector<RowSource> rowsrc;  // the blocks of every contraction row, indexed as rowk
   std::vector<int8_t> half_diag;  // half entries on the diagonal p == q (get the +1 of c)
   long long cg_terms = 0;       // CG products evaluated per channel (half outputs)
   long long cg_terms_full = 0;  // CG products of the unfolded contraction (reference count)
@@ -142,10 +177,21 @@ struct Bso4Tables {
 bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err);
 double cg_coefficient(int j1, int m1, int j2, int m2, int j, int m);  // doubled indices
 
+// A half-layer entry's generator weights and weight in full-layer sums (Bso4Tables::gen).
+template <typename T>
+struct alignas(16) GenEntry {
+  T cm, cp, q, w;
+};
+
 // Device copies of the tables.
 struct DevTables {
   int J = 0, NU = 0, HU = 0, K = 0, NS = 0, NYP = 0, NTILE = 0, NZT = 0, NROWS = 0;
   int NCG = 0;  // entries of the 1-D CG coefficient table
+  int NBLK = 0;
+  int blk_off[kMaxJ + 2] = {0};
+  int zoff[kMaxJ + 1] = {0};
+  TripleZ* trz = nullptr;         // K
+  RowSource* rowsrc = nullptr;    // NROWS
   int hoff[kMaxJ + 2] = {0};
   int Mp[kMaxJ + 1] = {0};
   int yoff[kMaxJ + 1] = {0};
@@ -165,6 +211,11 @@ struct DevTables {
   SlotEntry* slots = nullptr;   // NS
   int* bk_off = nullptr;        // K + 1
   BkItem* bk_items = nullptr;
+  // tables of the derivatives and the evaluation (fill_deriv_tables)
+  GenEntry<float>* gen32 = nullptr;   // HU
+  GenEntry<double>* gen64 = nullptr;  // HU
+  int* gam_off = nullptr;       // NBLK + 1
+  GammaItem* gam = nullptr;
 };
 
 // Packed recursion records from the table vectors.
@@ -194,6 +245,9 @@ cudaError_t fill_dev_tables(const Bso4Tables& t, DevTables* d, Put put) {
   d->NZT = t.nzu;
   d->NROWS = (int)t.rowk.size();
   d->NCG = (int)t.cg.size();
+  d->NBLK = t.nblk;
+  for (int j = 0; j <= t.J + 1; ++j) d->blk_off[j] = t.blk_off[j];
+  for (int j = 0; j <= t.J; ++j) d->zoff[j] = t.zoff[j];
   for (int j = 0; j <= t.J + 1; ++j) {
     d->hoff[j] = t.hoff[j];
     d->rowk_off[j] = t.rowk_off[j];
@@ -223,10 +277,29 @@ cudaError_t fill_dev_tables(const Bso4Tables& t, DevTables* d, Put put) {
   if (e == cudaSuccess) e = put(r32, &d->rec32);
   if (e == cudaSuccess) e = put(r64, &d->rec64);
   if (e == cudaSuccess) e = put(t.zitems, &d->zitems);
+  if (e == cudaSuccess) e = put(t.trz, &d->trz);
+  if (e == cudaSuccess) e = put(t.rowsrc, &d->rowsrc);
   if (e == cudaSuccess) e = put(t.zitem_off, &d->zitem_off);
   if (e == cudaSuccess) e = put(t.slots, &d->slots);
   if (e == cudaSuccess) e = put(t.bk_off, &d->bk_off);
   if (e == cudaSuccess) e = put(t.bk_items, &d->bk_items);
+  return e;
+}
+
+// Device tables that only derivatives and evaluation need, placed like those of fill_dev_tables.
+template <class Put>
+cudaError_t fill_deriv_tables(const Bso4Tables& t, DevTables* d, Put put) {
+  std::vector<GenEntry<float>> g32(t.HU);
+  std::vector<GenEntry<double>> g64(t.HU);
+  for (int h = 0; h < t.HU; ++h) {
+    const double* g = &t.gen[4 * (size_t)h];
+    g32[h] = {(float)g[0], (float)g[1], (float)g[2], (float)g[3]};
+    g64[h] = {g[0], g[1], g[2], g[3]};
+  }
+  cudaError_t e = put(g32, &d->gen32);
+  if (e == cudaSuccess) e = put(g64, &d->gen64);
+  if (e == cudaSuccess) e = put(t.gam_off, &d->gam_off);
+  if (e == cudaSuccess) e = put(t.gam, &d->gam);
   return e;
 }
 
@@ -309,17 +382,18 @@ cudaError_t launch_sort_lists(const DevBatch& b, cudaStream_t st);
 // does not fit in shared memory, and preferred (unless only_if_required) when it would cost a
 // resident CTA per SM; 0 otherwise.
 size_t bso4_y_scratch_bytes(const DevTables& tb, int nch, int eb, int max_ctas, bool only_if_required = false);
-// Evaluation with fitted weights instead of design rows: per-pair force and stress
-// contributions of dE/dB_a (beta_a = w_lin for the linear model; w_lin + (W + W^T) B_a for the
-// quadratic one), gathered into E/F/S by launch_eval_gather.
+// Evaluation with fitted weights (bispectrum_eval.cu): per-pair forces and per-atom stress of
+// dE/dB_a (beta_a = w_lin for the linear model; w_lin + (W + W^T) B_a for the quadratic one),
+// gathered into E/F/S by launch_eval_gather.  The weights come as gamma, per Z block and channel.
 template <typename T>
 struct DevEval {
-  const T* beta = nullptr;       // one vector (nch*K) or one per atom (A x nch*K)
-  int beta_per_atom = 0;
+  const T* gamma = nullptr;      // one vector (nch * NBLK) or one per atom
+  int per_atom = 0;
   const double* wlin = nullptr;  // linear weights: the kernel writes Eatom = w0 + w_lin . B_a (linear model)
   double w0 = 0.0;
-  double* pair = nullptr;        // P x 9: force contribution f_q (3), stress contribution (6: xx yy zz yz xz xy)
-  double* Eatom = nullptr;       // A: energy of each atom (linear model; may be null)
+  T* pair = nullptr;             // P x 3: the pair's force contribution
+  double* Satom = nullptr;       // A x 6: sum over the atom's pairs of the stress products (xx yy zz yz xz xy)
+  double* Eatom = nullptr;       // A: energy of each atom (written for the linear model)
 };
 
 // Launch shape of the descriptor kernel, chosen per handle by the autotuner (api.cu); every
@@ -330,29 +404,35 @@ struct Bso4Launch {
   int sorted_queue = 1;  // atoms longest first (1) or in index order (0)
 };
 // Descriptor kernel (bispectrum.cu): B (A x nch*K) and w_ch * dB (P x 3 x nch*K) of the batch,
-// either may be null; or evaluation (ev->pair set, dBout null).  Atoms are taken in `order`
-// (null: index order) through `counter` (one int of device memory, reset by the launch).
+// either may be null.  Atoms are taken in `order` (null: index order) through `counter` (one int
+// of device memory, reset by the launch).
 template <typename T>
 cudaError_t launch_bso4(const DevTables& tb, const DevBatch& b, const BsoParams& p, T* Bout, T* dBout,
-                        const DevEval<T>* ev, const int* order, int* counter, cudaStream_t st,
-                        void* yscratch = nullptr, size_t yscratch_bytes = 0, const Bso4Launch* shape = nullptr);
+                        const int* order, int* counter, cudaStream_t st, void* yscratch = nullptr,
+                        size_t yscratch_bytes = 0, const Bso4Launch* shape = nullptr);
+// Evaluation kernel (bispectrum_eval.cu) of the batch.
+template <typename T>
+cudaError_t launch_bso4_eval(const DevTables& tb, const DevBatch& b, const BsoParams& p, const DevEval<T>& ev,
+                             const int* order, int* counter, cudaStream_t st);
 // Linear design rows of the batch from B, w_ch * dB and the reverse pairs (rows.cu); Sp is a
 // workspace of A x 6 x KK stress partials.  Columns [1, 1 + KK) of the energy, force and stress
 // rows are written.
 template <typename T>
 cudaError_t launch_lin_rows(const DevBatch& b, const DevRows& rows, const BsoParams& p, int KK, const int* rev,
                             const T* B, const T* dB, T* Sp, T* X, cudaStream_t st);
-// E (S; from Eatom when given), F (3A) and S (6S) from the per-pair contributions of evaluation.
-cudaError_t launch_eval_gather(const DevBatch& b, const BsoParams& p, const int* rev, const double* pair,
-                               const double* Eatom, double* E, double* F, double* S, cudaStream_t st);
+// E (S), F (3A) and S (6S) from the atoms' energies and stresses and the pairs' forces of evaluation.
+template <typename T>
+cudaError_t launch_eval_gather(const DevBatch& b, const BsoParams& p, const int* rev, const DevEval<T>& ev, double* E,
+                               double* F, double* S, cudaStream_t st);
 // Atoms ordered by descending neighbour count (the descriptor kernel's queue); tmp holds
 // atom_order_tmp_ints(maxnn) ints.
 size_t atom_order_tmp_ints(int maxnn);
 cudaError_t launch_atom_order(const int* nn, int A, int maxnn, int* order, int* tmp, cudaStream_t st);
-// beta_a = w_lin + Wsym B_a and Eatom_a = w0 + B_a . (beta_a + w_lin) / 2   (eval.cu)
+// The block weights gamma (nch * NBLK per atom) of beta_a = w_lin + Wsym B_a and the energies
+// Eatom_a = w0 + B_a . (beta_a + w_lin) / 2; with B null those of beta = w_lin, once (eval.cu)
 template <typename T>
-cudaError_t launch_eval_beta(const T* B, int A, int nchK, const double* wlin, const double* wsym, double w0, T* beta,
-                             double* Eatom, cudaStream_t st);
+cudaError_t launch_eval_gamma(const DevTables& tb, const T* B, int A, int nch, const double* wlin, const double* wsym,
+                              double w0, T* gamma, double* Eatom, cudaStream_t st);
 
 // FP64 Gram and rhs on the CUDA cores; with ws (gram_workspace_doubles(M, D) doubles) the
 // row-chunk partials are summed in a fixed order (bitwise reproducible), else with atomics

@@ -300,12 +300,12 @@ extern "C" int mld_gpu_descriptors_noalloc(const mld_gpu_config* cfg, int nat, c
   prm.sign_stress = cfg->sign_stress;
   prm.sign_big = cfg->sign_stress_big_box;
   if (mixed) {
-    CKN(launch_bso4<float>(dt, b, prm, bstage, (float*)nullptr, nullptr, nullptr, qcount, st, yscr, ysb));
+    CKN(launch_bso4<float>(dt, b, prm, bstage, (float*)nullptr, nullptr, qcount, st, yscr, ysb));
     const size_t n = (size_t)nat * KK;
     k_widen<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(bstage, B, n);
     CKN(cudaGetLastError());
   } else {
-    CKN(launch_bso4<double>(dt, b, prm, B, (double*)nullptr, nullptr, nullptr, qcount, st, yscr, ysb));
+    CKN(launch_bso4<double>(dt, b, prm, B, (double*)nullptr, nullptr, qcount, st, yscr, ysb));
   }
 #undef CKN
   return MLD_OK;

@@ -104,50 +104,54 @@ __global__ void __launch_bounds__(kRowThreads) k_lin_struct_rows(int KK, const i
   }
 }
 
-// Evaluation: F_i[a] = sum_q pair_q[a] - pair_rev(q)[a], one thread per (atom, component).
+// Evaluation: F_i[a] = sum_q pair_q[a] - pair_rev(q)[a] in FP64, one thread per (atom, component).
+template <typename T>
 __global__ void k_eval_forces(int A, const int* __restrict__ nbr_off, const int* __restrict__ rev,
-                              const double* __restrict__ pair, double* __restrict__ F) {
+                              const T* __restrict__ pair, double* __restrict__ F) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 3LL * A) return;
   const int i = (int)(t / 3), a = (int)(t - 3LL * i);
   double sum = 0.0;
-  for (int q = nbr_off[i]; q < nbr_off[i + 1]; ++q) {
+  const int q1 = nbr_off[i + 1];
+#pragma unroll 8
+  for (int q = nbr_off[i]; q < q1; ++q) {
     const int b = rev[q];
-    sum += pair[(size_t)q * 9 + a] - (b >= 0 ? pair[(size_t)b * 9 + a] : 0.0);
+    sum += (double)pair[(size_t)q * 3 + a] - (b >= 0 ? (double)pair[(size_t)b * 3 + a] : 0.0);
   }
   F[t] = sum;
 }
 
-// Evaluation, one CTA per structure: E_s = sum_i Eatom_i (when given), S_s = sign_stress*3/V *
-// sum_i sum_q pair_q[3 + c]; per-thread sums over a fixed atom stride, then a fixed tree.
-__global__ void __launch_bounds__(kRowThreads) k_eval_struct(const int* __restrict__ atom_start,
-                                                             const int* __restrict__ nbr_off,
-                                                             const double* __restrict__ pair,
-                                                             const double* __restrict__ Eatom,
-                                                             const double* __restrict__ volume, double sign_stress,
-                                                             double* __restrict__ E, double* __restrict__ S) {
-  __shared__ double red[7][kRowThreads];
+// Evaluation, one CTA per structure: E_s = sum_i Eatom_i, S_s = sign_stress*3/V * sum_i Satom_i;
+// per-thread sums over a fixed atom stride, then a fixed tree over the lanes and the warps.
+constexpr int kStructThreads = 1024;
+__global__ void __launch_bounds__(kStructThreads) k_eval_struct(const int* __restrict__ atom_start,
+                                                                const double* __restrict__ Satom,
+                                                                const double* __restrict__ Eatom,
+                                                                const double* __restrict__ volume, double sign_stress,
+                                                                double* __restrict__ E, double* __restrict__ S) {
+  __shared__ double red[7][kStructThreads / 32];
   const int s = blockIdx.x, tid = threadIdx.x;
   double v[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int i = atom_start[s] + tid; i < atom_start[s + 1]; i += kRowThreads) {
-    if (Eatom) v[0] += Eatom[i];
-    for (int q = nbr_off[i]; q < nbr_off[i + 1]; ++q)
+  const int a1 = atom_start[s + 1];
+  for (int i = atom_start[s] + tid; i < a1; i += kStructThreads) {
+    v[0] += Eatom[i];
 #pragma unroll
-      for (int c = 0; c < 6; ++c) v[1 + c] += pair[(size_t)q * 9 + 3 + c];
+    for (int c = 0; c < 6; ++c) v[1 + c] += Satom[(size_t)i * 6 + c];
   }
 #pragma unroll
-  for (int c = 0; c < 7; ++c) red[c][tid] = v[c];
+  for (int c = 0; c < 7; ++c) {
+    for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
+    if ((tid & 31) == 0) red[c][tid >> 5] = v[c];
+  }
   __syncthreads();
-  for (int o = kRowThreads / 2; o > 0; o >>= 1) {
-    if (tid < o)
-#pragma unroll
-      for (int c = 0; c < 7; ++c) red[c][tid] += red[c][tid + o];
-    __syncthreads();
-  }
-  if (tid == 0) {
-    if (Eatom) E[s] = red[0][0];
-    const double sc = sign_stress * 3.0 / volume[s];
-    for (int c = 0; c < 6; ++c) S[6 * (size_t)s + c] = sc * red[1 + c][0];
+  const int c = tid >> 5;
+  if (c < 7) {
+    double t = red[c][tid & 31];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((tid & 31) == 0) {
+      if (c == 0) E[s] = t;
+      else S[6 * (size_t)s + c - 1] = sign_stress * 3.0 / volume[s] * t;
+    }
   }
 }
 
@@ -229,17 +233,22 @@ cudaError_t launch_lin_rows(const DevBatch& b, const DevRows& rows, const BsoPar
   return cudaGetLastError();
 }
 
-cudaError_t launch_eval_gather(const DevBatch& b, const BsoParams& p, const int* rev, const double* pair,
-                               const double* Eatom, double* E, double* F, double* S, cudaStream_t st) {
+template <typename T>
+cudaError_t launch_eval_gather(const DevBatch& b, const BsoParams& p, const int* rev, const DevEval<T>& ev, double* E,
+                               double* F, double* S, cudaStream_t st) {
   if (b.A == 0) return cudaSuccess;
   const long long n = 3LL * b.A;
-  k_eval_forces<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(b.A, b.nbr_off, rev, pair, F);
+  k_eval_forces<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(b.A, b.nbr_off, rev, ev.pair, F);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_eval_struct<<<b.S, kRowThreads, 0, st>>>(b.atom_start, b.nbr_off, pair, Eatom, b.volume, p.sign_stress, E, S);
+  k_eval_struct<<<b.S, kStructThreads, 0, st>>>(b.atom_start, ev.Satom, ev.Eatom, b.volume, p.sign_stress, E, S);
   return cudaGetLastError();
 }
 
+template cudaError_t launch_eval_gather<double>(const DevBatch&, const BsoParams&, const int*, const DevEval<double>&,
+                                                double*, double*, double*, cudaStream_t);
+template cudaError_t launch_eval_gather<float>(const DevBatch&, const BsoParams&, const int*, const DevEval<float>&,
+                                               double*, double*, double*, cudaStream_t);
 template cudaError_t launch_lin_rows<double>(const DevBatch&, const DevRows&, const BsoParams&, int, const int*,
                                              const double*, const double*, double*, double*, cudaStream_t);
 template cudaError_t launch_lin_rows<float>(const DevBatch&, const DevRows&, const BsoParams&, int, const int*,
