@@ -238,19 +238,19 @@ inline unsigned long long chain_order(int J) {
 // of consecutive neighbours use distinct banks.
 __host__ __device__ constexpr int u_stride(int HU) { return HU | 1; }
 
-// U (all half layers) of neighbours 0..count-1 into Us[n][u_stride]; zp, xp come from the geometry
-// records rec(n).  Work items (chain, 32 neighbours) go to the warps longest first, every second
+// U (all half layers but the first, which is 1) of neighbours 0..count-1 into Us[n][u_stride]; zx(n)
+// points to the neighbour's zp and xp.  Work items (chain, 32 neighbours) go to the warps longest first, every second
 // round in reverse.  No synchronisation inside.
-template <typename T, class Rec>
+template <typename T, class Zx>
 __device__ __forceinline__ void u_store(cx<T>* Us, int HS, int count, int J, unsigned long long order, int warp,
-                                        int lane, Rec rec) {
+                                        int lane, Zx zx) {
   const int nb = (count + 31) >> 5, nitem = J * nb;
   for (int r = 0; r * kNW < nitem; ++r) {
     const int it = (r & 1) ? (r + 1) * kNW - 1 - warp : r * kNW + warp;
     if (it >= nitem) continue;
     const int ci = it / nb, n = (it - ci * nb) * 32 + lane;
     if (n < count) {
-      const T* g = rec(n) + kGeoZx;
+      const T* g = zx(n);
       const cx<T> z = {g[0], g[1]}, x = {g[2], g[3]};
       cx<T>* u = Us + (size_t)n * HS;
       switch ((int)(order >> (4 * ci)) & 15) {
@@ -386,20 +386,30 @@ struct PairSource {
   int ntypes, has_rin;
 };
 
-// Geometry record of pair q with a centre of type ti.
+// Geometry record of pair q with a centre of type ti, but for the neighbour's index and type, which
+// come back in *nb and *tn (put_pair stores them).
 template <typename T>
-__device__ __forceinline__ void pair_geometry(const PairSource<T>& s, const T* rin, size_t q, int ti, T* g) {
-  const int nb = s.nbr_idx[q];
-  const int tn = s.types[nb];
+__device__ __forceinline__ void pair_geometry(const PairSource<T>& s, const T* rin, size_t q, int ti, T* g, int* nb,
+                                              int* tn) {
+  *nb = s.nbr_idx[q];
+  *tn = s.types[*nb];
   T x[3], rinv;
   pair_u_rinv<T>(s.nbr_u, s.u32, q, x, &rinv);
-  nbr_geometry<T>(x[0], x[1], x[2], rinv, s.rcut, s.inv_r0, s.has_rin ? rin[ti * s.ntypes + tn] : T(0), s.rin_w, g);
+  nbr_geometry<T>(x[0], x[1], x[2], rinv, s.rcut, s.inv_r0, s.has_rin ? rin[ti * s.ntypes + *tn] : T(0), s.rin_w, g);
   g[kGeoU + 0] = x[0];
   g[kGeoU + 1] = x[1];
   g[kGeoU + 2] = x[2];
   g[kGeoU + 3] = rinv;
+}
+
+template <typename T>
+__device__ __forceinline__ void put_pair(T* g, int nb, int tn) {
   reinterpret_cast<int*>(g + kGeoIdx)[0] = nb;
   reinterpret_cast<int*>(g + kGeoIdx)[1] = tn;
+}
+template <typename T>
+__device__ __forceinline__ int pair_type(const T* g) {
+  return reinterpret_cast<const int*>(g + kGeoIdx)[1];
 }
 
 // c on half layers from the U store of neighbours 0..count-1 of a pass: chalf += sum over them in

@@ -189,13 +189,14 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
     auto load_pass = [&](int base, int count) {
       for (int n = tid; n < count; n += nth) {
         T* g = geo(n);
-        pair_geometry<T>(args.src, args.rin, (size_t)(p0 + base + n), ti, g);
-        const int tn = reinterpret_cast<int*>(g + kGeoIdx)[1];
+        int nb, tn;
+        pair_geometry<T>(args.src, args.rin, (size_t)(p0 + base + n), ti, g, &nb, &tn);
+        put_pair<T>(g, nb, tn);
         for (int ch = 0; ch < nch; ++ch) fcw[n * nch + ch] = g[kGeoFc] * args.chw[ch * args.src.ntypes + tn];
         Us[(size_t)n * HS] = {T(1), T(0)};
       }
       __syncthreads();
-      u_store<T>(Us, HS, count, J, args.chains, warp, lane, geo);
+      u_store<T>(Us, HS, count, J, args.chains, warp, lane, [&](int n) { return geo(n) + kGeoZx; });
       __syncthreads();
     };
     // ---- c -----------------------------------------------------------------------------------
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
           }
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const int tn = reinterpret_cast<const int*>(geo(min(g4 + i, count - 1)) + kGeoIdx)[1];
+            const int tn = pair_type<T>(geo(min(g4 + i, count - 1)));
             const T w = args.chw[ch * args.src.ntypes + tn];
 #pragma unroll
             for (int b = 0; b < 4; ++b) tot[i * 4 + b] = fma(w, acc[i][b].x + acc[i][b].y, tot[i * 4 + b]);
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
             __syncthreads();
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              const int tn = reinterpret_cast<const int*>(geo(min(c0 + nt * 4 + i, count - 1)) + kGeoIdx)[1];
+              const int tn = pair_type<T>(geo(min(c0 + nt * 4 + i, count - 1)));
               wn[i] = args.chw[ch * args.src.ntypes + tn];
             }
             const cx<T>* zc = tbuf + (size_t)ch * tb.NZT;

@@ -358,7 +358,7 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
         }
         s.ufull = (uint16_t)uidx(j, p, q);
         s.k = (uint16_t)k;
-        s.ypos = (uint16_t)(t->yoff[j] + e * t->Mp[j] + r);
+        s.ypos = (uint16_t)(t->yoff[j] + ((r / kRowTile) * H(j) + e) * kRowTile + r % kRowTile);
         s.wgt = (uint8_t)((p == 0 && q == 0) ? 1 : 2);
         se.ypos = s.ypos;
         se.nterm = s.nterm;

@@ -104,21 +104,6 @@ struct alignas(16) RowSource {
 };
 static_assert(sizeof(RowSource) == 16, "row sources are 16 bytes");
 
-// Packed per-entry recursion record of the half layers (one 16-byte load per entry).  tz and tx
-// (>= 0 in the tables) are stored with the sign that selects the entry's Z / conj(Z) and X
-// (+ for qneg != 0), so the kernel takes their magnitudes with fabs.
-struct RecEntry32 {
-  float tz, tx;
-  int16_t sz, sx;
-  int32_t qneg;
-};
-struct RecEntry64 {
-  double tz, tx;
-  int16_t sz, sx;
-  int32_t qneg;
-  int64_t pad;
-};
-
 constexpr int kZWarps = 8;   // warps of the phase-2 schedule (= warps of a k_bso4 CTA)
 constexpr int kRounds = 3;   // ranks of a triple's layer rows (its distinct layers in ascending order)
 constexpr int kRankShift = 12;  // row destination code: (rank << kRankShift) | index within the rank's buffer
@@ -137,7 +122,7 @@ struct Bso4Tables {
   std::vector<ZTerm> zterms;    // ZA/ZB/ZC outputs on half layers
   int nzu = 0;                  // distinct Z computations among them (the term buffer's entries)
   std::vector<YSlot> yslots;    // folded slots
-  std::vector<SlotEntry> slots; // the same slots in the kernel's form
+  std::vector<SlotEntry> slots; // the same slots with their distinct terms and Y positions
   std::vector<int> bk_off;      // K + 1 offsets into bk_items
   std::vector<BkItem> bk_items; // ZA entries of each triple
   // per layer-block row: destination code (rank << kRankShift) | index, -1 for padding; the
@@ -185,7 +170,7 @@ struct alignas(16) GenEntry {
 
 // Device copies of the tables.
 struct DevTables {
-  int J = 0, NU = 0, HU = 0, K = 0, NS = 0, NYP = 0, NTILE = 0, NZT = 0, NROWS = 0;
+  int J = 0, NU = 0, HU = 0, K = 0, NYP = 0, NTILE = 0, NZT = 0, NROWS = 0;
   int NCG = 0;  // entries of the 1-D CG coefficient table
   int NBLK = 0;
   int blk_off[kMaxJ + 2] = {0};
@@ -204,31 +189,14 @@ struct DevTables {
   float* cg32 = nullptr;
   int16_t* expand = nullptr;
   int8_t* half_diag = nullptr;
-  RecEntry32* rec32 = nullptr;  // packed recursion records (FP32 method)
-  RecEntry64* rec64 = nullptr;  // packed recursion records (FP64 method)
   ZItem* zitems = nullptr;
   int* zitem_off = nullptr;     // kZWarps + 1
-  SlotEntry* slots = nullptr;   // NS
-  int* bk_off = nullptr;        // K + 1
-  BkItem* bk_items = nullptr;
   // tables of the derivatives and the evaluation (fill_deriv_tables)
   GenEntry<float>* gen32 = nullptr;   // HU
   GenEntry<double>* gen64 = nullptr;  // HU
   int* gam_off = nullptr;       // NBLK + 1
   GammaItem* gam = nullptr;
 };
-
-// Packed recursion records from the table vectors.
-inline void pack_recursion(const Bso4Tables& t, std::vector<RecEntry32>* r32, std::vector<RecEntry64>* r64) {
-  r32->resize(t.HU);
-  r64->resize(t.HU);
-  for (int h = 0; h < t.HU; ++h) {
-    // tz, tx >= 0 carry the sign of the entry's q (+ for q >= 0), which selects Z / conj(Z) and X
-    const double sq = t.rec_qneg[h] ? 1.0 : -1.0;
-    (*r32)[h] = RecEntry32{(float)(sq * t.rec_tz[h]), (float)(sq * t.rec_tx[h]), t.rec_sz[h], t.rec_sx[h], (int32_t)t.rec_qneg[h]};
-    (*r64)[h] = RecEntry64{sq * t.rec_tz[h], sq * t.rec_tx[h], t.rec_sz[h], t.rec_sx[h], (int32_t)t.rec_qneg[h], 0};
-  }
-}
 
 // Fill the scalar part of *d from t and place every device table through put(vector, &ptr),
 // which allocates (or carves) device memory of the vector's size and copies it there.
@@ -239,7 +207,6 @@ cudaError_t fill_dev_tables(const Bso4Tables& t, DevTables* d, Put put) {
   d->NU = t.NU;
   d->HU = t.HU;
   d->K = t.K;
-  d->NS = (int)t.slots.size();
   d->NYP = t.NYP;
   d->NTILE = (int)t.tiles.size();
   d->NZT = t.nzu;
@@ -263,9 +230,6 @@ cudaError_t fill_dev_tables(const Bso4Tables& t, DevTables* d, Put put) {
   cg64.resize((cg64.size() + 1) / 2 * 2, 0.0);
   std::vector<float> cg32(t.cg.begin(), t.cg.end());
   cg32.resize((cg32.size() + 3) / 4 * 4, 0.0f);
-  std::vector<RecEntry32> r32;
-  std::vector<RecEntry64> r64;
-  pack_recursion(t, &r32, &r64);
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = put(t.rowk, &d->rowk);
   if (e == cudaSuccess) e = put(t.rank_slot, &d->rank_slot);
@@ -274,15 +238,10 @@ cudaError_t fill_dev_tables(const Bso4Tables& t, DevTables* d, Put put) {
   if (e == cudaSuccess) e = put(cg32, &d->cg32);
   if (e == cudaSuccess) e = put(t.expand, &d->expand);
   if (e == cudaSuccess) e = put(t.half_diag, &d->half_diag);
-  if (e == cudaSuccess) e = put(r32, &d->rec32);
-  if (e == cudaSuccess) e = put(r64, &d->rec64);
   if (e == cudaSuccess) e = put(t.zitems, &d->zitems);
   if (e == cudaSuccess) e = put(t.trz, &d->trz);
   if (e == cudaSuccess) e = put(t.rowsrc, &d->rowsrc);
   if (e == cudaSuccess) e = put(t.zitem_off, &d->zitem_off);
-  if (e == cudaSuccess) e = put(t.slots, &d->slots);
-  if (e == cudaSuccess) e = put(t.bk_off, &d->bk_off);
-  if (e == cudaSuccess) e = put(t.bk_items, &d->bk_items);
   return e;
 }
 
