@@ -123,6 +123,7 @@ struct mld_gpu_handle {
     B_GWS, B_TERR, B_PCG, B_POS32, B_YSCR, B_RINV, B_KZD, B_KZF, B_KWS, B_WSERVE, B_P32,
     B_EW, B_EBETA, B_EB, B_EOUT, B_KTC, B_SKW, B_ORDER, B_QCNT, B_SP, B_EPAIR, B_EATOM, B_GP,
     B_CNC, B_CELLOFF, B_CELLOF, B_CELLSTART, B_CELLATOMS, B_SORTTMP, B_NBR_U32, B_MVWS, B_GTCP, B_NBRTMP,
+    B_CHALF, B_EY,
     B_COUNT
   };
   static_assert(B_COUNT <= 80, "buffer table too small");
@@ -346,13 +347,13 @@ int y_scratch(mld_gpu_handle* h, void** p, size_t* bytes) {
 constexpr int kTuneMinAtoms = 64;
 
 template <typename T>
-int tuned_launch(mld_gpu_handle* h, int mode, T* Bout, T* dB, void* ys, size_t ysb) {
-  auto& tn = h->tune[mode];
+int tuned_launch(mld_gpu_handle* h, T* Bout, T* dB, void* ys, size_t ysb) {
+  auto& tn = h->tune[0];
   const int* order = bp_<int>(h, mld_gpu_handle::B_ORDER);
   int* counter = bp_<int>(h, mld_gpu_handle::B_QCNT);
   // only the design-row stage of a fit is tuned: it is repeated on the same batch, while
   // evaluation batches (serving) and descriptor dumps change from call to call
-  if (tn.done || mode != 0 || h->A < kTuneMinAtoms * std::max(1, h->nsm)) {
+  if (tn.done || h->A < kTuneMinAtoms * std::max(1, h->nsm)) {
     CK(launch_bso4<T>(h->dt, h->b, h->bp, Bout, dB, order, counter, h->st, ys, ysb, &tn.best));
     return MLD_OK;
   }
@@ -386,23 +387,31 @@ int tuned_launch(mld_gpu_handle* h, int mode, T* Bout, T* dB, void* ys, size_t y
 }
 
 template <typename T>
-int prepare_descriptors(mld_gpu_handle* h, bool want_dB, void** ys, size_t* ysb) {
+int prepare_descriptors(mld_gpu_handle* h, void** ys, size_t* ysb) {
   int rcy = y_scratch<T>(h, ys, ysb);
   if (rcy) return rcy;
-  if (want_dB) CK(ensure(h, mld_gpu_handle::B_DBOUT, sizeof(T) * std::max<size_t>((size_t)h->b.P * 3 * h->KK, 1)));
+  CK(ensure(h, mld_gpu_handle::B_DBOUT, sizeof(T) * std::max<size_t>((size_t)h->b.P * 3 * h->KK, 1)));
   return MLD_OK;
 }
 
-// B and w_ch * dB of the staged batch into B_BOUT / B_DBOUT (dB optional) through the
-// descriptor kernel's queue
+// B of the staged batch into Bout and, if asked, w_ch * dB into B_DBOUT: both from the descriptor
+// kernel, B alone from the atoms-on-lanes sums
 template <typename T>
 int run_descriptors(mld_gpu_handle* h, bool want_dB, T* Bout) {
+  if (!want_dB) {
+    CK(ensure(h, mld_gpu_handle::B_CHALF, sizeof(T) * 2 * (size_t)std::max(1, h->A) * h->nch * h->dt.HU));
+    void* c = bp_<void>(h, mld_gpu_handle::B_CHALF);
+    CK(launch_c_half<T>(h->dt, h->b, h->bp, 0, h->A, bp_<int>(h, mld_gpu_handle::B_ORDER),
+                        bp_<int>(h, mld_gpu_handle::B_QCNT), c, h->st));
+    CK(launch_lane_descriptors<T>(h->dt, h->b, h->bp, 0, h->A, c, Bout, h->st));
+    nl(h, 2);
+    return MLD_OK;
+  }
   void* ys = nullptr;
   size_t ysb = 0;
-  int rcy = prepare_descriptors<T>(h, want_dB, &ys, &ysb);
+  int rcy = prepare_descriptors<T>(h, &ys, &ysb);
   if (rcy) return rcy;
-  T* dB = want_dB ? bp_<T>(h, mld_gpu_handle::B_DBOUT) : nullptr;
-  int rc = tuned_launch<T>(h, want_dB ? 0 : 2, Bout, dB, ys, ysb);
+  int rc = tuned_launch<T>(h, Bout, bp_<T>(h, mld_gpu_handle::B_DBOUT), ys, ysb);
   if (rc) return rc;
   nl(h, 1);
   return MLD_OK;
@@ -463,7 +472,7 @@ int run_rows(mld_gpu_handle* h, const RowLayout& L, bool with_labels, T** Xout) 
     T* Bq = bp_<T>(h, mld_gpu_handle::B_BOUT);
     void* ys = nullptr;
     size_t ysb = 0;
-    int rcd = prepare_descriptors<T>(h, true, &ys, &ysb);
+    int rcd = prepare_descriptors<T>(h, &ys, &ysb);
     if (rcd) return rcd;
     T* dBq = bp_<T>(h, mld_gpu_handle::B_DBOUT);
     // the stage of this batch: descriptor kernel, reverse pairs, linear (and quadratic) rows
@@ -1646,7 +1655,7 @@ int eval_weights_upload(mld_gpu_handle* h, const double* w_full) {
       for (int j = 0; j < KK; ++j) hw[KK + (size_t)i * KK + j] = W[(size_t)i * KK + j] + W[(size_t)j * KK + i];
   }
   const size_t eb = h->mixed ? sizeof(float) : sizeof(double);
-  CK(ensure(h, mld_gpu_handle::B_EW, sizeof(double) * hw.size() + eb * h->nch * h->dt.NBLK + 256));
+  CK(ensure(h, mld_gpu_handle::B_EW, sizeof(double) * hw.size() + eb * h->nch * h->dt.NBLKP + 256));
   double* dw = bp_<double>(h, mld_gpu_handle::B_EW);
   CK(cudaMemcpyAsync(dw, hw.data(), sizeof(double) * hw.size(), cudaMemcpyHostToDevice, h->st));
   if (!h->quad) {
@@ -1672,6 +1681,8 @@ static int eval_run(mld_gpu_handle* h, double* out) {
   CK(ensure(h, mld_gpu_handle::B_EPAIR, sizeof(T) * 3 * (size_t)std::max<long long>(1, h->b.P)));
   CK(ensure(h, mld_gpu_handle::B_EATOM, sizeof(double) * 7 * (size_t)std::max(1, h->A)));
   CK(ensure(h, mld_gpu_handle::B_REV, sizeof(int) * (size_t)std::max<long long>(1, h->b.P)));
+  const int* order = bp_<int>(h, mld_gpu_handle::B_ORDER);
+  int* counter = bp_<int>(h, mld_gpu_handle::B_QCNT);
   DevEval<T> ev;
   ev.pair = bp_<T>(h, mld_gpu_handle::B_EPAIR);
   ev.Eatom = bp_<double>(h, mld_gpu_handle::B_EATOM);
@@ -1688,14 +1699,19 @@ static int eval_run(mld_gpu_handle* h, double* out) {
     if (rc) return rc;
     CK(launch_eval_gamma<T>(h->dt, B, h->A, h->nch, wlin, wsym, h->ew0, gamma, ev.Eatom, h->st));
     ev.gamma = gamma;
-    ev.per_atom = 1;
     nl(h, 1);
   } else {
-    ev.gamma = gammaT;
-    ev.wlin = wlin;
+    // c and y of every atom
+    const size_t nc = (size_t)std::max(1, h->A) * h->nch * h->dt.HU * 2;
+    CK(ensure(h, mld_gpu_handle::B_CHALF, sizeof(T) * nc));
+    CK(ensure(h, mld_gpu_handle::B_EY, sizeof(T) * nc));
+    ev.c = bp_<void>(h, mld_gpu_handle::B_CHALF);
+    ev.y = bp_<void>(h, mld_gpu_handle::B_EY);
+    CK(launch_c_half<T>(h->dt, h->b, h->bp, 0, h->A, order, counter, bp_<void>(h, mld_gpu_handle::B_CHALF), h->st));
+    CK(launch_lane_y<T>(h->dt, h->b, h->bp, 0, h->A, ev.c, gammaT, bp_<void>(h, mld_gpu_handle::B_EY), h->st));
+    nl(h, 2);
   }
-  CK(launch_bso4_eval<T>(h->dt, h->b, h->bp, ev, bp_<int>(h, mld_gpu_handle::B_ORDER), bp_<int>(h, mld_gpu_handle::B_QCNT),
-                         h->st));
+  CK(launch_bso4_eval<T>(h->dt, h->b, h->bp, ev, order, counter, h->st));
   CK(launch_reverse_pairs(h->b, bp_<int>(h, mld_gpu_handle::B_REV), h->st));
   CK(launch_eval_gather<T>(h->b, h->bp, bp_<int>(h, mld_gpu_handle::B_REV), ev, E, F, S, h->st));
   nl(h, 4);

@@ -10,18 +10,19 @@
 // A pair then costs its U (computed once, kept in shared memory from the sum for c) and four dot
 // products of HU complex entries.
 //
-// Persistent CTAs take atoms from a queue.  Per atom: geometry and U of the neighbours (column
-// chains), c, the Z terms, y, the energy (linear model: B from the Z terms), the generators' y_b,
-// the pairs.  An atom with more neighbours than the U store holds is done in passes, whose U is
-// computed again for the pairs.
+// Linear model: c and y come from the atoms-on-lanes kernels (bispectrum_lanes.cu); here, per atom,
+// the energy (c . y / 3: the energy is of third degree in c), the generators' y_b, and in passes of
+// as many neighbours as the U store holds their geometry, U and dot products.  Bound: latency of
+// the short phases and shared-memory reads.
 //
-// The quadratic model's stress takes the neighbour's beta (the neighbour's B in the quadratic stress
+// Quadratic model: its stress takes the neighbour's beta (the neighbour's B in the quadratic stress
 // rows, mld_stress.F90:580-603): y is formed per neighbour from the Z terms of all channels (one
 // real by complex product per term, a third of a dB contraction), and its dot products are taken
-// with the generators applied to U.
+// with the generators applied to U.  The Z terms of the atom are therefore formed in the CTA, from c
+// summed over the same U store.  Bound: FP32 arithmetic and shared memory of the Z terms.
 //
-// Bound: FP32 arithmetic and shared memory; most of an atom's time is its Z terms.  Every sum has a
-// fixed order that does not depend on the batch.
+// Persistent CTAs take atoms from a queue.  Every sum has a fixed order that does not depend on the
+// batch.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -38,27 +39,27 @@ constexpr int kChunk = 16;  // neighbours whose own y is formed at a time (quadr
 template <typename T>
 constexpr int kGrow = sizeof(T) == 4 ? 20 : 18;
 
-// A stress sum: FP64, or a double-FP32 pair (the products and sums of FP32 forces and lever arms are
-// then as exact as FP64 ones without its 64 times slower issue).
+// A sum of products of three: FP64, or a double-FP32 pair (products and sums of FP32 values are then
+// as exact as FP64 ones without its 64 times slower issue).
 template <typename T>
-struct StressSum;
+struct ExactSum;
 template <>
-struct StressSum<double> {
+struct ExactSum<double> {
   double v = 0.0;
   __device__ __forceinline__ void add(double f, double u, double rinv) { v += f * rinv * u; }
-  __device__ __forceinline__ void add(const StressSum& o) { v += o.v; }
-  __device__ __forceinline__ StressSum down(int d) const { return {__shfl_down_sync(0xffffffffu, v, d)}; }
+  __device__ __forceinline__ void add(const ExactSum& o) { v += o.v; }
+  __device__ __forceinline__ ExactSum down(int d) const { return {__shfl_down_sync(0xffffffffu, v, d)}; }
   __device__ __forceinline__ double value() const { return v; }
 };
 template <>
-struct StressSum<float> {
+struct ExactSum<float> {
   float h = 0.f, l = 0.f;
   __device__ __forceinline__ void add(float f, float u, float rinv) {
     const float p = f * rinv, pe = fmaf(f, rinv, -p);
     ds_fma(h, l, u, p, pe);
   }
-  __device__ __forceinline__ void add(const StressSum& o) { ds_add(h, l, o.h, o.l); }
-  __device__ __forceinline__ StressSum down(int d) const {
+  __device__ __forceinline__ void add(const ExactSum& o) { ds_add(h, l, o.h, o.l); }
+  __device__ __forceinline__ ExactSum down(int d) const {
     return {__shfl_down_sync(0xffffffffu, h, d), __shfl_down_sync(0xffffffffu, l, d)};
   }
   __device__ __forceinline__ double value() const { return (double)h + (double)l; }
@@ -85,7 +86,7 @@ struct EvalArgs {
 };
 
 struct EvalPlan {
-  size_t hoff, exp, hd, sj, cfull, chalf, gamma, bk, cg, tbuf, yb, yt, geo, fcw, red, grow, next, U, total;
+  size_t hoff, exp, hd, sj, cfull, chalf, gamma, cg, tbuf, yb, yt, geo, fcw, red, grow, next, U, total;
 };
 
 __host__ __device__ inline size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
@@ -98,18 +99,14 @@ __host__ __device__ inline EvalPlan eval_plan(const DevTables& tb, int nch, int 
   s.exp = o;   o = up16(o + sizeof(int16_t) * tb.NU);
   s.hd = o;    o = up16(o + tb.HU);
   s.sj = o;    o = up16(o + tb.HU);
-  s.cfull = o; o = up16(o + cxb * nch * tb.NU);
-  s.chalf = o; o = up16(o + cxb * nch * tb.HU);
-  s.gamma = o; o = up16(o + (size_t)eb * nch * tb.NBLK);
-  s.bk = o;    o = up16(o + (size_t)eb * nch * tb.K);
-  s.cg = o;    o = up16(o + up16((size_t)eb * tb.NCG));
-  // Z terms (of every channel for the quadratic stress) and the generators' y_b (4 * nch * HU complex),
-  // which take the place of the Z terms in the linear model
-  const size_t ny = (size_t)4 * nch * tb.HU, nz = quad ? (size_t)nch * tb.NZT : (tb.NZT > (int)ny ? (size_t)tb.NZT : ny);
-  s.tbuf = o;  o = up16(o + cxb * nz);
-  s.yb = quad ? o : s.tbuf;
-  o = up16(o + (quad ? cxb * ny : 0));
-  s.yt = o;    o = up16(o + cxb * nch * tb.HU);
+  s.cfull = o; o = up16(o + (quad ? cxb * nch * tb.NU : 0));
+  s.chalf = o; o = up16(o + (quad ? cxb * nch * tb.HU : 0));
+  s.gamma = o; o = up16(o + (quad ? (size_t)eb * nch * tb.NBLK : 0));
+  s.cg = o;    o = up16(o + (quad ? (size_t)eb * tb.NCG : 0));
+  // Z terms of every channel, y, and the generators' y_b
+  s.tbuf = o;  o = up16(o + (quad ? cxb * nch * tb.NZT : 0));
+  s.yt = o;    o = up16(o + (quad ? cxb * nch * tb.HU : 0));
+  s.yb = o;    o = up16(o + cxb * 4 * nch * tb.HU);
   s.geo = o;   o = up16(o + (size_t)eb * kGeo * slots);
   s.fcw = o;   o = up16(o + (size_t)eb * nch * slots);
   s.red = o;   o = up16(o + (size_t)eb * (kNW * kChunk * 4));
@@ -128,8 +125,8 @@ template <typename T, bool kQuad>
 __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(EvalArgs<T> args, int A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DevTables& tb = args.tb;
-  const int J = tb.J, NU = tb.NU, HU = tb.HU, K = tb.K;
-  const int nch = args.nch, nchK = nch * K, nchG = nch * tb.NBLK;
+  const int J = tb.J, NU = tb.NU, HU = tb.HU;
+  const int nch = args.nch, nchG = nch * tb.NBLK;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int nth = kNW * 32;
   const EvalPlan sp = eval_plan(tb, nch, (int)sizeof(T), args.slots, kQuad);
@@ -140,7 +137,6 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
   cx<T>* cfull = reinterpret_cast<cx<T>*>(smem_raw + sp.cfull);
   cx<T>* chalf = reinterpret_cast<cx<T>*>(smem_raw + sp.chalf);
   T* sgam = reinterpret_cast<T*>(smem_raw + sp.gamma);
-  T* Bk = reinterpret_cast<T*>(smem_raw + sp.bk);
   T* scg = reinterpret_cast<T*>(smem_raw + sp.cg);
   cx<T>* tbuf = reinterpret_cast<cx<T>*>(smem_raw + sp.tbuf);
   cx<T>* yb = reinterpret_cast<cx<T>*>(smem_raw + sp.yb);  // [nch][HU][4]
@@ -163,11 +159,9 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
     while (j < J && tb.hoff[j + 1] <= e) ++j;
     sj[e] = (int8_t)j;
   }
-  for (int e = tid; e < tb.NCG; e += nth) scg[e] = args.cg[e];
-  if constexpr (!kQuad) {
-    for (int e = tid; e < nchG; e += nth) sgam[e] = args.ev.gamma[e];
-  }
-  const int zr0 = tb.zitem_off[warp], zr1 = tb.zitem_off[warp + 1];
+  if constexpr (kQuad)
+    for (int e = tid; e < tb.NCG; e += nth) scg[e] = args.cg[e];
+  const int zr0 = kQuad ? tb.zitem_off[warp] : 0, zr1 = kQuad ? tb.zitem_off[warp + 1] : 0;
 
   int nxt = 0;
   if (tid == 0) nxt = atomicAdd(args.counter, 1);
@@ -199,33 +193,36 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
       u_store<T>(Us, HS, count, J, args.chains, warp, lane, [&](int n) { return geo(n) + kGeoZx; });
       __syncthreads();
     };
-    // ---- c -----------------------------------------------------------------------------------
-    for (int ps = 0; ps < npass; ++ps) {
-      const int base = ps * args.slots, count = min(args.slots, nn - base);
-      load_pass(base, count);
-      c_sum<T>(chalf, Us, HS, fcw, shd, count, nch, HU, ps == 0, ps == npass - 1, tid);
+    // ---- y = dE/dc: quadratic model, from c and the Z terms of this atom ------------------------
+    const cx<T>* ysrc = yt;
+    if constexpr (kQuad) {
+      for (int ps = 0; ps < npass; ++ps) {
+        const int base = ps * args.slots, count = min(args.slots, nn - base);
+        load_pass(base, count);
+        c_sum<T>(chalf, Us, HS, fcw, shd, count, nch, HU, ps == 0, ps == npass - 1, tid);
+        __syncthreads();
+      }
+    }
+    if (nn == 0) {  // no neighbours: the constant alone
+      if (tid < 6) args.ev.Satom[(size_t)atom * 6 + tid] = 0.0;
+      if (!kQuad && tid == 0) args.ev.Eatom[atom] = args.ev.w0;
+      continue;
+    }
+    if constexpr (kQuad) {
+      for (int e = tid; e < nch * NU; e += nth) {
+        const int ch = e / NU, f = e - ch * NU;
+        cfull[e] = fetch(chalf + ch * HU, sexp[f]);
+      }
       __syncthreads();
-    }
-    if (npass == 0) {  // no neighbours: c is the identity
-      for (int e = tid; e < nch * HU; e += nth) chalf[e] = {shd[e % HU] ? T(1) : T(0), T(0)};
-      __syncthreads();
-    }
-    for (int e = tid; e < nch * NU; e += nth) {
-      const int ch = e / NU, f = e - ch * NU;
-      cfull[e] = fetch(chalf + ch * HU, sexp[f]);
-    }
-    __syncthreads();
-    // ---- Z terms, y, and B (linear model) ------------------------------------------------------
-    for (int ch = 0; ch < nch; ++ch) {
-      cx<T>* zt = tbuf + (kQuad ? (size_t)ch * tb.NZT : 0);
-      z_rounds<T>(tb.zitems, zr0, zr1, cfull + ch * NU, scg, zt, lane);
+      for (int ch = 0; ch < nch; ++ch)
+        z_rounds<T>(tb.zitems, zr0, zr1, cfull + ch * NU, scg, tbuf + (size_t)ch * tb.NZT, lane);
       __syncthreads();
       // y of each half entry: the blocks of its layer with their weights, in order
-      const T* gc = sgam + ch * tb.NBLK;
-      for (int h = tid; h < HU; h += nth) {
+      for (int i = tid; i < nch * HU; i += nth) {
+        const int ch = i / HU, h = i - ch * HU;
         const int j = sj[h], H = shoff[j + 1] - shoff[j];
-        const cx<T>* z = zt + tb.zoff[j] + (h - shoff[j]);
-        const T* g = gc + tb.blk_off[j];
+        const cx<T>* z = tbuf + (size_t)ch * tb.NZT + tb.zoff[j] + (h - shoff[j]);
+        const T* g = sgam + ch * tb.NBLK + tb.blk_off[j];
         const int nb = tb.blk_off[j + 1] - tb.blk_off[j];
         cx<T> v = {T(0), T(0)};
 #pragma unroll 4
@@ -234,32 +231,30 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
           v.x = fma(g[r], zr.x, v.x);
           v.y = fma(g[r], zr.y, v.y);
         }
-        yt[ch * HU + h] = v;
+        yt[i] = v;
       }
-      if constexpr (!kQuad) {
-        b_sums<T>(tb.trz, K, shoff, chalf + ch * HU, zt, warp, lane, Bk + ch * K);
-        __syncthreads();
+      __syncthreads();
+    } else {
+      ysrc = static_cast<const cx<T>*>(args.ev.y) + (size_t)atom * nch * HU;
+      if (warp == kNW - 1) {  // energy of the atom, w0 + w_lin . B = w0 + c . y / 3
+        const cx<T>* c = static_cast<const cx<T>*>(args.ev.c) + (size_t)atom * nch * HU;
+        ExactSum<T> s;
+        for (int e = lane; e < nch * HU; e += 32) {
+          const T w = args.gen[e % HU].w;
+          const cx<T> cv = c[e], yv = ysrc[e];
+          s.add(cv.x, yv.x, w);
+          s.add(cv.y, yv.y, w);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s.add(s.down(o));
+        if (lane == 0) args.ev.Eatom[atom] = args.ev.w0 + s.value() / 3.0;
       }
-    }
-    if constexpr (kQuad) __syncthreads();
-    if constexpr (!kQuad) {
-      if (warp == 0) {  // energy of the atom, w0 + w_lin . B_a (FP64, fixed lane order)
-        double e = 0.0;
-        if (nn > 0)
-          for (int k = lane; k < nchK; k += 32) e += args.ev.wlin[k] * (double)Bk[k];
-        for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-        if (lane == 0) args.ev.Eatom[atom] = e + args.ev.w0;
-      }
-    }
-    if (nn == 0) {
-      if (tid < 6) args.ev.Satom[(size_t)atom * 6 + tid] = 0.0;
-      continue;
     }
     // ---- the generators' y_b, weighted for sums over the half layers ---------------------------
     for (int e = tid; e < nch * HU; e += nth) {
       const int ch = e / HU, h = e - ch * HU;
       const GenEntry<T> g = args.gen[h];
-      const cx<T>* y = yt + ch * HU;
+      const cx<T>* y = ysrc + ch * HU;
       const cx<T> y0 = y[h], ym = y[max(h - 1, 0)];
       cx<T> yp = y[min(h + 1, HU - 1)];
       if (g.w == T(1)) yp = {-ym.x, ym.y};  // centre of an even layer: y(0, 2) = -conj y(0, -2)
@@ -271,13 +266,13 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
       o[2] = {w * (a.y + b.y), -w * (a.x + b.x)};
       o[3] = {w * (b.x - a.x), w * (b.y - a.y)};
     }
-    __syncthreads();
+    if constexpr (kQuad) __syncthreads();  // (the linear model's passes begin with a barrier)
     // ---- pairs: forces (and, linear model, stress) ---------------------------------------------
     const T lev = args.small[args.atom_struct[atom]] ? T(1) : -args.sign_big;  // stress lever arm: sign * u
-    StressSum<T> sacc;  // of this thread's (pair slot, component)
+    ExactSum<T> sacc;  // of this thread's (pair slot, component)
     for (int ps = npass - 1; ps >= 0; --ps) {
       const int base = ps * args.slots, count = min(args.slots, nn - base);
-      if (ps != npass - 1) load_pass(base, count);  // (the last pass is still in shared memory)
+      if (!kQuad || ps != npass - 1) load_pass(base, count);  // (quadratic: the last pass is still there)
       for (int g4 = warp * 4; g4 < count; g4 += kNW * 4) {
         // a warp takes four pairs, its lanes the half entries
         T tot[16];
@@ -437,13 +432,13 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
       if (ps > 0) __syncthreads();  // the pass's U and geometry have been read
     }
     // stress of the atom: the partial sums of (slot, component), slots in order
-    StressSum<T>* sred = reinterpret_cast<StressSum<T>*>(red);
+    ExactSum<T>* sred = reinterpret_cast<ExactSum<T>*>(red);
     if constexpr (kQuad) {
       __syncthreads();
       if (tid < kChunk * 6) sred[tid] = sacc;
       __syncthreads();
       if (tid < 6) {
-        StressSum<T> v;
+        ExactSum<T> v;
         for (int n = 0; n < kChunk; ++n) v.add(sred[n * 6 + tid]);
         args.ev.Satom[(size_t)atom * 6 + tid] = v.value();
       }
@@ -451,7 +446,7 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
       if (lane < 24) sred[warp * 24 + lane] = sacc;
       __syncthreads();
       if (warp == 0) {
-        StressSum<T> v;
+        ExactSum<T> v;
         if (lane < 24)
           for (int w = 0; w < kNW; ++w) v.add(sred[w * 24 + lane]);
         v.add(v.down(12));  // slots (0 + 2) and (1 + 3), then both
@@ -478,8 +473,8 @@ template <typename T>
 cudaError_t launch_bso4_eval(const DevTables& tb, const DevBatch& b, const BsoParams& p, const DevEval<T>& ev,
                              const int* order, int* counter, cudaStream_t st) {
   if (b.A == 0) return cudaSuccess;
-  if (!counter || !ev.pair || !ev.Satom || !tb.gen32) return cudaErrorInvalidValue;
-  const bool quad = ev.per_atom != 0;
+  if (!counter || !ev.pair || !ev.Satom || !tb.gen32 || (!ev.gamma && (!ev.c || !ev.y))) return cudaErrorInvalidValue;
+  const bool quad = ev.gamma != nullptr;
   EvalArgs<T> a{};
   a.tb = tb;
   if constexpr (sizeof(T) == 8) {

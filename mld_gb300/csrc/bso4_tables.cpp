@@ -246,6 +246,123 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
     t->gam_off.push_back((int)t->gam.size());
   }
 
+  // atoms-on-lanes sums: operand pairs in descending order (exchanging the operands of a block changes
+  // the sign of both its CG factors alike), all output layers of a pair from one set of products
+  {
+    std::map<std::pair<int, int>, std::vector<int>> outs;  // pair -> output layers, descending
+    for (const auto& kb : kblocks)
+      for (const Block& B : kb) {
+        std::vector<int>& v = outs[{std::max(B.jA, B.jB), std::min(B.jA, B.jB)}];
+        if (std::find(v.begin(), v.end(), B.jO) == v.end()) v.push_back(B.jO);
+      }
+    struct Part { long long cost; LaneRec r; };
+    // a job's records in four parts, each record to the least loaded one, longest first
+    auto add_job = [](std::vector<Part>& recs, LaneJob job, std::vector<LaneRec>* out, std::vector<LaneJob>* jobs) {
+      std::stable_sort(recs.begin(), recs.end(), [](const Part& x, const Part& y) { return x.cost > y.cost; });
+      std::vector<LaneRec> part[4];
+      long long load[4] = {0, 0, 0, 0};
+      for (const Part& p : recs) {
+        const int q = (int)(std::min_element(load, load + 4) - load);
+        load[q] += p.cost;
+        part[q].push_back(p.r);
+      }
+      for (int q = 0; q < 4; ++q) {
+        job.rec[q] = (int)out->size();
+        out->insert(out->end(), part[q].begin(), part[q].end());
+      }
+      job.rec[4] = (int)out->size();
+      jobs->push_back(job);
+    };
+    std::map<std::tuple<int, int, int>, int> pblk;  // pair block -> its number
+    std::vector<std::vector<GammaItem>> gam;
+    for (int k = 0; k < t->K; ++k)
+      for (const Block& B : kblocks[k]) {
+        const auto ins = pblk.emplace(std::make_tuple(std::max(B.jA, B.jB), std::min(B.jA, B.jB), B.jO), (int)pblk.size());
+        if (ins.second) gam.emplace_back();
+        gam[ins.first->second].push_back(GammaItem{(uint16_t)k, (uint8_t)B.snum, (uint8_t)B.sden});
+      }
+    t->nblk_pair = (int)gam.size();
+    for (const auto& v : gam) {
+      t->gamp_off.push_back((int)t->gamp.size());
+      t->gamp.insert(t->gamp.end(), v.begin(), v.end());
+    }
+    t->gamp_off.push_back((int)t->gamp.size());
+    std::map<std::tuple<int, int, int>, int> triple;
+    for (int k = 0; k < t->K; ++k) triple[std::make_tuple(t->l1[k], t->l2[k], t->l[k])] = k;
+    std::map<std::pair<int, int>, std::vector<Part>> ypos;  // output position -> records
+    struct BJob { long long cost; std::vector<Part> recs; LaneJob job; };
+    std::vector<BJob> bjobs;
+    for (auto& pr : outs) {
+      const int jA = pr.first.first, jB = pr.first.second;
+      std::vector<int>& os = pr.second;
+      std::sort(os.begin(), os.end(), [](int x, int y) { return x > y; });
+      const int jm = os[0];
+      std::map<int, std::pair<int, int>> cgo;  // m -> offset, stride
+      for (int m = -jm; m <= jm; m += 2) {
+        int n = 0;
+        while (n < (int)os.size() && os[n] >= std::abs(m)) ++n;
+        cgo[m] = {(int)t->cgv.size(), n};
+        for (int ma = std::max(-jA, m - jB); ma <= std::min(jA, m + jB); ma += 2)
+          for (int o = 0; o < n; ++o) t->cgv.push_back(cg_coefficient(jA, ma, jB, m - ma, os[o], m));
+      }
+      BJob bj{};
+      for (int o : os)
+        if (o >= jA) bj.job.out[bj.job.nout++] = (uint16_t)triple.at(std::make_tuple(jA, jB, o));
+      for (int m1 = -jm; m1 <= jm; m1 += 2)
+        for (int m2 = -jm; m2 <= jm; m2 += 2) {
+          if (loc(jm, m1, m2) >= H(jm)) continue;
+          const int malo = std::max(-jA, m1 - jB), mahi = std::min(jA, m1 + jB);
+          const int mblo = std::max(-jA, m2 - jB), mbhi = std::min(jA, m2 + jB);
+          const int mu = std::max(std::abs(m1), std::abs(m2));
+          LaneRec r{};
+          r.na = (uint8_t)((mahi - malo) / 2 + 1);
+          r.nb = (uint8_t)((mbhi - mblo) / 2 + 1);
+          r.s1 = (uint8_t)(jA + 1);
+          r.s2 = (uint8_t)(jB + 1);
+          r.i1 = (uint16_t)uidx(jA, malo, mblo);
+          r.i2 = (uint16_t)uidx(jB, m1 - malo, m2 - mblo);
+          r.cg1 = (uint16_t)cgo[m1].first;
+          r.cg2 = (uint16_t)cgo[m2].first;
+          r.st1 = (uint8_t)cgo[m1].second;
+          r.st2 = (uint8_t)cgo[m2].second;
+          LaneRec y = r, b = r;
+          const int top = J - ((J ^ m1) & 1);  // highest layer with this position
+          y.off = (uint8_t)((top - jm) / 2);
+          for (int o : os)
+            if (o >= mu) y.out[y.nj++] = (uint16_t)pblk.at(std::make_tuple(jA, jB, o));
+          b.w = (uint16_t)((m1 == 0 && m2 == 0) ? 1 : 2);
+          for (int o : os)
+            if (o >= mu && o >= jA) b.out[b.nj++] = (uint16_t)uidx(o, m1, m2);
+          auto cost = [](const LaneRec& x) { return (long long)x.na * (x.nb * (4 + 2 * x.nj) + 2 * x.nj) + 16; };
+          ypos[{m1, m2}].push_back(Part{cost(y), y});
+          if (b.nj) {
+            bj.recs.push_back(Part{cost(b), b});
+            bj.cost += cost(b);
+          }
+        }
+      if (!bj.recs.empty()) bjobs.push_back(std::move(bj));
+    }
+    if (t->cgv.size() >= 65535) {
+      *err = "contraction tables exceed 16-bit offsets";
+      return false;
+    }
+    std::stable_sort(bjobs.begin(), bjobs.end(), [](const BJob& x, const BJob& y) { return x.cost > y.cost; });
+    for (BJob& b : bjobs) add_job(b.recs, b.job, &t->brecs, &t->bjobs);
+    std::vector<std::pair<long long, std::pair<int, int>>> yorder;
+    for (const auto& yp : ypos) {
+      long long c = 0;
+      for (const Part& p : yp.second) c += p.cost;
+      yorder.push_back({-c, yp.first});
+    }
+    std::sort(yorder.begin(), yorder.end());
+    for (const auto& yo : yorder) {
+      const int m1 = yo.second.first, m2 = yo.second.second, mu = std::max(std::abs(m1), std::abs(m2));
+      LaneJob job{};
+      for (int o = J - ((J ^ m1) & 1); o >= mu; o -= 2) job.out[job.nout++] = (uint16_t)(t->hoff[o] + loc(o, m1, m2));
+      add_job(ypos[yo.second], job, &t->yrecs, &t->yjobs);
+    }
+  }
+
   // layer-blocked Y: rows of layer j are the triples using layer j (any of l, l1, l2).  A
   // triple's distinct layers in ascending order have ranks 0, 1, 2; within a layer the rows are
   // grouped by rank, the layer padded to whole row tiles.  The dB contraction writes a row's

@@ -65,8 +65,12 @@ template <typename T>
 cudaError_t launch_eval_gamma(const DevTables& tb, const T* B, int A, int nch, const double* wlin, const double* wsym,
                               double w0, T* gamma, double* Eatom, cudaStream_t st) {
   if (A <= 0) return cudaSuccess;
-  k_eval_gamma<T><<<B ? A : 1, kGammaThreads, sizeof(double) * 2 * nch * tb.K, st>>>(tb.gam_off, tb.gam, tb.NBLK, nch, tb.K, B,
-                                                                                     wlin, wsym, w0, gamma, Eatom);
+  const size_t smem = sizeof(double) * 2 * nch * tb.K;
+  if (B)
+    k_eval_gamma<T><<<A, kGammaThreads, smem, st>>>(tb.gam_off, tb.gam, tb.NBLK, nch, tb.K, B, wlin, wsym, w0, gamma, Eatom);
+  else
+    k_eval_gamma<T><<<1, kGammaThreads, smem, st>>>(tb.gamp_off, tb.gamp, tb.NBLKP, nch, tb.K, nullptr, wlin, nullptr, w0,
+                                                    gamma, nullptr);
   return cudaGetLastError();
 }
 

@@ -85,6 +85,31 @@ struct BkItem {
 static_assert(sizeof(BkItem) == 8, "B items are 8 bytes");
 static_assert(offsetof(BkItem, ufull) == 2 && offsetof(BkItem, wgt) == 4, "BkItem layout (decoded by the descriptor kernel)");
 
+// A record of the atoms-on-lanes sums (bispectrum_lanes.cu; 32 bytes): for an operand pair jA >= jB and
+// an output position (m1, m2), the Z terms of nj of the pair's output layers in descending jO,
+//   Z_o = sum_{a<na} cgv[cg1 + a st1 + o] sum_{b<nb} cgv[cg2 + b st2 + o] c[i1 + a s1 + b] c[i2 - a s2 - b].
+constexpr int kMaxZOut = kMaxJ / 2 + 1;
+struct alignas(16) LaneRec {
+  uint16_t i1, i2, cg1, cg2;
+  uint8_t na, nb, s1, s2;
+  uint8_t st1, st2, nj, off;  // off (y): the job's output of Z_0
+  uint16_t out[kMaxZOut];     // y: the terms' blocks; B: c indices of the output position
+  uint16_t w;                 // B: weight of the position in a sum over full layers
+  uint16_t pad;
+};
+static_assert(sizeof(LaneRec) == 32, "lane records are two 16-byte words");
+static_assert(offsetof(LaneRec, na) == 8 && offsetof(LaneRec, st1) == 12 && offsetof(LaneRec, out) == 16 &&
+                  offsetof(LaneRec, w) == 28,
+              "LaneRec layout (decoded from its words)");
+// A job: its records in four parts of about equal work, and its outputs (y: half entries of the
+// layers jO in descending order; B: triples)
+struct LaneJob {
+  int rec[5];
+  uint16_t nout;
+  uint16_t out[kMaxZOut];
+  uint16_t pad;
+};
+
 // Layer l of a triple and the first term of its ZA block: B_k = sum_e w_e Re(conj(c^l[e]) Z[za + e]).
 struct TripleZ {
   uint16_t za;
@@ -151,6 +176,16 @@ struct Bso4Tables {
   // (snum / sden) beta_k
   std::vector<int> gam_off;
   std::vector<GammaItem> gam;
+  // the blocks with their operands in descending order (blocks that differ by the exchange are one),
+  // as the atoms-on-lanes sums count them
+  int nblk_pair = 0;
+  std::vector<int> gamp_off;
+  std::vector<GammaItem> gamp;
+  // atoms-on-lanes sums: CG coefficients of a pair by (m, first index, jO descending), the records and
+  // jobs of B (a job per operand pair) and y (a job per output position), heaviest jobs first
+  std::vector<double> cgv;
+  std::vector<LaneRec> brecs, yrecs;
+  std::vector<LaneJob> bjobs, yjobs;
   std::vector<TripleZ> trz;       // the ZA block and layer of each triple
   std::vector<RowSource> rowsrc;  // the blocks of every contraction row, indexed as rowk
   std::vector<int8_t> half_diag;  // half entries on the diagonal p == q (get the +1 of c)
@@ -175,6 +210,13 @@ struct DevTables {
   int NBLK = 0;
   int blk_off[kMaxJ + 2] = {0};
   int zoff[kMaxJ + 1] = {0};
+  int NCGV = 0, NBJ = 0, NYJ = 0, NBLKP = 0;
+  double* cgv64 = nullptr;        // NCGV
+  float* cgv32 = nullptr;
+  LaneRec* brecs = nullptr;
+  LaneJob* bjobs = nullptr;       // NBJ
+  LaneRec* yrecs = nullptr;       // (fill_deriv_tables)
+  LaneJob* yjobs = nullptr;       // NYJ
   TripleZ* trz = nullptr;         // K
   RowSource* rowsrc = nullptr;    // NROWS
   int hoff[kMaxJ + 2] = {0};
@@ -196,6 +238,8 @@ struct DevTables {
   GenEntry<double>* gen64 = nullptr;  // HU
   int* gam_off = nullptr;       // NBLK + 1
   GammaItem* gam = nullptr;
+  int* gamp_off = nullptr;      // NBLKP + 1
+  GammaItem* gamp = nullptr;
 };
 
 // Fill the scalar part of *d from t and place every device table through put(vector, &ptr),
@@ -239,6 +283,13 @@ cudaError_t fill_dev_tables(const Bso4Tables& t, DevTables* d, Put put) {
   if (e == cudaSuccess) e = put(t.expand, &d->expand);
   if (e == cudaSuccess) e = put(t.half_diag, &d->half_diag);
   if (e == cudaSuccess) e = put(t.zitems, &d->zitems);
+  d->NCGV = (int)t.cgv.size();
+  d->NBJ = (int)t.bjobs.size();
+  std::vector<float> cgv32(t.cgv.begin(), t.cgv.end());
+  if (e == cudaSuccess) e = put(t.cgv, &d->cgv64);
+  if (e == cudaSuccess) e = put(cgv32, &d->cgv32);
+  if (e == cudaSuccess) e = put(t.brecs, &d->brecs);
+  if (e == cudaSuccess) e = put(t.bjobs, &d->bjobs);
   if (e == cudaSuccess) e = put(t.trz, &d->trz);
   if (e == cudaSuccess) e = put(t.rowsrc, &d->rowsrc);
   if (e == cudaSuccess) e = put(t.zitem_off, &d->zitem_off);
@@ -259,6 +310,12 @@ cudaError_t fill_deriv_tables(const Bso4Tables& t, DevTables* d, Put put) {
   if (e == cudaSuccess) e = put(g64, &d->gen64);
   if (e == cudaSuccess) e = put(t.gam_off, &d->gam_off);
   if (e == cudaSuccess) e = put(t.gam, &d->gam);
+  d->NBLKP = t.nblk_pair;
+  if (e == cudaSuccess) e = put(t.gamp_off, &d->gamp_off);
+  if (e == cudaSuccess) e = put(t.gamp, &d->gamp);
+  d->NYJ = (int)t.yjobs.size();
+  if (e == cudaSuccess) e = put(t.yrecs, &d->yrecs);
+  if (e == cudaSuccess) e = put(t.yjobs, &d->yjobs);
   return e;
 }
 
@@ -341,15 +398,30 @@ cudaError_t launch_sort_lists(const DevBatch& b, cudaStream_t st);
 // does not fit in shared memory, and preferred (unless only_if_required) when it would cost a
 // resident CTA per SM; 0 otherwise.
 size_t bso4_y_scratch_bytes(const DevTables& tb, int nch, int eb, int max_ctas, bool only_if_required = false);
+// c (count x nch x HU complex of T) of atoms first .. first + count - 1; with `order` (all atoms, in
+// that order) first = 0.  counter: one int of device memory, reset by the launch.
+template <typename T>
+cudaError_t launch_c_half(const DevTables& tb, const DevBatch& b, const BsoParams& p, int first, int count,
+                          const int* order, int* counter, void* c, cudaStream_t st);
+// B (whole-batch array) of the same atoms from their c.
+template <typename T>
+cudaError_t launch_lane_descriptors(const DevTables& tb, const DevBatch& b, const BsoParams& p, int first, int count,
+                                    const void* c, T* B, cudaStream_t st);
+// y = dE/dc (as c) of the same atoms with the pair-block weights gamma (nch * NBLKP).
+template <typename T>
+cudaError_t launch_lane_y(const DevTables& tb, const DevBatch& b, const BsoParams& p, int first, int count,
+                          const void* c, const T* gamma, void* y, cudaStream_t st);
+
 // Evaluation with fitted weights (bispectrum_eval.cu): per-pair forces and per-atom stress of
 // dE/dB_a (beta_a = w_lin for the linear model; w_lin + (W + W^T) B_a for the quadratic one),
-// gathered into E/F/S by launch_eval_gather.  The weights come as gamma, per Z block and channel.
+// gathered into E/F/S by launch_eval_gather.
 template <typename T>
 struct DevEval {
-  const T* gamma = nullptr;      // one vector (nch * NBLK) or one per atom
-  int per_atom = 0;
-  const double* wlin = nullptr;  // linear weights: the kernel writes Eatom = w0 + w_lin . B_a (linear model)
+  // linear model: c and y of every atom (A x nch x HU complex of T); the kernel writes Eatom
+  const void* c = nullptr;
+  const void* y = nullptr;
   double w0 = 0.0;
+  const T* gamma = nullptr;      // quadratic model: Z-block weights, nch * NBLK per atom
   T* pair = nullptr;             // P x 3: the pair's force contribution
   double* Satom = nullptr;       // A x 6: sum over the atom's pairs of the stress products (xx yy zz yz xz xy)
   double* Eatom = nullptr;       // A: energy of each atom (written for the linear model)
@@ -388,7 +460,8 @@ cudaError_t launch_eval_gather(const DevBatch& b, const BsoParams& p, const int*
 size_t atom_order_tmp_ints(int maxnn);
 cudaError_t launch_atom_order(const int* nn, int A, int maxnn, int* order, int* tmp, cudaStream_t st);
 // The block weights gamma (nch * NBLK per atom) of beta_a = w_lin + Wsym B_a and the energies
-// Eatom_a = w0 + B_a . (beta_a + w_lin) / 2; with B null those of beta = w_lin, once (eval.cu)
+// Eatom_a = w0 + B_a . (beta_a + w_lin) / 2; with B null the pair-block weights (nch * NBLKP) of
+// beta = w_lin, once (eval.cu)
 template <typename T>
 cudaError_t launch_eval_gamma(const DevTables& tb, const T* B, int A, int nch, const double* wlin, const double* wsym,
                               double w0, T* gamma, double* Eatom, cudaStream_t st);

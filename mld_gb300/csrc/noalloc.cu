@@ -233,17 +233,17 @@ extern "C" int mld_gpu_descriptors_noalloc(const mld_gpu_config* cfg, int nat, c
   int* dmax = reinterpret_cast<int*>(take(sizeof(int) * 2));
   int* qcount = reinterpret_cast<int*>(take(sizeof(int)));  // descriptor kernel's queue counter
   float* bstage = mixed ? reinterpret_cast<float*>(take(sizeof(float) * (size_t)nat * KK)) : nullptr;
-  // global Y slices of the descriptor kernel only when they do not fit in shared memory (FP64
-  // with several channels); at most 64 persistent CTAs
-  const size_t ysb = bso4_y_scratch_bytes(dt, nch, mixed ? 4 : 8, 64, true);
-  void* yscr = ysb ? take(ysb) : nullptr;
+  // c of a chunk of atoms (at least kMinChunk, as many as the space behind the pairs holds)
+  constexpr int kMinChunk = 32;
+  const size_t per_atom = (size_t)nch * dt.HU * 2 * (mixed ? 4 : 8);
+  const size_t reserve = align256(per_atom * std::min(nat, kMinChunk));
   const size_t fixed = (size_t)(p - S->base);
-  if (fixed > kScratchBytes) {
+  if (fixed + reserve + 512 > kScratchBytes) {
     set_err(err, err_len, "descriptor staging exceeds the scratch array");
     return MLD_ERR_NOALLOC_LIMIT;
   }
   // remaining space holds the neighbour list: 4 B index + 24 B displacement per pair
-  const long long pair_cap = std::min<long long>((long long)(kScratchBytes - fixed - 512) / 28,
+  const long long pair_cap = std::min<long long>((long long)(kScratchBytes - fixed - reserve - 512) / 28,
                                                  (long long)MLD_NOALLOC_MAX_PAIRS);
 
 #define CKN(call)                                                            \
@@ -299,13 +299,23 @@ extern "C" int mld_gpu_descriptors_noalloc(const mld_gpu_config* cfg, int nat, c
   prm.rin_width = cfg->r_cut_width_in;
   prm.sign_stress = cfg->sign_stress;
   prm.sign_big = cfg->sign_stress_big_box;
+  p = S->base + align256((size_t)(p - S->base));
+  const int chunk = (int)std::min<size_t>(nat, (size_t)(S->base + kScratchBytes - p) / per_atom);
+  void* c = take(per_atom * chunk);
+  for (int a0 = 0; a0 < nat; a0 += chunk) {
+    const int na = std::min(chunk, nat - a0);
+    if (mixed) {
+      CKN(launch_c_half<float>(dt, b, prm, a0, na, nullptr, qcount, c, st));
+      CKN(launch_lane_descriptors<float>(dt, b, prm, a0, na, c, bstage, st));
+    } else {
+      CKN(launch_c_half<double>(dt, b, prm, a0, na, nullptr, qcount, c, st));
+      CKN(launch_lane_descriptors<double>(dt, b, prm, a0, na, c, B, st));
+    }
+  }
   if (mixed) {
-    CKN(launch_bso4<float>(dt, b, prm, bstage, (float*)nullptr, nullptr, qcount, st, yscr, ysb));
     const size_t n = (size_t)nat * KK;
     k_widen<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(bstage, B, n);
     CKN(cudaGetLastError());
-  } else {
-    CKN(launch_bso4<double>(dt, b, prm, B, (double*)nullptr, nullptr, qcount, st, yscr, ysb));
   }
 #undef CKN
   return MLD_OK;
