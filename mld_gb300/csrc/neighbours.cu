@@ -113,11 +113,30 @@ __global__ void __launch_bounds__(256) k_neighbours(
     const int lo0 = n0 >= 3 ? -1 : 0, hi0 = n0 >= 3 ? 1 : n0 - 1;
     const int lo1 = n1 >= 3 ? -1 : 0, hi1 = n1 >= 3 ? 1 : n1 - 1;
     const int lo2 = n2 >= 3 ? -1 : 0, hi2 = n2 >= 3 ? 1 : n2 - 1;
+    // the cells of a row along the last direction are consecutive: one range of atoms, or two
+    // where the row wraps around, instead of three of a few atoms each (27 scans with a quarter of
+    // the lanes busy)
+    const int w0 = c2 + lo2, w1 = c2 + hi2;  // cells w0 .. w1 of the row, before wrapping
     for (int d0 = lo0; d0 <= hi0; ++d0)
-      for (int d1 = lo1; d1 <= hi1; ++d1)
-        for (int d2 = lo2; d2 <= hi2; ++d2) {
-          const int cell = cell_off[s] + (((c0 + d0 + n0) % n0) * n1 + (c1 + d1 + n1) % n1) * n2 + (c2 + d2 + n2) % n2;
-          const int e0 = cell_start[cell], e1 = cell_start[cell + 1];
+      for (int d1 = lo1; d1 <= hi1; ++d1) {
+        const int row = cell_off[s] + (((c0 + d0 + n0) % n0) * n1 + (c1 + d1 + n1) % n1) * n2;
+        for (int seg = 0; seg < 2; ++seg) {
+          int f, t;  // first and last cell of the segment
+          if (n2 < 3) {
+            f = 0;
+            t = seg == 0 ? n2 - 1 : -1;
+          } else if (w0 < 0) {
+            f = seg == 0 ? 0 : w0 + n2;
+            t = seg == 0 ? w1 : n2 - 1;
+          } else if (w1 >= n2) {
+            f = seg == 0 ? w0 : 0;
+            t = seg == 0 ? n2 - 1 : w1 - n2;
+          } else {
+            f = w0;
+            t = seg == 0 ? w1 : -1;
+          }
+          if (t < f) continue;
+          const int e0 = cell_start[row + f], e1 = cell_start[row + t + 1];
           for (int base = e0; base < e1; base += 32) {
             const int e = base + lane;
             bool ok = false;
@@ -156,12 +175,99 @@ __global__ void __launch_bounds__(256) k_neighbours(
             count += __popc(m);
           }
         }
+      }
     if (pass != 1 && lane == 0) {
       counts[g] = count;
       atomicMax(maxcount, count);
     }
     return;
   }
+  if (sm) {
+    // Small box.  An image n of atom j lies at least |f_k + n_k| w_k away (f = fractional x_j - x_i, w_k the
+    // perpendicular widths), so along each direction only the n_k with |f_k + n_k| w_k < r_cut + margin
+    // are candidates: one or two of 2 nsize + 1.  A lane takes one (j, n1) and keeps its accepted
+    // (n2, n3) as bits; the lanes' counts give their places, in the order (j, n1, n2, n3).
+    float b32[9], iw[3];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) b32[k] = (float)bg[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)  // (r_cut + margin) / w_k; the margin covers the FP32 rounding of f
+      iw[k] = (rcb + kBand) * sqrtf(b32[3 * k] * b32[3 * k] + b32[3 * k + 1] * b32[3 * k + 1] + b32[3 * k + 2] * b32[3 * k + 2]);
+    const int c2m = (int)(2.f * iw[1]) + 2, c3m = (int)(2.f * iw[2]) + 2;  // most n2, n3 of a lane
+    if (c2m * c3m <= 64) {
+      const int w1n = 2 * n1s + 1;
+      const long long nitem = (long long)nat * w1n;
+      for (long long base = 0; base < nitem; base += 32) {
+        const long long it = base + lane;
+        unsigned long long hit = 0ull;
+        int jj = 0, n1 = 0, lo2 = 0, lo3 = 0, cnt3 = 1;
+        if (it < nitem) {
+          if (nitem < 0x7fffffffLL) jj = (int)it / w1n;
+          else jj = (int)(it / w1n);
+          n1 = (int)(it - (long long)jj * w1n) - n1s;
+          const float4 pj = pos32[a0 + jj];
+          const float x0 = pj.x - pi.x, x1 = pj.y - pi.y, x2 = pj.z - pi.z;
+          const float f0 = b32[0] * x0 + b32[1] * x1 + b32[2] * x2;
+          const float f1 = b32[3] * x0 + b32[4] * x1 + b32[5] * x2;
+          const float f2 = b32[6] * x0 + b32[7] * x1 + b32[8] * x2;
+          if (fabsf(f0 + (float)n1) < iw[0]) {
+            lo2 = max(-n2s, (int)ceilf(-iw[1] - f1));
+            lo3 = max(-n3s, (int)ceilf(-iw[2] - f2));
+            const int hi2 = min(n2s, (int)floorf(iw[1] - f1)), hi3 = min(n3s, (int)floorf(iw[2] - f2));
+            cnt3 = max(1, hi3 - lo3 + 1);
+            int bit = 0;
+            for (int n2 = lo2; n2 <= hi2; ++n2)
+              for (int n3 = lo3; n3 <= hi3; ++n3, ++bit) {
+                const float d0 = (pi.x - pj.x) - (c32[0] * n1 + c32[3] * n2 + c32[6] * n3);
+                const float d1 = (pi.y - pj.y) - (c32[1] * n1 + c32[4] * n2 + c32[7] * n3);
+                const float d2 = (pi.z - pj.z) - (c32[2] * n1 + c32[5] * n2 + c32[8] * n3);
+                const float r2f = d0 * d0 + d1 * d1 + d2 * d2;
+                bool ok = false;
+                if (r2f < rci2 && r2f > kSelf2) {
+                  ok = true;
+                } else if (r2f < rcb2) {
+                  const double* xj = pos + 3 * (size_t)(a0 + jj);
+                  const double t0 = xi0 - (xj[0] + cl[0] * n1 + cl[3] * n2 + cl[6] * n3);
+                  const double t1 = xi1 - (xj[1] + cl[1] * n1 + cl[4] * n2 + cl[7] * n3);
+                  const double t2 = xi2 - (xj[2] + cl[2] * n1 + cl[5] * n2 + cl[8] * n3);
+                  const double r2 = t0 * t0 + t1 * t1 + t2 * t2;
+                  ok = (r2 >= 1e-15) && (r2 <= rc2) && (sqrt(r2) < rcut);
+                }
+                if (ok) hit |= 1ull << bit;
+              }
+          }
+        }
+        const int mine = __popcll(hit);
+        int pre = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, pre, o);
+          if (lane >= o) pre += v;
+        }
+        const int total = __shfl_sync(0xffffffffu, pre, 31);
+        if (pass != 0) {
+          int k = count + pre - mine;
+          for (unsigned long long m = hit; m; m &= m - 1, ++k) {
+            const int bit = __ffsll((long long)m) - 1, n2 = lo2 + bit / cnt3, n3 = lo3 + bit % cnt3;
+            if (pass == 1) {
+              nbr_idx[wbase + k] = a0 + jj;
+              nbr_u[3 * (size_t)(wbase + k)] = (double)g;
+              nbr_u[3 * (size_t)(wbase + k) + 1] = (double)pack_image(n1, n2, n3);
+            } else if (k < cap) {
+              tmp[(size_t)g * cap + k] = make_int2(a0 + jj, pack_image(n1, n2, n3));
+            }
+          }
+        }
+        count += total;
+      }
+      if (pass != 1 && lane == 0) {
+        counts[g] = count;
+        atomicMax(maxcount, count);
+      }
+      return;
+    }
+  }
+  // all atoms (and, in a box thinner than the bits allow, all images)
   const long long ncand = (long long)nat * nimg;
   for (long long base = 0; base < ncand; base += 32) {
     const long long cidx = base + lane;
