@@ -1341,7 +1341,7 @@ int mld_gpu_descriptors(mld_gpu_handle* h, double* B_out, int* n_neigh_out) {
   const size_t nB = (size_t)h->A * h->KK;
   if (h->mixed) {
     CK(ensure(h, mld_gpu_handle::B_BOUT, sizeof(float) * std::max<size_t>(nB, 1)));
-    rc = run_descriptors<float>(h, true, bp_<float>(h, mld_gpu_handle::B_BOUT));
+    rc = run_descriptors<float>(h, false, bp_<float>(h, mld_gpu_handle::B_BOUT));
     if (rc) return rc;
     if (B_out) {
       std::vector<float> tmp(nB);
@@ -1352,7 +1352,7 @@ int mld_gpu_descriptors(mld_gpu_handle* h, double* B_out, int* n_neigh_out) {
     }
   } else {
     CK(ensure(h, mld_gpu_handle::B_BOUT, sizeof(double) * std::max<size_t>(nB, 1)));
-    rc = run_descriptors<double>(h, true, bp_<double>(h, mld_gpu_handle::B_BOUT));
+    rc = run_descriptors<double>(h, false, bp_<double>(h, mld_gpu_handle::B_BOUT));
     if (rc) return rc;
     if (B_out)
       CK(cudaMemcpyAsync(B_out, bp_<double>(h, mld_gpu_handle::B_BOUT), sizeof(double) * nB, cudaMemcpyDeviceToHost,
@@ -1378,6 +1378,12 @@ int mld_gpu_descriptor_derivatives(mld_gpu_handle* h, long long* P_inout, int* n
   if (u_out) CK(cudaMemcpyAsync(u_out, h->b.nbr_u, sizeof(double) * 3 * P, cudaMemcpyDeviceToHost, h->st));
   const size_t nd = (size_t)P * 3 * h->KK;
   if (dB_out) {
+    // the derivatives of the staged batch; its B come along
+    const size_t nB = std::max<size_t>((size_t)h->A * h->KK, 1);
+    CK(ensure(h, mld_gpu_handle::B_BOUT, (h->mixed ? sizeof(float) : sizeof(double)) * nB));
+    const int rc = h->mixed ? run_descriptors<float>(h, true, bp_<float>(h, mld_gpu_handle::B_BOUT))
+                            : run_descriptors<double>(h, true, bp_<double>(h, mld_gpu_handle::B_BOUT));
+    if (rc) return rc;
     if (h->mixed) {
       std::vector<float> tmp(nd);
       CK(cudaMemcpyAsync(tmp.data(), bp_<float>(h, mld_gpu_handle::B_DBOUT), sizeof(float) * nd,

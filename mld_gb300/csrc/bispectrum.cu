@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
   T* ssc = reinterpret_cast<T*>(smem_raw + sp.sc);  // ssc[16 n + d] = n / d, the row scales
 
   // tables, once per CTA
-  for (int e = tid; e < HU; e += nth) sgen[e] = args.gen ? args.gen[e] : GenEntry<T>{};
+  for (int e = tid; e < HU; e += nth) sgen[e] = args.gen[e];
   for (int e = tid; e < kMaxJ + 2; e += nth) shoff[e] = tb.hoff[e];
   int* sMp = snext + 4;
   int* syoff = sMp + (kMaxJ + 1);
@@ -179,7 +179,6 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
   for (int e = tid; e < HU; e += nth) shd[e] = tb.half_diag[e];
   const int zr0 = tb.zitem_off[warp], zr1 = tb.zitem_off[warp + 1];  // this warp's Z rounds
 
-  const bool need_d = args.dBout != nullptr;
   const int slots = phase1_slots(args.g1);
 
   // thread 0 takes the next queue position while the current atom runs; it publishes it at the
@@ -248,48 +247,45 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
     for (int ch = 0; ch < nch; ++ch) {
       z_rounds<T>(tb.zitems, zr0, zr1, cfull + ch * NU, scg, tbuf, lane);
       __syncthreads();
-      if (need_d) {
-        // Y rows by tiles of four, [tile][entry][row]: a warp per tile, lanes over (entry, row), so a
-        // lane keeps its row's sources and a warp stores 32 consecutive values
-        cx<T>* Yc = Y + (size_t)ch * NYP;
-        for (int t = warp; t < tb.NTILE; t += kNW) {
-          const int tile = stile[t], j = tile >> 8, rt = tile & 255;
-          const int H = shoff[j + 1] - shoff[j];
-          const uint4 rs = __ldg(reinterpret_cast<const uint4*>(tb.rowsrc) + srko[j] + rt * kRowTile + (lane & 3));
-          // x = z0 | z1 << 16, y = z2 | nterm << 16, z = snum0..2 | sden0 << 24, w = sden1 | sden2 << 8
-          const int nterm = rs.y >> 16;
-          const int z0 = rs.x & 0xFFFF, z1 = rs.x >> 16, z2 = rs.y & 0xFFFF;
-          const T s0 = nterm > 0 ? ssc[(rs.z & 0xFF) * 16 + (rs.z >> 24)] : T(0);
-          const T s1 = nterm > 1 ? ssc[((rs.z >> 8) & 0xFF) * 16 + (rs.w & 0xFF)] : T(0);
-          const T s2 = nterm > 2 ? ssc[((rs.z >> 16) & 0xFF) * 16 + ((rs.w >> 8) & 0xFF)] : T(0);
-          cx<T>* o = Yc + syoff[j] + rt * kRowTile * H;
-          const int centre = (j & 1) ? -1 : H - 1;  // the only entry of weight 1
-          for (int i = lane; i < kRowTile * H; i += 32) {
-            const int e = i >> 2;
-            cx<T> v = {T(0), T(0)};
-            if (nterm > 0) {
-              const cx<T> z = tbuf[z0 + e];
-              v = {s0 * z.x, s0 * z.y};
-            }
-            if (nterm > 1) {
-              const cx<T> z = tbuf[z1 + e];
-              v = {fma(s1, z.x, v.x), fma(s1, z.y, v.y)};
-            }
-            if (nterm > 2) {
-              const cx<T> z = tbuf[z2 + e];
-              v = {fma(s2, z.x, v.x), fma(s2, z.y, v.y)};
-            }
-            const T w = e == centre ? T(1) : T(2);
-            o[i] = {w * v.x, w * v.y};
+      // Y rows by tiles of four, [tile][entry][row]: a warp per tile, lanes over (entry, row), so a
+      // lane keeps its row's sources and a warp stores 32 consecutive values
+      cx<T>* Yc = Y + (size_t)ch * NYP;
+      for (int t = warp; t < tb.NTILE; t += kNW) {
+        const int tile = stile[t], j = tile >> 8, rt = tile & 255;
+        const int H = shoff[j + 1] - shoff[j];
+        const uint4 rs = __ldg(reinterpret_cast<const uint4*>(tb.rowsrc) + srko[j] + rt * kRowTile + (lane & 3));
+        // x = z0 | z1 << 16, y = z2 | nterm << 16, z = snum0..2 | sden0 << 24, w = sden1 | sden2 << 8
+        const int nterm = rs.y >> 16;
+        const int z0 = rs.x & 0xFFFF, z1 = rs.x >> 16, z2 = rs.y & 0xFFFF;
+        const T s0 = nterm > 0 ? ssc[(rs.z & 0xFF) * 16 + (rs.z >> 24)] : T(0);
+        const T s1 = nterm > 1 ? ssc[((rs.z >> 8) & 0xFF) * 16 + (rs.w & 0xFF)] : T(0);
+        const T s2 = nterm > 2 ? ssc[((rs.z >> 16) & 0xFF) * 16 + ((rs.w >> 8) & 0xFF)] : T(0);
+        cx<T>* o = Yc + syoff[j] + rt * kRowTile * H;
+        const int centre = (j & 1) ? -1 : H - 1;  // the only entry of weight 1
+        for (int i = lane; i < kRowTile * H; i += 32) {
+          const int e = i >> 2;
+          cx<T> v = {T(0), T(0)};
+          if (nterm > 0) {
+            const cx<T> z = tbuf[z0 + e];
+            v = {s0 * z.x, s0 * z.y};
           }
+          if (nterm > 1) {
+            const cx<T> z = tbuf[z1 + e];
+            v = {fma(s1, z.x, v.x), fma(s1, z.y, v.y)};
+          }
+          if (nterm > 2) {
+            const cx<T> z = tbuf[z2 + e];
+            v = {fma(s2, z.x, v.x), fma(s2, z.y, v.y)};
+          }
+          const T w = e == centre ? T(1) : T(2);
+          o[i] = {w * v.x, w * v.y};
         }
       }
-      if (args.Bout) b_sums<T>(tb.trz, K, shoff, p1c + ch * HU, tbuf, warp, lane, Bk + ch * K);
+      b_sums<T>(tb.trz, K, shoff, p1c + ch * HU, tbuf, warp, lane, Bk + ch * K);
       __syncthreads();
     }
-    if (args.Bout)
-      for (int e = tid; e < nchK; e += nth) args.Bout[(size_t)atom * nchK + e] = nn == 0 ? T(0) : Bk[e];
-    if (!need_d || nn == 0) continue;
+    for (int e = tid; e < nchK; e += nth) args.Bout[(size_t)atom * nchK + e] = nn == 0 ? T(0) : Bk[e];
+    if (nn == 0) continue;
 
     // ---------------- phase 3: dB per neighbour chunk (kNB neighbours, the last one the rest) -
     cx<T>* Us = reinterpret_cast<cx<T>*>(W);
@@ -463,7 +459,7 @@ cudaError_t launch_bso4(const DevTables& tb, const DevBatch& b, const BsoParams&
     a.gen = tb.gen32;
     a.cg = reinterpret_cast<const T*>(tb.cg32);
   }
-  if (dBout && !a.gen) return cudaErrorInvalidValue;
+  if (!Bout || !dBout || !a.gen) return cudaErrorInvalidValue;
   a.src = {b.types, b.nbr_idx, b.nbr_u, sizeof(T) == 4 ? b.nbr_u32 : nullptr, (T)p.rcut, (T)p.inv_r0,
            (T)p.rin_width, p.ntypes, p.has_rin};
   a.nbr_off = b.nbr_off;

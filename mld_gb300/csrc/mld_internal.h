@@ -434,8 +434,7 @@ struct Bso4Launch {
   int ctas_per_sm = 0;   // persistent CTAs per SM (0: as many as fit)
   int sorted_queue = 1;  // atoms longest first (1) or in index order (0)
 };
-// Descriptor kernel (bispectrum.cu): B (A x nch*K) and w_ch * dB (P x 3 x nch*K) of the batch,
-// either may be null.  Atoms are taken in `order` (null: index order) through `counter` (one int
+// Descriptor kernel (bispectrum.cu): B (A x nch*K) and w_ch * dB (P x 3 x nch*K) of the batch.  Atoms are taken in `order` (null: index order) through `counter` (one int
 // of device memory, reset by the launch).
 template <typename T>
 cudaError_t launch_bso4(const DevTables& tb, const DevBatch& b, const BsoParams& p, T* Bout, T* dBout,
