@@ -1,24 +1,27 @@
-// Sums over the Clebsch-Gordan (Z) terms with a lane per atom: the descriptors B, and y = dE/dc for
+// Sums over the Clebsch-Gordan (Z) terms with atoms on lanes: the descriptors B, and y = dE/dc for
 // the evaluation.
 //
 // Inside a CTA that works on one atom, the Z terms are lanes: their index lists, extents and
 // coefficients differ, so operands are gathered with bank conflicts, lanes idle where extents
-// differ, and every term forms its own products of c.  Here the 32 lanes of a warp hold 32 atoms
-// and run the same term: control flow is uniform, coefficients are broadcast, c (entry, atom) is
-// read without conflicts, and the products of an operand pair (jA, jB) are formed once for all its
+// differ, and every term forms its own products of c.  Here the lanes of a warp hold atoms and run
+// the same term: control flow is uniform, coefficients are broadcast, c (entry, atom) is read
+// without conflicts, and the products of an operand pair (jA, jB) are formed once for all its
 // output layers jO,
 //   Z_jO(m1,m2) = sum_a CG_jO(a; m1) sum_b CG_jO(b; m2) c^jA[a, b] c^jB[m1 - a, m2 - b]
 // (17.3k products and 163k FMAs per channel at j_max 4, against 42.6k and 255k of the term lists).
+// In FP32 a lane holds two atoms, whose values are packed for the two-wide FP32 instructions: half
+// the instructions per atom for the products, and half the loads of coefficients and records.
 // The sums that the terms feed stay in registers: no term is stored.
 //   B  a job is an operand pair: B_k = sum_m w Re(conj(c^l(m)) Z_l(m)) of its triples (l >= jA)
 //   y  a job is an output position (m1, m2): y_jO(m1,m2) = sum over the pairs of gamma Z_jO(m1,m2)
 // Four warps share a job (its records in four fixed parts of equal work, added in order), so the
 // sums do not depend on the number of atoms or on how the jobs fall on the CTAs.
 //
-// Bound: shared-memory reads in FP32 (two 8-byte operands per product), the FP64 pipe in FP64.
+// Bound: instruction issue and shared-memory reads in FP32, the FP64 pipe in FP64.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "bispectrum.cuh"
 
@@ -26,7 +29,60 @@ namespace mld {
 
 namespace {
 
-constexpr int kGroups = kNW / 4;  // four warps share a job
+// The values of a lane's atoms: two FP32 packed in a register pair, or one FP64.
+struct F2 {
+  unsigned long long v;
+};
+template <typename T>
+struct LaneVec;
+template <>
+struct LaneVec<float> {
+  using type = F2;
+  static constexpr int atoms = 2, warps = 16;
+};
+template <>
+struct LaneVec<double> {
+  using type = double;
+  static constexpr int atoms = 1, warps = 8;  // (the FP64 pipe needs fewer warps, the terms more registers)
+};
+__device__ __forceinline__ F2 pack(float a, float b) {
+  F2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d.v) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ void unpack(F2 a, float* v) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(a.v));
+}
+__device__ __forceinline__ void unpack(double a, double* v) { v[0] = a; }
+__device__ __forceinline__ F2 vmul(F2 a, F2 b) {
+  F2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ F2 vadd(F2 a, F2 b) {
+  F2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ F2 vfma(F2 a, F2 b, F2 c) {
+  F2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return d;
+}
+__device__ __forceinline__ F2 vneg(F2 a) { return vmul(a, F2{0xBF800000BF800000ull}); }  // one instruction
+__device__ __forceinline__ double vmul(double a, double b) { return a * b; }
+__device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ double vneg(double a) { return -a; }
+__device__ __forceinline__ double vadd(double a, double b) { return a + b; }
+__device__ __forceinline__ F2 vdup(float a, F2) { return pack(a, a); }
+__device__ __forceinline__ double vdup(double a, double) { return a; }
+
+// complex value of a lane's atoms (16 bytes)
+template <typename V>
+struct alignas(16) vcx {
+  V x, y;
+};
+
 
 template <typename T>
 struct LaneArgs {
@@ -43,58 +99,58 @@ struct LaneArgs {
   cx<T>* y;             // A x nch x HU
 };
 
-// lanes that hold atoms: 32, or 16 where the c of 32 atoms does not fit in shared memory
+// lanes that hold atoms: 32, or 16 where their c does not fit in shared memory; a padded row per entry
+// (16-byte values) so that the transposing stores spread over the banks
 struct LanePlan {
-  int width, stride;
+  int stride;
   size_t c, cg, gamma, part, total;
 };
 
 __host__ __device__ inline size_t upl(size_t x) { return (x + 15) & ~(size_t)15; }
 
-__host__ __device__ inline LanePlan lane_plan(const DevTables& tb, int eb, int width) {
+__host__ __device__ inline LanePlan lane_plan(const DevTables& tb, int eb, int lanes) {
   LanePlan s;
-  s.width = width;
-  s.stride = width + 1;
+  s.stride = lanes + 1;
   size_t o = 0;
-  s.c = o;     o = upl(o + (size_t)2 * eb * tb.NU * s.stride);
-  s.cg = o;    o = upl(o + (eb == 4 ? (size_t)eb * tb.NCGV : 0));  // FP64 reads them through the cache
-  s.gamma = o; o = upl(o + (size_t)eb * tb.NBLKP);
-  s.part = o;  o = upl(o + (size_t)kGroups * 4 * (tb.J / 2 + 1) * 32 * 2 * eb);
+  s.c = o;     o = upl(o + (size_t)16 * tb.NU * s.stride);
+  s.cg = o;    o = upl(o + (eb == 4 ? (size_t)8 * tb.NCGV : 0));  // FP32: doubled; FP64 reads through the cache
+  s.gamma = o; o = upl(o + (size_t)8 * tb.NBLKP);
+  s.part = o;  o = upl(o + (size_t)16 * (eb == 4 ? LaneVec<float>::warps : LaneVec<double>::warps) * (tb.J / 2 + 1) * 32);
   s.total = o;
   return s;
 }
 
 // C consecutive b of a record, all its a: zs[o] += sum_a c1[a][o] sum_{b<C} c2[b][o] c c, o < NJ
-template <int NJ, int C, typename T>
-__device__ __forceinline__ void lane_chunk(const cx<T>* __restrict__ pa, const cx<T>* __restrict__ pb, int ST, int da,
-                                           int db, int na, const T* __restrict__ c1p, int st1,
-                                           const T* __restrict__ c2p, int st2, cx<T>* zs) {
-  T c2[C][NJ];
+template <int NJ, int C, typename V>
+__device__ __forceinline__ void lane_chunk(const vcx<V>* __restrict__ pa, const vcx<V>* __restrict__ pb, int ST, int da,
+                                           int db, int na, const V* __restrict__ c1p, int st1,
+                                           const V* __restrict__ c2p, int st2, vcx<V>* zs) {
+  V c2[C][NJ];
 #pragma unroll
   for (int b = 0; b < C; ++b)
 #pragma unroll
     for (int o = 0; o < NJ; ++o) c2[b][o] = c2p[b * st2 + o];
   for (int a = 0; a < na; ++a) {
-    cx<T> part[NJ];
+    vcx<V> part[NJ];
 #pragma unroll
     for (int b = 0; b < C; ++b) {
-      const cx<T> u = pa[b * ST], v = pb[-b * ST];
-      const cx<T> pr = {fma(u.x, v.x, -(u.y * v.y)), fma(u.x, v.y, u.y * v.x)};
+      const vcx<V> u = pa[b * ST], v = pb[-b * ST];
+      const vcx<V> pr = {vfma(vneg(u.y), v.y, vmul(u.x, v.x)), vfma(u.x, v.y, vmul(u.y, v.x))};
 #pragma unroll
       for (int o = 0; o < NJ; ++o) {
         if (b == 0) {
-          part[o] = {c2[b][o] * pr.x, c2[b][o] * pr.y};
+          part[o] = {vmul(c2[b][o], pr.x), vmul(c2[b][o], pr.y)};
         } else {
-          part[o].x = fma(c2[b][o], pr.x, part[o].x);
-          part[o].y = fma(c2[b][o], pr.y, part[o].y);
+          part[o].x = vfma(c2[b][o], pr.x, part[o].x);
+          part[o].y = vfma(c2[b][o], pr.y, part[o].y);
         }
       }
     }
 #pragma unroll
     for (int o = 0; o < NJ; ++o) {
-      const T c1 = c1p[o];
-      zs[o].x = fma(c1, part[o].x, zs[o].x);
-      zs[o].y = fma(c1, part[o].y, zs[o].y);
+      const V c1 = c1p[o];
+      zs[o].x = vfma(c1, part[o].x, zs[o].x);
+      zs[o].y = vfma(c1, part[o].y, zs[o].y);
     }
     c1p += st1;
     pa += da;
@@ -103,28 +159,31 @@ __device__ __forceinline__ void lane_chunk(const cx<T>* __restrict__ pa, const c
 }
 
 // Z of the NJ output layers of a record
-template <int NJ, typename T>
-__device__ __forceinline__ void lane_terms(uint4 z0, const cx<T>* __restrict__ cl, int ST, const T* __restrict__ cg,
-                                           cx<T>* zs) {
+template <int NJ, typename V>
+__device__ __forceinline__ void lane_terms(uint4 z0, const vcx<V>* __restrict__ cl, int ST, const V* __restrict__ cg,
+                                           vcx<V>* zs) {
+  constexpr int C = NJ <= 3 || std::is_same<V, double>::value ? 4 : 2;  // C * NJ coefficients in registers
   // x = i1 | i2 << 16, y = cg1 | cg2 << 16, z = na | nb << 8 | s1 << 16 | s2 << 24, w = st1 | st2 << 8 | ..
-  const cx<T>* pa = cl + (size_t)(z0.x & 0xFFFF) * ST;
-  const cx<T>* pb = cl + (size_t)(z0.x >> 16) * ST;
+  const vcx<V>* pa = cl + (z0.x & 0xFFFF) * ST;
+  const vcx<V>* pb = cl + (z0.x >> 16) * ST;
   const int na = z0.z & 0xFF, da = ((z0.z >> 16) & 0xFF) * ST, db = (z0.z >> 24) * ST;
   const int st1 = z0.w & 0xFF, st2 = (z0.w >> 8) & 0xFF;
-  const T* c1p = cg + (z0.y & 0xFFFF);
-  const T* c2p = cg + (z0.y >> 16);
+  const V* c1p = cg + (z0.y & 0xFFFF);
+  const V* c2p = cg + (z0.y >> 16);
   int nb = (z0.z >> 8) & 0xFF;
 #pragma unroll
-  for (int o = 0; o < NJ; ++o) zs[o] = {T(0), T(0)};
-  for (; nb >= 4; nb -= 4) {
-    lane_chunk<NJ, 4>(pa, pb, ST, da, db, na, c1p, st1, c2p, st2, zs);
-    pa += 4 * ST;
-    pb -= 4 * ST;
-    c2p += 4 * st2;
+  for (int o = 0; o < NJ; ++o) zs[o] = {V{}, V{}};
+  for (; nb >= C; nb -= C) {
+    lane_chunk<NJ, C, V>(pa, pb, ST, da, db, na, c1p, st1, c2p, st2, zs);
+    pa += C * ST;
+    pb -= C * ST;
+    c2p += C * st2;
   }
-  if (nb == 1) lane_chunk<NJ, 1>(pa, pb, ST, da, db, na, c1p, st1, c2p, st2, zs);
-  else if (nb == 2) lane_chunk<NJ, 2>(pa, pb, ST, da, db, na, c1p, st1, c2p, st2, zs);
-  else if (nb == 3) lane_chunk<NJ, 3>(pa, pb, ST, da, db, na, c1p, st1, c2p, st2, zs);
+  if (nb == 1) lane_chunk<NJ, 1, V>(pa, pb, ST, da, db, na, c1p, st1, c2p, st2, zs);
+  if constexpr (C > 2) {
+    if (nb == 2) lane_chunk<NJ, 2, V>(pa, pb, ST, da, db, na, c1p, st1, c2p, st2, zs);
+    else if (nb == 3) lane_chunk<NJ, 3, V>(pa, pb, ST, da, db, na, c1p, st1, c2p, st2, zs);
+  }
 }
 
 __device__ __forceinline__ int out_of(uint4 z1, int o) {
@@ -133,73 +192,93 @@ __device__ __forceinline__ int out_of(uint4 z1, int o) {
 }
 
 // A record into the job's sums.  y: acc[off + o] += gamma[out_o] Z_o; B: acc[o].x += w Re(conj(c[out_o]) Z_o)
-template <int NJ, bool kY, typename T>
-__device__ __forceinline__ void lane_record(uint4 z0, uint4 z1, const cx<T>* __restrict__ cl, int ST,
-                                            const T* __restrict__ cg, const T* __restrict__ gam, cx<T>* acc) {
-  cx<T> zs[NJ];
-  lane_terms<NJ, T>(z0, cl, ST, cg, zs);
+template <int NJ, bool kY, typename V>
+__device__ __forceinline__ void lane_record(uint4 z0, uint4 z1, const vcx<V>* __restrict__ cl, int ST,
+                                            const V* __restrict__ cg, const V* __restrict__ gam, vcx<V>* acc) {
+  vcx<V> zs[NJ];
+  lane_terms<NJ, V>(z0, cl, ST, cg, zs);
   if constexpr (kY) {
     const int off = z0.w >> 24;
+    if (off == 0) {  // pairs that reach the highest layers: most of the work
 #pragma unroll
-    for (int o = 0; o < NJ; ++o) {
-      const T g = gam[out_of(z1, o)];
+      for (int o = 0; o < NJ; ++o) {
+        const V g = gam[out_of(z1, o)];
+        acc[o].x = vfma(g, zs[o].x, acc[o].x);
+        acc[o].y = vfma(g, zs[o].y, acc[o].y);
+      }
+    } else {
 #pragma unroll
-      for (int k = 0; k + o < kMaxZOut; ++k)
-        if (k == off) {
-          acc[k + o].x = fma(g, zs[o].x, acc[k + o].x);
-          acc[k + o].y = fma(g, zs[o].y, acc[k + o].y);
-        }
+      for (int o = 0; o < NJ; ++o) {
+        const V g = gam[out_of(z1, o)];
+#pragma unroll
+        for (int k = 1; k + o < kMaxZOut; ++k)
+          if (k == off) {
+            acc[k + o].x = vfma(g, zs[o].x, acc[k + o].x);
+            acc[k + o].y = vfma(g, zs[o].y, acc[k + o].y);
+          }
+      }
     }
   } else {
-    const T w = (T)(z1.w & 0xFFFF);
+    const int wi = z1.w & 0xFFFF;
 #pragma unroll
     for (int o = 0; o < NJ; ++o) {
-      const cx<T> c = cl[(size_t)out_of(z1, o) * ST];
-      acc[o].x = fma(w, fma(c.x, zs[o].x, c.y * zs[o].y), acc[o].x);
+      const vcx<V> c = cl[out_of(z1, o) * ST];
+      const V t = vfma(c.x, zs[o].x, vmul(c.y, zs[o].y));
+      acc[o].x = vadd(acc[o].x, wi == 2 ? vadd(t, t) : t);
     }
   }
 }
 
 template <typename T, bool kY>
-__global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_lanes(LaneArgs<T> args, int width) {
+__global__ void __launch_bounds__(LaneVec<T>::warps * 32, 1) k_lanes(LaneArgs<T> args, int lanes) {
+  using V = typename LaneVec<T>::type;
+  constexpr int kPer = LaneVec<T>::atoms, kLaneWarps = LaneVec<T>::warps;
+  constexpr int kGroups = kLaneWarps / 4;  // four warps share a job
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DevTables& tb = args.tb;
-  const LanePlan sp = lane_plan(tb, (int)sizeof(T), width);
+  const LanePlan sp = lane_plan(tb, (int)sizeof(T), lanes);
   const int ST = sp.stride, HU = tb.HU, K = tb.K;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ch = blockIdx.z, a0 = blockIdx.x * width;
-  const int na = min(width, args.A - a0);
-  cx<T>* sc = reinterpret_cast<cx<T>*>(smem_raw + sp.c);
-  T* sg = reinterpret_cast<T*>(smem_raw + sp.gamma);
-  cx<T>* part = reinterpret_cast<cx<T>*>(smem_raw + sp.part);
-  const T* cg = args.cg;
+  constexpr int nth = kLaneWarps * 32;
+  const int ch = blockIdx.z, a0 = blockIdx.x * lanes * kPer;
+  const int na = min(lanes * kPer, args.A - a0);
+  vcx<V>* sc = reinterpret_cast<vcx<V>*>(smem_raw + sp.c);
+  V* sg = reinterpret_cast<V*>(smem_raw + sp.gamma);
+  vcx<V>* part = reinterpret_cast<vcx<V>*>(smem_raw + sp.part);
   // c of the atoms, expanded to full layers; a warp per atom
-  for (int a = warp; a < width; a += kNW) {
+  for (int a = warp; a < lanes * kPer; a += kLaneWarps) {
     const cx<T>* src = args.c + ((size_t)(a0 + min(a, na - 1)) * args.nch + ch) * HU;
-    for (int f = lane; f < tb.NU; f += 32) sc[(size_t)f * ST + a] = fetch(src, tb.expand[f]);
+    T* dst = reinterpret_cast<T*>(sc + a / kPer) + a % kPer;  // re, im of atom a: kPer values apart
+    for (int f = lane; f < tb.NU; f += 32) {
+      const cx<T> v = fetch(src, tb.expand[f]);
+      T* d = dst + (size_t)f * ST * 2 * kPer;
+      d[0] = v.x;
+      d[kPer] = v.y;
+    }
   }
+  const V* cg;
   if constexpr (sizeof(T) == 4) {
-    T* scg = reinterpret_cast<T*>(smem_raw + sp.cg);
-    for (int e = tid; e < tb.NCGV; e += kNW * 32) scg[e] = args.cg[e];
+    V* scg = reinterpret_cast<V*>(smem_raw + sp.cg);
+    for (int e = tid; e < tb.NCGV; e += nth) scg[e] = vdup(args.cg[e], V{});
     cg = scg;
+  } else {
+    cg = args.cg;
   }
   if constexpr (kY) {
-    for (int b = tid; b < tb.NBLKP; b += kNW * 32) sg[b] = args.gamma[ch * tb.NBLKP + b];
+    for (int b = tid; b < tb.NBLKP; b += nth) sg[b] = vdup(args.gamma[ch * tb.NBLKP + b], V{});
   }
   __syncthreads();
-  const int al = lane < width ? lane : lane - width;  // (16 atoms: both halves of the warp hold them)
-  const int atom = a0 + al;
-  const bool mine = lane < width && al < na;
-  const cx<T>* cl = sc + al;
+  const int al = lane < lanes ? lane : lane - lanes;  // (16 lanes: both halves of the warp hold the same atoms)
+  const vcx<V>* cl = sc + al;
   const int group = warp >> 2, q = warp & 3, no = tb.J / 2 + 1;
-  const bool alone = !kY && (mine ? args.nbr_off[atom + 1] == args.nbr_off[atom] : false);
-  cx<T>* mypart = part + (size_t)group * 4 * no * 32;
+  vcx<V>* mypart = part + (size_t)group * 4 * no * 32;
   for (int job = blockIdx.y * kGroups + group; job < args.njobs; job += gridDim.y * kGroups) {
     const LaneJob& jb = args.jobs[job];
-    cx<T> acc[kMaxZOut];
+    vcx<V> acc[kMaxZOut];
 #pragma unroll
-    for (int o = 0; o < kMaxZOut; ++o) acc[o] = {T(0), T(0)};
+    for (int o = 0; o < kMaxZOut; ++o) acc[o] = {V{}, V{}};
     const int r0 = jb.rec[q], r1 = jb.rec[q + 1];
+    constexpr int kAhead = 6;
     const uint4* rp = reinterpret_cast<const uint4*>(args.recs);
     uint4 n0 = make_uint4(0, 0, 0, 0), n1 = n0;
     if (r0 < r1) {
@@ -208,17 +287,19 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_lanes(Lane
     }
     for (int r = r0; r < r1; ++r) {
       const uint4 z0 = n0, z1 = n1;
+      // every record is read once per CTA: fetch ahead of the register prefetch
+      if (r + kAhead < r1) asm volatile("prefetch.global.L1 [%0];" ::"l"(rp + 2 * (size_t)(r + kAhead)));
       if (r + 1 < r1) {
         n0 = __ldg(rp + 2 * (size_t)(r + 1));
         n1 = __ldg(rp + 2 * (size_t)(r + 1) + 1);
       }
       switch ((z0.w >> 16) & 0xFF) {
-        case 1: lane_record<1, kY, T>(z0, z1, cl, ST, cg, sg, acc); break;
-        case 2: lane_record<2, kY, T>(z0, z1, cl, ST, cg, sg, acc); break;
-        case 3: lane_record<3, kY, T>(z0, z1, cl, ST, cg, sg, acc); break;
-        case 4: lane_record<4, kY, T>(z0, z1, cl, ST, cg, sg, acc); break;
-        case 5: lane_record<5, kY, T>(z0, z1, cl, ST, cg, sg, acc); break;
-        default: lane_record<6, kY, T>(z0, z1, cl, ST, cg, sg, acc); break;
+        case 1: lane_record<1, kY, V>(z0, z1, cl, ST, cg, sg, acc); break;
+        case 2: lane_record<2, kY, V>(z0, z1, cl, ST, cg, sg, acc); break;
+        case 3: lane_record<3, kY, V>(z0, z1, cl, ST, cg, sg, acc); break;
+        case 4: lane_record<4, kY, V>(z0, z1, cl, ST, cg, sg, acc); break;
+        case 5: lane_record<5, kY, V>(z0, z1, cl, ST, cg, sg, acc); break;
+        default: lane_record<6, kY, V>(z0, z1, cl, ST, cg, sg, acc); break;
       }
     }
 #pragma unroll
@@ -226,15 +307,23 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_lanes(Lane
       if (o < no) mypart[(q * no + o) * 32 + lane] = acc[o];
     asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
     for (int o = q; o < jb.nout; o += 4) {
-      cx<T> v = mypart[o * 32 + lane];
+      vcx<V> v = mypart[o * 32 + lane];
 #pragma unroll
       for (int p = 1; p < 4; ++p) {
-        const cx<T> w = mypart[(p * no + o) * 32 + lane];
-        v = {v.x + w.x, v.y + w.y};
+        const vcx<V> w = mypart[(p * no + o) * 32 + lane];
+        v = {vadd(v.x, w.x), vadd(v.y, w.y)};
       }
-      if (mine) {
-        if constexpr (kY) args.y[((size_t)atom * args.nch + ch) * HU + jb.out[o]] = v;
-        else args.B[((size_t)atom * args.nch + ch) * K + jb.out[o]] = alone ? T(0) : v.x;
+      T re[kPer], im[kPer];
+      unpack(v.x, re);
+      unpack(v.y, im);
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const int a = al * kPer + k;
+        if (lane < lanes && a < na) {
+          const size_t row = (size_t)(a0 + a) * args.nch + ch;
+          if constexpr (kY) args.y[row * HU + jb.out[o]] = {re[k], im[k]};
+          else args.B[row * K + jb.out[o]] = args.nbr_off[a0 + a + 1] == args.nbr_off[a0 + a] ? T(0) : re[k];
+        }
       }
     }
     asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
@@ -347,23 +436,32 @@ cudaError_t sm_count(int* nsm) {
 template <typename T, bool kY>
 cudaError_t launch_lanes(LaneArgs<T>& a, cudaStream_t st) {
   if (a.A <= 0 || a.njobs <= 0) return cudaSuccess;
-  int width = 32;
-  size_t smem = lane_plan(a.tb, (int)sizeof(T), width).total;
-  if (smem > (size_t)optin()) {
-    width = 16;
-    smem = lane_plan(a.tb, (int)sizeof(T), width).total;
-  }
+  int lanes = 32;
+  if (lane_plan(a.tb, (int)sizeof(T), lanes).total > (size_t)optin()) lanes = 16;
+  const size_t smem = lane_plan(a.tb, (int)sizeof(T), lanes).total;
   if (smem > (size_t)optin()) return cudaErrorInvalidConfiguration;
   cudaError_t e = cudaFuncSetAttribute(k_lanes<T, kY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int nsm = 0;
   if ((e = sm_count(&nsm)) != cudaSuccess) return e;
-  // the jobs of a tile of atoms are spread over CTAs until about four rounds of CTAs fill the GPU; a
-  // CTA keeps at least two jobs per group, or its load of c would outweigh them
-  const int tiles = (a.A + width - 1) / width;
-  const int most = std::max(1, a.njobs / (2 * kGroups));
-  const int slices = std::min(most, std::max(1, 8 * nsm / (tiles * a.nch)));
-  k_lanes<T, kY><<<dim3(tiles, slices, a.nch), kNW * 32, smem, st>>>(a, width);
+  // The jobs of a tile of atoms may be spread over several CTAs (slices), each of which loads the
+  // tile's c: worth it where the tiles do not fill the GPU or leave its last round of CTAs nearly
+  // empty.  Loading c costs about 1/20 of a tile's jobs in FP32, a tenth of that share in FP64.
+  constexpr int kGroups = LaneVec<T>::warps / 4;
+  const int per = lanes * LaneVec<T>::atoms, tiles = (a.A + per - 1) / per;
+  const int most = std::max(1, (a.njobs + kGroups - 1) / kGroups);
+  int slices = 1;
+  double best = 0.0;
+  for (int s = 1; s <= most; ++s) {
+    const long long rounds = ((long long)tiles * a.nch * s + nsm - 1) / nsm;
+    const double jobs = (double)((a.njobs + kGroups * s - 1) / (kGroups * s)) * kGroups / a.njobs;
+    const double t = (double)rounds * (jobs + (sizeof(T) == 4 ? 0.05 : 0.005));
+    if (s == 1 || t < best) {
+      best = t;
+      slices = s;
+    }
+  }
+  k_lanes<T, kY><<<dim3(tiles, slices, a.nch), LaneVec<T>::warps * 32, smem, st>>>(a, lanes);
   return cudaGetLastError();
 }
 

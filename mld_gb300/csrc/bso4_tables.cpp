@@ -267,6 +267,10 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
         part[q].push_back(p.r);
       }
       for (int q = 0; q < 4; ++q) {
+        // records of equal shape one after the other: they run the same code
+        std::stable_sort(part[q].begin(), part[q].end(), [](const LaneRec& x, const LaneRec& y) {
+          return x.nj != y.nj ? x.nj > y.nj : (x.nb != y.nb ? x.nb > y.nb : x.na > y.na);
+        });
         job.rec[q] = (int)out->size();
         out->insert(out->end(), part[q].begin(), part[q].end());
       }
