@@ -1661,13 +1661,19 @@ int eval_weights_upload(mld_gpu_handle* h, const double* w_full) {
       for (int j = 0; j < KK; ++j) hw[KK + (size_t)i * KK + j] = W[(size_t)i * KK + j] + W[(size_t)j * KK + i];
   }
   const size_t eb = h->mixed ? sizeof(float) : sizeof(double);
-  CK(ensure(h, mld_gpu_handle::B_EW, sizeof(double) * hw.size() + eb * h->nch * h->dt.NBLKP + 256));
+  const size_t next = h->quad ? (h->mixed ? sizeof(float2) * n2 : 0) : eb * h->nch * h->dt.NBLKP;
+  CK(ensure(h, mld_gpu_handle::B_EW, sizeof(double) * hw.size() + next + 256));
   double* dw = bp_<double>(h, mld_gpu_handle::B_EW);
   CK(cudaMemcpyAsync(dw, hw.data(), sizeof(double) * hw.size(), cudaMemcpyHostToDevice, h->st));
-  if (!h->quad) {
-    void* g = dw + hw.size();
-    if (h->mixed) CK(launch_eval_gamma<float>(h->dt, nullptr, 1, h->nch, dw, nullptr, 0.0, (float*)g, nullptr, h->st));
-    else CK(launch_eval_gamma<double>(h->dt, nullptr, 1, h->nch, dw, nullptr, 0.0, (double*)g, nullptr, h->st));
+  void* ext = dw + hw.size();
+  if (h->quad) {
+    if (h->mixed) CK(launch_split_pairs(dw + KK, static_cast<float2*>(ext), n2, h->st));
+  } else if (h->mixed) {
+    CK(launch_eval_gamma<float>(h->dt, nullptr, 1, h->nch, dw, nullptr, nullptr, 0.0, static_cast<float*>(ext), nullptr,
+                                h->st));
+  } else {
+    CK(launch_eval_gamma<double>(h->dt, nullptr, 1, h->nch, dw, nullptr, nullptr, 0.0, static_cast<double*>(ext), nullptr,
+                                 h->st));
   }
   CK(cudaStreamSynchronize(h->st));
   h->ew0 = w_full[0];
@@ -1683,7 +1689,8 @@ static int eval_run(mld_gpu_handle* h, double* out) {
   double* S = F + 3 * (size_t)h->A;
   const double* wlin = bp_<double>(h, mld_gpu_handle::B_EW);
   const double* wsym = wlin + KK;
-  const T* gammaT = reinterpret_cast<const T*>(wlin + KK + (h->quad ? (size_t)KK * KK : 0));
+  // behind the FP64 weights: the linear model's block weights, the quadratic model's Wsym as FP32 pairs
+  const void* wext = wlin + KK + (h->quad ? (size_t)KK * KK : 0);
   CK(ensure(h, mld_gpu_handle::B_EPAIR, sizeof(T) * 3 * (size_t)std::max<long long>(1, h->b.P)));
   CK(ensure(h, mld_gpu_handle::B_EATOM, sizeof(double) * 7 * (size_t)std::max(1, h->A)));
   CK(ensure(h, mld_gpu_handle::B_REV, sizeof(int) * (size_t)std::max<long long>(1, h->b.P)));
@@ -1703,7 +1710,9 @@ static int eval_run(mld_gpu_handle* h, double* out) {
     T* gamma = bp_<T>(h, mld_gpu_handle::B_EBETA);
     int rc = run_descriptors<T>(h, false, B);
     if (rc) return rc;
-    CK(launch_eval_gamma<T>(h->dt, B, h->A, h->nch, wlin, wsym, h->ew0, gamma, ev.Eatom, h->st));
+    CK(launch_eval_gamma<T>(h->dt, B, h->A, h->nch, wlin, wsym, static_cast<const float2*>(wext), h->ew0, gamma, ev.Eatom,
+                            h->st));
+    ev.c = bp_<void>(h, mld_gpu_handle::B_CHALF);  // left there by the pass for B
     ev.gamma = gamma;
     nl(h, 1);
   } else {
@@ -1714,7 +1723,7 @@ static int eval_run(mld_gpu_handle* h, double* out) {
     ev.c = bp_<void>(h, mld_gpu_handle::B_CHALF);
     ev.y = bp_<void>(h, mld_gpu_handle::B_EY);
     CK(launch_c_half<T>(h->dt, h->b, h->bp, 0, h->A, order, counter, bp_<void>(h, mld_gpu_handle::B_CHALF), h->st));
-    CK(launch_lane_y<T>(h->dt, h->b, h->bp, 0, h->A, ev.c, gammaT, bp_<void>(h, mld_gpu_handle::B_EY), h->st));
+    CK(launch_lane_y<T>(h->dt, h->b, h->bp, 0, h->A, ev.c, static_cast<const T*>(wext), bp_<void>(h, mld_gpu_handle::B_EY), h->st));
     nl(h, 2);
   }
   CK(launch_bso4_eval<T>(h->dt, h->b, h->bp, ev, order, counter, h->st));

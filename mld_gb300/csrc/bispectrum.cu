@@ -59,6 +59,7 @@ struct KernelArgs {
 };
 
 constexpr int kNB = 16;  // neighbours per phase-3 chunk
+constexpr int kScale = kMaxJ + 2;  // row scales n / d, n and d <= kMaxJ + 1
 
 // Shared-memory carve-up, in order (every region 16-byte aligned):
 //   gen[HU]  hoff[kMaxJ+2]  rowk[NROWS]  tiles[NTILE]  rank_slot[2K]  cfull[nch*NU]
@@ -68,8 +69,8 @@ constexpr int kNB = 16;  // neighbours per phase-3 chunk
 //   W region (phase 2: CG coefficients; phase 3: U of the chunk, then the chunk's contractions by
 //   rank: rank 0 [cols][K], rank 1 [cols][nrank1], rank 2 [cols][nrank2])
 //   Bk[nch*K]  nwt[nch*NB]  next atom
-//   expand[NU]  half_diag[HU] (tables staged once per CTA)  sc[256] (row scales)
-//   crec[NB*kGeo] (records of a chunk's neighbours beyond geo_cap)
+//   expand[NU]  half_diag[HU] (tables staged once per CTA)  sc[kScale^2] (row scales)
+//   crec[NB*kGeoDeriv] (records of a chunk's neighbours beyond geo_cap)
 //   geo[geo_cap*kGeo] (geometry records of the atom's first geo_cap neighbours)
 struct SmemPlan {
   size_t gen, hoff, rowk, tiles, rslot, cfull, Y, V, p1z, p1w, p1c, W, Bk, nwt, next, sc, exp, hd, crec, geo, total;
@@ -113,10 +114,10 @@ __host__ __device__ inline SmemPlan smem_plan(const DevTables& tb, int nch, int 
   s.Bk = o;    o = al16(o + (size_t)eb * nch * tb.K);
   s.nwt = o;   o = al16(o + (size_t)eb * nch * kNB);
   s.next = o;  o = al16(o + sizeof(int) * (4 + 3 * kMaxJ + 4 + kRounds));
-  s.sc = o;    o = al16(o + (size_t)eb * 256);
+  s.sc = o;    o = al16(o + (size_t)eb * kScale * kScale);
   s.exp = o;   o = al16(o + sizeof(int16_t) * tb.NU);
   s.hd = o;    o = al16(o + tb.HU);
-  s.crec = o;  o = al16(o + (size_t)eb * kGeo * kNB);
+  s.crec = o;  o = al16(o + (size_t)eb * kGeoDeriv * kNB);
   s.geo = o;   o = al16(o + (size_t)eb * kGeo * geo_cap);
   s.total = o;
   return s;
@@ -157,7 +158,7 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
   int* snext = reinterpret_cast<int*>(smem_raw + sp.next);
   T* crec = reinterpret_cast<T*>(smem_raw + sp.crec);
   T* sgeo = reinterpret_cast<T*>(smem_raw + sp.geo);
-  T* ssc = reinterpret_cast<T*>(smem_raw + sp.sc);  // ssc[16 n + d] = n / d, the row scales
+  T* ssc = reinterpret_cast<T*>(smem_raw + sp.sc);  // ssc[kScale n + d] = n / d, the row scales
 
   // tables, once per CTA
   for (int e = tid; e < HU; e += nth) sgen[e] = args.gen[e];
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
   for (int e = tid; e < tb.NROWS; e += nth) srowk[e] = tb.rowk[e];
   for (int e = tid; e < tb.NTILE; e += nth) stile[e] = tb.tiles[e];
   for (int e = tid; e < (kRounds - 1) * K; e += nth) srslot[e] = tb.rank_slot[e];
-  for (int e = tid; e < 256; e += nth) ssc[e] = (e & 15) ? (T)(e >> 4) / (T)(e & 15) : T(0);
+  for (int e = tid; e < kScale * kScale; e += nth) ssc[e] = e % kScale ? (T)(e / kScale) / (T)(e % kScale) : T(0);
   int16_t* sexp = reinterpret_cast<int16_t*>(smem_raw + sp.exp);
   int8_t* shd = reinterpret_cast<int8_t*>(smem_raw + sp.hd);
   for (int e = tid; e < NU; e += nth) sexp[e] = tb.expand[e];
@@ -257,9 +258,9 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
         // x = z0 | z1 << 16, y = z2 | nterm << 16, z = snum0..2 | sden0 << 24, w = sden1 | sden2 << 8
         const int nterm = rs.y >> 16;
         const int z0 = rs.x & 0xFFFF, z1 = rs.x >> 16, z2 = rs.y & 0xFFFF;
-        const T s0 = nterm > 0 ? ssc[(rs.z & 0xFF) * 16 + (rs.z >> 24)] : T(0);
-        const T s1 = nterm > 1 ? ssc[((rs.z >> 8) & 0xFF) * 16 + (rs.w & 0xFF)] : T(0);
-        const T s2 = nterm > 2 ? ssc[((rs.z >> 16) & 0xFF) * 16 + ((rs.w >> 8) & 0xFF)] : T(0);
+        const T s0 = nterm > 0 ? ssc[(rs.z & 0xFF) * kScale + (rs.z >> 24)] : T(0);
+        const T s1 = nterm > 1 ? ssc[((rs.z >> 8) & 0xFF) * kScale + (rs.w & 0xFF)] : T(0);
+        const T s2 = nterm > 2 ? ssc[((rs.z >> 16) & 0xFF) * kScale + ((rs.w >> 8) & 0xFF)] : T(0);
         cx<T>* o = Yc + syoff[j] + rt * kRowTile * H;
         const int centre = (j & 1) ? -1 : H - 1;  // the only entry of weight 1
         for (int i = lane; i < kRowTile * H; i += 32) {
@@ -294,13 +295,16 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
       const int nb_here = min(kNB, nn - base);
       // record of the chunk's neighbour n: phase 1's, else computed again
       auto rec = [&](int n) {
-        return base + n < args.geo_cap ? sgeo + (size_t)(base + n) * kGeo : crec + (size_t)n * kGeo;
+        return base + n < args.geo_cap ? sgeo + (size_t)(base + n) * kGeo : crec + (size_t)n * kGeoDeriv;
       };
       if (tid < nb_here) {
         T* r = rec(tid);
         if (base + tid >= args.geo_cap) {
+          T g[kGeo];
           int nb, tn;
-          pair_geometry<T>(args.src, args.rin, (size_t)(p0 + base + tid), ti, r, &nb, &tn);
+          pair_geometry<T>(args.src, args.rin, (size_t)(p0 + base + tid), ti, g, &nb, &tn);
+#pragma unroll
+          for (int k = 0; k < kGeoIdx; ++k) r[k] = g[k];
           put_pair<T>(r, nb, tn);
         }
         for (int ch = 0; ch < nch; ++ch) nwt[ch * kNB + tid] = args.chw[ch * args.src.ntypes + pair_type<T>(r)];

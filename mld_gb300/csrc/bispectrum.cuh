@@ -47,13 +47,14 @@ constexpr int kNW = 8;  // warps per CTA (== kZWarps)
 static_assert(kNW == kZWarps, "phase-2 schedule is built for the CTA's warps");
 
 // ---- neighbour geometry --------------------------------------------------------------------
-// Record of a neighbour (kGeo values, a multiple of 4 so that records stay 16-byte aligned):
+// Record of a neighbour (kGeo values, a multiple of 4 so that records stay 16-byte aligned); the first
+// kGeoDeriv are what the derivatives need:
 //   kGeoXi   xi[3][3]: d/du_a of U is U sum_b xi[a][b] rho(T_b) (the generators below)
-//   kGeoFc   f_c, kGeoKap kappa[3] with f_c' e_a = sum_b xi[a][b] kappa[b], kGeoDfr f_c' e_a
-//   kGeoZx   zp and xp, the matrix of U^1
-//   kGeoU    displacement u and 1/r; kGeoIdx the neighbour's index and type (two ints)
-constexpr int kGeo = 28;
-constexpr int kGeoXi = 0, kGeoFc = 9, kGeoKap = 10, kGeoDfr = 13, kGeoZx = 16, kGeoU = 20, kGeoIdx = 24;
+//   kGeoFc   f_c, kGeoKap kappa[3] with f_c' e_a = sum_b xi[a][b] kappa[b]
+//   kGeoZx   zp and xp, the matrix of U^1; kGeoIdx the neighbour's index and type (two ints)
+//   kGeoDfr  f_c' e_a; kGeoU displacement u and 1/r
+constexpr int kGeo = 28, kGeoDeriv = 20;
+constexpr int kGeoXi = 0, kGeoFc = 9, kGeoKap = 10, kGeoZx = 13, kGeoIdx = 17, kGeoDfr = 20, kGeoU = 23;
 
 // angular_functions.f90:66-107 (the geometric set-up of spherical_4d) and the cutoff of
 // compute_bispectrum_so4.F90:337-377 (type-2 cosine outer cut times (1 - inner type-3 cut)).
@@ -405,11 +406,11 @@ __device__ __forceinline__ void pair_geometry(const PairSource<T>& s, const T* r
 template <typename T>
 __device__ __forceinline__ void put_pair(T* g, int nb, int tn) {
   reinterpret_cast<int*>(g + kGeoIdx)[0] = nb;
-  reinterpret_cast<int*>(g + kGeoIdx)[1] = tn;
+  reinterpret_cast<int*>(g + kGeoIdx + 1)[0] = tn;
 }
 template <typename T>
 __device__ __forceinline__ int pair_type(const T* g) {
-  return reinterpret_cast<const int*>(g + kGeoIdx)[1];
+  return reinterpret_cast<const int*>(g + kGeoIdx + 1)[0];
 }
 
 // c on half layers from the U store of neighbours 0..count-1 of a pass: chalf += sum over them in

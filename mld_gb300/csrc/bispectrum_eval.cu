@@ -16,10 +16,12 @@
 // the short phases and shared-memory reads.
 //
 // Quadratic model: its stress takes the neighbour's beta (the neighbour's B in the quadratic stress
-// rows, mld_stress.F90:580-603): y is formed per neighbour from the Z terms of all channels (one
-// real by complex product per term, a third of a dB contraction), and its dot products are taken
-// with the generators applied to U.  The Z terms of the atom are therefore formed in the CTA, from c
-// summed over the same U store.  Bound: FP32 arithmetic and shared memory of the Z terms.
+// rows, mld_stress.F90:580-603): y is formed per neighbour from the Z terms (one real by complex
+// product per term, a third of a dB contraction), and its dot products are taken with the generators
+// applied to U.  Neighbours are lanes and four half entries a step of a warp, so the Z terms are
+// broadcast, a neighbour's block weights are read without conflicts, and its y never leaves the
+// registers.  The Z terms of the atom are formed in the CTA, a channel at a time.  Bound: FP32
+// arithmetic and shared memory of the Z terms.
 //
 // Persistent CTAs take atoms from a queue.  Every sum has a fixed order that does not depend on the
 // batch.
@@ -34,10 +36,9 @@ namespace mld {
 
 namespace {
 
-constexpr int kChunk = 16;  // neighbours whose own y is formed at a time (quadratic stress)
-// row stride of the chunk's gamma: 16-byte aligned, few store conflicts
-template <typename T>
-constexpr int kGrow = sizeof(T) == 4 ? 20 : 18;
+constexpr int kBatch = 32;              // neighbours (lanes) whose own y is formed at a time
+constexpr int kGrow = kBatch + 1;       // row stride of their block weights (odd: no bank conflicts)
+constexpr int kStressRows = 42;         // neighbours per round of the stress sums, times six components
 
 // A sum of products of three: FP64, or a double-FP32 pair (products and sums of FP32 values are then
 // as exact as FP64 ones without its 64 times slower issue).
@@ -86,7 +87,7 @@ struct EvalArgs {
 };
 
 struct EvalPlan {
-  size_t hoff, exp, hd, sj, cfull, chalf, gamma, cg, tbuf, yb, yt, geo, fcw, red, grow, next, U, total;
+  size_t hoff, exp, quads, cfull, gamma, cg, tbuf, yb, yt, geo, red, grow, next, U, total;
 };
 
 __host__ __device__ inline size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
@@ -97,20 +98,24 @@ __host__ __device__ inline EvalPlan eval_plan(const DevTables& tb, int nch, int 
   size_t o = 0;
   s.hoff = o;  o = up16(o + sizeof(int) * (kMaxJ + 2));
   s.exp = o;   o = up16(o + sizeof(int16_t) * tb.NU);
-  s.hd = o;    o = up16(o + tb.HU);
-  s.sj = o;    o = up16(o + tb.HU);
+  s.quads = o; o = up16(o + sizeof(int16_t) * (tb.HU / 4 + kMaxJ + 2));
   s.cfull = o; o = up16(o + (quad ? cxb * nch * tb.NU : 0));
-  s.chalf = o; o = up16(o + (quad ? cxb * nch * tb.HU : 0));
   s.gamma = o; o = up16(o + (quad ? (size_t)eb * nch * tb.NBLK : 0));
   s.cg = o;    o = up16(o + (quad ? (size_t)eb * tb.NCG : 0));
-  // Z terms of every channel, y, and the generators' y_b
-  s.tbuf = o;  o = up16(o + (quad ? cxb * nch * tb.NZT : 0));
+  // Z terms of a channel, y, and the block weights of a batch, which the generators' y_b and the
+  // sums over the warps follow in the same place
+  s.tbuf = o;  o = up16(o + (quad ? cxb * tb.NZT : 0));
   s.yt = o;    o = up16(o + (quad ? cxb * nch * tb.HU : 0));
-  s.yb = o;    o = up16(o + cxb * 4 * nch * tb.HU);
+  size_t w = cxb * 4 * nch * tb.HU;
+  if (quad) {
+    const size_t g = (size_t)eb * tb.NBLK * kGrow, r = (size_t)eb * kNW * 2 * kBatch * 4;
+    w = w > g ? w : g;
+    w = w > r ? w : r;
+  }
+  s.yb = o;
+  s.grow = o;  o = up16(o + w);
   s.geo = o;   o = up16(o + (size_t)eb * kGeo * slots);
-  s.fcw = o;   o = up16(o + (size_t)eb * nch * slots);
-  s.red = o;   o = up16(o + (size_t)eb * (kNW * kChunk * 4));
-  s.grow = o;  o = up16(o + (quad ? (size_t)eb * tb.NBLK * (eb == 4 ? 20 : 18) : 0));
+  s.red = o;   o = up16(o + 8 * 256);
   s.next = o;  o = up16(o + 16);
   s.U = o;     o = up16(o + cxb * u_stride(tb.HU) * slots);
   s.total = o;
@@ -132,18 +137,15 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
   const EvalPlan sp = eval_plan(tb, nch, (int)sizeof(T), args.slots, kQuad);
   int* shoff = reinterpret_cast<int*>(smem_raw + sp.hoff);
   int16_t* sexp = reinterpret_cast<int16_t*>(smem_raw + sp.exp);
-  int8_t* shd = reinterpret_cast<int8_t*>(smem_raw + sp.hd);
-  int8_t* sj = reinterpret_cast<int8_t*>(smem_raw + sp.sj);  // layer of each half entry
+  int16_t* squad = reinterpret_cast<int16_t*>(smem_raw + sp.quads);  // four half entries: layer << 8 | quad
   cx<T>* cfull = reinterpret_cast<cx<T>*>(smem_raw + sp.cfull);
-  cx<T>* chalf = reinterpret_cast<cx<T>*>(smem_raw + sp.chalf);
   T* sgam = reinterpret_cast<T*>(smem_raw + sp.gamma);
   T* scg = reinterpret_cast<T*>(smem_raw + sp.cg);
   cx<T>* tbuf = reinterpret_cast<cx<T>*>(smem_raw + sp.tbuf);
   cx<T>* yb = reinterpret_cast<cx<T>*>(smem_raw + sp.yb);  // [nch][HU][4]
   cx<T>* yt = reinterpret_cast<cx<T>*>(smem_raw + sp.yt);
   T* sgeo = reinterpret_cast<T*>(smem_raw + sp.geo);
-  T* fcw = reinterpret_cast<T*>(smem_raw + sp.fcw);
-  T* red = reinterpret_cast<T*>(smem_raw + sp.red);
+  ExactSum<T>* sred = reinterpret_cast<ExactSum<T>*>(smem_raw + sp.red);
   T* grow = reinterpret_cast<T*>(smem_raw + sp.grow);
   int* snext = reinterpret_cast<int*>(smem_raw + sp.next);
   cx<T>* Us = reinterpret_cast<cx<T>*>(smem_raw + sp.U);
@@ -153,11 +155,11 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
   // tables, once per CTA
   for (int e = tid; e < kMaxJ + 2; e += nth) shoff[e] = tb.hoff[e];
   for (int e = tid; e < NU; e += nth) sexp[e] = tb.expand[e];
-  for (int e = tid; e < HU; e += nth) {
-    shd[e] = tb.half_diag[e];
-    int j = 0;
-    while (j < J && tb.hoff[j + 1] <= e) ++j;
-    sj[e] = (int8_t)j;
+  int nquad = 0;
+  for (int j = J; j >= 0; --j) {  // heaviest layers first
+    const int c = (tb.hoff[j + 1] - tb.hoff[j] + 3) >> 2;
+    for (int q = tid; q < c; q += nth) squad[nquad + q] = (int16_t)((j << 8) | q);
+    nquad += c;
   }
   if constexpr (kQuad)
     for (int e = tid; e < tb.NCG; e += nth) scg[e] = args.cg[e];
@@ -186,93 +188,170 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
         int nb, tn;
         pair_geometry<T>(args.src, args.rin, (size_t)(p0 + base + n), ti, g, &nb, &tn);
         put_pair<T>(g, nb, tn);
-        for (int ch = 0; ch < nch; ++ch) fcw[n * nch + ch] = g[kGeoFc] * args.chw[ch * args.src.ntypes + tn];
         Us[(size_t)n * HS] = {T(1), T(0)};
       }
       __syncthreads();
       u_store<T>(Us, HS, count, J, args.chains, warp, lane, [&](int n) { return geo(n) + kGeoZx; });
       __syncthreads();
     };
-    // ---- y = dE/dc: quadratic model, from c and the Z terms of this atom ------------------------
-    const cx<T>* ysrc = yt;
-    if constexpr (kQuad) {
-      for (int ps = 0; ps < npass; ++ps) {
-        const int base = ps * args.slots, count = min(args.slots, nn - base);
-        load_pass(base, count);
-        c_sum<T>(chalf, Us, HS, fcw, shd, count, nch, HU, ps == 0, ps == npass - 1, tid);
-        __syncthreads();
-      }
-    }
     if (nn == 0) {  // no neighbours: the constant alone
       if (tid < 6) args.ev.Satom[(size_t)atom * 6 + tid] = 0.0;
       if (!kQuad && tid == 0) args.ev.Eatom[atom] = args.ev.w0;
       continue;
     }
+    const cx<T>* ysrc = kQuad ? yt : static_cast<const cx<T>*>(args.ev.y) + (size_t)atom * nch * HU;
+    const cx<T>* csrc = static_cast<const cx<T>*>(args.ev.c) + (size_t)atom * nch * HU;
     if constexpr (kQuad) {
       for (int e = tid; e < nch * NU; e += nth) {
         const int ch = e / NU, f = e - ch * NU;
-        cfull[e] = fetch(chalf + ch * HU, sexp[f]);
+        cfull[e] = fetch(csrc + ch * HU, sexp[f]);
       }
-      __syncthreads();
-      for (int ch = 0; ch < nch; ++ch)
-        z_rounds<T>(tb.zitems, zr0, zr1, cfull + ch * NU, scg, tbuf + (size_t)ch * tb.NZT, lane);
-      __syncthreads();
-      // y of each half entry: the blocks of its layer with their weights, in order
-      for (int i = tid; i < nch * HU; i += nth) {
-        const int ch = i / HU, h = i - ch * HU;
-        const int j = sj[h], H = shoff[j + 1] - shoff[j];
-        const cx<T>* z = tbuf + (size_t)ch * tb.NZT + tb.zoff[j] + (h - shoff[j]);
-        const T* g = sgam + ch * tb.NBLK + tb.blk_off[j];
-        const int nb = tb.blk_off[j + 1] - tb.blk_off[j];
-        cx<T> v = {T(0), T(0)};
-#pragma unroll 4
-        for (int r = 0; r < nb; ++r) {
-          const cx<T> zr = z[r * H];
-          v.x = fma(g[r], zr.x, v.x);
-          v.y = fma(g[r], zr.y, v.y);
-        }
-        yt[i] = v;
+    } else if (warp == kNW - 1) {  // energy of the atom, w0 + w_lin . B = w0 + c . y / 3
+      ExactSum<T> s;
+      for (int e = lane; e < nch * HU; e += 32) {
+        const T w = args.gen[e % HU].w;
+        const cx<T> cv = csrc[e], yv = ysrc[e];
+        s.add(cv.x, yv.x, w);
+        s.add(cv.y, yv.y, w);
       }
-      __syncthreads();
-    } else {
-      ysrc = static_cast<const cx<T>*>(args.ev.y) + (size_t)atom * nch * HU;
-      if (warp == kNW - 1) {  // energy of the atom, w0 + w_lin . B = w0 + c . y / 3
-        const cx<T>* c = static_cast<const cx<T>*>(args.ev.c) + (size_t)atom * nch * HU;
-        ExactSum<T> s;
-        for (int e = lane; e < nch * HU; e += 32) {
-          const T w = args.gen[e % HU].w;
-          const cx<T> cv = c[e], yv = ysrc[e];
-          s.add(cv.x, yv.x, w);
-          s.add(cv.y, yv.y, w);
-        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s.add(s.down(o));
-        if (lane == 0) args.ev.Eatom[atom] = args.ev.w0 + s.value() / 3.0;
+      for (int o = 16; o > 0; o >>= 1) s.add(s.down(o));
+      if (lane == 0) args.ev.Eatom[atom] = args.ev.w0 + s.value() / 3.0;
+    }
+    // the generators' y_b, weighted for sums over the half layers
+    auto form_yb = [&]() {
+      for (int e = tid; e < nch * HU; e += nth) {
+        const int ch = e / HU, h = e - ch * HU;
+        const GenEntry<T> g = args.gen[h];
+        const cx<T>* y = ysrc + ch * HU;
+        const cx<T> y0 = y[h], ym = y[max(h - 1, 0)];
+        cx<T> yp = y[min(h + 1, HU - 1)];
+        if (g.w == T(1)) yp = {-ym.x, ym.y};  // centre of an even layer: y(0, 2) = -conj y(0, -2)
+        const cx<T> a = {g.cm * ym.x, g.cm * ym.y}, b = {g.cp * yp.x, g.cp * yp.y};
+        const T w = g.w, qw = g.q * g.w;
+        cx<T>* o = yb + (size_t)e * 4;
+        o[0] = {w * y0.x, w * y0.y};
+        o[1] = {-qw * y0.y, qw * y0.x};
+        o[2] = {w * (a.y + b.y), -w * (a.x + b.x)};
+        o[3] = {w * (b.x - a.x), w * (b.y - a.y)};
       }
-    }
-    // ---- the generators' y_b, weighted for sums over the half layers ---------------------------
-    for (int e = tid; e < nch * HU; e += nth) {
-      const int ch = e / HU, h = e - ch * HU;
-      const GenEntry<T> g = args.gen[h];
-      const cx<T>* y = ysrc + ch * HU;
-      const cx<T> y0 = y[h], ym = y[max(h - 1, 0)];
-      cx<T> yp = y[min(h + 1, HU - 1)];
-      if (g.w == T(1)) yp = {-ym.x, ym.y};  // centre of an even layer: y(0, 2) = -conj y(0, -2)
-      const cx<T> a = {g.cm * ym.x, g.cm * ym.y}, b = {g.cp * yp.x, g.cp * yp.y};
-      const T w = g.w, qw = g.q * g.w;
-      cx<T>* o = yb + (size_t)e * 4;
-      o[0] = {w * y0.x, w * y0.y};
-      o[1] = {-qw * y0.y, qw * y0.x};
-      o[2] = {w * (a.y + b.y), -w * (a.x + b.x)};
-      o[3] = {w * (b.x - a.x), w * (b.y - a.y)};
-    }
-    if constexpr (kQuad) __syncthreads();  // (the linear model's passes begin with a barrier)
+    };
+    if constexpr (!kQuad) form_yb();  // (each pass begins with barriers)
     // ---- pairs: forces (and, linear model, stress) ---------------------------------------------
     const T lev = args.small[args.atom_struct[atom]] ? T(1) : -args.sign_big;  // stress lever arm: sign * u
     ExactSum<T> sacc;  // of this thread's (pair slot, component)
+    const int srow = tid / 6, scomp = tid - srow * 6;  // quadratic model: its neighbours and component
     for (int ps = npass - 1; ps >= 0; --ps) {
       const int base = ps * args.slots, count = min(args.slots, nn - base);
-      if (!kQuad || ps != npass - 1) load_pass(base, count);  // (quadratic: the last pass is still there)
+      load_pass(base, count);
+      if constexpr (kQuad) {
+        // stress sums S_b of the pass's neighbours with their own beta, channel by channel
+        T st[2][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) st[i >> 2][i & 3] = T(0);
+        for (int ch = 0; ch < nch; ++ch) {
+          z_rounds<T>(tb.zitems, zr0, zr1, cfull + ch * NU, scg, tbuf, lane);
+          __syncthreads();
+          if (ps == npass - 1) {
+            // y of the atom: the blocks of each layer with its own weights, in order
+            for (int h = tid; h < HU; h += nth) {
+              int j = 0;
+              while (shoff[j + 1] <= h) ++j;
+              const int H = shoff[j + 1] - shoff[j];
+              const cx<T>* z = tbuf + tb.zoff[j] + (h - shoff[j]);
+              const T* g = sgam + ch * tb.NBLK + tb.blk_off[j];
+              const int nb = tb.blk_off[j + 1] - tb.blk_off[j];
+              cx<T> v = {T(0), T(0)};
+#pragma unroll 4
+              for (int r = 0; r < nb; ++r) {
+                const cx<T> zr = z[r * H];
+                v.x = fma(g[r], zr.x, v.x);
+                v.y = fma(g[r], zr.y, v.y);
+              }
+              yt[ch * HU + h] = v;
+            }
+          }
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            const int b0 = b * kBatch;
+            if (b0 >= count) continue;
+            for (int n = warp; n < min(kBatch, count - b0); n += kNW) {
+              const int nb = reinterpret_cast<const int*>(geo(b0 + n) + kGeoIdx)[0];
+              const T* src = args.ev.gamma + (size_t)nb * nchG + ch * tb.NBLK;
+              for (int r = lane; r < tb.NBLK; r += 32) grow[r * kGrow + n] = src[r];
+            }
+            __syncthreads();
+            const int n = min(b0 + lane, count - 1);
+            const cx<T>* u = Us + (size_t)n * HS;
+            const T wn = args.chw[ch * args.src.ntypes + pair_type<T>(geo(n))];
+            for (int it = warp; it < nquad; it += kNW) {
+              const int q = squad[it], j = q >> 8, e0 = (q & 255) * 4;
+              const int H = shoff[j + 1] - shoff[j], nb = tb.blk_off[j + 1] - tb.blk_off[j];
+              const cx<T>* z = tbuf + tb.zoff[j] + e0;
+              const T* g = grow + tb.blk_off[j] * kGrow + (n - b0);
+              cx<T> y[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) y[i] = {T(0), T(0)};
+              // (the last step of a layer reads up to three values past its entries; they are not used)
+#pragma unroll 2
+              for (int r = 0; r < nb; ++r) {
+                const T w = g[r * kGrow];
+                const cx<T> ww = {w, w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) y[i] = fma2(ww, z[r * H + i], y[i]);
+              }
+              const int h0 = shoff[j] + e0;
+              cx<T> um = u[max(h0 - 1, 0)], u0 = u[h0];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                if (e0 + i < H) {
+                  const GenEntry<T> ge = args.gen[h0 + i];
+                  const cx<T> up = u[min(h0 + i + 1, HU - 1)];
+                  // w y . (U, T1 U, T2 U, T3 U)
+                  cx<T> uq = up;
+                  if (ge.w == T(1)) uq = {-um.x, um.y};
+                  const cx<T> a = {ge.cm * um.x, ge.cm * um.y}, c = {ge.cp * uq.x, ge.cp * uq.y};
+                  const cx<T> s = {a.x + c.x, a.y + c.y}, d = {a.x - c.x, a.y - c.y};
+                  const T wg = ge.w * wn;
+                  const cx<T> yw = {wg * y[i].x, wg * y[i].y};
+                  st[b][0] = fma(yw.x, u0.x, fma(yw.y, u0.y, st[b][0]));
+                  st[b][1] = fma(ge.q, fma(yw.x, u0.y, -(yw.y * u0.x)), st[b][1]);
+                  st[b][2] = fma(-yw.x, s.y, fma(yw.y, s.x, st[b][2]));
+                  st[b][3] = fma(yw.x, d.x, fma(yw.y, d.y, st[b][3]));
+                  um = u0;
+                  u0 = up;
+                }
+              }
+            }
+            __syncthreads();  // the weights have been read (and, after the last batch, the Z terms)
+          }
+        }
+        // sums over the warps, in order; then the stress of (neighbour, component)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) grow[((warp * 2 + b) * kBatch + lane) * 4 + i] = st[b][i];
+        __syncthreads();
+        if (srow < kStressRows) {
+          const int aa = stress_a(scomp), bb = stress_b(scomp);
+          for (int n = srow; n < count; n += kStressRows) {
+            T S[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+              S[b] = T(0);
+#pragma unroll
+              for (int w = 0; w < kNW; ++w) S[b] += grow[((w * 2 + n / kBatch) * kBatch + n % kBatch) * 4 + b];
+            }
+            const T* g = geo(n);
+            const T* xi = g + kGeoXi + 3 * aa;
+            const T f = fma(g[kGeoFc], fma(xi[0], S[1], fma(xi[1], S[2], xi[2] * S[3])), g[kGeoDfr + aa] * S[0]);
+            sacc.add(f, lev * g[kGeoU + bb], g[kGeoU + 3]);
+          }
+        }
+        __syncthreads();
+        form_yb();  // where the sums were
+        __syncthreads();
+      }
       for (int g4 = warp * 4; g4 < count; g4 += kNW * 4) {
         // a warp takes four pairs, its lanes the half entries
         T tot[16];
@@ -334,112 +413,15 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
             sacc.add(fs, lev * gs[kGeoU + stress_b(sc)], gs[kGeoU + 3]);
         }
       }
-      if constexpr (kQuad) {
-        // stress with the neighbours' beta, kChunk neighbours at a time: thread (4 neighbours, entry)
-        const int nt = tid & 3;
-        for (int c0 = 0; c0 < count; c0 += kChunk) {
-          T tot[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) tot[i] = T(0);
-          const cx<T>* up[4];
-          T wn[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) up[i] = Us + (size_t)min(c0 + nt * 4 + i, count - 1) * HS;
-          for (int ch = 0; ch < nch; ++ch) {
-            __syncthreads();  // the previous weights have been read
-            for (int e = tid; e < kChunk * tb.NBLK; e += nth) {
-              const int n = e / tb.NBLK, r = e - n * tb.NBLK;
-              T g = T(0);
-              if (c0 + n < count) {
-                const int nb = reinterpret_cast<const int*>(geo(c0 + n) + kGeoIdx)[0];
-                g = args.ev.gamma[(size_t)nb * nchG + ch * tb.NBLK + r];
-              }
-              grow[r * kGrow<T> + n] = g;
-            }
-            __syncthreads();
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int tn = pair_type<T>(geo(min(c0 + nt * 4 + i, count - 1)));
-              wn[i] = args.chw[ch * args.src.ntypes + tn];
-            }
-            const cx<T>* zc = tbuf + (size_t)ch * tb.NZT;
-            for (int e = tid >> 2; e < HU; e += nth / 4) {
-              const int j = sj[e], H = shoff[j + 1] - shoff[j], nb = tb.blk_off[j + 1] - tb.blk_off[j];
-              const cx<T>* z = zc + tb.zoff[j] + (e - shoff[j]);
-              const T* gr = grow + (size_t)tb.blk_off[j] * kGrow<T> + nt * 4;
-              cx<T> y[4];
-#pragma unroll
-              for (int i = 0; i < 4; ++i) y[i] = {T(0), T(0)};
-#pragma unroll 4
-              for (int r = 0; r < nb; ++r) {
-                const cx<T> zr = z[r * H];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  const T b = gr[r * kGrow<T> + i];
-                  y[i].x = fma(b, zr.x, y[i].x);
-                  y[i].y = fma(b, zr.y, y[i].y);
-                }
-              }
-              const GenEntry<T> g = args.gen[e];
-              const int em = max(e - 1, 0), ep = min(e + 1, HU - 1);
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                // w y . (U, T1 U, T2 U, T3 U)
-                const cx<T> u = up[i][e], um = up[i][em];
-                cx<T> uq = up[i][ep];
-                if (g.w == T(1)) uq = {-um.x, um.y};
-                const cx<T> a = {g.cm * um.x, g.cm * um.y}, b = {g.cp * uq.x, g.cp * uq.y};
-                const cx<T> s = {a.x + b.x, a.y + b.y}, d = {a.x - b.x, a.y - b.y};
-                const T wg = g.w * wn[i];
-                const cx<T> yw = {wg * y[i].x, wg * y[i].y};
-                tot[i * 4 + 0] = fma(yw.x, u.x, fma(yw.y, u.y, tot[i * 4 + 0]));
-                tot[i * 4 + 1] = fma(g.q, fma(yw.x, u.y, -(yw.y * u.x)), tot[i * 4 + 1]);
-                tot[i * 4 + 2] = fma(-yw.x, s.y, fma(yw.y, s.x, tot[i * 4 + 2]));
-                tot[i * 4 + 3] = fma(yw.x, d.x, fma(yw.y, d.y, tot[i * 4 + 3]));
-              }
-            }
-          }
-          // sums over the lanes of equal nt: a lane ends with two of its 16 values
-#pragma unroll
-          for (int s = 8; s > 1; s >>= 1) {
-            const bool hi = lane & (2 * s);
-#pragma unroll
-            for (int i = 0; i < s; ++i) {
-              const T keep = hi ? tot[i + s] : tot[i], send = hi ? tot[i] : tot[i + s];
-              tot[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * s);
-            }
-          }
-          const int vi = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2;
-          __syncthreads();  // red is free
-          red[(warp * kChunk + nt * 4 + (vi >> 2)) * 4 + (vi & 3)] = tot[0];
-          red[(warp * kChunk + nt * 4 + (vi >> 2)) * 4 + (vi & 3) + 1] = tot[1];
-          __syncthreads();
-          if (tid < kChunk * 6 && c0 + tid / 6 < count) {
-            const int n = tid / 6, sc = tid - n * 6, aa = stress_a(sc);
-            T S[4];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-              S[b] = T(0);
-              for (int w = 0; w < kNW; ++w) S[b] += red[(w * kChunk + n) * 4 + b];
-            }
-            const T* g = geo(c0 + n);
-            const T* xi = g + kGeoXi + 3 * aa;
-            const T f = fma(g[kGeoFc], fma(xi[0], S[1], fma(xi[1], S[2], xi[2] * S[3])), g[kGeoDfr + aa] * S[0]);
-            sacc.add(f, lev * g[kGeoU + stress_b(sc)], g[kGeoU + 3]);
-          }
-        }
-      }
       if (ps > 0) __syncthreads();  // the pass's U and geometry have been read
     }
     // stress of the atom: the partial sums of (slot, component), slots in order
-    ExactSum<T>* sred = reinterpret_cast<ExactSum<T>*>(red);
     if constexpr (kQuad) {
-      __syncthreads();
-      if (tid < kChunk * 6) sred[tid] = sacc;
+      if (srow < kStressRows) sred[tid] = sacc;
       __syncthreads();
       if (tid < 6) {
         ExactSum<T> v;
-        for (int n = 0; n < kChunk; ++n) v.add(sred[n * 6 + tid]);
+        for (int n = 0; n < kStressRows; ++n) v.add(sred[n * 6 + tid]);
         args.ev.Satom[(size_t)atom * 6 + tid] = v.value();
       }
     } else {
@@ -473,7 +455,7 @@ template <typename T>
 cudaError_t launch_bso4_eval(const DevTables& tb, const DevBatch& b, const BsoParams& p, const DevEval<T>& ev,
                              const int* order, int* counter, cudaStream_t st) {
   if (b.A == 0) return cudaSuccess;
-  if (!counter || !ev.pair || !ev.Satom || !tb.gen32 || (!ev.gamma && (!ev.c || !ev.y))) return cudaErrorInvalidValue;
+  if (!counter || !ev.pair || !ev.Satom || !tb.gen32 || !ev.c || (!ev.gamma && !ev.y)) return cudaErrorInvalidValue;
   const bool quad = ev.gamma != nullptr;
   EvalArgs<T> a{};
   a.tb = tb;

@@ -90,7 +90,7 @@ struct LaneArgs {
   const LaneRec* recs;
   const LaneJob* jobs;
   int njobs;
-  const T* cg;
+  const void* cg;       // FP32: every coefficient twice (for the packed instructions)
   const cx<T>* c;       // A x nch x HU
   const int* nbr_off;   // of the first atom
   const T* gamma;       // y: nch * NBLKP
@@ -101,6 +101,7 @@ struct LaneArgs {
 
 // lanes that hold atoms: 32, or 16 where their c does not fit in shared memory; a padded row per entry
 // (16-byte values) so that the transposing stores spread over the banks
+// The coefficients go to shared memory in FP32 where there is room, else they are read through the cache.
 struct LanePlan {
   int stride;
   size_t c, cg, gamma, part, total;
@@ -108,12 +109,12 @@ struct LanePlan {
 
 __host__ __device__ inline size_t upl(size_t x) { return (x + 15) & ~(size_t)15; }
 
-__host__ __device__ inline LanePlan lane_plan(const DevTables& tb, int eb, int lanes) {
+__host__ __device__ inline LanePlan lane_plan(const DevTables& tb, int eb, int lanes, bool cg_shared) {
   LanePlan s;
   s.stride = lanes + 1;
   size_t o = 0;
   s.c = o;     o = upl(o + (size_t)16 * tb.NU * s.stride);
-  s.cg = o;    o = upl(o + (eb == 4 ? (size_t)8 * tb.NCGV : 0));  // FP32: doubled; FP64 reads through the cache
+  s.cg = o;    o = upl(o + (cg_shared ? (size_t)8 * tb.NCGV : 0));
   s.gamma = o; o = upl(o + (size_t)8 * tb.NBLKP);
   s.part = o;  o = upl(o + (size_t)16 * (eb == 4 ? LaneVec<float>::warps : LaneVec<double>::warps) * (tb.J / 2 + 1) * 32);
   s.total = o;
@@ -230,13 +231,13 @@ __device__ __forceinline__ void lane_record(uint4 z0, uint4 z1, const vcx<V>* __
 }
 
 template <typename T, bool kY>
-__global__ void __launch_bounds__(LaneVec<T>::warps * 32, 1) k_lanes(LaneArgs<T> args, int lanes) {
+__global__ void __launch_bounds__(LaneVec<T>::warps * 32, 1) k_lanes(LaneArgs<T> args, int lanes, bool cg_shared) {
   using V = typename LaneVec<T>::type;
   constexpr int kPer = LaneVec<T>::atoms, kLaneWarps = LaneVec<T>::warps;
   constexpr int kGroups = kLaneWarps / 4;  // four warps share a job
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DevTables& tb = args.tb;
-  const LanePlan sp = lane_plan(tb, (int)sizeof(T), lanes);
+  const LanePlan sp = lane_plan(tb, (int)sizeof(T), lanes, cg_shared);
   const int ST = sp.stride, HU = tb.HU, K = tb.K;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int nth = kLaneWarps * 32;
@@ -256,13 +257,11 @@ __global__ void __launch_bounds__(LaneVec<T>::warps * 32, 1) k_lanes(LaneArgs<T>
       d[kPer] = v.y;
     }
   }
-  const V* cg;
-  if constexpr (sizeof(T) == 4) {
+  const V* cg = static_cast<const V*>(args.cg);
+  if (cg_shared) {
     V* scg = reinterpret_cast<V*>(smem_raw + sp.cg);
-    for (int e = tid; e < tb.NCGV; e += nth) scg[e] = vdup(args.cg[e], V{});
+    for (int e = tid; e < tb.NCGV; e += nth) scg[e] = cg[e];
     cg = scg;
-  } else {
-    cg = args.cg;
   }
   if constexpr (kY) {
     for (int b = tid; b < tb.NBLKP; b += nth) sg[b] = vdup(args.gamma[ch * tb.NBLKP + b], V{});
@@ -437,8 +436,11 @@ template <typename T, bool kY>
 cudaError_t launch_lanes(LaneArgs<T>& a, cudaStream_t st) {
   if (a.A <= 0 || a.njobs <= 0) return cudaSuccess;
   int lanes = 32;
-  if (lane_plan(a.tb, (int)sizeof(T), lanes).total > (size_t)optin()) lanes = 16;
-  const size_t smem = lane_plan(a.tb, (int)sizeof(T), lanes).total;
+  bool cg_shared = sizeof(T) == 4;
+  auto bytes = [&]() { return lane_plan(a.tb, (int)sizeof(T), lanes, cg_shared).total; };
+  if (bytes() > (size_t)optin()) lanes = 16;
+  if (bytes() > (size_t)optin()) cg_shared = false;
+  const size_t smem = bytes();
   if (smem > (size_t)optin()) return cudaErrorInvalidConfiguration;
   cudaError_t e = cudaFuncSetAttribute(k_lanes<T, kY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -461,7 +463,7 @@ cudaError_t launch_lanes(LaneArgs<T>& a, cudaStream_t st) {
       slices = s;
     }
   }
-  k_lanes<T, kY><<<dim3(tiles, slices, a.nch), LaneVec<T>::warps * 32, smem, st>>>(a, lanes);
+  k_lanes<T, kY><<<dim3(tiles, slices, a.nch), LaneVec<T>::warps * 32, smem, st>>>(a, lanes, cg_shared);
   return cudaGetLastError();
 }
 
@@ -514,7 +516,7 @@ static LaneArgs<T> lane_args(const DevTables& tb, const DevBatch& b, const BsoPa
   LaneArgs<T> a{};
   a.tb = tb;
   if constexpr (sizeof(T) == 8) a.cg = tb.cgv64;
-  else a.cg = tb.cgv32;
+  else a.cg = tb.cgv32x2;
   a.c = static_cast<const cx<T>*>(c);
   a.nbr_off = b.nbr_off + first;
   a.A = count;

@@ -9,6 +9,7 @@
 // that use block b: the evaluation kernel takes gamma instead of beta.
 #include <cuda_runtime.h>
 
+#include "ds.cuh"
 #include "mld_internal.h"
 
 namespace mld {
@@ -16,67 +17,124 @@ namespace mld {
 namespace {
 
 constexpr int kGammaThreads = 128;
+constexpr int kGammaAtoms = 4;  // atoms per CTA: each reads Wsym once for all of them
 
-// One CTA per atom: beta[k] = w_lin[k] + sum_j Wsym[j][k] B[j] (Wsym symmetric, read by rows j
-// so that consecutive threads read consecutive k), the atom's energy w0 + B . (beta + w_lin) / 2 and
-// gamma of every channel and block.  B null: beta = w_lin, no energy.
+__global__ void k_split_pairs(const double* __restrict__ in, float2* __restrict__ out, size_t n) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float h, l;
+  ds_split(in[i], h, l);
+  out[i] = make_float2(h, l);
+}
+
+// beta[k] = w_lin[k] + sum_j Wsym[j][k] B[j] (Wsym symmetric, read by rows j so that consecutive threads
+// read consecutive k), the atom's energy w0 + B . (beta + w_lin) / 2 and gamma of every channel and
+// block.  The sums over j run in double-FP32 for FP32 descriptors (2^-44 relative; FP64 issues at 1/64
+// of the FP32 rate and took 182 us of a 4,001-atom step with K = 110, 2 channels), in FP64 for FP64
+// ones.  B null: beta = w_lin, no energy.
 template <typename T>
 __global__ void __launch_bounds__(kGammaThreads) k_eval_gamma(const int* __restrict__ gam_off,
                                                               const GammaItem* __restrict__ gam, int nblk, int nch,
-                                                              int K, const T* __restrict__ B,
+                                                              int K, int A, const T* __restrict__ B,
                                                               const double* __restrict__ wlin,
-                                                              const double* __restrict__ wsym, double w0,
+                                                              const double* __restrict__ wsym,
+                                                              const float2* __restrict__ wsym32, double w0,
                                                               T* __restrict__ gamma, double* __restrict__ Eatom) {
-  extern __shared__ double bsh[];  // B, then beta: 2 * nch * K
-  __shared__ double red[4];
-  const int a = blockIdx.x, tid = threadIdx.x, nchK = nch * K;
-  double* beta = bsh + nchK;
+  extern __shared__ double beta[];  // [kGammaAtoms][nchK], then B as T
+  __shared__ double red[kGammaAtoms][kGammaThreads / 32];
+  const int tid = threadIdx.x, nchK = nch * K, a0 = blockIdx.x * kGammaAtoms;
+  const int na = B ? min(kGammaAtoms, A - a0) : 1;
+  T* bsh = reinterpret_cast<T*>(beta + kGammaAtoms * nchK);
   if (B) {
-    for (int j = tid; j < nchK; j += kGammaThreads) bsh[j] = (double)B[(size_t)a * nchK + j];
+    for (int j = tid; j < kGammaAtoms * nchK; j += kGammaThreads)
+      bsh[j] = j < na * nchK ? B[(size_t)a0 * nchK + j] : T(0);
     __syncthreads();
   }
-  double e = 0.0;
+  double e[kGammaAtoms];
+#pragma unroll
+  for (int a = 0; a < kGammaAtoms; ++a) e[a] = 0.0;
   for (int k = tid; k < nchK; k += kGammaThreads) {
-    double v = wlin[k];
+    double v[kGammaAtoms];
+#pragma unroll
+    for (int a = 0; a < kGammaAtoms; ++a) v[a] = wlin[k];
     if (B) {
-      for (int j = 0; j < nchK; ++j) v = fma(wsym[(size_t)j * nchK + k], bsh[j], v);
-      e = fma(0.5 * bsh[k], v + wlin[k], e);
+      if constexpr (sizeof(T) == 4) {
+        float h[kGammaAtoms], l[kGammaAtoms];
+#pragma unroll
+        for (int a = 0; a < kGammaAtoms; ++a) h[a] = l[a] = 0.f;
+#pragma unroll 2
+        for (int j = 0; j < nchK; ++j) {
+          const float2 w = wsym32[(size_t)j * nchK + k];
+#pragma unroll
+          for (int a = 0; a < kGammaAtoms; ++a) ds_fma(h[a], l[a], bsh[a * nchK + j], w.x, w.y);
+        }
+#pragma unroll
+        for (int a = 0; a < kGammaAtoms; ++a) v[a] += (double)h[a] + (double)l[a];
+      } else {
+        for (int j = 0; j < nchK; ++j) {
+          const double w = wsym[(size_t)j * nchK + k];
+#pragma unroll
+          for (int a = 0; a < kGammaAtoms; ++a) v[a] = fma(w, (double)bsh[a * nchK + j], v[a]);
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < kGammaAtoms; ++a) e[a] = fma(0.5 * (double)bsh[a * nchK + k], v[a] + wlin[k], e[a]);
     }
-    beta[k] = (double)(T)v;  // the weights in the method's precision
+#pragma unroll
+    for (int a = 0; a < kGammaAtoms; ++a) beta[a * nchK + k] = (double)(T)v[a];  // in the method's precision
   }
   __syncthreads();
   for (int b = tid; b < nch * nblk; b += kGammaThreads) {
     const int ch = b / nblk, i = b - ch * nblk;
-    double g = 0.0;
-    for (int t = gam_off[i]; t < gam_off[i + 1]; ++t)
-      g = fma((double)gam[t].snum / (double)gam[t].sden, beta[ch * K + gam[t].k], g);
-    gamma[(size_t)a * nch * nblk + b] = (T)g;
+    const int t0 = gam_off[i], t1 = gam_off[i + 1];
+    double g[kGammaAtoms];
+#pragma unroll
+    for (int a = 0; a < kGammaAtoms; ++a) g[a] = 0.0;
+    for (int t = t0; t < t1; ++t) {
+      const GammaItem it = gam[t];
+      const double sc = it.snum == it.sden ? 1.0 : (double)it.snum / (double)it.sden;
+#pragma unroll
+      for (int a = 0; a < kGammaAtoms; ++a) g[a] = fma(sc, beta[a * nchK + ch * K + it.k], g[a]);
+    }
+#pragma unroll
+    for (int a = 0; a < kGammaAtoms; ++a)
+      if (a < na) gamma[(size_t)(a0 + a) * nch * nblk + b] = (T)g[a];
   }
   if (!B) return;
-  for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-  if ((tid & 31) == 0) red[tid >> 5] = e;
+#pragma unroll
+  for (int a = 0; a < kGammaAtoms; ++a) {
+    for (int o = 16; o > 0; o >>= 1) e[a] += __shfl_xor_sync(0xffffffffu, e[a], o);
+    if ((tid & 31) == 0) red[a][tid >> 5] = e[a];
+  }
   __syncthreads();
-  if (tid == 0) Eatom[a] = w0 + red[0] + red[1] + red[2] + red[3];
+  if (tid < na) Eatom[a0 + tid] = w0 + red[tid][0] + red[tid][1] + red[tid][2] + red[tid][3];
 }
 
 }  // namespace
 
+cudaError_t launch_split_pairs(const double* in, float2* out, size_t n, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  k_split_pairs<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(in, out, n);
+  return cudaGetLastError();
+}
+
 template <typename T>
 cudaError_t launch_eval_gamma(const DevTables& tb, const T* B, int A, int nch, const double* wlin, const double* wsym,
-                              double w0, T* gamma, double* Eatom, cudaStream_t st) {
+                              const float2* wsym32, double w0, T* gamma, double* Eatom, cudaStream_t st) {
   if (A <= 0) return cudaSuccess;
-  const size_t smem = sizeof(double) * 2 * nch * tb.K;
+  const size_t smem = (sizeof(double) + sizeof(T)) * kGammaAtoms * nch * tb.K;
   if (B)
-    k_eval_gamma<T><<<A, kGammaThreads, smem, st>>>(tb.gam_off, tb.gam, tb.NBLK, nch, tb.K, B, wlin, wsym, w0, gamma, Eatom);
+    k_eval_gamma<T><<<(A + kGammaAtoms - 1) / kGammaAtoms, kGammaThreads, smem, st>>>(
+        tb.gam_off, tb.gam, tb.NBLK, nch, tb.K, A, B, wlin, wsym, wsym32, w0, gamma, Eatom);
   else
-    k_eval_gamma<T><<<1, kGammaThreads, smem, st>>>(tb.gamp_off, tb.gamp, tb.NBLKP, nch, tb.K, nullptr, wlin, nullptr, w0,
-                                                    gamma, nullptr);
+    k_eval_gamma<T><<<1, kGammaThreads, smem, st>>>(tb.gamp_off, tb.gamp, tb.NBLKP, nch, tb.K, 1, nullptr, wlin, nullptr,
+                                                    nullptr, w0, gamma, nullptr);
   return cudaGetLastError();
 }
 
 template cudaError_t launch_eval_gamma<double>(const DevTables&, const double*, int, int, const double*, const double*,
-                                               double, double*, double*, cudaStream_t);
+                                               const float2*, double, double*, double*, cudaStream_t);
 template cudaError_t launch_eval_gamma<float>(const DevTables&, const float*, int, int, const double*, const double*,
-                                              double, float*, double*, cudaStream_t);
+                                              const float2*, double, float*, double*, cudaStream_t);
 
 }  // namespace mld

@@ -212,7 +212,7 @@ struct DevTables {
   int zoff[kMaxJ + 1] = {0};
   int NCGV = 0, NBJ = 0, NYJ = 0, NBLKP = 0;
   double* cgv64 = nullptr;        // NCGV
-  float* cgv32 = nullptr;
+  float2* cgv32x2 = nullptr;      // every coefficient twice
   LaneRec* brecs = nullptr;
   LaneJob* bjobs = nullptr;       // NBJ
   LaneRec* yrecs = nullptr;       // (fill_deriv_tables)
@@ -285,9 +285,10 @@ cudaError_t fill_dev_tables(const Bso4Tables& t, DevTables* d, Put put) {
   if (e == cudaSuccess) e = put(t.zitems, &d->zitems);
   d->NCGV = (int)t.cgv.size();
   d->NBJ = (int)t.bjobs.size();
-  std::vector<float> cgv32(t.cgv.begin(), t.cgv.end());
+  std::vector<float2> cgv32x2;
+  for (double v : t.cgv) cgv32x2.push_back(make_float2((float)v, (float)v));
   if (e == cudaSuccess) e = put(t.cgv, &d->cgv64);
-  if (e == cudaSuccess) e = put(cgv32, &d->cgv32);
+  if (e == cudaSuccess) e = put(cgv32x2, &d->cgv32x2);
   if (e == cudaSuccess) e = put(t.brecs, &d->brecs);
   if (e == cudaSuccess) e = put(t.bjobs, &d->bjobs);
   if (e == cudaSuccess) e = put(t.trz, &d->trz);
@@ -417,9 +418,8 @@ cudaError_t launch_lane_y(const DevTables& tb, const DevBatch& b, const BsoParam
 // gathered into E/F/S by launch_eval_gather.
 template <typename T>
 struct DevEval {
-  // linear model: c and y of every atom (A x nch x HU complex of T); the kernel writes Eatom
-  const void* c = nullptr;
-  const void* y = nullptr;
+  const void* c = nullptr;       // c of every atom (A x nch x HU complex of T)
+  const void* y = nullptr;       // linear model: y of every atom, as c; the kernel writes Eatom
   double w0 = 0.0;
   const T* gamma = nullptr;      // quadratic model: Z-block weights, nch * NBLK per atom
   T* pair = nullptr;             // P x 3: the pair's force contribution
@@ -460,10 +460,11 @@ size_t atom_order_tmp_ints(int maxnn);
 cudaError_t launch_atom_order(const int* nn, int A, int maxnn, int* order, int* tmp, cudaStream_t st);
 // The block weights gamma (nch * NBLK per atom) of beta_a = w_lin + Wsym B_a and the energies
 // Eatom_a = w0 + B_a . (beta_a + w_lin) / 2; with B null the pair-block weights (nch * NBLKP) of
-// beta = w_lin, once (eval.cu)
+// beta = w_lin, once (eval.cu).  wsym32: Wsym as double-FP32 pairs (launch_split_pairs), for T = float.
 template <typename T>
 cudaError_t launch_eval_gamma(const DevTables& tb, const T* B, int A, int nch, const double* wlin, const double* wsym,
-                              double w0, T* gamma, double* Eatom, cudaStream_t st);
+                              const float2* wsym32, double w0, T* gamma, double* Eatom, cudaStream_t st);
+cudaError_t launch_split_pairs(const double* in, float2* out, size_t n, cudaStream_t st);
 
 // FP64 Gram and rhs on the CUDA cores; with ws (gram_workspace_doubles(M, D) doubles) the
 // row-chunk partials are summed in a fixed order (bitwise reproducible), else with atomics
