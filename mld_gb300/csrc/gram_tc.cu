@@ -12,8 +12,13 @@
 //
 // Grid: (upper-triangle tile pairs) x (row splits), split-major so that the CTAs resident at one
 // time read the same rows (L2 reuse).  Per CTA: warp 0 issues TMA loads into a 3-stage ring,
-// warp 1 allocates two 128-column TMEM accumulators and issues tcgen05.mma from one thread,
-// warps 2-17 drain the accumulators with tcgen05.ld into compensated FP32 sums.  With several
+// warp 1 allocates four 128-column TMEM accumulators and issues tcgen05.mma from one thread,
+// warps 2-17 drain the accumulators with tcgen05.ld into compensated FP32 sums.
+//
+// 60,000 rows x 1541 columns: k_gram_tc 705 -> 495 us (1.1 PFLOP/s of the three products), k_split_bf16
+// 336 -> 175 us.  Of the first, 125 us were the last of three rounds of CTAs (gram_tc_splits); with
+// two accumulators the MMAs waited for the epilogue's chain of load, wait and add.  What bounds it
+// now is the operand traffic, 64 KB per 64-row slice of a tile: 11 TB/s from L2.  With several
 // row splits each split writes its tile to a partial buffer and k_gram_tc_reduce adds the splits
 // into the FP64 Gram in split order (without that buffer: FP64 atomics, order not fixed); with
 // one split the CTA adds its tile directly.  Every mbarrier wait
@@ -39,6 +44,7 @@ using tc::kTileBytes;
 constexpr int kStages = 3;
 constexpr int kStageBytes = 4 * kTileBytes;    // A_hi, A_lo, B_hi, B_lo
 constexpr int kFlush = 1;                      // K slices per TMEM accumulation (64 design rows)
+constexpr int kAcc = 4;                        // TMEM accumulators: the MMAs run ahead of the epilogue
 constexpr int kEpiWarps = 16;                  // four per TMEM lane quarter, 32 columns each
 constexpr int kGramThreads = 32 * (2 + kEpiWarps);
 constexpr size_t kGramSmem = (size_t)kStages * kStageBytes + 1024 + 256;
@@ -52,41 +58,100 @@ using tc::mma_bf16;
 using tc::mma_commit;
 using tc::sw128_desc;
 
+// two FP32 values in one 64-bit register
+__device__ __forceinline__ uint64_t pack2(uint32_t a, uint32_t b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ float part2(uint64_t v, int i) {
+  uint32_t a, b;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v));
+  return __uint_as_float(i ? b : a);
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// eight TMEM columns of the warp's lanes; the registers are valid after tmem_wait8
+__device__ __forceinline__ void tmem_ld8(uint32_t (&v)[8], uint32_t taddr) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait8(uint32_t (&v)[8]) {
+  // the registers are operands so that nothing that reads them moves above the wait
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])::"memory");
+}
+
 }  // namespace
 
 // Transpose rows [r0, r0 + rows) of X (row stride ldx, columns [c0, c0 + D)) into the K-major
 // bf16 planes hi/lo (D x Mp), scaling row r by sqrt(w[r]); design rows [rows, Mp) are zeroed.
-// grid.x: 32-row blocks of the chunk, grid.y: 32-column blocks.
+// grid.x: 64-row blocks of the chunk, grid.y: blocks of kSplitTiles tiles of 64 columns.
+//
+// A thread carries two rows of a column through shared memory as one float2 (row pair p at
+// [p][column], odd stride: no bank conflicts either way), so a warp reads 128 bytes of a row of X
+// and writes 128 bytes of a plane row; the next tile's loads are issued before this one's stores.
+constexpr int kSplitTiles = 4;
+
 template <typename T>
 __global__ void __launch_bounds__(256) k_split_bf16(const T* __restrict__ X, int ldx, int c0, int D,
                                                     const double* __restrict__ w, long long r0, long long rows,
                                                     long long Mp, __nv_bfloat16* __restrict__ hi,
                                                     __nv_bfloat16* __restrict__ lo) {
-  __shared__ float tile[32][33];
-  __shared__ float sw[32];
-  const long long rb = (long long)blockIdx.x * 32;
-  const int cb = blockIdx.y * 32;
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+  __shared__ float2 tile[32][65];
+  __shared__ float sw[64];
+  const long long rb = (long long)blockIdx.x * 64;
+  const int lane = threadIdx.x, wy = threadIdx.y;  // block (32, 8)
+  const int tid = wy * 32 + lane;
+  const int nrow = (int)min((long long)64, rows - rb);  // may be <= 0 in the zeroed rows
   // sqrt(w) and x' in FP32: the split keeps about 17 bits of x', and FP64 runs at 1/64 rate
-  if (tid < 32) sw[tid] = (rb + tid < rows) ? (float)sqrt(w[r0 + rb + tid]) : 0.f;
+  if (tid < 64) sw[tid] = tid < nrow ? (float)sqrt(w[r0 + rb + tid]) : 0.f;
   __syncthreads();
-  for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-    const long long r = rb + y;
-    const int c = cb + threadIdx.x;
-    float v = 0.f;
-    if (r < rows && c < D) v = (float)X[(r0 + r) * ldx + c0 + c] * sw[y];
-    tile[y][threadIdx.x] = v;
-  }
-  __syncthreads();
-  for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-    const int c = cb + y;
-    const long long r = rb + threadIdx.x;
-    if (c < D && r < Mp) {
-      const float v = tile[threadIdx.x][y];
-      const __nv_bfloat16 h = __float2bfloat16_rn(v);
-      hi[(size_t)c * Mp + r] = h;
-      lo[(size_t)c * Mp + r] = __float2bfloat16_rn(v - __bfloat162float(h));
+  const T* Xb = X + (r0 + rb) * ldx + c0;
+  // warp wy holds row pairs wy, wy + 8, ... and column halves 0, 1 of a tile
+  float2 v[4][2];
+  auto load = [&](int cb) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = 2 * (wy + 8 * i), c = cb + 32 * h + lane;
+        v[i][h].x = r < nrow && c < D ? (float)Xb[(long long)r * ldx + c] * sw[r] : 0.f;
+        v[i][h].y = r + 1 < nrow && c < D ? (float)Xb[(long long)(r + 1) * ldx + c] * sw[r + 1] : 0.f;
+      }
+  };
+  const int cbeg = blockIdx.y * (64 * kSplitTiles), cend = min(D, cbeg + 64 * kSplitTiles);
+  const bool in = rb + 2 * lane < Mp;  // Mp is even
+  load(cbeg);
+  for (int cb = cbeg; cb < cend; cb += 64) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) tile[wy + 8 * i][32 * h + lane] = v[i][h];
+    __syncthreads();
+    if (cb + 64 < cend) load(cb + 64);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int cl = wy + 8 * i, c = cb + cl;
+      if (c < cend && in) {
+        const float2 x = tile[lane][cl];
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x.x, x.y);
+        const size_t o = (size_t)c * Mp + rb + 2 * lane;
+        *reinterpret_cast<__nv_bfloat162*>(hi + o) = h;
+        *reinterpret_cast<__nv_bfloat162*>(lo + o) =
+            __floats2bfloat162_rn(x.x - __low2float(h), x.y - __high2float(h));
+      }
     }
+    __syncthreads();
   }
 }
 
@@ -95,7 +160,7 @@ __global__ void __launch_bounds__(256) k_split_bf16(const T* __restrict__ X, int
 //
 // The FP32 accumulator lives in TMEM for `flush` K slices only (kFlush = 1: 64 design rows), because
 // the tensor core rounds its FP32 accumulation toward zero (a bias that grows with the chain): the MMA issuer
-// alternates between two 128-column TMEM buffers, and the epilogue warps drain the idle buffer
+// cycles through kAcc 128-column TMEM buffers, and the epilogue warps drain the full ones
 // into compensated (Kahan) FP32 register sums, so the error of the whole split stays at the
 // level of one short FP32 accumulation.  Epilogue warp w reads TMEM lane quarter w % 4 and one
 // quarter (32 columns) of the tile.
@@ -107,9 +172,9 @@ __global__ void __launch_bounds__(kGramThreads, 1)
   unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = reinterpret_cast<uint64_t*>(tiles + kStages * kStageBytes);
   uint64_t* empty = full + kStages;
-  uint64_t* tfull = empty + kStages;  // [2] accumulator buffer ready for the epilogue
-  uint64_t* tempty = tfull + 2;       // [2] accumulator buffer drained
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+  uint64_t* tfull = empty + kStages;  // [kAcc] accumulator buffer ready for the epilogue
+  uint64_t* tempty = tfull + kAcc;    // [kAcc] accumulator buffer drained
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + kAcc);
 
   int t = blockIdx.x % ntile, ti = 0;
   const int split = blockIdx.x / ntile;
@@ -128,7 +193,7 @@ __global__ void __launch_bounds__(kGramThreads, 1)
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kAcc; ++b) {
       mbar_init(&tfull[b], 1);
       mbar_init(&tempty[b], kEpiWarps);
     }
@@ -136,7 +201,7 @@ __global__ void __launch_bounds__(kGramThreads, 1)
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(2 * kTM));
+                 "r"(kAcc * kTM));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -166,10 +231,10 @@ __global__ void __launch_bounds__(kGramThreads, 1)
     // the copies issued last may still be in flight: wait for them (bounded) before leaving
     for (int k = max(0, issued - kStages); k < issued; ++k) mbar_wait(&full[k % kStages], (k / kStages) & 1, wait_limit);
   } else if (warp == 1 && lane == 0) {
-    // MMA issuer: K-slice group g accumulates into TMEM buffer g & 1
+    // MMA issuer: K-slice group g accumulates into TMEM buffer g % kAcc
     for (int g = 0; g < ngrp && ok; ++g) {
-      const int b = g & 1;
-      if (g >= 2 && !mbar_wait(&tempty[b], ((g >> 1) - 1) & 1, wait_limit)) {
+      const int b = g % kAcc;
+      if (g >= kAcc && !mbar_wait(&tempty[b], ((g / kAcc) - 1) & 1, wait_limit)) {
         ok = false;
         break;
       }
@@ -200,44 +265,54 @@ __global__ void __launch_bounds__(kGramThreads, 1)
   } else if (warp >= 2) {
     // epilogue: Kahan sums of 32 columns of one TMEM lane quarter
     const int q = warp & 3, cq = (warp - 2) >> 2;
-    float sum[32], cmp[32];
+    uint64_t sum[16], cmp[16];  // column pairs
 #pragma unroll
-    for (int c = 0; c < 32; ++c) sum[c] = cmp[c] = 0.f;
-    bool got = true;
-    for (int g = 0; g < ngrp; ++g) {
-      const int b = g & 1;
-      if (!mbar_wait(&tfull[b], (g >> 1) & 1, wait_limit)) {
-        got = false;
-        break;
-      }
+    for (int c = 0; c < 16; ++c) sum[c] = cmp[c] = 0;
+    // Eight columns at a time, the next eight (of this or the next accumulator) on their way while
+    // these are added; an accumulator is given back as soon as its last columns are in registers.
+    const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cq * 32);
+    uint32_t v[2][8];
+    bool got = mbar_wait(&tfull[0], 0, wait_limit);
+    if (got) {
       asm volatile("tcgen05.fence::after_thread_sync;");
+      tmem_ld8(v[0], tbase);
+    }
+    for (int g = 0; g < ngrp && got; ++g) {
+      const uint32_t tb = tbase + (uint32_t)(g % kAcc * kTM);
 #pragma unroll
-      for (int h2 = 0; h2 < 4; ++h2) {
-        uint32_t v[8];
-        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * kTM + cq * 32 + h2 * 8);
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                     : "r"(taddr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      for (int h = 0; h < 4; ++h) {
+        tmem_wait8(v[h & 1]);
+        if (h < 3) {
+          tmem_ld8(v[(h + 1) & 1], tb + (h + 1) * 8);
+        } else {
+          asm volatile("tcgen05.fence::before_thread_sync;");
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&tempty[g % kAcc]);
+          if (g + 1 < ngrp) {
+            got = mbar_wait(&tfull[(g + 1) % kAcc], ((g + 1) / kAcc) & 1, wait_limit);
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            if (got) tmem_ld8(v[0], tbase + (uint32_t)((g + 1) % kAcc * kTM));
+          }
+        }
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const int e = h2 * 8 + c;
-          const float y = __uint_as_float(v[c]) - cmp[e];
-          const float tt = sum[e] + y;
-          cmp[e] = (tt - sum[e]) - y;
+        for (int c = 0; c < 4; ++c) {
+          const int e = h * 4 + c;
+          const uint64_t y = sub2(pack2(v[h & 1][2 * c], v[h & 1][2 * c + 1]), cmp[e]);
+          const uint64_t tt = add2(sum[e], y);
+          cmp[e] = sub2(sub2(tt, sum[e]), y);
           sum[e] = tt;
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;");
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(&tempty[b]);
     }
     if (got && part) {
       // this split's tile, added to G in split order by k_gram_tc_reduce
       double* pt = part + ((size_t)split * ntile + blockIdx.x % ntile) * (kTM * kTM) + (size_t)(q * 32 + lane) * kTM +
                    cq * 32;
 #pragma unroll
-      for (int c = 0; c < 32; ++c) pt[c] = (double)sum[c] - (double)cmp[c];
+      for (int c = 0; c < 16; ++c)
+        *reinterpret_cast<double2*>(pt + 2 * c) =
+            make_double2((double)part2(sum[c], 0) - (double)part2(cmp[c], 0),
+                         (double)part2(sum[c], 1) - (double)part2(cmp[c], 1));
     } else if (got) {
       // straight into G: with a single split the CTA is the only writer of these elements
       const int i = ti * kTM + q * 32 + lane;
@@ -245,7 +320,8 @@ __global__ void __launch_bounds__(kGramThreads, 1)
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
           const int j = tj * kTM + cq * 32 + c;
-          if (j < D && j >= i) atomicAdd(&G[(size_t)i * D + j], (double)sum[c] - (double)cmp[c]);
+          if (j < D && j >= i)
+            atomicAdd(&G[(size_t)i * D + j], (double)part2(sum[c >> 1], c & 1) - (double)part2(cmp[c >> 1], c & 1));
         }
       }
     } else if (lane == 0) {
@@ -257,7 +333,7 @@ __global__ void __launch_bounds__(kGramThreads, 1)
   __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kTM));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kAcc * kTM));
   }
 }
 
@@ -277,12 +353,27 @@ void gram_tc_test_timeout(int skip_loads, long long wait_limit) {
 size_t gram_tc_min_workspace(int D) { return (size_t)4 * D * kTK + 256; }
 
 namespace {
-// row splits of one chunk of nk 64-row slices: at least two waves of CTAs where the tile count
-// alone does not give them, every split non-empty
+// Row splits of one chunk of nk 64-row slices.  One CTA runs per SM, so the chunk takes
+// rounds(ns) = ceil(ntile ns / nsm) times the slices of a split plus a CTA's own cost (ring fill,
+// partial tile), about kSplitCost slices; ns makes that least among those whose partials fit
+// (gram_tc_max_splits).  1541 columns x 60,000 rows: 91 tiles, 5 splits fill 2.99 rounds; the 4 that
+// "two waves of CTAs" asks for filled 2.39 of 3.
+constexpr int kSplitCost = 8;
+int gram_tc_max_splits(int ntile, int nsm) { return std::max(1, (3 * nsm + ntile / 2) / ntile); }
 int gram_tc_splits(int nk, int ntile, int nsm, int* kps) {
-  const int ns = std::max(1, std::min(nk, (2 * nsm + ntile - 1) / ntile));
-  *kps = (nk + ns - 1) / ns;
-  return (nk + *kps - 1) / *kps;
+  const int most = std::min(nk, gram_tc_max_splits(ntile, nsm));
+  long long best = 0;
+  int ns = 1;
+  for (int s = 1; s <= most; ++s) {
+    const long long per = (nk + s - 1) / s, n = (nk + per - 1) / per;  // n splits, none empty
+    const long long t = ((long long)ntile * n + nsm - 1) / nsm * (per + kSplitCost);
+    if (s == 1 || t < best) {
+      best = t;
+      ns = (int)n;
+      *kps = (int)per;
+    }
+  }
+  return ns;
 }
 
 // G[i][j] += sum over the splits of their tile partials, in split order (upper triangle).
@@ -300,6 +391,7 @@ __global__ void k_gram_tc_reduce(const double* __restrict__ part, int nt, int nt
   const int i = ti * kTM + e / kTM, j = tj * kTM + e % kTM;
   if (i >= D || j >= D || j < i) return;
   double s = 0.0;
+#pragma unroll 16
   for (int sp = 0; sp < nsplit; ++sp) s += part[((size_t)sp * ntile + tile) * (kTM * kTM) + e];
   G[(size_t)i * D + j] += s;
 }
@@ -307,8 +399,8 @@ __global__ void k_gram_tc_reduce(const double* __restrict__ part, int nt, int nt
 
 size_t gram_tc_part_doubles(int D, int nsm) {
   const int nt = (D + kTM - 1) / kTM, ntile = nt * (nt + 1) / 2;
-  if (ntile >= 2 * nsm) return 0;  // one split per chunk: no partials
-  return (size_t)(2 * nsm + ntile) * kTM * kTM;
+  const int ns = gram_tc_max_splits(ntile, nsm);
+  return ns > 1 ? (size_t)ns * ntile * kTM * kTM : 0;  // one split per chunk: no partials
 }
 
 bool gram_tc_available() { return tc::encode_fn() != nullptr; }
@@ -337,7 +429,7 @@ cudaError_t launch_gram_tc(const T* X, int ldx, int c0, int D, const double* w, 
     const long long rows = std::min(chunk, M - r0);
     const long long Mp = (rows + 7) / 8 * 8;  // 16-byte plane row stride
     __nv_bfloat16* lo = hi + (size_t)D * Mp;
-    dim3 g1((unsigned)((Mp + 31) / 32), (unsigned)((D + 31) / 32));
+    dim3 g1((unsigned)((Mp + 63) / 64), (unsigned)((D + 64 * kSplitTiles - 1) / (64 * kSplitTiles)));
     k_split_bf16<T><<<g1, dim3(32, 8), 0, st>>>(X, ldx, c0, D, w, r0, rows, Mp, hi, lo);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
