@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <functional>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -14,6 +15,8 @@
 
 
 using namespace mld;
+
+static void rows_pool_trim(int dev);  // mld_gpu_gram_rows
 
 namespace {
 
@@ -157,6 +160,11 @@ cudaError_t ensure(mld_gpu_handle* h, int id, size_t bytes) {
   size_t want = std::max<size_t>(bytes, 256);
   want = want + want / 8;  // headroom for slowly growing batches
   cudaError_t e = cudaMalloc(&bf.p, want);
+  if (e == cudaErrorMemoryAllocation) {  // memory kept by mld_gpu_gram_rows may be what is missing
+    (void)cudaGetLastError();
+    rows_pool_trim(h->device);
+    e = cudaMalloc(&bf.p, want);
+  }
   if (e != cudaSuccess) return e;
   bf.cap = want;
   return cudaSuccess;
@@ -175,14 +183,31 @@ cudaError_t upload(mld_gpu_handle* h, int id, const V* src, size_t n) {
   return cudaMemcpyAsync(h->bufs[id].p, src, sizeof(V) * n, cudaMemcpyHostToDevice, h->st);
 }
 
-template <typename V>
-cudaError_t dev_alloc_copy(mld_gpu_handle* h, V** dst, const V* src, size_t n) {
-  cudaError_t e = cudaMalloc((void**)dst, sizeof(V) * std::max<size_t>(n, 1));
-  if (e != cudaSuccess) return e;
-  h->owned.push_back(*dst);
-  if (n) e = cudaMemcpy(*dst, src, sizeof(V) * n, cudaMemcpyHostToDevice);
-  return e;
-}
+// Device tables of a handle, laid out one after another and moved by one allocation and one copy
+// (31 tables: a copy each was half of the time of mld_gpu_create).
+struct TablePack {
+  std::vector<unsigned char> bytes;
+  std::vector<std::pair<void*, size_t>> slots;  // pointer to set, offset of its table
+  template <typename V>
+  cudaError_t put(const std::vector<V>& v, V** dst) {
+    const size_t off = (bytes.size() + 255) / 256 * 256;
+    bytes.resize(off + sizeof(V) * std::max<size_t>(v.size(), 1));
+    if (!v.empty()) std::memcpy(bytes.data() + off, v.data(), sizeof(V) * v.size());
+    slots.emplace_back(dst, off);
+    return cudaSuccess;
+  }
+  cudaError_t upload(mld_gpu_handle* h) {
+    unsigned char* base = nullptr;
+    cudaError_t e = cudaMalloc((void**)&base, bytes.size());
+    if (e != cudaSuccess) return e;
+    h->owned.push_back(base);
+    for (const auto& s : slots) {
+      void* q = base + s.second;
+      std::memcpy(s.first, &q, sizeof(q));
+    }
+    return cudaMemcpy(base, bytes.data(), bytes.size(), cudaMemcpyHostToDevice);
+  }
+};
 
 void recips(const double* cell, double* bg) {
   const double *a1 = cell, *a2 = cell + 3, *a3 = cell + 6;
@@ -1130,9 +1155,11 @@ int mld_gpu_create(const mld_gpu_config* cfg, mld_gpu_handle** out) {
   h->Dfull = h->DL + (h->quad ? h->KK * h->KK : 0);           // reference layout (dim_design_line)
   h->ldx = round_up4(h->D);
   // device tables
-  auto put = [h](const auto& vec, auto** dst) { return dev_alloc_copy(h, dst, vec.data(), vec.size()); };
+  TablePack pack;
+  auto put = [&pack](const auto& vec, auto** dst) { return pack.put(vec, dst); };
   e = fill_dev_tables(t, &h->dt, put);
   if (e == cudaSuccess) e = fill_deriv_tables(t, &h->dt, put);
+  if (e == cudaSuccess) e = pack.upload(h);
   if (e != cudaSuccess) {
     int code = cuda_fail(h, e, "table upload");
     mld_gpu_destroy(h);
@@ -1177,6 +1204,7 @@ void mld_gpu_destroy(mld_gpu_handle* h) {
   for (auto& e : h->tev)
     if (e) cudaEventDestroy(e);
   if (h->st) cudaStreamDestroy(h->st);
+  rows_pool_trim(h->device);
   delete h;
 }
 
@@ -1961,6 +1989,64 @@ int set_err(char* err, int err_len, int code, const std::string& msg) {
 }
 }  // namespace
 
+namespace {
+// Workspace of mld_gpu_gram_rows, which has no handle to keep it in: stream-ordered memory of a pool
+// of this library's own (any thread and stream may take from it), of which at most kRowsPoolKeep
+// stays mapped between calls; mld_gpu_destroy gives that back (rows_pool_trim).  Mapping and
+// unmapping the planes of 60,000 rows x 1541 columns on each call took 0.6 ms beside 1.2 ms of
+// kernels.
+constexpr size_t kRowsPoolKeep = size_t(512) << 20;
+constexpr int kRowsPoolDevices = 64;
+std::mutex g_rows_pool_mutex;
+cudaMemPool_t g_rows_pool[kRowsPoolDevices] = {};
+
+cudaError_t rows_pool(int dev, cudaMemPool_t* out) {
+  if (dev < 0 || dev >= kRowsPoolDevices) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(g_rows_pool_mutex);
+  if (!g_rows_pool[dev]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = cudaMemPoolCreate(&pool, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t keep = kRowsPoolKeep;
+    e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return e;
+    }
+    g_rows_pool[dev] = pool;
+  }
+  *out = g_rows_pool[dev];
+  return cudaSuccess;
+}
+
+struct RowsWorkspace {
+  void* p = nullptr;
+  cudaStream_t st = nullptr;
+  cudaError_t get(int dev, size_t bytes, cudaStream_t stream) {
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = rows_pool(dev, &pool);
+    st = stream;
+    return e == cudaSuccess ? cudaMallocFromPoolAsync(&p, bytes, pool, st) : e;
+  }
+  // after the last launch that uses it and before the stream is waited for: what exceeds
+  // kRowsPoolKeep is unmapped by that wait
+  void release() {
+    if (p) cudaFreeAsync(p, st);
+    p = nullptr;
+  }
+  ~RowsWorkspace() { release(); }
+};
+}  // namespace
+
+static void rows_pool_trim(int dev) {
+  std::lock_guard<std::mutex> lock(g_rows_pool_mutex);
+  if (dev >= 0 && dev < kRowsPoolDevices && g_rows_pool[dev]) cudaMemPoolTrimTo(g_rows_pool[dev], 0);
+}
+
 extern "C" int mld_gpu_gram_rows(int method, const void* X, int x_is_fp32, long long M, int D, int ldx,
                                  const double* w, const double* y, double* G, double* rhs, void* stream, char* err,
                                  int err_len) {
@@ -1972,83 +2058,72 @@ extern "C" int mld_gpu_gram_rows(int method, const void* X, int x_is_fp32, long 
   int dev = 0, nsm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  void* ws = nullptr;
-  double* hbuf = nullptr;
-  int* terr = nullptr;
-  double* part = nullptr;  // tensor-core split partials and right-hand-side partials
-  auto cleanup = [&]() {
-    if (ws) cudaFree(ws);
-    if (hbuf) cudaFree(hbuf);
-    if (terr) cudaFree(terr);
-    if (part) cudaFree(part);
+  if (e != cudaSuccess) return set_err(err, err_len, MLD_ERR_CUDA, std::string("device query: ") + cudaGetErrorString(e));
+  // one stream-ordered allocation, carved below
+  const size_t rows = (size_t)std::max<long long>(M, 1);
+  const bool plain = method == MLD_PRECISION_PLAIN_FP64;
+  size_t off_part = 0, off_vec = 0, off_err = 0, total = 0, wsb = 0, npart = 0;
+  auto carve = [&total](size_t bytes) {
+    const size_t o = total;
+    total += (bytes + 1023) / 1024 * 1024;
+    return o;
   };
-  auto cuda_err = [&](cudaError_t ce, const char* where) {
-    cleanup();
-    return set_err(err, err_len, ce == cudaErrorMemoryAllocation ? MLD_ERR_OOM : MLD_ERR_CUDA,
-                   std::string(where) + ": " + cudaGetErrorString(ce));
-  };
-  if (e != cudaSuccess) return cuda_err(e, "device query");
-  if (method == MLD_PRECISION_PLAIN_FP64) {
-    double* hv = rhs;
-    const double* yy = y;
-    if (!hv) {
-      e = cudaMalloc(&hbuf, sizeof(double) * (size_t)D + sizeof(double) * (size_t)std::max<long long>(M, 1));
-      if (e != cudaSuccess) return cuda_err(e, "cudaMalloc");
-      hv = hbuf;
-      double* yz = hbuf + D;
-      e = cudaMemsetAsync(yz, 0, sizeof(double) * (size_t)std::max<long long>(M, 1), st);
-      if (e != cudaSuccess) return cuda_err(e, "cudaMemsetAsync");
-      yy = yz;
-    }
-    e = cudaMalloc(&ws, sizeof(double) * gram_workspace_doubles(M, D));
-    if (e != cudaSuccess) return cuda_err(e, "workspace");
-    double* gws = static_cast<double*>(ws);
-    e = x_is_fp32 ? launch_gram<float>(static_cast<const float*>(X), ldx, w, yy, M, D, G, hv, st, gws)
-                  : launch_gram<double>(static_cast<const double*>(X), ldx, w, yy, M, D, G, hv, st, gws);
-    if (e != cudaSuccess) return cuda_err(e, "launch_gram");
+  if (plain) {
+    wsb = sizeof(double) * gram_workspace_doubles(M, D);
+    carve(wsb);
+    if (!rhs) off_vec = carve(sizeof(double) * ((size_t)D + rows));  // right-hand side, zero labels
   } else {
     if (!gram_tc_available())
       return set_err(err, err_len, MLD_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    const size_t need = (size_t)4 * D * (size_t)((std::max<long long>(M, 1) + 63) / 64 * 64) + 256;
-    const size_t wsb = std::max(gram_tc_min_workspace(D), std::min(need, kGramWorkspaceCap));
-    const size_t npart = gram_tc_part_doubles(D, nsm);
-    const size_t nrhs = rhs ? gram_workspace_doubles(M, D) : 0;
-    e = cudaMalloc(&ws, wsb);
-    if (e == cudaSuccess) e = cudaMalloc(&part, sizeof(double) * std::max<size_t>(std::max(npart, nrhs), 1));
-    if (e == cudaSuccess) e = cudaMalloc(&terr, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemsetAsync(terr, 0, sizeof(int), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(G, 0, sizeof(double) * (size_t)D * D, st);
-    if (e != cudaSuccess) return cuda_err(e, "workspace");
-    e = x_is_fp32 ? launch_gram_tc<float>(static_cast<const float*>(X), ldx, 0, D, w, M, G, ws, wsb, terr, nsm, st,
-                                          part, npart)
-                  : launch_gram_tc<double>(static_cast<const double*>(X), ldx, 0, D, w, M, G, ws, wsb, terr, nsm, st,
-                                           part, npart);
-    if (e == cudaSuccess) e = launch_symmetrize(G, D, st);
-    float2* sv = nullptr;
-    // the right-hand side reuses the partial buffer after the Gram (same stream)
-    if (e == cudaSuccess && rhs && x_is_fp32) {
-      e = cudaMalloc(&sv, sizeof(float2) * (size_t)std::max<long long>(M, 1));
-      if (e == cudaSuccess)
-        e = launch_rhs<float>(static_cast<const float*>(X), ldx, w, y, M, D, rhs, nsm, st, sv, part);
-    } else if (e == cudaSuccess && rhs) {
-      e = launch_rhs<double>(static_cast<const double*>(X), ldx, w, y, M, D, rhs, nsm, st, nullptr, part);
-    }
-    if (sv) {
-      cudaStreamSynchronize(st);
-      cudaFree(sv);
-    }
-    if (e != cudaSuccess) return cuda_err(e, "launch_gram_tc");
-    int herr = 0;
-    e = cudaMemcpyAsync(&herr, terr, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_err(e, "synchronize");
-    if (herr) {
-      cleanup();
-      return set_err(err, err_len, MLD_ERR_TIMEOUT, "tensor-core Gram: a pipeline wait timed out");
-    }
+    const size_t need = (size_t)4 * D * ((rows + 63) / 64 * 64) + 256;
+    wsb = std::max(gram_tc_min_workspace(D), std::min(need, kGramWorkspaceCap));
+    npart = gram_tc_part_doubles(D, nsm);
+    carve(wsb);
+    off_part = carve(sizeof(double) * std::max(npart, rhs ? gram_workspace_doubles(M, D) : 0));
+    if (rhs && x_is_fp32) off_vec = carve(sizeof(float2) * rows);
+    off_err = carve(sizeof(int));
   }
-  e = cudaStreamSynchronize(st);
-  cleanup();
-  if (e != cudaSuccess) return set_err(err, err_len, MLD_ERR_CUDA, cudaGetErrorString(e));
+  RowsWorkspace wsp;
+  e = wsp.get(dev, total, st);
+  if (e != cudaSuccess)
+    return set_err(err, err_len, e == cudaErrorMemoryAllocation ? MLD_ERR_OOM : MLD_ERR_CUDA,
+                   std::string("workspace: ") + cudaGetErrorString(e));
+  unsigned char* base = static_cast<unsigned char*>(wsp.p);
+  int herr = 0;
+  if (plain) {
+    double* hv = rhs;
+    const double* yy = y;
+    if (!rhs) {
+      hv = reinterpret_cast<double*>(base + off_vec);
+      e = cudaMemsetAsync(hv + D, 0, sizeof(double) * rows, st);
+      yy = hv + D;
+    }
+    double* gws = reinterpret_cast<double*>(base);
+    if (e == cudaSuccess)
+      e = x_is_fp32 ? launch_gram<float>(static_cast<const float*>(X), ldx, w, yy, M, D, G, hv, st, gws)
+                    : launch_gram<double>(static_cast<const double*>(X), ldx, w, yy, M, D, G, hv, st, gws);
+  } else {
+    double* part = reinterpret_cast<double*>(base + off_part);  // split partials, then those of the right-hand side
+    int* terr = reinterpret_cast<int*>(base + off_err);
+    e = cudaMemsetAsync(terr, 0, sizeof(int), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(G, 0, sizeof(double) * (size_t)D * D, st);
+    if (e == cudaSuccess)
+      e = x_is_fp32 ? launch_gram_tc<float>(static_cast<const float*>(X), ldx, 0, D, w, M, G, base, wsb, terr, nsm, st,
+                                            part, npart)
+                    : launch_gram_tc<double>(static_cast<const double*>(X), ldx, 0, D, w, M, G, base, wsb, terr, nsm,
+                                             st, part, npart);
+    if (e == cudaSuccess) e = launch_symmetrize(G, D, st);
+    if (e == cudaSuccess && rhs)
+      e = x_is_fp32 ? launch_rhs<float>(static_cast<const float*>(X), ldx, w, y, M, D, rhs, nsm, st,
+                                        reinterpret_cast<float2*>(base + off_vec), part)
+                    : launch_rhs<double>(static_cast<const double*>(X), ldx, w, y, M, D, rhs, nsm, st, nullptr, part);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, terr, sizeof(int), cudaMemcpyDeviceToHost, st);
+  }
+  wsp.release();
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = es;
+  if (e != cudaSuccess)
+    return set_err(err, err_len, MLD_ERR_CUDA, std::string("normal matrix: ") + cudaGetErrorString(e));
+  if (herr) return set_err(err, err_len, MLD_ERR_TIMEOUT, "tensor-core Gram: a pipeline wait timed out");
   return set_err(err, err_len, MLD_OK, "");
 }
