@@ -12,6 +12,7 @@
 // other half follows by conjugation and the sums over a full layer fold into 2*Re over the half
 // (plus the self-symmetric centre of even layers).
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdlib>
 #include <map>
@@ -22,9 +23,13 @@
 namespace mld {
 
 static double factorial(int n) {
-  double r = 1.0;
-  for (int i = 2; i <= n; ++i) r *= (double)i;
-  return r;
+  static const std::array<double, 171> table = [] {
+    std::array<double, 171> f{};
+    f[0] = 1.0;
+    for (int i = 1; i < (int)f.size(); ++i) f[i] = f[i - 1] * (double)i;
+    return f;
+  }();
+  return table[n];
 }
 
 // Clebsch-Gordan coefficient <j1 m1 j2 m2 | j m> in the Condon-Shortley phase convention, from
@@ -174,6 +179,9 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
     for (int b = 0; b < 3; ++b) {
       Block& B = bl[b];
       B.first = (int)t->zterms.size();
+      int cgm[2 * kMaxJ + 1];  // m + jO -> list, looked up once per block
+      std::fill(cgm, cgm + 2 * B.jO + 1, -1);
+      auto cgl = [&](int m) { return cgm[m + B.jO] >= 0 ? cgm[m + B.jO] : (cgm[m + B.jO] = cglist(B.jA, B.jB, B.jO, m)); };
       for (int m1 = -B.jO; m1 <= B.jO; m1 += 2)
         for (int m2 = -B.jO; m2 <= B.jO; m2 += 2) {
           int malo = std::max(-B.jA, m1 - B.jB), mahi = std::min(B.jA, m1 + B.jB);
@@ -188,8 +196,8 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
           z.s2 = (uint8_t)(B.jB + 1);
           z.i1 = (uint16_t)uidx(B.jA, malo, mblo);
           z.i2 = (uint16_t)uidx(B.jB, m1 - malo, m2 - mblo);
-          z.cg1 = (uint16_t)cglist(B.jA, B.jB, B.jO, m1);
-          z.cg2 = (uint16_t)cglist(B.jA, B.jB, B.jO, m2);
+          z.cg1 = (uint16_t)cgl(m1);
+          z.cg2 = (uint16_t)cgl(m2);
           z.snum = (uint8_t)B.snum;
           z.sden = (uint8_t)B.sden;
           t->cg_terms += nt;
@@ -258,21 +266,24 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
     struct Part { long long cost; LaneRec r; };
     // a job's records in four parts, each record to the least loaded one, longest first
     auto add_job = [](std::vector<Part>& recs, LaneJob job, std::vector<LaneRec>* out, std::vector<LaneJob>* jobs) {
-      std::stable_sort(recs.begin(), recs.end(), [](const Part& x, const Part& y) { return x.cost > y.cost; });
-      std::vector<LaneRec> part[4];
+      std::vector<const Part*> order;
+      order.reserve(recs.size());
+      for (const Part& p : recs) order.push_back(&p);
+      std::stable_sort(order.begin(), order.end(), [](const Part* x, const Part* y) { return x->cost > y->cost; });
+      std::vector<const LaneRec*> part[4];
       long long load[4] = {0, 0, 0, 0};
-      for (const Part& p : recs) {
+      for (const Part* p : order) {
         const int q = (int)(std::min_element(load, load + 4) - load);
-        load[q] += p.cost;
-        part[q].push_back(p.r);
+        load[q] += p->cost;
+        part[q].push_back(&p->r);
       }
       for (int q = 0; q < 4; ++q) {
         // records of equal shape one after the other: they run the same code
-        std::stable_sort(part[q].begin(), part[q].end(), [](const LaneRec& x, const LaneRec& y) {
-          return x.nj != y.nj ? x.nj > y.nj : (x.nb != y.nb ? x.nb > y.nb : x.na > y.na);
+        std::stable_sort(part[q].begin(), part[q].end(), [](const LaneRec* x, const LaneRec* y) {
+          return x->nj != y->nj ? x->nj > y->nj : (x->nb != y->nb ? x->nb > y->nb : x->na > y->na);
         });
         job.rec[q] = (int)out->size();
-        out->insert(out->end(), part[q].begin(), part[q].end());
+        for (const LaneRec* r : part[q]) out->push_back(*r);
       }
       job.rec[4] = (int)out->size();
       jobs->push_back(job);
@@ -293,7 +304,8 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
     t->gamp_off.push_back((int)t->gamp.size());
     std::map<std::tuple<int, int, int>, int> triple;
     for (int k = 0; k < t->K; ++k) triple[std::make_tuple(t->l1[k], t->l2[k], t->l[k])] = k;
-    std::map<std::pair<int, int>, std::vector<Part>> ypos;  // output position -> records
+    const int ML = 2 * J + 1;
+    std::vector<std::vector<Part>> ypos((size_t)ML * ML);  // output position (m1 + J, m2 + J) -> records
     struct BJob { long long cost; std::vector<Part> recs; LaneJob job; };
     std::vector<BJob> bjobs;
     for (auto& pr : outs) {
@@ -301,11 +313,13 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
       std::vector<int>& os = pr.second;
       std::sort(os.begin(), os.end(), [](int x, int y) { return x > y; });
       const int jm = os[0];
-      std::map<int, std::pair<int, int>> cgo;  // m -> offset, stride
+      std::vector<std::pair<int, int>> cgo(2 * jm + 1);  // m + jm -> offset, stride
+      int pb[kMaxJ + 1] = {0};                           // output layer -> pair block
+      for (int o : os) pb[o] = pblk.at(std::make_tuple(jA, jB, o));
       for (int m = -jm; m <= jm; m += 2) {
         int n = 0;
         while (n < (int)os.size() && os[n] >= std::abs(m)) ++n;
-        cgo[m] = {(int)t->cgv.size(), n};
+        cgo[m + jm] = {(int)t->cgv.size(), n};
         for (int ma = std::max(-jA, m - jB); ma <= std::min(jA, m + jB); ma += 2)
           for (int o = 0; o < n; ++o) t->cgv.push_back(cg_coefficient(jA, ma, jB, m - ma, os[o], m));
       }
@@ -325,20 +339,20 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
           r.s2 = (uint8_t)(jB + 1);
           r.i1 = (uint16_t)uidx(jA, malo, mblo);
           r.i2 = (uint16_t)uidx(jB, m1 - malo, m2 - mblo);
-          r.cg1 = (uint16_t)cgo[m1].first;
-          r.cg2 = (uint16_t)cgo[m2].first;
-          r.st1 = (uint8_t)cgo[m1].second;
-          r.st2 = (uint8_t)cgo[m2].second;
+          r.cg1 = (uint16_t)cgo[m1 + jm].first;
+          r.cg2 = (uint16_t)cgo[m2 + jm].first;
+          r.st1 = (uint8_t)cgo[m1 + jm].second;
+          r.st2 = (uint8_t)cgo[m2 + jm].second;
           LaneRec y = r, b = r;
           const int top = J - ((J ^ m1) & 1);  // highest layer with this position
           y.off = (uint8_t)((top - jm) / 2);
           for (int o : os)
-            if (o >= mu) y.out[y.nj++] = (uint16_t)pblk.at(std::make_tuple(jA, jB, o));
+            if (o >= mu) y.out[y.nj++] = (uint16_t)pb[o];
           b.w = (uint16_t)((m1 == 0 && m2 == 0) ? 1 : 2);
           for (int o : os)
             if (o >= mu && o >= jA) b.out[b.nj++] = (uint16_t)uidx(o, m1, m2);
           auto cost = [](const LaneRec& x) { return (long long)x.na * (x.nb * (4 + 2 * x.nj) + 2 * x.nj) + 16; };
-          ypos[{m1, m2}].push_back(Part{cost(y), y});
+          ypos[(size_t)(m1 + J) * ML + m2 + J].push_back(Part{cost(y), y});
           if (b.nj) {
             bj.recs.push_back(Part{cost(b), b});
             bj.cost += cost(b);
@@ -352,15 +366,15 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
     }
     std::stable_sort(bjobs.begin(), bjobs.end(), [](const BJob& x, const BJob& y) { return x.cost > y.cost; });
     for (BJob& b : bjobs) add_job(b.recs, b.job, &t->brecs, &t->bjobs);
-    std::vector<std::pair<long long, std::pair<int, int>>> yorder;
-    for (const auto& yp : ypos) {
+    std::vector<std::pair<long long, size_t>> yorder;
+    for (size_t i = 0; i < ypos.size(); ++i) {
       long long c = 0;
-      for (const Part& p : yp.second) c += p.cost;
-      yorder.push_back({-c, yp.first});
+      for (const Part& p : ypos[i]) c += p.cost;
+      if (c) yorder.push_back({-c, i});
     }
     std::sort(yorder.begin(), yorder.end());
     for (const auto& yo : yorder) {
-      const int m1 = yo.second.first, m2 = yo.second.second, mu = std::max(std::abs(m1), std::abs(m2));
+      const int m1 = (int)(yo.second / ML) - J, m2 = (int)(yo.second % ML) - J, mu = std::max(std::abs(m1), std::abs(m2));
       LaneJob job{};
       for (int o = J - ((J ^ m1) & 1); o >= mu; o -= 2) job.out[job.nout++] = (uint16_t)(t->hoff[o] + loc(o, m1, m2));
       add_job(ypos[yo.second], job, &t->yrecs, &t->yjobs);
