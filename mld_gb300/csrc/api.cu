@@ -126,7 +126,7 @@ struct mld_gpu_handle {
     B_GWS, B_TERR, B_PCG, B_POS32, B_YSCR, B_RINV, B_KZD, B_KZF, B_KWS, B_WSERVE, B_P32,
     B_EW, B_EBETA, B_EB, B_EOUT, B_KTC, B_SKW, B_ORDER, B_QCNT, B_SP, B_EPAIR, B_EATOM, B_GP,
     B_CNC, B_CELLOFF, B_CELLOF, B_CELLSTART, B_CELLATOMS, B_SORTTMP, B_NBR_U32, B_MVWS, B_GTCP, B_NBRTMP,
-    B_CHALF, B_EY,
+    B_CHALF, B_ZT, B_EY,
     B_COUNT
   };
   static_assert(B_COUNT <= 80, "buffer table too small");
@@ -352,14 +352,60 @@ int build_neighbours(mld_gpu_handle* h) {
 // workspace of the tensor-core kernel-row product (derivative-vector planes of one atom chunk)
 constexpr size_t kKrrTcWorkspaceCap = size_t(6) << 30;
 
-// global Y scratch of the descriptor kernel when its per-atom Y does not fit in shared memory
+// Route of B with dB.  More atoms than SMs: Z terms with atoms on lanes, Y rows, derivatives
+// (bispectrum_deriv.cu).  Up to an atom per SM, and for tables too large for it, the one kernel that
+// forms Z itself, a CTA per atom (bispectrum.cu): the tiles of lanes are then few and three launches go.
+// Design rows of one Fe structure at j_max 4, one kernel / three: 100 atoms FP64 0.69 / 1.00 ms, FP32
+// 309 / 349 us; 250 atoms 1.33 / 1.28 ms, 426 / 418 us; 1000 atoms FP64 3.38 / 3.12 ms; 23,000 FP32
+// atoms in 60 structures at j_max 2, FP64: 5.2 / 3.2 ms.
+constexpr size_t kZCap = size_t(2) << 30;  // Z terms and Y rows held at a time
+
 template <typename T>
-int y_scratch(mld_gpu_handle* h, void** p, size_t* bytes) {
-  *bytes = bso4_y_scratch_bytes(h->dt, h->nch, (int)sizeof(T), 2 * std::max(1, h->nsm));
-  *p = nullptr;
-  if (*bytes) {
-    CK(ensure(h, mld_gpu_handle::B_YSCR, *bytes));
-    *p = bp_<void>(h, mld_gpu_handle::B_YSCR);
+bool deriv_route(const mld_gpu_handle* h) {
+  // (a configuration is taken or refused whatever the batch)
+  return h->A > h->nsm && bso4_available(h->dt, h->nch, (int)sizeof(T)) && deriv_available(h->dt, h->nch, (int)sizeof(T));
+}
+
+// atoms of a pass of the derivative route: whole tiles within kZCap, passes of equal size
+template <typename T>
+int deriv_pass(const mld_gpu_handle* h, size_t* zbytes, size_t* ybytes) {
+  const int tile = lane_tile(h->dt, (int)sizeof(T)), A = std::max(1, h->A);
+  const size_t yper = (size_t)h->nch * h->dt.NYP * 2 * sizeof(T) * tile;
+  const size_t zper = (size_t)h->nch * h->dt.NZTP * 2 * sizeof(T) * tile;
+  const long long tiles = (A + tile - 1) / tile, most = std::max<long long>(1, (long long)(kZCap / (zper + yper)));
+  const long long passes = (tiles + most - 1) / most, n = (tiles + passes - 1) / passes;
+  *zbytes = (size_t)n * zper;
+  *ybytes = (size_t)n * yper;
+  return (int)std::min<long long>(n * tile, A);
+}
+
+// B of the staged batch into Bout and w_ch * dB into dB, with one launch shape
+template <typename T>
+int launch_rows_descriptors(mld_gpu_handle* h, T* Bout, T* dB, const Bso4Launch& shape, int* launches) {
+  const int* order = bp_<int>(h, mld_gpu_handle::B_ORDER);
+  int* counter = bp_<int>(h, mld_gpu_handle::B_QCNT);
+  if (!deriv_route<T>(h)) {
+    const size_t ysb = bso4_y_scratch_bytes(h->dt, h->nch, (int)sizeof(T), 2 * std::max(1, h->nsm));
+    void* ys = ysb ? bp_<void>(h, mld_gpu_handle::B_YSCR) : nullptr;
+    CK(launch_bso4<T>(h->dt, h->b, h->bp, Bout, dB, order, counter, h->st, ys, ysb, &shape));
+    *launches = 1;
+    return MLD_OK;
+  }
+  size_t zb = 0, yb = 0;
+  const int pass = deriv_pass<T>(h, &zb, &yb);
+  void* c = bp_<void>(h, mld_gpu_handle::B_CHALF);
+  void* z = bp_<void>(h, mld_gpu_handle::B_ZT);
+  void* y = bp_<void>(h, mld_gpu_handle::B_YSCR);
+  *launches = 0;
+  for (int a0 = 0; a0 < h->A; a0 += pass) {
+    const int n = std::min(pass, h->A - a0);
+    const int* q = order && shape.sorted_queue ? order + a0 : nullptr;
+    const int first = q ? 0 : a0;
+    CK(launch_c_half<T>(h->dt, h->b, h->bp, first, n, q, true, counter, c, h->st));
+    CK(launch_lane_z<T>(h->dt, h->nch, n, c, z, h->st));
+    CK(launch_y_rows<T>(h->dt, h->nch, n, z, y, h->st));
+    CK(launch_deriv<T>(h->dt, h->b, h->bp, first, n, q, counter, c, y, Bout, dB, shape, h->st));
+    *launches += 4;
   }
   return MLD_OK;
 }
@@ -372,15 +418,15 @@ int y_scratch(mld_gpu_handle* h, void** p, size_t* bytes) {
 constexpr int kTuneMinAtoms = 64;
 
 template <typename T>
-int tuned_launch(mld_gpu_handle* h, T* Bout, T* dB, void* ys, size_t ysb) {
+int tuned_launch(mld_gpu_handle* h, T* Bout, T* dB) {
   auto& tn = h->tune[0];
-  const int* order = bp_<int>(h, mld_gpu_handle::B_ORDER);
-  int* counter = bp_<int>(h, mld_gpu_handle::B_QCNT);
+  int launches = 0;
   // only the design-row stage of a fit is tuned: it is repeated on the same batch, while
   // evaluation batches (serving) and descriptor dumps change from call to call
   if (tn.done || h->A < kTuneMinAtoms * std::max(1, h->nsm)) {
-    CK(launch_bso4<T>(h->dt, h->b, h->bp, Bout, dB, order, counter, h->st, ys, ysb, &tn.best));
-    return MLD_OK;
+    const int rc = launch_rows_descriptors<T>(h, Bout, dB, tn.best, &launches);
+    nl(h, launches);
+    return rc;
   }
   tn.cand.clear();
   tn.ms.clear();
@@ -393,7 +439,9 @@ int tuned_launch(mld_gpu_handle* h, T* Bout, T* dB, void* ys, size_t ysb) {
   float best = 0.f;
   for (const Bso4Launch& c : tn.cand) {
     CK(cudaEventRecord(ev0, h->st));
-    CK(launch_bso4<T>(h->dt, h->b, h->bp, Bout, dB, order, counter, h->st, ys, ysb, &c));
+    const int rc = launch_rows_descriptors<T>(h, Bout, dB, c, &launches);
+    nl(h, launches);
+    if (rc) return rc;
     CK(cudaEventRecord(ev1, h->st));
     CK(cudaEventSynchronize(ev1));
     float ms = 0.f;
@@ -406,40 +454,41 @@ int tuned_launch(mld_gpu_handle* h, T* Bout, T* dB, void* ys, size_t ysb) {
   }
   cudaEventDestroy(ev0);
   cudaEventDestroy(ev1);
-  nl(h, (long long)tn.cand.size() - 1);
   tn.done = true;
   return MLD_OK;
 }
 
+// buffers of run_descriptors with derivatives
 template <typename T>
-int prepare_descriptors(mld_gpu_handle* h, void** ys, size_t* ysb) {
-  int rcy = y_scratch<T>(h, ys, ysb);
-  if (rcy) return rcy;
+int prepare_descriptors(mld_gpu_handle* h) {
+  size_t zb = 0, yb = 0;
+  if (deriv_route<T>(h)) {
+    const int pass = deriv_pass<T>(h, &zb, &yb);
+    CK(ensure(h, mld_gpu_handle::B_ZT, zb));
+    CK(ensure(h, mld_gpu_handle::B_CHALF, sizeof(T) * 2 * (size_t)pass * h->nch * h->dt.HU));
+  } else {
+    yb = bso4_y_scratch_bytes(h->dt, h->nch, (int)sizeof(T), 2 * std::max(1, h->nsm));
+  }
+  if (yb) CK(ensure(h, mld_gpu_handle::B_YSCR, yb));
   CK(ensure(h, mld_gpu_handle::B_DBOUT, sizeof(T) * std::max<size_t>((size_t)h->b.P * 3 * h->KK, 1)));
   return MLD_OK;
 }
 
-// B of the staged batch into Bout and, if asked, w_ch * dB into B_DBOUT: both from the descriptor
-// kernel, B alone from the atoms-on-lanes sums
+// B of the staged batch into Bout and, if asked, w_ch * dB into B_DBOUT
 template <typename T>
 int run_descriptors(mld_gpu_handle* h, bool want_dB, T* Bout) {
   if (!want_dB) {
     CK(ensure(h, mld_gpu_handle::B_CHALF, sizeof(T) * 2 * (size_t)std::max(1, h->A) * h->nch * h->dt.HU));
     void* c = bp_<void>(h, mld_gpu_handle::B_CHALF);
-    CK(launch_c_half<T>(h->dt, h->b, h->bp, 0, h->A, bp_<int>(h, mld_gpu_handle::B_ORDER),
+    CK(launch_c_half<T>(h->dt, h->b, h->bp, 0, h->A, bp_<int>(h, mld_gpu_handle::B_ORDER), false,
                         bp_<int>(h, mld_gpu_handle::B_QCNT), c, h->st));
     CK(launch_lane_descriptors<T>(h->dt, h->b, h->bp, 0, h->A, c, Bout, h->st));
     nl(h, 2);
     return MLD_OK;
   }
-  void* ys = nullptr;
-  size_t ysb = 0;
-  int rcy = prepare_descriptors<T>(h, &ys, &ysb);
+  int rcy = prepare_descriptors<T>(h);
   if (rcy) return rcy;
-  int rc = tuned_launch<T>(h, Bout, bp_<T>(h, mld_gpu_handle::B_DBOUT), ys, ysb);
-  if (rc) return rc;
-  nl(h, 1);
-  return MLD_OK;
+  return tuned_launch<T>(h, Bout, bp_<T>(h, mld_gpu_handle::B_DBOUT));
 }
 
 template <typename T>
@@ -495,9 +544,7 @@ int run_rows(mld_gpu_handle* h, const RowLayout& L, bool with_labels, T** Xout) 
     CK(ensure(h, mld_gpu_handle::B_SP, sizeof(T) * nB * 6));
     if (h->quad) CK(ensure(h, mld_gpu_handle::B_HQ, sizeof(T) * (size_t)std::max(1, h->A) * 6 * h->KK));
     T* Bq = bp_<T>(h, mld_gpu_handle::B_BOUT);
-    void* ys = nullptr;
-    size_t ysb = 0;
-    int rcd = prepare_descriptors<T>(h, &ys, &ysb);
+    int rcd = prepare_descriptors<T>(h);
     if (rcd) return rcd;
     T* dBq = bp_<T>(h, mld_gpu_handle::B_DBOUT);
     // the stage of this batch: descriptor kernel, reverse pairs, linear (and quadratic) rows
@@ -1750,7 +1797,7 @@ static int eval_run(mld_gpu_handle* h, double* out) {
     CK(ensure(h, mld_gpu_handle::B_EY, sizeof(T) * nc));
     ev.c = bp_<void>(h, mld_gpu_handle::B_CHALF);
     ev.y = bp_<void>(h, mld_gpu_handle::B_EY);
-    CK(launch_c_half<T>(h->dt, h->b, h->bp, 0, h->A, order, counter, bp_<void>(h, mld_gpu_handle::B_CHALF), h->st));
+    CK(launch_c_half<T>(h->dt, h->b, h->bp, 0, h->A, order, false, counter, bp_<void>(h, mld_gpu_handle::B_CHALF), h->st));
     CK(launch_lane_y<T>(h->dt, h->b, h->bp, 0, h->A, ev.c, static_cast<const T*>(wext), bp_<void>(h, mld_gpu_handle::B_EY), h->st));
     nl(h, 2);
   }

@@ -441,6 +441,13 @@ static bool y_shared(const DevTables& tb, int nch, int eb) {
   return ss <= (size_t)max_optin_smem() && per_sm / (ss + 1024) >= per_sm / (sg + 1024);
 }
 
+bool bso4_available(const DevTables& tb, int nch, int eb) {
+  for (int g1 : {4, 6, 8, 16})
+    for (bool y : {true, false})
+      if (smem_plan(tb, nch, eb, y, g1).total <= (size_t)max_optin_smem()) return true;
+  return false;
+}
+
 size_t bso4_y_scratch_bytes(const DevTables& tb, int nch, int eb, int max_ctas, bool only_if_required) {
   const bool fits = smem_plan(tb, nch, eb, true).total <= (size_t)max_optin_smem();
   if (fits && (only_if_required || y_shared(tb, nch, eb))) return 0;

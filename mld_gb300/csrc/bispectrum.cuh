@@ -239,9 +239,27 @@ inline unsigned long long chain_order(int J) {
 // of consecutive neighbours use distinct banks.
 __host__ __device__ constexpr int u_stride(int HU) { return HU | 1; }
 
+// Chain d of a neighbour with zp, xp at zx into its row u of the store.
+template <typename T>
+__device__ __forceinline__ void u_chain_of(int d, const T* zx, int J, cx<T>* u) {
+  const cx<T> z = {zx[0], zx[1]}, x = {zx[2], zx[3]};
+  switch (d) {
+    case 1: u_chain<1>(z, x, J, u); break;
+    case 2: u_chain<2>(z, x, J, u); break;
+    case 3: u_chain<3>(z, x, J, u); break;
+    case 4: u_chain<4>(z, x, J, u); break;
+    case 5: u_chain<5>(z, x, J, u); break;
+    case 6: u_chain<6>(z, x, J, u); break;
+    case 7: u_chain<7>(z, x, J, u); break;
+    case 8: u_chain<8>(z, x, J, u); break;
+    case 9: u_chain<9>(z, x, J, u); break;
+    default: u_chain<10>(z, x, J, u); break;
+  }
+}
+
 // U (all half layers but the first, which is 1) of neighbours 0..count-1 into Us[n][u_stride]; zx(n)
-// points to the neighbour's zp and xp.  Work items (chain, 32 neighbours) go to the warps longest first, every second
-// round in reverse.  No synchronisation inside.
+// points to the neighbour's zp and xp.  Work items (chain, 32 neighbours) go to the warps longest
+// first, every second round in reverse.  No synchronisation inside.
 template <typename T, class Zx>
 __device__ __forceinline__ void u_store(cx<T>* Us, int HS, int count, int J, unsigned long long order, int warp,
                                         int lane, Zx zx) {
@@ -250,23 +268,7 @@ __device__ __forceinline__ void u_store(cx<T>* Us, int HS, int count, int J, uns
     const int it = (r & 1) ? (r + 1) * kNW - 1 - warp : r * kNW + warp;
     if (it >= nitem) continue;
     const int ci = it / nb, n = (it - ci * nb) * 32 + lane;
-    if (n < count) {
-      const T* g = zx(n);
-      const cx<T> z = {g[0], g[1]}, x = {g[2], g[3]};
-      cx<T>* u = Us + (size_t)n * HS;
-      switch ((int)(order >> (4 * ci)) & 15) {
-        case 1: u_chain<1>(z, x, J, u); break;
-        case 2: u_chain<2>(z, x, J, u); break;
-        case 3: u_chain<3>(z, x, J, u); break;
-        case 4: u_chain<4>(z, x, J, u); break;
-        case 5: u_chain<5>(z, x, J, u); break;
-        case 6: u_chain<6>(z, x, J, u); break;
-        case 7: u_chain<7>(z, x, J, u); break;
-        case 8: u_chain<8>(z, x, J, u); break;
-        case 9: u_chain<9>(z, x, J, u); break;
-        default: u_chain<10>(z, x, J, u); break;
-      }
-    }
+    if (n < count) u_chain_of<T>((int)(order >> (4 * ci)) & 15, zx(n), J, Us + (size_t)n * HS);
     __syncwarp();
   }
 }

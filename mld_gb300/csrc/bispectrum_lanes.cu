@@ -11,9 +11,10 @@
 // (17.3k products and 163k FMAs per channel at j_max 4, against 42.6k and 255k of the term lists).
 // In FP32 a lane holds two atoms, whose values are packed for the two-wide FP32 instructions: half
 // the instructions per atom for the products, and half the loads of coefficients and records.
-// The sums that the terms feed stay in registers: no term is stored.
+// For B and y the sums that the terms feed stay in registers: no term is stored.
 //   B  a job is an operand pair: B_k = sum_m w Re(conj(c^l(m)) Z_l(m)) of its triples (l >= jA)
 //   y  a job is an output position (m1, m2): y_jO(m1,m2) = sum over the pairs of gamma Z_jO(m1,m2)
+//   z  the terms themselves, [tile of atoms][channel][term][atom], for the derivative kernel
 // Four warps share a job (its records in four fixed parts of equal work, added in order), so the
 // sums do not depend on the number of atoms or on how the jobs fall on the CTAs.
 //
@@ -84,6 +85,15 @@ struct alignas(16) vcx {
 };
 
 
+// the atoms' values one after the other, (re, im) each
+__device__ __forceinline__ vcx<F2> interleave(vcx<F2> v) {
+  float re[2], im[2];
+  unpack(v.x, re);
+  unpack(v.y, im);
+  return {pack(re[0], im[0]), pack(re[1], im[1])};
+}
+__device__ __forceinline__ vcx<double> interleave(vcx<double> v) { return v; }
+
 template <typename T>
 struct LaneArgs {
   DevTables tb;
@@ -97,7 +107,10 @@ struct LaneArgs {
   int A, nch;
   T* B;                 // A x nch*K
   cx<T>* y;             // A x nch x HU
+  cx<T>* z;             // tiles x nch x NZTP x atoms of a tile
 };
+
+enum { kLaneB = 0, kLaneY = 1, kLaneZ = 2 };
 
 // lanes that hold atoms: 32, or 16 where their c does not fit in shared memory; a padded row per entry
 // (16-byte values) so that the transposing stores spread over the banks
@@ -193,12 +206,18 @@ __device__ __forceinline__ int out_of(uint4 z1, int o) {
 }
 
 // A record into the job's sums.  y: acc[off + o] += gamma[out_o] Z_o; B: acc[o].x += w Re(conj(c[out_o]) Z_o)
-template <int NJ, bool kY, typename V>
+// z: the terms to zo[out_o][atoms of the tile]
+template <int NJ, int kMode, typename V>
 __device__ __forceinline__ void lane_record(uint4 z0, uint4 z1, const vcx<V>* __restrict__ cl, int ST,
-                                            const V* __restrict__ cg, const V* __restrict__ gam, vcx<V>* acc) {
+                                            const V* __restrict__ cg, const V* __restrict__ gam, vcx<V>* acc,
+                                            vcx<V>* zo, int zst, bool store) {
   vcx<V> zs[NJ];
   lane_terms<NJ, V>(z0, cl, ST, cg, zs);
-  if constexpr (kY) {
+  if constexpr (kMode == kLaneZ) {
+    if (store)
+#pragma unroll
+      for (int o = 0; o < NJ; ++o) zo[(size_t)out_of(z1, o) * zst] = interleave(zs[o]);
+  } else if constexpr (kMode == kLaneY) {
     const int off = z0.w >> 24;
     if (off == 0) {  // pairs that reach the highest layers: most of the work
 #pragma unroll
@@ -230,7 +249,7 @@ __device__ __forceinline__ void lane_record(uint4 z0, uint4 z1, const vcx<V>* __
   }
 }
 
-template <typename T, bool kY>
+template <typename T, int kMode>
 __global__ void __launch_bounds__(LaneVec<T>::warps * 32, 1) k_lanes(LaneArgs<T> args, int lanes, bool cg_shared) {
   using V = typename LaneVec<T>::type;
   constexpr int kPer = LaneVec<T>::atoms, kLaneWarps = LaneVec<T>::warps;
@@ -263,13 +282,16 @@ __global__ void __launch_bounds__(LaneVec<T>::warps * 32, 1) k_lanes(LaneArgs<T>
     for (int e = tid; e < tb.NCGV; e += nth) scg[e] = cg[e];
     cg = scg;
   }
-  if constexpr (kY) {
+  if constexpr (kMode == kLaneY) {
     for (int b = tid; b < tb.NBLKP; b += nth) sg[b] = vdup(args.gamma[ch * tb.NBLKP + b], V{});
   }
   __syncthreads();
   const int al = lane < lanes ? lane : lane - lanes;  // (16 lanes: both halves of the warp hold the same atoms)
   const vcx<V>* cl = sc + al;
   const int group = warp >> 2, q = warp & 3, no = tb.J / 2 + 1;
+  vcx<V>* zo = nullptr;
+  if constexpr (kMode == kLaneZ)
+    zo = reinterpret_cast<vcx<V>*>(args.z) + ((size_t)blockIdx.x * args.nch + ch) * tb.NZTP * lanes + al;
   vcx<V>* mypart = part + (size_t)group * 4 * no * 32;
   for (int job = blockIdx.y * kGroups + group; job < args.njobs; job += gridDim.y * kGroups) {
     const LaneJob& jb = args.jobs[job];
@@ -293,14 +315,15 @@ __global__ void __launch_bounds__(LaneVec<T>::warps * 32, 1) k_lanes(LaneArgs<T>
         n1 = __ldg(rp + 2 * (size_t)(r + 1) + 1);
       }
       switch ((z0.w >> 16) & 0xFF) {
-        case 1: lane_record<1, kY, V>(z0, z1, cl, ST, cg, sg, acc); break;
-        case 2: lane_record<2, kY, V>(z0, z1, cl, ST, cg, sg, acc); break;
-        case 3: lane_record<3, kY, V>(z0, z1, cl, ST, cg, sg, acc); break;
-        case 4: lane_record<4, kY, V>(z0, z1, cl, ST, cg, sg, acc); break;
-        case 5: lane_record<5, kY, V>(z0, z1, cl, ST, cg, sg, acc); break;
-        default: lane_record<6, kY, V>(z0, z1, cl, ST, cg, sg, acc); break;
+        case 1: lane_record<1, kMode, V>(z0, z1, cl, ST, cg, sg, acc, zo, lanes, lane < lanes); break;
+        case 2: lane_record<2, kMode, V>(z0, z1, cl, ST, cg, sg, acc, zo, lanes, lane < lanes); break;
+        case 3: lane_record<3, kMode, V>(z0, z1, cl, ST, cg, sg, acc, zo, lanes, lane < lanes); break;
+        case 4: lane_record<4, kMode, V>(z0, z1, cl, ST, cg, sg, acc, zo, lanes, lane < lanes); break;
+        case 5: lane_record<5, kMode, V>(z0, z1, cl, ST, cg, sg, acc, zo, lanes, lane < lanes); break;
+        default: lane_record<6, kMode, V>(z0, z1, cl, ST, cg, sg, acc, zo, lanes, lane < lanes); break;
       }
     }
+    if constexpr (kMode == kLaneZ) continue;
 #pragma unroll
     for (int o = 0; o < kMaxZOut; ++o)
       if (o < no) mypart[(q * no + o) * 32 + lane] = acc[o];
@@ -320,7 +343,7 @@ __global__ void __launch_bounds__(LaneVec<T>::warps * 32, 1) k_lanes(LaneArgs<T>
         const int a = al * kPer + k;
         if (lane < lanes && a < na) {
           const size_t row = (size_t)(a0 + a) * args.nch + ch;
-          if constexpr (kY) args.y[row * HU + jb.out[o]] = {re[k], im[k]};
+          if constexpr (kMode == kLaneY) args.y[row * HU + jb.out[o]] = {re[k], im[k]};
           else args.B[row * K + jb.out[o]] = args.nbr_off[a0 + a + 1] == args.nbr_off[a0 + a] ? T(0) : re[k];
         }
       }
@@ -339,7 +362,7 @@ struct CArgs {
   T rin[kMaxTypes * kMaxTypes];
   int nch;
   const int* order;
-  int first;
+  int first, by_position;
   int* counter;
   unsigned long long chains;
   int slots;
@@ -408,7 +431,7 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_c_half(CAr
       c_sum<T>(chalf, Us, HS, fcw, shd, count, nch, HU, base == 0, base + args.slots >= nn, tid);
       if (base + args.slots < nn) __syncthreads();
     }
-    cx<T>* out = args.c + (size_t)(atom - args.first) * nch * HU;
+    cx<T>* out = args.c + (size_t)(args.by_position ? qi : atom - args.first) * nch * HU;
     // a thread writes the entries it has summed itself
     for (int e = tid; e < nch * HU; e += nth)
       out[e] = nn > 0 ? chalf[e] : cx<T>{shd[e % HU] ? T(1) : T(0), T(0)};
@@ -432,17 +455,24 @@ cudaError_t sm_count(int* nsm) {
   return e;
 }
 
-template <typename T, bool kY>
+// lanes per tile and where the coefficients go; the shared memory of a CTA (0: does not fit)
+size_t lane_shape(const DevTables& tb, int eb, int* lanes, bool* cg_shared) {
+  *lanes = 32;
+  *cg_shared = eb == 4;
+  auto bytes = [&]() { return lane_plan(tb, eb, *lanes, *cg_shared).total; };
+  if (bytes() > (size_t)optin()) *lanes = 16;
+  if (bytes() > (size_t)optin()) *cg_shared = false;
+  return bytes() <= (size_t)optin() ? bytes() : 0;
+}
+
+template <typename T, int kMode>
 cudaError_t launch_lanes(LaneArgs<T>& a, cudaStream_t st) {
   if (a.A <= 0 || a.njobs <= 0) return cudaSuccess;
-  int lanes = 32;
-  bool cg_shared = sizeof(T) == 4;
-  auto bytes = [&]() { return lane_plan(a.tb, (int)sizeof(T), lanes, cg_shared).total; };
-  if (bytes() > (size_t)optin()) lanes = 16;
-  if (bytes() > (size_t)optin()) cg_shared = false;
-  const size_t smem = bytes();
-  if (smem > (size_t)optin()) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaFuncSetAttribute(k_lanes<T, kY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int lanes;
+  bool cg_shared;
+  const size_t smem = lane_shape(a.tb, (int)sizeof(T), &lanes, &cg_shared);
+  if (!smem) return cudaErrorInvalidConfiguration;
+  cudaError_t e = cudaFuncSetAttribute(k_lanes<T, kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int nsm = 0;
   if ((e = sm_count(&nsm)) != cudaSuccess) return e;
@@ -463,7 +493,7 @@ cudaError_t launch_lanes(LaneArgs<T>& a, cudaStream_t st) {
       slices = s;
     }
   }
-  k_lanes<T, kY><<<dim3(tiles, slices, a.nch), LaneVec<T>::warps * 32, smem, st>>>(a, lanes, cg_shared);
+  k_lanes<T, kMode><<<dim3(tiles, slices, a.nch), LaneVec<T>::warps * 32, smem, st>>>(a, lanes, cg_shared);
   return cudaGetLastError();
 }
 
@@ -471,7 +501,7 @@ cudaError_t launch_lanes(LaneArgs<T>& a, cudaStream_t st) {
 
 template <typename T>
 cudaError_t launch_c_half(const DevTables& tb, const DevBatch& b, const BsoParams& p, int first, int count,
-                          const int* order, int* counter, void* c, cudaStream_t st) {
+                          const int* order, bool by_position, int* counter, void* c, cudaStream_t st) {
   if (count <= 0) return cudaSuccess;
   CArgs<T> a{};
   a.tb = tb;
@@ -483,6 +513,7 @@ cudaError_t launch_c_half(const DevTables& tb, const DevBatch& b, const BsoParam
   a.nch = p.nch;
   a.order = order;
   a.first = first;
+  a.by_position = by_position ? 1 : 0;
   a.counter = counter;
   a.chains = chain_order(tb.J);
   a.c = static_cast<cx<T>*>(c);
@@ -532,7 +563,7 @@ cudaError_t launch_lane_descriptors(const DevTables& tb, const DevBatch& b, cons
   a.jobs = tb.bjobs;
   a.njobs = tb.NBJ;
   a.B = B + (size_t)first * p.nch * tb.K;
-  return launch_lanes<T, false>(a, st);
+  return launch_lanes<T, kLaneB>(a, st);
 }
 
 template <typename T>
@@ -544,13 +575,38 @@ cudaError_t launch_lane_y(const DevTables& tb, const DevBatch& b, const BsoParam
   a.njobs = tb.NYJ;
   a.gamma = gamma;
   a.y = static_cast<cx<T>*>(y);
-  return launch_lanes<T, true>(a, st);
+  return launch_lanes<T, kLaneY>(a, st);
 }
 
+int lane_tile(const DevTables& tb, int eb) {
+  int lanes;
+  bool cg_shared;
+  if (!lane_shape(tb, eb, &lanes, &cg_shared)) return 0;
+  return lanes * (eb == 4 ? LaneVec<float>::atoms : LaneVec<double>::atoms);
+}
+
+template <typename T>
+cudaError_t launch_lane_z(const DevTables& tb, int nch, int count, const void* c, void* z, cudaStream_t st) {
+  LaneArgs<T> a{};
+  a.tb = tb;
+  if constexpr (sizeof(T) == 8) a.cg = tb.cgv64;
+  else a.cg = tb.cgv32x2;
+  a.c = static_cast<const cx<T>*>(c);
+  a.A = count;
+  a.nch = nch;
+  a.recs = tb.zrecs;
+  a.jobs = tb.yjobs;
+  a.njobs = tb.NYJ;
+  a.z = static_cast<cx<T>*>(z);
+  return launch_lanes<T, kLaneZ>(a, st);
+}
+
+template cudaError_t launch_lane_z<double>(const DevTables&, int, int, const void*, void*, cudaStream_t);
+template cudaError_t launch_lane_z<float>(const DevTables&, int, int, const void*, void*, cudaStream_t);
 template cudaError_t launch_c_half<double>(const DevTables&, const DevBatch&, const BsoParams&, int, int, const int*,
-                                           int*, void*, cudaStream_t);
+                                           bool, int*, void*, cudaStream_t);
 template cudaError_t launch_c_half<float>(const DevTables&, const DevBatch&, const BsoParams&, int, int, const int*,
-                                          int*, void*, cudaStream_t);
+                                          bool, int*, void*, cudaStream_t);
 template cudaError_t launch_lane_descriptors<double>(const DevTables&, const DevBatch&, const BsoParams&, int, int,
                                                      const void*, double*, cudaStream_t);
 template cudaError_t launch_lane_descriptors<float>(const DevTables&, const DevBatch&, const BsoParams&, int, int,

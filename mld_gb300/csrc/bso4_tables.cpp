@@ -254,6 +254,7 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
     t->gam_off.push_back((int)t->gam.size());
   }
 
+  std::map<std::tuple<int, int, int>, int> pairz;  // pair block -> its first term
   // atoms-on-lanes sums: operand pairs in descending order (exchanging the operands of a block changes
   // the sign of both its CG factors alike), all output layers of a pair from one set of products
   {
@@ -297,6 +298,15 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
         gam[ins.first->second].push_back(GammaItem{(uint16_t)k, (uint8_t)B.snum, (uint8_t)B.sden});
       }
     t->nblk_pair = (int)gam.size();
+    // the terms of the pair blocks, block by block
+    std::vector<int> pz(pblk.size());
+    for (const auto& b : pblk) pz[b.second] = std::get<2>(b.first);
+    for (int& z : pz) {
+      const int n = H(z);
+      z = t->nztp;
+      t->nztp += n;
+    }
+    for (const auto& b : pblk) pairz[b.first] = pz[b.second];
     for (const auto& v : gam) {
       t->gamp_off.push_back((int)t->gamp.size());
       t->gamp.insert(t->gamp.end(), v.begin(), v.end());
@@ -377,7 +387,14 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
       const int m1 = (int)(yo.second / ML) - J, m2 = (int)(yo.second % ML) - J, mu = std::max(std::abs(m1), std::abs(m2));
       LaneJob job{};
       for (int o = J - ((J ^ m1) & 1); o >= mu; o -= 2) job.out[job.nout++] = (uint16_t)(t->hoff[o] + loc(o, m1, m2));
+      const size_t first = t->yrecs.size();
       add_job(ypos[yo.second], job, &t->yrecs, &t->yjobs);
+      for (size_t i = first; i < t->yrecs.size(); ++i) {
+        LaneRec z = t->yrecs[i];
+        for (int o = 0; o < z.nj; ++o)
+          z.out[o] = (uint16_t)(pz[z.out[o]] + loc(J - ((J ^ m1) & 1) - 2 * (z.off + o), m1, m2));
+        t->zrecs.push_back(z);
+      }
     }
   }
 
@@ -470,6 +487,13 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
           ++rs.nterm;
         }
       t->rowsrc.push_back(rs);
+      if (k >= 0) {
+        int n = 0;
+        for (const Block& B : kblocks[k])
+          if (B.jO == j)
+            rs.z[n++] = (uint16_t)pairz.at(std::make_tuple(std::max(B.jA, B.jB), std::min(B.jA, B.jB), B.jO));
+      }
+      t->rowsrc2.push_back(rs);
     }
 
   // folded slots; the kernel's slot entries; the ZA entries of every triple for B

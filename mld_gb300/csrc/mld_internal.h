@@ -184,10 +184,12 @@ struct Bso4Tables {
   // atoms-on-lanes sums: CG coefficients of a pair by (m, first index, jO descending), the records and
   // jobs of B (a job per operand pair) and y (a job per output position), heaviest jobs first
   std::vector<double> cgv;
-  std::vector<LaneRec> brecs, yrecs;
+  std::vector<LaneRec> brecs, yrecs, zrecs;  // zrecs: yrecs with the terms' places in place of their blocks
+  int nztp = 0;                   // terms of the pair blocks, block by block (rowsrc2)
   std::vector<LaneJob> bjobs, yjobs;
   std::vector<TripleZ> trz;       // the ZA block and layer of each triple
   std::vector<RowSource> rowsrc;  // the blocks of every contraction row, indexed as rowk
+  std::vector<RowSource> rowsrc2; // the same on the terms of the pair blocks
   std::vector<int8_t> half_diag;  // half entries on the diagonal p == q (get the +1 of c)
   long long cg_terms = 0;       // CG products evaluated per channel (half outputs)
   long long cg_terms_full = 0;  // CG products of the unfolded contraction (reference count)
@@ -210,13 +212,15 @@ struct DevTables {
   int NBLK = 0;
   int blk_off[kMaxJ + 2] = {0};
   int zoff[kMaxJ + 1] = {0};
-  int NCGV = 0, NBJ = 0, NYJ = 0, NBLKP = 0;
+  int NCGV = 0, NBJ = 0, NYJ = 0, NBLKP = 0, NZTP = 0;
   double* cgv64 = nullptr;        // NCGV
   float2* cgv32x2 = nullptr;      // every coefficient twice
   LaneRec* brecs = nullptr;
   LaneJob* bjobs = nullptr;       // NBJ
   LaneRec* yrecs = nullptr;       // (fill_deriv_tables)
   LaneJob* yjobs = nullptr;       // NYJ
+  LaneRec* zrecs = nullptr;
+  RowSource* rowsrc2 = nullptr;
   TripleZ* trz = nullptr;         // K
   RowSource* rowsrc = nullptr;    // NROWS
   int hoff[kMaxJ + 2] = {0};
@@ -317,6 +321,9 @@ cudaError_t fill_deriv_tables(const Bso4Tables& t, DevTables* d, Put put) {
   d->NYJ = (int)t.yjobs.size();
   if (e == cudaSuccess) e = put(t.yrecs, &d->yrecs);
   if (e == cudaSuccess) e = put(t.yjobs, &d->yjobs);
+  d->NZTP = t.nztp;
+  if (e == cudaSuccess) e = put(t.zrecs, &d->zrecs);
+  if (e == cudaSuccess) e = put(t.rowsrc2, &d->rowsrc2);
   return e;
 }
 
@@ -399,11 +406,21 @@ cudaError_t launch_sort_lists(const DevBatch& b, cudaStream_t st);
 // does not fit in shared memory, and preferred (unless only_if_required) when it would cost a
 // resident CTA per SM; 0 otherwise.
 size_t bso4_y_scratch_bytes(const DevTables& tb, int nch, int eb, int max_ctas, bool only_if_required = false);
-// c (count x nch x HU complex of T) of atoms first .. first + count - 1; with `order` (all atoms, in
-// that order) first = 0.  counter: one int of device memory, reset by the launch.
+// whether the kernel's shared memory fits at all (FP64 at j_max 5 does not)
+bool bso4_available(const DevTables& tb, int nch, int eb);
+// Launch shape of the descriptor kernel, chosen per handle by the autotuner (api.cu); every
+// shape gives bitwise the same results.
+struct Bso4Launch {
+  int col_tile = 4;      // columns per register tile of the dB contraction: 2 or 4
+  int ctas_per_sm = 0;   // persistent CTAs per SM (0: as many as fit)
+  int sorted_queue = 1;  // atoms longest first (1) or in index order (0)
+};
+// c (count x nch x HU complex of T) of atoms first .. first + count - 1, or of order[0 .. count - 1]
+// (first = 0).  Rows by atom (atom - first) or by position in the queue.  counter: one int of device
+// memory, reset by the launch.
 template <typename T>
 cudaError_t launch_c_half(const DevTables& tb, const DevBatch& b, const BsoParams& p, int first, int count,
-                          const int* order, int* counter, void* c, cudaStream_t st);
+                          const int* order, bool by_position, int* counter, void* c, cudaStream_t st);
 // B (whole-batch array) of the same atoms from their c.
 template <typename T>
 cudaError_t launch_lane_descriptors(const DevTables& tb, const DevBatch& b, const BsoParams& p, int first, int count,
@@ -412,6 +429,22 @@ cudaError_t launch_lane_descriptors(const DevTables& tb, const DevBatch& b, cons
 template <typename T>
 cudaError_t launch_lane_y(const DevTables& tb, const DevBatch& b, const BsoParams& p, int first, int count,
                           const void* c, const T* gamma, void* y, cudaStream_t st);
+
+// Y rows of `count` rows of Z terms, [position][nch][NYP], and from them and c (by position) B and
+// w_ch * dB (whole-batch arrays) of atoms first .. first + count - 1, or of order[0 .. count - 1]
+// (bispectrum_deriv.cu).
+template <typename T>
+cudaError_t launch_y_rows(const DevTables& tb, int nch, int count, const void* z, void* y, cudaStream_t st);
+template <typename T>
+cudaError_t launch_deriv(const DevTables& tb, const DevBatch& b, const BsoParams& p, int first, int count,
+                         const int* order, int* counter, const void* c, const void* y, T* Bout, T* dBout,
+                         const Bso4Launch& shape, cudaStream_t st);
+bool deriv_available(const DevTables& tb, int nch, int eb);
+// Z terms of `count` rows of c, [tile][nch][NZTP][atoms of a tile] complex of T; lane_tile: atoms of a
+// tile (0: the tables do not fit).
+int lane_tile(const DevTables& tb, int eb);
+template <typename T>
+cudaError_t launch_lane_z(const DevTables& tb, int nch, int count, const void* c, void* z, cudaStream_t st);
 
 // Evaluation with fitted weights (bispectrum_eval.cu): per-pair forces and per-atom stress of
 // dE/dB_a (beta_a = w_lin for the linear model; w_lin + (W + W^T) B_a for the quadratic one),
@@ -427,13 +460,6 @@ struct DevEval {
   double* Eatom = nullptr;       // A: energy of each atom (written for the linear model)
 };
 
-// Launch shape of the descriptor kernel, chosen per handle by the autotuner (api.cu); every
-// shape gives bitwise the same results.
-struct Bso4Launch {
-  int col_tile = 4;      // columns per register tile of the dB contraction: 2 or 4
-  int ctas_per_sm = 0;   // persistent CTAs per SM (0: as many as fit)
-  int sorted_queue = 1;  // atoms longest first (1) or in index order (0)
-};
 // Descriptor kernel (bispectrum.cu): B (A x nch*K) and w_ch * dB (P x 3 x nch*K) of the batch.  Atoms are taken in `order` (null: index order) through `counter` (one int
 // of device memory, reset by the launch).
 template <typename T>

@@ -305,10 +305,10 @@ extern "C" int mld_gpu_descriptors_noalloc(const mld_gpu_config* cfg, int nat, c
   for (int a0 = 0; a0 < nat; a0 += chunk) {
     const int na = std::min(chunk, nat - a0);
     if (mixed) {
-      CKN(launch_c_half<float>(dt, b, prm, a0, na, nullptr, qcount, c, st));
+      CKN(launch_c_half<float>(dt, b, prm, a0, na, nullptr, false, qcount, c, st));
       CKN(launch_lane_descriptors<float>(dt, b, prm, a0, na, c, bstage, st));
     } else {
-      CKN(launch_c_half<double>(dt, b, prm, a0, na, nullptr, qcount, c, st));
+      CKN(launch_c_half<double>(dt, b, prm, a0, na, nullptr, false, qcount, c, st));
       CKN(launch_lane_descriptors<double>(dt, b, prm, a0, na, c, B, st));
     }
   }
