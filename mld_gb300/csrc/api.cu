@@ -1777,19 +1777,41 @@ static int eval_run(mld_gpu_handle* h, double* out) {
   ev.Satom = ev.Eatom + std::max(1, h->A);
   ev.w0 = h->ew0;
   if (h->quad) {
-    // B of every atom; its weights and energy; then the evaluation kernel
+    // c and Z terms of every atom, B from them; its weights and energy; then the evaluation kernel on
+    // the same terms, which are formed again where one pass (kZCap) does not hold them all
     const size_t na = (size_t)std::max(1, h->A);
+    size_t zb = 0, yb = 0;
+    const int pass = deriv_pass<T>(h, &zb, &yb);
     CK(ensure(h, mld_gpu_handle::B_EB, sizeof(T) * na * KK));
-    CK(ensure(h, mld_gpu_handle::B_EBETA, sizeof(T) * na * h->nch * h->dt.NBLK));
+    CK(ensure(h, mld_gpu_handle::B_EBETA, sizeof(T) * na * h->nch * h->dt.NBLKP));
+    CK(ensure(h, mld_gpu_handle::B_CHALF, sizeof(T) * 2 * na * h->nch * h->dt.HU));
+    CK(ensure(h, mld_gpu_handle::B_ZT, zb));
     T* B = bp_<T>(h, mld_gpu_handle::B_EB);
     T* gamma = bp_<T>(h, mld_gpu_handle::B_EBETA);
-    int rc = run_descriptors<T>(h, false, B);
-    if (rc) return rc;
+    T* c = bp_<T>(h, mld_gpu_handle::B_CHALF);
+    const size_t crow = 2 * (size_t)h->nch * h->dt.HU;
+    ev.z = bp_<void>(h, mld_gpu_handle::B_ZT);
+    ev.gamma = gamma;
+    CK(launch_c_half<T>(h->dt, h->b, h->bp, 0, h->A, order, true, counter, c, h->st));
+    nl(h, 1);
+    for (int a0 = 0; a0 < h->A; a0 += pass) {
+      const int n = std::min(pass, h->A - a0);
+      CK(launch_lane_z<T>(h->dt, h->nch, n, c + crow * a0, bp_<void>(h, mld_gpu_handle::B_ZT), h->st));
+      CK(launch_z_descriptors<T>(h->dt, h->b, h->bp, order + a0, n, c + crow * a0, ev.z, B, h->st));
+      nl(h, 2);
+    }
     CK(launch_eval_gamma<T>(h->dt, B, h->A, h->nch, wlin, wsym, static_cast<const float2*>(wext), h->ew0, gamma, ev.Eatom,
                             h->st));
-    ev.c = bp_<void>(h, mld_gpu_handle::B_CHALF);  // left there by the pass for B
-    ev.gamma = gamma;
     nl(h, 1);
+    for (int a0 = 0; a0 < h->A; a0 += pass) {
+      const int n = std::min(pass, h->A - a0);
+      if (pass < h->A) {
+        CK(launch_lane_z<T>(h->dt, h->nch, n, c + crow * a0, bp_<void>(h, mld_gpu_handle::B_ZT), h->st));
+        nl(h, 1);
+      }
+      CK(launch_bso4_eval<T>(h->dt, h->b, h->bp, ev, order + a0, n, counter, h->st));
+      nl(h, 1);
+    }
   } else {
     // c and y of every atom
     const size_t nc = (size_t)std::max(1, h->A) * h->nch * h->dt.HU * 2;
@@ -1799,12 +1821,12 @@ static int eval_run(mld_gpu_handle* h, double* out) {
     ev.y = bp_<void>(h, mld_gpu_handle::B_EY);
     CK(launch_c_half<T>(h->dt, h->b, h->bp, 0, h->A, order, false, counter, bp_<void>(h, mld_gpu_handle::B_CHALF), h->st));
     CK(launch_lane_y<T>(h->dt, h->b, h->bp, 0, h->A, ev.c, static_cast<const T*>(wext), bp_<void>(h, mld_gpu_handle::B_EY), h->st));
-    nl(h, 2);
+    CK(launch_bso4_eval<T>(h->dt, h->b, h->bp, ev, order, h->A, counter, h->st));
+    nl(h, 3);
   }
-  CK(launch_bso4_eval<T>(h->dt, h->b, h->bp, ev, order, counter, h->st));
   CK(launch_reverse_pairs(h->b, bp_<int>(h, mld_gpu_handle::B_REV), h->st));
   CK(launch_eval_gather<T>(h->b, h->bp, bp_<int>(h, mld_gpu_handle::B_REV), ev, E, F, S, h->st));
-  nl(h, 4);
+  nl(h, 3);
   return MLD_OK;
 }
 

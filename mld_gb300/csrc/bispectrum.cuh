@@ -127,6 +127,14 @@ __device__ __forceinline__ void nbr_geometry(T x0, T x1, T x2, T rinv, T rcut, T
   g[kGeoKap + 2] = dk * e[1];
 }
 
+// one complex value from global to shared memory, asynchronously (cp.async)
+__device__ __forceinline__ void copy_async(cx<float>* dst, const cx<float>* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async(cx<double>* dst, const cx<double>* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
 // ---- U by column chains --------------------------------------------------------------------
 // Column q of layer j follows from column q - 1 of layer j - 1 alone (angular_functions.f90:108-272),
 // so the layers fall into independent chains: chain d starts with column 0 (q = -j) of layer d, a

@@ -20,8 +20,9 @@
 // product per term, a third of a dB contraction), and its dot products are taken with the generators
 // applied to U.  Neighbours are lanes and four half entries a step of a warp, so the Z terms are
 // broadcast, a neighbour's block weights are read without conflicts, and its y never leaves the
-// registers.  The Z terms of the atom are formed in the CTA, a channel at a time.  Bound: FP32
-// arithmetic and shared memory of the Z terms.
+// registers.  The Z terms come from the atoms-on-lanes kernel, a channel at a time and asynchronously:
+// formed here, they took 37 % of the kernel.  Bound: shared memory reads and FP32 arithmetic of the
+// neighbours' y.
 //
 // Persistent CTAs take atoms from a queue.  Every sum has a fixed order that does not depend on the
 // batch.
@@ -70,7 +71,6 @@ template <typename T>
 struct EvalArgs {
   DevTables tb;
   const GenEntry<T>* gen;
-  const T* cg;
   PairSource<T> src;
   const int* atom_struct;
   const int* small;
@@ -83,11 +83,12 @@ struct EvalArgs {
   int* counter;
   unsigned long long chains;
   int slots;  // neighbours of the U store
+  int tile;   // atoms of a tile of Z terms
   DevEval<T> ev;
 };
 
 struct EvalPlan {
-  size_t hoff, exp, quads, cfull, gamma, cg, tbuf, yb, yt, geo, red, grow, next, U, total;
+  size_t hoff, quads, gamma, tbuf, yb, yt, geo, red, grow, next, U, total;
 };
 
 __host__ __device__ inline size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
@@ -97,18 +98,15 @@ __host__ __device__ inline EvalPlan eval_plan(const DevTables& tb, int nch, int 
   EvalPlan s;
   size_t o = 0;
   s.hoff = o;  o = up16(o + sizeof(int) * (kMaxJ + 2));
-  s.exp = o;   o = up16(o + sizeof(int16_t) * tb.NU);
   s.quads = o; o = up16(o + sizeof(int16_t) * (tb.HU / 4 + kMaxJ + 2));
-  s.cfull = o; o = up16(o + (quad ? cxb * nch * tb.NU : 0));
-  s.gamma = o; o = up16(o + (quad ? (size_t)eb * nch * tb.NBLK : 0));
-  s.cg = o;    o = up16(o + (quad ? (size_t)eb * tb.NCG : 0));
+  s.gamma = o; o = up16(o + (quad ? (size_t)eb * nch * tb.NBLKP : 0));
   // Z terms of a channel, y, and the block weights of a batch, which the generators' y_b and the
   // sums over the warps follow in the same place
-  s.tbuf = o;  o = up16(o + (quad ? cxb * tb.NZT : 0));
+  s.tbuf = o;  o = up16(o + (quad ? cxb * tb.NZTP : 0));
   s.yt = o;    o = up16(o + (quad ? cxb * nch * tb.HU : 0));
   size_t w = cxb * 4 * nch * tb.HU;
   if (quad) {
-    const size_t g = (size_t)eb * tb.NBLK * kGrow, r = (size_t)eb * kNW * 2 * kBatch * 4;
+    const size_t g = (size_t)eb * tb.NBLKP * kGrow, r = (size_t)eb * kNW * 2 * kBatch * 4;
     w = w > g ? w : g;
     w = w > r ? w : r;
   }
@@ -130,17 +128,14 @@ template <typename T, bool kQuad>
 __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(EvalArgs<T> args, int A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DevTables& tb = args.tb;
-  const int J = tb.J, NU = tb.NU, HU = tb.HU;
-  const int nch = args.nch, nchG = nch * tb.NBLK;
+  const int J = tb.J, HU = tb.HU;
+  const int nch = args.nch, nchG = nch * tb.NBLKP;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int nth = kNW * 32;
   const EvalPlan sp = eval_plan(tb, nch, (int)sizeof(T), args.slots, kQuad);
   int* shoff = reinterpret_cast<int*>(smem_raw + sp.hoff);
-  int16_t* sexp = reinterpret_cast<int16_t*>(smem_raw + sp.exp);
   int16_t* squad = reinterpret_cast<int16_t*>(smem_raw + sp.quads);  // four half entries: layer << 8 | quad
-  cx<T>* cfull = reinterpret_cast<cx<T>*>(smem_raw + sp.cfull);
   T* sgam = reinterpret_cast<T*>(smem_raw + sp.gamma);
-  T* scg = reinterpret_cast<T*>(smem_raw + sp.cg);
   cx<T>* tbuf = reinterpret_cast<cx<T>*>(smem_raw + sp.tbuf);
   cx<T>* yb = reinterpret_cast<cx<T>*>(smem_raw + sp.yb);  // [nch][HU][4]
   cx<T>* yt = reinterpret_cast<cx<T>*>(smem_raw + sp.yt);
@@ -154,16 +149,12 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
 
   // tables, once per CTA
   for (int e = tid; e < kMaxJ + 2; e += nth) shoff[e] = tb.hoff[e];
-  for (int e = tid; e < NU; e += nth) sexp[e] = tb.expand[e];
   int nquad = 0;
   for (int j = J; j >= 0; --j) {  // heaviest layers first
     const int c = (tb.hoff[j + 1] - tb.hoff[j] + 3) >> 2;
     for (int q = tid; q < c; q += nth) squad[nquad + q] = (int16_t)((j << 8) | q);
     nquad += c;
   }
-  if constexpr (kQuad)
-    for (int e = tid; e < tb.NCG; e += nth) scg[e] = args.cg[e];
-  const int zr0 = kQuad ? tb.zitem_off[warp] : 0, zr1 = kQuad ? tb.zitem_off[warp + 1] : 0;
 
   int nxt = 0;
   if (tid == 0) nxt = atomicAdd(args.counter, 1);
@@ -200,13 +191,15 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
       continue;
     }
     const cx<T>* ysrc = kQuad ? yt : static_cast<const cx<T>*>(args.ev.y) + (size_t)atom * nch * HU;
-    const cx<T>* csrc = static_cast<const cx<T>*>(args.ev.c) + (size_t)atom * nch * HU;
-    if constexpr (kQuad) {
-      for (int e = tid; e < nch * NU; e += nth) {
-        const int ch = e / NU, f = e - ch * NU;
-        cfull[e] = fetch(csrc + ch * HU, sexp[f]);
-      }
-    } else if (warp == kNW - 1) {  // energy of the atom, w0 + w_lin . B = w0 + c . y / 3
+    // quadratic model: the atom's Z terms of a channel into tbuf, a copy per term
+    auto load_z = [&](int ch) {
+      const cx<T>* z = static_cast<const cx<T>*>(args.ev.z) +
+                       ((size_t)(qi / args.tile) * nch + ch) * tb.NZTP * args.tile + qi % args.tile;
+      for (int t = tid; t < tb.NZTP; t += nth) copy_async(tbuf + t, z + (size_t)t * args.tile);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (!kQuad && warp == kNW - 1) {  // energy of the atom, w0 + w_lin . B = w0 + c . y / 3
+      const cx<T>* csrc = static_cast<const cx<T>*>(args.ev.c) + (size_t)atom * nch * HU;
       ExactSum<T> s;
       for (int e = lane; e < nch * HU; e += 32) {
         const T w = args.gen[e % HU].w;
@@ -243,6 +236,7 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
     const int srow = tid / 6, scomp = tid - srow * 6;  // quadratic model: its neighbours and component
     for (int ps = npass - 1; ps >= 0; --ps) {
       const int base = ps * args.slots, count = min(args.slots, nn - base);
+      if constexpr (kQuad) load_z(0);  // (arrives beside the geometry and U)
       load_pass(base, count);
       if constexpr (kQuad) {
         // stress sums S_b of the pass's neighbours with their own beta, channel by channel
@@ -250,7 +244,7 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
 #pragma unroll
         for (int i = 0; i < 8; ++i) st[i >> 2][i & 3] = T(0);
         for (int ch = 0; ch < nch; ++ch) {
-          z_rounds<T>(tb.zitems, zr0, zr1, cfull + ch * NU, scg, tbuf, lane);
+          asm volatile("cp.async.wait_group 0;" ::: "memory");
           __syncthreads();
           if (ps == npass - 1) {
             // y of the atom: the blocks of each layer with its own weights, in order
@@ -258,9 +252,9 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
               int j = 0;
               while (shoff[j + 1] <= h) ++j;
               const int H = shoff[j + 1] - shoff[j];
-              const cx<T>* z = tbuf + tb.zoff[j] + (h - shoff[j]);
-              const T* g = sgam + ch * tb.NBLK + tb.blk_off[j];
-              const int nb = tb.blk_off[j + 1] - tb.blk_off[j];
+              const cx<T>* z = tbuf + tb.zoffp[j] + (h - shoff[j]);
+              const T* g = sgam + ch * tb.NBLKP + tb.blkp_off[j];
+              const int nb = tb.blkp_off[j + 1] - tb.blkp_off[j];
               cx<T> v = {T(0), T(0)};
 #pragma unroll 4
               for (int r = 0; r < nb; ++r) {
@@ -277,8 +271,8 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
             if (b0 >= count) continue;
             for (int n = warp; n < min(kBatch, count - b0); n += kNW) {
               const int nb = reinterpret_cast<const int*>(geo(b0 + n) + kGeoIdx)[0];
-              const T* src = args.ev.gamma + (size_t)nb * nchG + ch * tb.NBLK;
-              for (int r = lane; r < tb.NBLK; r += 32) grow[r * kGrow + n] = src[r];
+              const T* src = args.ev.gamma + (size_t)nb * nchG + ch * tb.NBLKP;
+              for (int r = lane; r < tb.NBLKP; r += 32) grow[r * kGrow + n] = src[r];
             }
             __syncthreads();
             const int n = min(b0 + lane, count - 1);
@@ -286,9 +280,9 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
             const T wn = args.chw[ch * args.src.ntypes + pair_type<T>(geo(n))];
             for (int it = warp; it < nquad; it += kNW) {
               const int q = squad[it], j = q >> 8, e0 = (q & 255) * 4;
-              const int H = shoff[j + 1] - shoff[j], nb = tb.blk_off[j + 1] - tb.blk_off[j];
-              const cx<T>* z = tbuf + tb.zoff[j] + e0;
-              const T* g = grow + tb.blk_off[j] * kGrow + (n - b0);
+              const int H = shoff[j + 1] - shoff[j], nb = tb.blkp_off[j + 1] - tb.blkp_off[j];
+              const cx<T>* z = tbuf + tb.zoffp[j] + e0;
+              const T* g = grow + tb.blkp_off[j] * kGrow + (n - b0);
               cx<T> y[4];
 #pragma unroll
               for (int i = 0; i < 4; ++i) y[i] = {T(0), T(0)};
@@ -325,6 +319,7 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
             }
             __syncthreads();  // the weights have been read (and, after the last batch, the Z terms)
           }
+          if (ch + 1 < nch) load_z(ch + 1);
         }
         // sums over the warps, in order; then the stress of (neighbour, component)
 #pragma unroll
@@ -453,18 +448,16 @@ int max_optin() {
 
 template <typename T>
 cudaError_t launch_bso4_eval(const DevTables& tb, const DevBatch& b, const BsoParams& p, const DevEval<T>& ev,
-                             const int* order, int* counter, cudaStream_t st) {
-  if (b.A == 0) return cudaSuccess;
-  if (!counter || !ev.pair || !ev.Satom || !tb.gen32 || !ev.c || (!ev.gamma && !ev.y)) return cudaErrorInvalidValue;
+                             const int* order, int count, int* counter, cudaStream_t st) {
+  if (count <= 0) return cudaSuccess;
   const bool quad = ev.gamma != nullptr;
+  if (!counter || !ev.pair || !ev.Satom || !tb.gen32 || (quad ? !ev.z : !ev.c || !ev.y)) return cudaErrorInvalidValue;
   EvalArgs<T> a{};
   a.tb = tb;
   if constexpr (sizeof(T) == 8) {
     a.gen = reinterpret_cast<const GenEntry<T>*>(tb.gen64);
-    a.cg = reinterpret_cast<const T*>(tb.cg64);
   } else {
     a.gen = reinterpret_cast<const GenEntry<T>*>(tb.gen32);
-    a.cg = reinterpret_cast<const T*>(tb.cg32);
   }
   a.src = {b.types, b.nbr_idx, b.nbr_u, sizeof(T) == 4 ? b.nbr_u32 : nullptr, (T)p.rcut, (T)p.inv_r0,
            (T)p.rin_width, p.ntypes, p.has_rin};
@@ -479,6 +472,8 @@ cudaError_t launch_bso4_eval(const DevTables& tb, const DevBatch& b, const BsoPa
   a.counter = counter;
   a.chains = chain_order(tb.J);
   a.ev = ev;
+  a.tile = quad ? lane_tile(tb, (int)sizeof(T)) : 1;
+  if (!a.tile) return cudaErrorInvalidConfiguration;
   // the largest U store (up to 64 neighbours) that keeps the CTAs per SM of a 32-neighbour one (at
   // most two: registers); it depends on the configuration only, not on the batch
   const size_t per_sm = 228 * 1024;
@@ -501,16 +496,16 @@ cudaError_t launch_bso4_eval(const DevTables& tb, const DevBatch& b, const BsoPa
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kNW * 32, smem);
   if (e != cudaSuccess) return e;
   if (occ < 1) return cudaErrorInvalidConfiguration;
-  const long long grid = std::min<long long>((long long)b.A, (long long)nsm * occ);
+  const long long grid = std::min<long long>(count, (long long)nsm * occ);
   e = cudaMemsetAsync(counter, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
-  kern<<<(unsigned)grid, kNW * 32, smem, st>>>(a, b.A);
+  kern<<<(unsigned)grid, kNW * 32, smem, st>>>(a, count);
   return cudaGetLastError();
 }
 
 template cudaError_t launch_bso4_eval<double>(const DevTables&, const DevBatch&, const BsoParams&,
-                                              const DevEval<double>&, const int*, int*, cudaStream_t);
+                                              const DevEval<double>&, const int*, int, int*, cudaStream_t);
 template cudaError_t launch_bso4_eval<float>(const DevTables&, const DevBatch&, const BsoParams&,
-                                             const DevEval<float>&, const int*, int*, cudaStream_t);
+                                             const DevEval<float>&, const int*, int, int*, cudaStream_t);
 
 }  // namespace mld

@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 #include <type_traits>
 
 #include "bispectrum.cuh"
@@ -438,6 +439,72 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_c_half(CAr
   }
 }
 
+// ---- B from stored terms -----------------------------------------------------------------------
+// A CTA per tile of atoms and channel, c of the tile turned around in shared memory, a warp per triple
+// with lanes on atoms: B_k = sum w Re(conj(c^l) Z_A).  Bound: reading a third of the terms once.
+constexpr int kZBWarps = 16;
+
+template <typename T>
+struct ZBArgs {
+  DevTables tb;
+  const cx<T>* c;
+  const cx<T>* z;
+  const int* order;
+  const int* nbr_off;
+  T* B;
+  int count, nch, tile;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kZBWarps * 32) k_z_descriptors(ZBArgs<T> a) {
+  constexpr int kPer = 16 / (2 * (int)sizeof(T));  // atoms of a lane
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const DevTables& tb = a.tb;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, HU = tb.HU, K = tb.K;
+  const int CS = a.tile + kPer;  // row of an entry, 16 bytes longer: fewer bank conflicts while turning
+  cx<T>* sc = reinterpret_cast<cx<T>*>(smem_raw);
+  T* sb = reinterpret_cast<T*>(sc + (size_t)HU * CS);  // [atom][K + 1]
+  const int t0 = blockIdx.x / a.nch, ch = blockIdx.x - t0 * a.nch;
+  const int na = min(a.tile, a.count - t0 * a.tile), lanes = a.tile / kPer;
+  for (int i = warp; i < a.tile; i += kZBWarps) {
+    const cx<T>* src = a.c + ((size_t)(t0 * a.tile + min(i, na - 1)) * a.nch + ch) * HU;
+    for (int e = lane; e < HU; e += 32) copy_async(sc + (size_t)e * CS + i, src + e);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const cx<T>* z = a.z + ((size_t)t0 * a.nch + ch) * tb.NZTP * a.tile + kPer * lane;
+  for (int k = warp; k < K; k += kZBWarps) {
+    if (lane >= lanes) break;
+    const TripleZ t = tb.trzp[k];
+    const int l = t.l, h0 = tb.hoff[l], H = tb.hoff[l + 1] - h0;
+    const int centre = (l & 1) ? -1 : H - 1;
+    T b[kPer];
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) b[p] = T(0);
+#pragma unroll 8
+    for (int e = 0; e < H; ++e) {
+      const uint4 zr = *reinterpret_cast<const uint4*>(z + (size_t)(t.za + e) * a.tile);
+      const uint4 cr = *reinterpret_cast<const uint4*>(sc + (size_t)(h0 + e) * CS + kPer * lane);
+      cx<T> zv[kPer], cv[kPer];
+      memcpy(zv, &zr, 16);
+      memcpy(cv, &cr, 16);
+      const T w = e == centre ? T(1) : T(2);
+#pragma unroll
+      for (int p = 0; p < kPer; ++p) b[p] = fma(w, fma(cv[p].x, zv[p].x, cv[p].y * zv[p].y), b[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) sb[(kPer * lane + p) * (K + 1) + k] = b[p];
+  }
+  __syncthreads();
+  for (int i = warp; i < na; i += kZBWarps) {
+    const int pos = t0 * a.tile + i, atom = a.order ? a.order[pos] : pos;
+    const bool alone = a.nbr_off[atom + 1] == a.nbr_off[atom];
+    for (int k = lane; k < K; k += 32)
+      a.B[((size_t)atom * a.nch + ch) * K + k] = alone ? T(0) : sb[i * (K + 1) + k];
+  }
+}
+
 int optin() {
   static int v = 0;
   if (!v) {
@@ -601,6 +668,34 @@ cudaError_t launch_lane_z(const DevTables& tb, int nch, int count, const void* c
   return launch_lanes<T, kLaneZ>(a, st);
 }
 
+template <typename T>
+cudaError_t launch_z_descriptors(const DevTables& tb, const DevBatch& b, const BsoParams& p, const int* order, int count,
+                                 const void* c, const void* z, T* B, cudaStream_t st) {
+  if (count <= 0) return cudaSuccess;
+  ZBArgs<T> a{};
+  a.tb = tb;
+  a.c = static_cast<const cx<T>*>(c);
+  a.z = static_cast<const cx<T>*>(z);
+  a.order = order;
+  a.nbr_off = b.nbr_off;
+  a.B = B;
+  a.count = count;
+  a.nch = p.nch;
+  a.tile = lane_tile(tb, (int)sizeof(T));
+  constexpr int kPer = 16 / (2 * (int)sizeof(T));
+  const size_t smem = 2 * sizeof(T) * tb.HU * (a.tile + kPer) + sizeof(T) * a.tile * (tb.K + 1);
+  if (!a.tile || smem > (size_t)optin()) return cudaErrorInvalidConfiguration;
+  cudaError_t e = cudaFuncSetAttribute(k_z_descriptors<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const unsigned grid = (unsigned)((count + a.tile - 1) / a.tile * p.nch);
+  k_z_descriptors<T><<<grid, kZBWarps * 32, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
+template cudaError_t launch_z_descriptors<double>(const DevTables&, const DevBatch&, const BsoParams&, const int*, int,
+                                                  const void*, const void*, double*, cudaStream_t);
+template cudaError_t launch_z_descriptors<float>(const DevTables&, const DevBatch&, const BsoParams&, const int*, int,
+                                                 const void*, const void*, float*, cudaStream_t);
 template cudaError_t launch_lane_z<double>(const DevTables&, int, int, const void*, void*, cudaStream_t);
 template cudaError_t launch_lane_z<float>(const DevTables&, int, int, const void*, void*, cudaStream_t);
 template cudaError_t launch_c_half<double>(const DevTables&, const DevBatch&, const BsoParams&, int, int, const int*,

@@ -298,6 +298,22 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
         gam[ins.first->second].push_back(GammaItem{(uint16_t)k, (uint8_t)B.snum, (uint8_t)B.sden});
       }
     t->nblk_pair = (int)gam.size();
+    {  // numbered layer by layer
+      std::vector<int> layer(gam.size()), number(gam.size());
+      for (const auto& b : pblk) layer[b.second] = std::get<2>(b.first);
+      std::vector<std::vector<GammaItem>> sorted;
+      for (int j = 0; j <= J; ++j) {
+        t->blkp_off[j] = (int)sorted.size();
+        for (size_t i = 0; i < gam.size(); ++i)
+          if (layer[i] == j) {
+            number[i] = (int)sorted.size();
+            sorted.push_back(std::move(gam[i]));
+          }
+      }
+      t->blkp_off[J + 1] = (int)sorted.size();
+      gam = std::move(sorted);
+      for (auto& b : pblk) b.second = number[b.second];
+    }
     // the terms of the pair blocks, block by block
     std::vector<int> pz(pblk.size());
     for (const auto& b : pblk) pz[b.second] = std::get<2>(b.first);
@@ -305,6 +321,15 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
       const int n = H(z);
       z = t->nztp;
       t->nztp += n;
+    }
+    for (int j = 0, z = 0; j <= J; ++j) {
+      t->zoffp[j] = z;
+      z += (t->blkp_off[j + 1] - t->blkp_off[j]) * H(j);
+    }
+    for (int k = 0; k < t->K; ++k) {
+      const Block& B = kblocks[k][0];
+      t->trzp.push_back(TripleZ{
+          (uint16_t)pz[pblk.at(std::make_tuple(std::max(B.jA, B.jB), std::min(B.jA, B.jB), B.jO))], (uint16_t)B.jO});
     }
     for (const auto& b : pblk) pairz[b.first] = pz[b.second];
     for (const auto& v : gam) {

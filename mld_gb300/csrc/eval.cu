@@ -125,7 +125,7 @@ cudaError_t launch_eval_gamma(const DevTables& tb, const T* B, int A, int nch, c
   const size_t smem = (sizeof(double) + sizeof(T)) * kGammaAtoms * nch * tb.K;
   if (B)
     k_eval_gamma<T><<<(A + kGammaAtoms - 1) / kGammaAtoms, kGammaThreads, smem, st>>>(
-        tb.gam_off, tb.gam, tb.NBLK, nch, tb.K, A, B, wlin, wsym, wsym32, w0, gamma, Eatom);
+        tb.gamp_off, tb.gamp, tb.NBLKP, nch, tb.K, A, B, wlin, wsym, wsym32, w0, gamma, Eatom);
   else
     k_eval_gamma<T><<<1, kGammaThreads, smem, st>>>(tb.gamp_off, tb.gamp, tb.NBLKP, nch, tb.K, 1, nullptr, wlin, nullptr,
                                                     nullptr, w0, gamma, nullptr);

@@ -185,7 +185,10 @@ struct Bso4Tables {
   // jobs of B (a job per operand pair) and y (a job per output position), heaviest jobs first
   std::vector<double> cgv;
   std::vector<LaneRec> brecs, yrecs, zrecs;  // zrecs: yrecs with the terms' places in place of their blocks
-  int nztp = 0;                   // terms of the pair blocks, block by block (rowsrc2)
+  int nztp = 0;                   // terms of the pair blocks, by layer, block and half entry
+  int blkp_off[kMaxJ + 2] = {0};  // first pair block and term of every layer
+  int zoffp[kMaxJ + 1] = {0};
+  std::vector<TripleZ> trzp;      // trz on these terms
   std::vector<LaneJob> bjobs, yjobs;
   std::vector<TripleZ> trz;       // the ZA block and layer of each triple
   std::vector<RowSource> rowsrc;  // the blocks of every contraction row, indexed as rowk
@@ -213,6 +216,8 @@ struct DevTables {
   int blk_off[kMaxJ + 2] = {0};
   int zoff[kMaxJ + 1] = {0};
   int NCGV = 0, NBJ = 0, NYJ = 0, NBLKP = 0, NZTP = 0;
+  int blkp_off[kMaxJ + 2] = {0};
+  int zoffp[kMaxJ + 1] = {0};
   double* cgv64 = nullptr;        // NCGV
   float2* cgv32x2 = nullptr;      // every coefficient twice
   LaneRec* brecs = nullptr;
@@ -221,6 +226,7 @@ struct DevTables {
   LaneJob* yjobs = nullptr;       // NYJ
   LaneRec* zrecs = nullptr;
   RowSource* rowsrc2 = nullptr;
+  TripleZ* trzp = nullptr;        // K
   TripleZ* trz = nullptr;         // K
   RowSource* rowsrc = nullptr;    // NROWS
   int hoff[kMaxJ + 2] = {0};
@@ -324,6 +330,9 @@ cudaError_t fill_deriv_tables(const Bso4Tables& t, DevTables* d, Put put) {
   d->NZTP = t.nztp;
   if (e == cudaSuccess) e = put(t.zrecs, &d->zrecs);
   if (e == cudaSuccess) e = put(t.rowsrc2, &d->rowsrc2);
+  if (e == cudaSuccess) e = put(t.trzp, &d->trzp);
+  for (int j = 0; j <= t.J + 1; ++j) d->blkp_off[j] = t.blkp_off[j];
+  for (int j = 0; j <= t.J; ++j) d->zoffp[j] = t.zoffp[j];
   return e;
 }
 
@@ -443,6 +452,10 @@ bool deriv_available(const DevTables& tb, int nch, int eb);
 // Z terms of `count` rows of c, [tile][nch][NZTP][atoms of a tile] complex of T; lane_tile: atoms of a
 // tile (0: the tables do not fit).
 int lane_tile(const DevTables& tb, int eb);
+// B (whole-batch array) of atoms order[0 .. count - 1] from their c and Z terms by position.
+template <typename T>
+cudaError_t launch_z_descriptors(const DevTables& tb, const DevBatch& b, const BsoParams& p, const int* order, int count,
+                                 const void* c, const void* z, T* B, cudaStream_t st);
 template <typename T>
 cudaError_t launch_lane_z(const DevTables& tb, int nch, int count, const void* c, void* z, cudaStream_t st);
 
@@ -454,7 +467,8 @@ struct DevEval {
   const void* c = nullptr;       // c of every atom (A x nch x HU complex of T)
   const void* y = nullptr;       // linear model: y of every atom, as c; the kernel writes Eatom
   double w0 = 0.0;
-  const T* gamma = nullptr;      // quadratic model: Z-block weights, nch * NBLK per atom
+  const T* gamma = nullptr;      // quadratic model: pair-block weights, nch * NBLKP per atom
+  const void* z = nullptr;       // quadratic model: Z terms by queue position (launch_lane_z)
   T* pair = nullptr;             // P x 3: the pair's force contribution
   double* Satom = nullptr;       // A x 6: sum over the atom's pairs of the stress products (xx yy zz yz xz xy)
   double* Eatom = nullptr;       // A: energy of each atom (written for the linear model)
@@ -469,7 +483,7 @@ cudaError_t launch_bso4(const DevTables& tb, const DevBatch& b, const BsoParams&
 // Evaluation kernel (bispectrum_eval.cu) of the batch.
 template <typename T>
 cudaError_t launch_bso4_eval(const DevTables& tb, const DevBatch& b, const BsoParams& p, const DevEval<T>& ev,
-                             const int* order, int* counter, cudaStream_t st);
+                             const int* order, int count, int* counter, cudaStream_t st);
 // Linear design rows of the batch from B, w_ch * dB and the reverse pairs (rows.cu); Sp is a
 // workspace of A x 6 x KK stress partials.  Columns [1, 1 + KK) of the energy, force and stress
 // rows are written.
@@ -484,7 +498,7 @@ cudaError_t launch_eval_gather(const DevBatch& b, const BsoParams& p, const int*
 // atom_order_tmp_ints(maxnn) ints.
 size_t atom_order_tmp_ints(int maxnn);
 cudaError_t launch_atom_order(const int* nn, int A, int maxnn, int* order, int* tmp, cudaStream_t st);
-// The block weights gamma (nch * NBLK per atom) of beta_a = w_lin + Wsym B_a and the energies
+// The pair-block weights gamma (nch * NBLKP per atom) of beta_a = w_lin + Wsym B_a and the energies
 // Eatom_a = w0 + B_a . (beta_a + w_lin) / 2; with B null the pair-block weights (nch * NBLKP) of
 // beta = w_lin, once (eval.cu).  wsym32: Wsym as double-FP32 pairs (launch_split_pairs), for T = float.
 template <typename T>
