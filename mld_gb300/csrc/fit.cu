@@ -122,7 +122,11 @@ __global__ void __launch_bounds__(256) k_gram(const T* __restrict__ X, int ldx, 
 
 // G (upper triangle of each tile pair) = sum over the row chunks of the partial tiles, in chunk
 // order; one CTA per tile pair, one thread per element.
-__global__ void __launch_bounds__(GT * GT) k_gram_reduce(const double* __restrict__ part, int npairs, int chunks, int D,
+// Grid (tile pairs, GT * GT / 32): 32 elements of a tile per block, a warp for every eighth chunk, the
+// warps' sums added in order.  (A thread that added all chunks waited out the FP64 adds one after the
+// other: 88 us for the linear fit of 60 structures, 14 so.)
+constexpr int kGramReduceWarps = 8;
+__global__ void __launch_bounds__(32 * kGramReduceWarps) k_gram_reduce(const double* __restrict__ part, int npairs, int chunks, int D,
                                                          double* __restrict__ G) {
   const int nt = (D + GT - 1) / GT;
   int t = blockIdx.x, ti = 0;
@@ -131,10 +135,17 @@ __global__ void __launch_bounds__(GT * GT) k_gram_reduce(const double* __restric
     ++ti;
   }
   const int tj = ti + t;
-  const int e = threadIdx.x, i = ti * GT + e / GT, j = tj * GT + e % GT;
-  if (i >= D || j >= D || (ti == tj && i > j)) return;
+  __shared__ double red[kGramReduceWarps][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int e = blockIdx.y * 32 + lane, i = ti * GT + e / GT, j = tj * GT + e % GT;
   double sum = 0.0;
-  for (int c = 0; c < chunks; ++c) sum += part[((size_t)c * npairs + blockIdx.x) * (GT * GT) + e];
+#pragma unroll 8
+  for (int c = warp; c < chunks; c += kGramReduceWarps) sum += part[((size_t)c * npairs + blockIdx.x) * (GT * GT) + e];
+  red[warp][lane] = sum;
+  __syncthreads();
+  if (warp > 0 || i >= D || j >= D || (ti == tj && i > j)) return;
+#pragma unroll
+  for (int w = 1; w < kGramReduceWarps; ++w) sum += red[w][lane];
   G[(size_t)i * D + j] = sum;
 }
 
@@ -205,7 +216,7 @@ cudaError_t launch_gram(const T* X, int ldx, const double* w, const double* y, l
   long long chunks = 0, rpb = 0;
   gram_chunks(M, D, nsm, &npairs, &chunks, &rpb);
   k_gram<T><<<dim3(npairs, (unsigned)chunks), 256, 0, st>>>(X, ldx, w, M, D, rpb, G, ws);
-  if (ws) k_gram_reduce<<<npairs, GT * GT, 0, st>>>(ws, npairs, (int)chunks, D, G);
+  if (ws) k_gram_reduce<<<dim3(npairs, GT * GT / 32), 32 * kGramReduceWarps, 0, st>>>(ws, npairs, (int)chunks, D, G);
   e = launch_rhs<T>(X, ldx, w, y, M, D, h, nsm, st, nullptr, ws);
   if (e != cudaSuccess) return e;
   k_symmetrize<<<D, 128, 0, st>>>(G, D);
@@ -382,17 +393,32 @@ __global__ void __launch_bounds__(256) k_xtv_ds(const float* __restrict__ X, int
   float ah[8], al[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) ah[k] = al[k] = 0.f;
-  for (long long r = r0 + warp; r < r1; r += 8) {
-    const float2 s = sv[r];
-    const float* xr = X + r * ldx + cb;
+  // three rows of loads in flight; the sums take the rows in order (60,000 rows x 1541: 112 -> 91 us)
+  constexpr int kAhead = 3;
+  for (long long rr = r0 + warp; rr < r1; rr += 8 * kAhead) {
+    float2 s[kAhead];
+    float x[kAhead][8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int c = lane + 32 * k;
-      if (cb + c < D) ds_fma(ah[k], al[k], xr[c], s.x, s.y);
+    for (int i = 0; i < kAhead; ++i) {
+      const long long r = min(rr + 8 * i, r1 - 1);
+      s[i] = sv[r];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int c = lane + 32 * k;
+        x[i][k] = cb + c < D ? X[r * ldx + cb + c] : 0.f;
+      }
     }
-    if (((r - r0) & 511) == 504) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) ds_norm(ah[k], al[k]);
+    for (int i = 0; i < kAhead; ++i) {
+      const long long r = rr + 8 * i;
+      if (r >= r1) break;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (cb + lane + 32 * k < D) ds_fma(ah[k], al[k], x[i][k], s[i].x, s[i].y);
+      if (((r - r0) & 511) == 504) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ds_norm(ah[k], al[k]);
+      }
     }
   }
 #pragma unroll
@@ -775,8 +801,7 @@ __global__ void __launch_bounds__(1024) k_jacobi_solve(const double* __restrict_
   double* cs = V + n * n;       // n/2 * 2
   int* pp = reinterpret_cast<int*>(cs + n);  // n/2
   int* qq = pp + n / 2;
-  int* perm = qq + n / 2;       // n
-  double* red = reinterpret_cast<double*>(perm + n);  // 2 doubles + flag
+  double* red = reinterpret_cast<double*>(qq + n / 2 + n);  // 2 doubles + flag
   const int tid = threadIdx.x, nth = blockDim.x;
   for (int e = tid; e < n * n; e += nth) {
     int i = e / n, j = e % n;
@@ -785,7 +810,6 @@ __global__ void __launch_bounds__(1024) k_jacobi_solve(const double* __restrict_
     A[e] = v;
     V[e] = (i == j) ? 1.0 : 0.0;
   }
-  for (int e = tid; e < n; e += nth) perm[e] = e;
   __syncthreads();
   const int npair = n / 2;
   int sweep = 0;
@@ -826,9 +850,13 @@ __global__ void __launch_bounds__(1024) k_jacobi_solve(const double* __restrict_
     if (red[0] <= 1e-28 * red[1] || red[1] == 0.0) break;
     __syncthreads();
     for (int round = 0; round < n - 1; ++round) {
-      // tournament pairing: perm[0] fixed, the rest rotate
+      // tournament pairing: place 0 holds index 0, the other indices move up one place a round
       if (tid < npair) {
-        int p = perm[tid], q = perm[n - 1 - tid];
+        auto at = [&](int place) {
+          const int k = place - 1 - round;
+          return place == 0 ? 0 : 1 + (k < 0 ? k + n - 1 : k);
+        };
+        int p = at(tid), q = at(n - 1 - tid);
         if (p > q) {
           int t = p;
           p = q;
@@ -872,12 +900,6 @@ __global__ void __launch_bounds__(1024) k_jacobi_solve(const double* __restrict_
         A[q * n + j] = s * apj + c * aqj;
       }
       __syncthreads();
-      if (tid == 0) {
-        int last = perm[n - 1];
-        for (int k = n - 1; k > 1; --k) perm[k] = perm[k - 1];
-        perm[1] = last;
-      }
-      __syncthreads();
     }
   }
   // min-norm solution: w = sum_{|lambda_i| > thr} (v_i . h / lambda_i) v_i
@@ -917,7 +939,10 @@ cudaError_t launch_solve_sym(double* G, const double* h, int D, double lambda, d
   size_t smem = sizeof(double) * (2 * (size_t)n * n + n) + sizeof(int) * (2 * n) + 4 * sizeof(double);
   cudaError_t e = cudaFuncSetAttribute(k_jacobi_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_jacobi_solve<<<1, 1024, smem, st>>>(G, h, D, lambda, rcond, wout, evals, info);
+  // a thread per rotated pair of elements, so that small matrices wait at narrow barriers (15 columns:
+  // 300 us with 1024 threads and the pairing shifted by one of them, 246 so)
+  const int threads = std::min(1024, std::max(128, (n * n / 2 + 31) / 32 * 32));
+  k_jacobi_solve<<<1, threads, smem, st>>>(G, h, D, lambda, rcond, wout, evals, info);
   return cudaGetLastError();
 }
 
@@ -982,13 +1007,15 @@ __global__ void __launch_bounds__(256) k_predict(const T* __restrict__ X, int ld
   }
 }
 
-// sq[0..5] = the per-CTA partials summed in CTA order
-__global__ void k_sq_reduce(double* __restrict__ sq, int blocks) {
-  const int k = threadIdx.x;
-  if (k >= 6) return;
+// sq[0..5] = the per-CTA partials in a fixed order: a warp per sum, lane l adds the CTAs l, l + 32, ...
+// in turn, then a fixed xor tree.  (One thread per sum waited out 1,216 loads: 91 us, 9 so.)
+__global__ void __launch_bounds__(192) k_sq_reduce(double* __restrict__ sq, int blocks) {
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double t = 0.0;
-  for (int b = 0; b < blocks; ++b) t += sq[kSqPartials + 6 * (size_t)b + k];
-  sq[k] = t;
+#pragma unroll 8
+  for (int b = lane; b < blocks; b += 32) t += sq[kSqPartials + 6 * (size_t)b + k];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) sq[k] = t;
 }
 
 template <typename T>
@@ -1009,7 +1036,7 @@ cudaError_t launch_predict_sq(const T* X, int ldx, const double* w, long long M,
     }
   }
   k_predict<T><<<blocks, 256, smem, st>>>(X, ldx, w, M, D, pred, y, kind, sq);
-  if (sq) k_sq_reduce<<<1, 32, 0, st>>>(sq, (int)blocks);
+  if (sq) k_sq_reduce<<<1, 192, 0, st>>>(sq, (int)blocks);
   return cudaGetLastError();
 }
 

@@ -23,20 +23,44 @@
 namespace mld {
 
 namespace {
-constexpr int kKT = 256;   // threads per CTA (one reference point each per pass)
 __constant__ int c_sa[6] = {0, 1, 2, 1, 0, 0};
 __constant__ int c_sb[6] = {0, 1, 2, 2, 2, 1};
 }  // namespace
 
+// x . x of a row of KK values by one warp, the same in every lane: lane l adds the values l, l + 32, ...
+// in turn, then a fixed xor tree (a thread per row read its row uncoalesced and one value at a time)
+template <typename T>
+__device__ __forceinline__ double warp_square(const T* __restrict__ x, int KK) {
+  double xx = 0.0;
+#pragma unroll 4
+  for (int c = threadIdx.x & 31; c < KK; c += 32) xx += (double)x[c] * (double)x[c];
+  for (int o = 16; o > 0; o >>= 1) xx += __shfl_xor_sync(0xffffffffu, xx, o);
+  return xx;
+}
+
+// Blocks of kKernelRows rows: the warps form the rows' squares, the first warp the powers of all of them
+// (a lane each: FP64 pow takes the FP64 pipe a few thousand clocks per warp, whatever its lanes).
+// 1,600 atoms x 110: 35 us with a thread per row, 19 so.
+constexpr int kKernelRows = 32, kKernelWarps = 8;
+template <typename T>
+__device__ __forceinline__ double block_squares(const T* __restrict__ X, int r0, int n, int KK, double* sq) {
+  for (int r = threadIdx.x >> 5; r < kKernelRows; r += kKernelWarps) {
+    const double v = r0 + r < n ? warp_square(X + (size_t)(r0 + r) * KK, KK) : 0.0;
+    if ((threadIdx.x & 31) == 0) sq[r] = v;
+  }
+  __syncthreads();
+  return sq[threadIdx.x & 31];
+}
+
 // per atom: [0] f(x,x), [1] sqrt f(x,x), [2] dker_xx, [3] 1 if the atom has neighbours
 template <typename T>
-__global__ void k_krr_atom(int A, int KK, const T* __restrict__ B, const int* __restrict__ nbr_off, double s2,
-                           double l2, double p, T* __restrict__ at) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= A) return;
-  const T* x = B + (size_t)a * KK;
-  double xx = 0.0;
-  for (int c = 0; c < KK; ++c) xx += (double)x[c] * (double)x[c];
+__global__ void __launch_bounds__(32 * kKernelWarps) k_krr_atom(int A, int KK, const T* __restrict__ B,
+                                                                const int* __restrict__ nbr_off, double s2, double l2,
+                                                                double p, T* __restrict__ at) {
+  __shared__ double sq[kKernelRows];
+  const double xx = block_squares(B, blockIdx.x * kKernelRows, A, KK, sq);
+  const int a = blockIdx.x * kKernelRows + threadIdx.x;
+  if (threadIdx.x >= kKernelRows || a >= A) return;
   const double base = s2 + xx / l2;
   const double kxx = pow(base, p);
   at[4 * (size_t)a] = (T)kxx;
@@ -47,12 +71,12 @@ __global__ void k_krr_atom(int A, int KK, const T* __restrict__ B, const int* __
 
 // per reference point: sqrt f(z,z)
 template <typename T>
-__global__ void k_krr_points(int nk, int KK, const T* __restrict__ Z, double s2, double l2, double p,
-                             T* __restrict__ szz) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nk) return;
-  double zz = 0.0;
-  for (int c = 0; c < KK; ++c) zz += (double)Z[(size_t)k * KK + c] * (double)Z[(size_t)k * KK + c];
+__global__ void __launch_bounds__(32 * kKernelWarps) k_krr_points(int nk, int KK, const T* __restrict__ Z, double s2,
+                                                                  double l2, double p, T* __restrict__ szz) {
+  __shared__ double sq[kKernelRows];
+  const double zz = block_squares(Z, blockIdx.x * kKernelRows, nk, KK, sq);
+  const int k = blockIdx.x * kKernelRows + threadIdx.x;
+  if (threadIdx.x >= kKernelRows || k >= nk) return;
   szz[k] = (T)sqrt(pow(s2 + zz / l2, p));
 }
 
@@ -96,22 +120,30 @@ __global__ void __launch_bounds__(256) k_krr_xz(int A, int nk, int KK, const T* 
 }
 
 
-// energy rows: grid (S, ceil(nk / kKT))
+// energy rows: grid (S, ceil(nk / 32)); lanes are reference points, warp w sums the structure's atoms
+// w, w + kEnergyWarps, ... in turn, and the warps' sums are added in order.  Bound: reading F once.  (A
+// thread that walked all atoms of the structure waited out a load and a division for each: eight
+// structures of up to 300 atoms x 1000 points 208 us, 20 so.)
+constexpr int kEnergyWarps = 16;
 template <typename T>
-__global__ void __launch_bounds__(kKT) k_krr_energy(int nk, const int* __restrict__ atom_start,
+__global__ void __launch_bounds__(32 * kEnergyWarps) k_krr_energy(int nk, const int* __restrict__ atom_start,
                                                     const long long* __restrict__ rowE, const T* __restrict__ F,
                                                     const T* __restrict__ at, const T* __restrict__ szz, double s2,
                                                     double l2, double p, int c0, int ldx, T* __restrict__ X) {
+  __shared__ double red[kEnergyWarps][32];
   const int s = blockIdx.x;
-  const int k = blockIdx.y * kKT + threadIdx.x;
-  if (rowE[s] < 0 || k >= nk) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = min(blockIdx.y * 32 + lane, nk - 1);
+  if (rowE[s] < 0) return;
+  const T zk = szz[k];
   // kernel values in the kernel's precision (FP64 runs at 1/64 rate), summed in double-FP32
   const T s2t = (T)s2, l2t = (T)l2, pt = (T)p;
   const int ip = (int)p;
   const bool ipow = (double)ip == p && ip >= 0 && ip <= 8;
   float sh = 0.f, sl = 0.f;
   double acc = 0.0;  // FP64 method
-  for (int a = atom_start[s]; a < atom_start[s + 1]; ++a) {
+  const int a1 = atom_start[s + 1];
+#pragma unroll 4
+  for (int a = atom_start[s] + warp; a < a1; a += kEnergyWarps) {
     const T* ata = at + 4 * (size_t)a;
     if (ata[3] == T(0)) continue;  // atoms without neighbours contribute zero
     const T base = s2t + F[(size_t)a * nk + k] / l2t;
@@ -121,7 +153,7 @@ __global__ void __launch_bounds__(kKT) k_krr_energy(int nk, const int* __restric
     } else {
       kt = (T)pow((double)base, (double)pt);
     }
-    const T kv = kt / (szz[k] * ata[1]);
+    const T kv = kt / (zk * ata[1]);
     if constexpr (sizeof(T) == 8) {
       acc += kv;
     } else {
@@ -131,7 +163,13 @@ __global__ void __launch_bounds__(kKT) k_krr_energy(int nk, const int* __restric
       sl += e;
     }
   }
-  X[rowE[s] * ldx + c0 + k] = sizeof(T) == 8 ? (T)acc : (T)((double)sh + (double)sl);
+  red[warp][lane] = sizeof(T) == 8 ? acc : (double)sh + (double)sl;
+  __syncthreads();
+  if (warp > 0 || blockIdx.y * 32 + lane >= nk) return;
+  double sum = 0.0;
+#pragma unroll
+  for (int w = 0; w < kEnergyWarps; ++w) sum += red[w][lane];
+  X[rowE[s] * ldx + c0 + k] = (T)sum;
 }
 
 // Force rows as a register-tiled product: CTA = (tile of NZ reference points, range of target
@@ -463,12 +501,12 @@ cudaError_t launch_krr_rows(const DevBatch& b, const DevRows& rows, const int* r
   T* F = szz + nk;
   T* Ts = F + (size_t)b.A * nk;
   T* tx = Ts + 6 * (size_t)b.A * KK;
-  k_krr_atom<T><<<(b.A + 255) / 256, 256, 0, st>>>(b.A, KK, Bq, b.nbr_off, s2, l2, power, at);
-  k_krr_points<T><<<(nk + 255) / 256, 256, 0, st>>>(nk, KK, Z, s2, l2, power, szz);
+  k_krr_atom<T><<<(b.A + kKernelRows - 1) / kKernelRows, 32 * kKernelWarps, 0, st>>>(b.A, KK, Bq, b.nbr_off, s2, l2, power, at);
+  k_krr_points<T><<<(unsigned)((nk + kKernelRows - 1) / kKernelRows), 32 * kKernelWarps, 0, st>>>(nk, KK, Z, s2, l2, power, szz);
   dim3 gx((nk + 63) / 64, (b.A + 63) / 64);
   k_krr_xz<T><<<gx, 256, 0, st>>>(b.A, nk, KK, Bq, Z, F);
-  dim3 gs(b.S, (nk + kKT - 1) / kKT);
-  k_krr_energy<T><<<gs, kKT, 0, st>>>(nk, b.atom_start, rows.rowE, F, at, szz, s2, l2, power, c0, rows.ldx, X);
+  dim3 gs(b.S, (nk + 31) / 32);
+  k_krr_energy<T><<<gs, 32 * kEnergyWarps, 0, st>>>(nk, b.atom_start, rows.rowE, F, at, szz, s2, l2, power, c0, rows.ldx, X);
   // stress partials T_s, T_s . x per atom (both paths)
   k_krr_stress_atom<T><<<b.A, 128, sizeof(T) * 3 * (size_t)std::max(1, b.maxnn), st>>>(
       KK, b.maxnn, b.atom_struct, b.small, b.nbr_off, b.nbr_u, Bq, dBq, sign_big, Ts, tx);

@@ -81,9 +81,12 @@ __global__ void __launch_bounds__(kRowThreads) k_lin_force_rows(
   }
 }
 
-// grid (S, 7): r = 0 energy row sum_i B_i; r = 1..6 stress rows sign_stress*3/V sum_i Sp_i.
+// grid (S, 7, columns / 32): r = 0 energy row sum_i B_i; r = 1..6 stress rows sign_stress*3/V sum_i Sp_i.
+// Lanes are columns; warp w sums the atoms w, w + 8, ... in turn, and the warps' sums are added in order.
+// (Threads that walked all atoms waited for each load: eight structures of up to 300 atoms 55 us, 9 so.)
+constexpr int kStructWarps = 8;
 template <typename T>
-__global__ void __launch_bounds__(kRowThreads) k_lin_struct_rows(int KK, const int* __restrict__ atom_start,
+__global__ void __launch_bounds__(32 * kStructWarps) k_lin_struct_rows(int KK, const int* __restrict__ atom_start,
                                                                  const T* __restrict__ B, const T* __restrict__ Sp,
                                                                  const double* __restrict__ volume, double sign_stress,
                                                                  const long long* __restrict__ rowE,
@@ -92,16 +95,22 @@ __global__ void __launch_bounds__(kRowThreads) k_lin_struct_rows(int KK, const i
   const int s = blockIdx.x, r = blockIdx.y;
   const long long row = (r == 0) ? rowE[s] : (rowS[s] >= 0 ? rowS[s] + (r - 1) : -1);
   if (row < 0) return;
+  __shared__ T red[kStructWarps][32];
   const int a0 = atom_start[s], a1 = atom_start[s + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.z * 32 + lane, kc = min(k, KK - 1);
+  const T* src = r == 0 ? B + kc : Sp + (size_t)(r - 1) * KK + kc;
+  const size_t step = r == 0 ? (size_t)KK : (size_t)6 * KK;
+  T sum = T(0);
+#pragma unroll 8
+  for (int a = a0 + warp; a < a1; a += kStructWarps) sum += src[a * step];
+  red[warp][lane] = sum;
+  __syncthreads();
+  if (warp > 0 || k >= KK) return;
   const T sc = (r == 0) ? T(1) : (T)(sign_stress * 3.0 / volume[s]);
-  for (int k = threadIdx.x; k < KK; k += kRowThreads) {
-    T sum = T(0);
-    if (r == 0)
-      for (int a = a0; a < a1; ++a) sum += B[(size_t)a * KK + k];
-    else
-      for (int a = a0; a < a1; ++a) sum += Sp[((size_t)a * 6 + (r - 1)) * KK + k];
-    X[row * ldx + 1 + k] = sc * sum;
-  }
+  sum = red[0][lane];
+#pragma unroll
+  for (int w = 1; w < kStructWarps; ++w) sum += red[w][lane];
+  X[row * ldx + 1 + k] = sc * sum;
 }
 
 // Evaluation: F_i[a] = sum_q pair_q[a] - pair_rev(q)[a] in FP64, one thread per (atom, component).
@@ -138,9 +147,12 @@ __global__ void __launch_bounds__(kStructThreads) k_eval_struct(const int* __res
 #pragma unroll
     for (int c = 0; c < 6; ++c) v[1 + c] += Satom[(size_t)i * 6 + c];
   }
+  // (warps without atoms add nothing: their sums are zero.  The FP64 pipe makes two sums a clock.)
+  const bool some = atom_start[s] + (tid & ~31) < a1;
 #pragma unroll
   for (int c = 0; c < 7; ++c) {
-    for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
+    if (some)
+      for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
     if ((tid & 31) == 0) red[c][tid >> 5] = v[c];
   }
   __syncthreads();
@@ -228,7 +240,7 @@ cudaError_t launch_lin_rows(const DevBatch& b, const DevRows& rows, const BsoPar
                                              p.sign_big, dB, rows.rowF, rows.rowS, X, rows.ldx, Sp);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_lin_struct_rows<T><<<dim3(b.S, 7), kRowThreads, 0, st>>>(KK, b.atom_start, B, Sp, b.volume, p.sign_stress,
+  k_lin_struct_rows<T><<<dim3(b.S, 7, (unsigned)((KK + 31) / 32)), 32 * kStructWarps, 0, st>>>(KK, b.atom_start, B, Sp, b.volume, p.sign_stress,
                                                              rows.rowE, rows.rowS, X, rows.ldx);
   return cudaGetLastError();
 }
@@ -238,7 +250,8 @@ cudaError_t launch_eval_gather(const DevBatch& b, const BsoParams& p, const int*
                                double* F, double* S, cudaStream_t st) {
   if (b.A == 0) return cudaSuccess;
   const long long n = 3LL * b.A;
-  k_eval_forces<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(b.A, b.nbr_off, rev, ev.pair, F);
+  // small blocks: a cell of some fifty atoms, whose sums take the FP64 pipe, spreads over several SMs
+  k_eval_forces<T><<<(unsigned)((n + 63) / 64), 64, 0, st>>>(b.A, b.nbr_off, rev, ev.pair, F);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_eval_struct<<<b.S, kStructThreads, 0, st>>>(b.atom_start, ev.Satom, ev.Eatom, b.volume, p.sign_stress, E, S);
