@@ -95,60 +95,63 @@ __device__ __forceinline__ void tmem_wait8(uint32_t (&v)[8]) {
 
 // Transpose rows [r0, r0 + rows) of X (row stride ldx, columns [c0, c0 + D)) into the K-major
 // bf16 planes hi/lo (D x Mp), scaling row r by sqrt(w[r]); design rows [rows, Mp) are zeroed.
-// grid.x: 64-row blocks of the chunk, grid.y: blocks of kSplitTiles tiles of 64 columns.
+// grid.x: kSplitRows-row blocks of the chunk, grid.y: blocks of kSplitTiles tiles of 64 columns.
 //
 // A thread carries two rows of a column through shared memory as one float2 (row pair p at
 // [p][column], odd stride: no bank conflicts either way), so a warp reads 128 bytes of a row of X
 // and writes 128 bytes of a plane row; the next tile's loads are issued before this one's stores.
-constexpr int kSplitTiles = 4;
+constexpr int kSplitTiles = 4, kSplitRows = 128, kSplitWarps = 16;
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_split_bf16(const T* __restrict__ X, int ldx, int c0, int D,
+__global__ void __launch_bounds__(32 * kSplitWarps) k_split_bf16(const T* __restrict__ X, int ldx, int c0, int D,
                                                     const double* __restrict__ w, long long r0, long long rows,
                                                     long long Mp, __nv_bfloat16* __restrict__ hi,
                                                     __nv_bfloat16* __restrict__ lo) {
-  __shared__ float2 tile[32][65];
-  __shared__ float sw[64];
-  const long long rb = (long long)blockIdx.x * 64;
-  const int lane = threadIdx.x, wy = threadIdx.y;  // block (32, 8)
+  __shared__ float2 tile[kSplitRows / 2][65];
+  __shared__ float sw[kSplitRows];
+  const long long rb = (long long)blockIdx.x * kSplitRows;
+  const int lane = threadIdx.x, wy = threadIdx.y;  // block (32, kSplitWarps)
   const int tid = wy * 32 + lane;
-  const int nrow = (int)min((long long)64, rows - rb);  // may be <= 0 in the zeroed rows
+  const int nrow = (int)min((long long)kSplitRows, rows - rb);  // may be <= 0 in the zeroed rows
   // sqrt(w) and x' in FP32: the split keeps about 17 bits of x', and FP64 runs at 1/64 rate
-  if (tid < 64) sw[tid] = tid < nrow ? (float)sqrt(w[r0 + rb + tid]) : 0.f;
+  if (tid < kSplitRows) sw[tid] = tid < nrow ? (float)sqrt(w[r0 + rb + tid]) : 0.f;
   __syncthreads();
   const T* Xb = X + (r0 + rb) * ldx + c0;
-  // warp wy holds row pairs wy, wy + 8, ... and column halves 0, 1 of a tile
+  // warp wy holds row pairs wy, wy + 16, ... and column halves 0, 1 of a tile
   float2 v[4][2];
   auto load = [&](int cb) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int r = 2 * (wy + 8 * i), c = cb + 32 * h + lane;
+        const int r = 2 * (wy + kSplitWarps * i), c = cb + 32 * h + lane;
         v[i][h].x = r < nrow && c < D ? (float)Xb[(long long)r * ldx + c] * sw[r] : 0.f;
         v[i][h].y = r + 1 < nrow && c < D ? (float)Xb[(long long)(r + 1) * ldx + c] * sw[r + 1] : 0.f;
       }
   };
   const int cbeg = blockIdx.y * (64 * kSplitTiles), cend = min(D, cbeg + 64 * kSplitTiles);
-  const bool in = rb + 2 * lane < Mp;  // Mp is even
   load(cbeg);
   for (int cb = cbeg; cb < cend; cb += 64) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) tile[wy + 8 * i][32 * h + lane] = v[i][h];
+      for (int h = 0; h < 2; ++h) tile[wy + kSplitWarps * i][32 * h + lane] = v[i][h];
     __syncthreads();
     if (cb + 64 < cend) load(cb + 64);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int cl = wy + 8 * i, c = cb + cl;
-      if (c < cend && in) {
-        const float2 x = tile[lane][cl];
-        const __nv_bfloat162 h = __floats2bfloat162_rn(x.x, x.y);
-        const size_t o = (size_t)c * Mp + rb + 2 * lane;
-        *reinterpret_cast<__nv_bfloat162*>(hi + o) = h;
-        *reinterpret_cast<__nv_bfloat162*>(lo + o) =
-            __floats2bfloat162_rn(x.x - __low2float(h), x.y - __high2float(h));
+    for (int i = 0; i < 64 / kSplitWarps; ++i) {
+      const int cl = wy + kSplitWarps * i, c = cb + cl;
+#pragma unroll
+      for (int g = 0; g < kSplitRows / 64; ++g) {
+        const long long r = rb + 64 * g + 2 * lane;
+        if (c < cend && r < Mp) {  // (Mp is even)
+          const float2 x = tile[32 * g + lane][cl];
+          const __nv_bfloat162 h = __floats2bfloat162_rn(x.x, x.y);
+          const size_t o = (size_t)c * Mp + r;
+          *reinterpret_cast<__nv_bfloat162*>(hi + o) = h;
+          *reinterpret_cast<__nv_bfloat162*>(lo + o) =
+              __floats2bfloat162_rn(x.x - __low2float(h), x.y - __high2float(h));
+        }
       }
     }
     __syncthreads();
@@ -429,8 +432,8 @@ cudaError_t launch_gram_tc(const T* X, int ldx, int c0, int D, const double* w, 
     const long long rows = std::min(chunk, M - r0);
     const long long Mp = (rows + 7) / 8 * 8;  // 16-byte plane row stride
     __nv_bfloat16* lo = hi + (size_t)D * Mp;
-    dim3 g1((unsigned)((Mp + 63) / 64), (unsigned)((D + 64 * kSplitTiles - 1) / (64 * kSplitTiles)));
-    k_split_bf16<T><<<g1, dim3(32, 8), 0, st>>>(X, ldx, c0, D, w, r0, rows, Mp, hi, lo);
+    dim3 g1((unsigned)((Mp + kSplitRows - 1) / kSplitRows), (unsigned)((D + 64 * kSplitTiles - 1) / (64 * kSplitTiles)));
+    k_split_bf16<T><<<g1, dim3(32, kSplitWarps), 0, st>>>(X, ldx, c0, D, w, r0, rows, Mp, hi, lo);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     CUtensorMap mh, ml;
