@@ -1858,6 +1858,13 @@ int eval_launch(mld_gpu_handle* h, cudaEvent_t done, double** pinned_out) {
   return MLD_OK;
 }
 
+// bytes of an atom in the buffers between the evaluation's kernels
+size_t eval_atom_bytes(const mld_gpu_handle* h) {
+  const size_t eb = h->mixed ? 4 : 8, c = 2 * eb * h->nch * h->dt.HU;
+  if (!h->quad) return 2 * c;  // c and y
+  return c + eb * (h->KK + (size_t)h->nch * h->dt.NBLKP + 2 * (size_t)h->nch * h->dt.NZTP);  // c, B, weights, Z terms
+}
+
 void eval_collect(const mld_gpu_handle* h, int s, double* E, double* F, double* Sout) {
   const double* hp = h->pinned;
   const int a0 = h->h_atom_start[s], nat = h->h_atom_start[s + 1] - a0;

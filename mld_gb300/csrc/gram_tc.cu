@@ -16,7 +16,7 @@
 // warps 2-17 drain the accumulators with tcgen05.ld into compensated FP32 sums.
 //
 // 60,000 rows x 1541 columns: k_gram_tc 705 -> 495 us (1.1 PFLOP/s of the three products), k_split_bf16
-// 336 -> 175 us.  Of the first, 125 us were the last of three rounds of CTAs (gram_tc_splits); with
+// 336 -> 165 us.  Of the first, 125 us were the last of three rounds of CTAs (gram_tc_splits); with
 // two accumulators the MMAs waited for the epilogue's chain of load, wait and add.  What bounds it
 // now is the operand traffic, 64 KB per 64-row slice of a tile: 11 TB/s from L2.  With several
 // row splits each split writes its tile to a partial buffer and k_gram_tc_reduce adds the splits

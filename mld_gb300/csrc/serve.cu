@@ -32,6 +32,7 @@ int eval_launch(mld_gpu_handle* h, cudaEvent_t done, double** pinned_out);
 void eval_collect(const mld_gpu_handle* h, int s, double* E, double* F, double* Sout);
 int eval_weights_upload(mld_gpu_handle* h, const double* w_full);
 int handle_dims(const mld_gpu_handle* h, int* D, int* ldx, int* KK, int* nch);
+size_t eval_atom_bytes(const mld_gpu_handle* h);
 void handle_release_buffers(mld_gpu_handle* h);
 }  // namespace mld
 
@@ -89,8 +90,7 @@ int sfail(mld_gpu_server* s, int code, const std::string& msg) {
 }
 
 // device bytes of one structure's batch buffers: neighbour pairs (expected neighbours from the
-// number density within r_cut, 1.5x margin), per-atom descriptors and effective weights, the
-// FP64 outputs (evaluation without design rows)
+// number density within r_cut, 1.5x margin), per-atom buffers of the evaluation, the FP64 outputs
 double request_bytes(const mld_gpu_server* s, int nat, const double* cell) {
   const double* c = cell;
   const double vol = std::fabs(c[0] * (c[4] * c[8] - c[5] * c[7]) - c[1] * (c[3] * c[8] - c[5] * c[6]) +
@@ -99,8 +99,9 @@ double request_bytes(const mld_gpu_server* s, int nat, const double* cell) {
   const double nn = std::min<double>(s->cfg.imm_neigh, 1.5 * nat / std::max(vol, 1e-9) * 4.18879 * rc * rc * rc + 8);
   const double eb = s->cfg.precision == MLD_PRECISION_MIXED ? 4.0 : 8.0;
   const double pairs = nat * nn;
-  // per pair: index, FP64 and FP32 displacement, reverse pair, the single-pass search row
-  return pairs * 44.0 + nat * (2.0 * s->KK * eb + 24.0 + 64.0) + 128.0;
+  // per pair: index, FP64 and FP32 displacement, reverse pair, the single-pass search row, the force;
+  // per atom: position and outputs, energy and stress, and what the evaluation kernels hand on
+  return pairs * (44.0 + 3.0 * eb) + nat * (24.0 + 64.0 + 56.0 + (double)mld::eval_atom_bytes(s->slots[0].h)) + 128.0;
 }
 
 void retire(mld_gpu_server* s, int idx) {
