@@ -1,4 +1,5 @@
-// Bispectrum-SO(4) descriptors and their derivatives: persistent CTAs, one centre atom at a time.
+// Bispectrum-SO(4) descriptors and their derivatives in one kernel, one centre atom at a time: the route
+// of batches of up to an atom per SM (larger ones: bispectrum_lanes.cu and bispectrum_deriv.cu).
 //
 // Per atom i with neighbours n (u_n = x_n - x_i, r_n < r_cut):
 //   phase 1  c^j(p,q) = delta_pq + sum_n w_ch(type_n) f_c(r_n) U^j_pq(u_n)           (compute_bispectrum_so4.F90:288-439)
@@ -123,11 +124,12 @@ __host__ __device__ inline SmemPlan smem_plan(const DevTables& tb, int nch, int 
   return s;
 }
 
+constexpr int kCT = 4;  // columns (neighbour, generator) per register tile of the dB contraction
+
 // kYShared: Y lives in shared memory (one channel); otherwise in the per-CTA global slice
 // args.yglobal (several channels), a separate instantiation so that the shared-memory
 // variant keeps shared-memory addressing.
-// kCT: columns (neighbour, generator) per register tile of the dB contraction (autotuned).
-template <typename T, bool kYShared, int kCT>
+template <typename T, bool kYShared>
 __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(KernelArgs<T> args, int A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DevTables& tb = args.tb;
@@ -524,8 +526,7 @@ cudaError_t launch_bso4(const DevTables& tb, const DevBatch& b, const BsoParams&
     }
   }
   a.yglobal = nullptr;
-  auto kern = sh.col_tile == 2 ? (y_in_smem ? k_bso4<T, true, 2> : k_bso4<T, false, 2>)
-                               : (y_in_smem ? k_bso4<T, true, 4> : k_bso4<T, false, 4>);
+  auto kern = y_in_smem ? k_bso4<T, true> : k_bso4<T, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int occ = 0;

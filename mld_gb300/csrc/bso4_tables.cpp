@@ -223,12 +223,9 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
         if (blkid.emplace(std::make_tuple(B.jA, B.jB, B.jO), nb[B.jO]).second) ++nb[B.jO];
     int z = 0;
     for (int j = 0; j <= J; ++j) {
-      t->blk_off[j] = t->nblk;
       t->zoff[j] = z;
-      t->nblk += nb[j];
       z += nb[j] * H(j);
     }
-    t->blk_off[J + 1] = t->nblk;
     t->nzu = z;
     zrep.assign(z, -1);
     for (int k = 0; k < t->K; ++k)
@@ -239,19 +236,11 @@ bool build_bso4_tables(double j_max, Bso4Tables* t, std::string* err) {
           if (zrep[u0 + e] < 0) zrep[u0 + e] = B.first + e;
         }
       }
-    std::vector<std::vector<GammaItem>> gam(t->nblk);
-    for (int k = 0; k < t->K; ++k)
-      for (int b = 0; b < 3; ++b) {
-        const Block& B = kblocks[k][b];
-        const int r = blkid[std::make_tuple(B.jA, B.jB, B.jO)];
-        gam[t->blk_off[B.jO] + r].push_back(GammaItem{(uint16_t)k, (uint8_t)B.snum, (uint8_t)B.sden});
-        if (b == 0) t->trz.push_back(TripleZ{(uint16_t)(t->zoff[B.jO] + r * H(B.jO)), (uint16_t)B.jO});
-      }
-    for (const auto& v : gam) {
-      t->gam_off.push_back((int)t->gam.size());
-      t->gam.insert(t->gam.end(), v.begin(), v.end());
+    for (int k = 0; k < t->K; ++k) {
+      const Block& B = kblocks[k][0];
+      const int r = blkid[std::make_tuple(B.jA, B.jB, B.jO)];
+      t->trz.push_back(TripleZ{(uint16_t)(t->zoff[B.jO] + r * H(B.jO)), (uint16_t)B.jO});
     }
-    t->gam_off.push_back((int)t->gam.size());
   }
 
   std::map<std::tuple<int, int, int>, int> pairz;  // pair block -> its first term

@@ -168,16 +168,11 @@ struct Bso4Tables {
   // q + 2 is -conj of the one at q - 2)
   std::vector<double> gen;
   // the distinct Z blocks (jA, jB -> jO), grouped by output layer: block r of layer j holds the terms
-  // zoff[j] + r * H_j + e of its half entries e, so sums over blocks or entries need no index lists
-  int nblk = 0;
-  int blk_off[kMaxJ + 2] = {0};
+  // zoff[j] + r * H_j + e of its half entries e
   int zoff[kMaxJ + 1] = {0};
-  // dE/dB_k = beta_k weighs block b with gamma_b = sum over [gam_off[b], gam_off[b + 1]) of
-  // (snum / sden) beta_k
-  std::vector<int> gam_off;
-  std::vector<GammaItem> gam;
   // the blocks with their operands in descending order (blocks that differ by the exchange are one),
-  // as the atoms-on-lanes sums count them
+  // as the atoms-on-lanes sums count them, layer by layer.  dE/dB_k = beta_k weighs block b with
+  // gamma_b = sum over [gamp_off[b], gamp_off[b + 1]) of (snum / sden) beta_k
   int nblk_pair = 0;
   std::vector<int> gamp_off;
   std::vector<GammaItem> gamp;
@@ -212,9 +207,6 @@ struct alignas(16) GenEntry {
 struct DevTables {
   int J = 0, NU = 0, HU = 0, K = 0, NYP = 0, NTILE = 0, NZT = 0, NROWS = 0;
   int NCG = 0;  // entries of the 1-D CG coefficient table
-  int NBLK = 0;
-  int blk_off[kMaxJ + 2] = {0};
-  int zoff[kMaxJ + 1] = {0};
   int NCGV = 0, NBJ = 0, NYJ = 0, NBLKP = 0, NZTP = 0;
   int blkp_off[kMaxJ + 2] = {0};
   int zoffp[kMaxJ + 1] = {0};
@@ -246,8 +238,6 @@ struct DevTables {
   // tables of the derivatives and the evaluation (fill_deriv_tables)
   GenEntry<float>* gen32 = nullptr;   // HU
   GenEntry<double>* gen64 = nullptr;  // HU
-  int* gam_off = nullptr;       // NBLK + 1
-  GammaItem* gam = nullptr;
   int* gamp_off = nullptr;      // NBLKP + 1
   GammaItem* gamp = nullptr;
 };
@@ -266,9 +256,6 @@ cudaError_t fill_dev_tables(const Bso4Tables& t, DevTables* d, Put put) {
   d->NZT = t.nzu;
   d->NROWS = (int)t.rowk.size();
   d->NCG = (int)t.cg.size();
-  d->NBLK = t.nblk;
-  for (int j = 0; j <= t.J + 1; ++j) d->blk_off[j] = t.blk_off[j];
-  for (int j = 0; j <= t.J; ++j) d->zoff[j] = t.zoff[j];
   for (int j = 0; j <= t.J + 1; ++j) {
     d->hoff[j] = t.hoff[j];
     d->rowk_off[j] = t.rowk_off[j];
@@ -319,8 +306,6 @@ cudaError_t fill_deriv_tables(const Bso4Tables& t, DevTables* d, Put put) {
   }
   cudaError_t e = put(g32, &d->gen32);
   if (e == cudaSuccess) e = put(g64, &d->gen64);
-  if (e == cudaSuccess) e = put(t.gam_off, &d->gam_off);
-  if (e == cudaSuccess) e = put(t.gam, &d->gam);
   d->NBLKP = t.nblk_pair;
   if (e == cudaSuccess) e = put(t.gamp_off, &d->gamp_off);
   if (e == cudaSuccess) e = put(t.gamp, &d->gamp);
@@ -420,7 +405,8 @@ bool bso4_available(const DevTables& tb, int nch, int eb);
 // Launch shape of the descriptor kernel, chosen per handle by the autotuner (api.cu); every
 // shape gives bitwise the same results.
 struct Bso4Launch {
-  int col_tile = 4;      // columns per register tile of the dB contraction: 2 or 4
+  int col_tile = 2;      // columns per register tile of k_deriv's contraction: 2 or 4 (492,000 Fe atoms: 58
+                         // against 62 ms; wider tiles leave long jobs to few warps at the end of a phase)
   int ctas_per_sm = 0;   // persistent CTAs per SM (0: as many as fit)
   int sorted_queue = 1;  // atoms longest first (1) or in index order (0)
 };
