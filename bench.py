@@ -13,7 +13,7 @@ design-row kernel, weighted Gram, ridge solve, train predictions/RMSE.
   e2e     the same through the C ABI with host buffers: each step stages positions, cells, types
           and labels from pinned host memory and reads back the coefficients and RMSE;
   plain   the all-FP64 method on the same data (the baseline named by the metric);
-  roofline  for the dominant kernel (fused descriptor kernel) against the measured FMA peak of
+  roofline  for the dominant stage (descriptor kernels) against the measured FMA peak of
           the pipe it runs on.
 """
 from __future__ import annotations
@@ -35,11 +35,11 @@ N_STRUCT = 2000
 RCUT = 4.7
 J_MAX = 4.0
 LAMBDA = 1e-8
-# DRAM bytes (read + write) of one k_bso4<float> launch per atom, from an ncu capture of the
-# 200-structure Fe case (45,702 atoms): 43.9 MB read (neighbour data, tables) + 1.017 GB written
-# (w*dB of every pair, the input of the row gather); both grow with the atoms (and their pairs),
-# so the figure is scaled by the atoms of the launch
-BSO4_DRAM_BYTES_PER_ATOM = (43.937024e6 + 1.017037e9) / 45702
+# DRAM bytes (read + write) of the descriptor kernels per atom, from an ncu capture of the
+# 200-structure Fe case (45,702 atoms): k_c_half 36 MB, k_lanes 807 MB (the Z terms written),
+# k_y_rows 1,661 MB (terms read, Y rows written), k_deriv 2,033 MB (rows read, w*dB of every pair
+# written); all grow with the atoms (and their pairs), so the figure is scaled by the atoms
+DESCRIPTOR_DRAM_BYTES_PER_ATOM = (36.194e6 + 806.902e6 + 1661.010e6 + 2033.390e6) / 45702
 
 
 def _args():
@@ -628,13 +628,13 @@ def main():
         "phase_ms": {k: v[0] / a.steps for k, v in res["prof"].items()},
         "mixed_solve": res["solve_info"],
         "descriptor_autotune": res["autotune"],
-        "roofline": {"kernel": "k_bso4<float> (fused descriptor + design rows)", "bound": "fp32",
+        "roofline": {"kernel": "k_c_half, k_lanes, k_y_rows, k_deriv <float> (descriptors and derivatives, with the row gathers)", "bound": "fp32",
                      "achieved": achieved, "peak": res["peak32"], "unit": "TFLOP/s", "frac": achieved / res["peak32"],
                      "peak_source": "measured in this run (FP32 FMA probe; not in MEASURED_PEAKS.json)",
                      "flops_per_launch": res["flops"], "flops_per_pair": res["per_pair"],
-                     "flops_per_atom": res["per_atom"], "traffic": BSO4_DRAM_BYTES_PER_ATOM * A,
+                     "flops_per_atom": res["per_atom"], "traffic": DESCRIPTOR_DRAM_BYTES_PER_ATOM * A,
                      "traffic_unit": "bytes per launch",
-                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on the "
+                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the four kernels on the "
                                        "200-structure case, scaled by atoms"},
         "gpu_launches": res["launches"],
         "clocks": res["clocks"],
