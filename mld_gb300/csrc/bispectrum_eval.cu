@@ -460,7 +460,8 @@ cudaError_t launch_bso4_eval(const DevTables& tb, const DevBatch& b, const BsoPa
     a.gen = reinterpret_cast<const GenEntry<T>*>(tb.gen32);
   }
   a.src = {b.types, b.nbr_idx, b.nbr_u, sizeof(T) == 4 ? b.nbr_u32 : nullptr, (T)p.rcut, (T)p.inv_r0,
-           (T)p.rin_width, p.ntypes, p.has_rin};
+           (T)p.rin_width, p.ntypes, p.has_rin, {}};
+  a.src.rates.set(p.rcut, p.inv_r0);
   a.atom_struct = b.atom_struct;
   a.small = b.small;
   a.nbr_off = b.nbr_off;

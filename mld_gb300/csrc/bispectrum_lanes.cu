@@ -573,7 +573,8 @@ cudaError_t launch_c_half(const DevTables& tb, const DevBatch& b, const BsoParam
   CArgs<T> a{};
   a.tb = tb;
   a.src = {b.types, b.nbr_idx, b.nbr_u, sizeof(T) == 4 ? b.nbr_u32 : nullptr, (T)p.rcut, (T)p.inv_r0,
-           (T)p.rin_width, p.ntypes, p.has_rin};
+           (T)p.rin_width, p.ntypes, p.has_rin, {}};
+  a.src.rates.set(p.rcut, p.inv_r0);
   a.nbr_off = b.nbr_off;
   for (int e = 0; e < kMaxCh * kMaxTypes; ++e) a.chw[e] = (T)p.chw[e];
   for (int e = 0; e < kMaxTypes * kMaxTypes; ++e) a.rin[e] = (T)p.rin[e];
