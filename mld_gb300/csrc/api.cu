@@ -1767,7 +1767,7 @@ static int eval_run(mld_gpu_handle* h, double* out) {
   // behind the FP64 weights: the linear model's block weights, the quadratic model's Wsym as FP32 pairs
   const void* wext = wlin + KK + (h->quad ? (size_t)KK * KK : 0);
   CK(ensure(h, mld_gpu_handle::B_EPAIR, sizeof(T) * 3 * (size_t)std::max<long long>(1, h->b.P)));
-  CK(ensure(h, mld_gpu_handle::B_EATOM, sizeof(double) * 7 * (size_t)std::max(1, h->A)));
+  CK(ensure(h, mld_gpu_handle::B_EATOM, sizeof(double) * (7 * (size_t)std::max(1, h->A) + eval_part_doubles(h->A, h->S))));
   CK(ensure(h, mld_gpu_handle::B_REV, sizeof(int) * (size_t)std::max<long long>(1, h->b.P)));
   const int* order = bp_<int>(h, mld_gpu_handle::B_ORDER);
   int* counter = bp_<int>(h, mld_gpu_handle::B_QCNT);
@@ -1775,6 +1775,9 @@ static int eval_run(mld_gpu_handle* h, double* out) {
   ev.pair = bp_<T>(h, mld_gpu_handle::B_EPAIR);
   ev.Eatom = bp_<double>(h, mld_gpu_handle::B_EATOM);
   ev.Satom = ev.Eatom + std::max(1, h->A);
+  ev.part = ev.Satom + 6 * (size_t)std::max(1, h->A);
+  int max_atoms = 0;
+  for (int s = 0; s < h->S; ++s) max_atoms = std::max(max_atoms, h->h_atom_start[s + 1] - h->h_atom_start[s]);
   ev.w0 = h->ew0;
   if (h->quad) {
     // c and Z terms of every atom, B from them; its weights and energy; then the evaluation kernel on
@@ -1825,7 +1828,7 @@ static int eval_run(mld_gpu_handle* h, double* out) {
     nl(h, 3);
   }
   CK(launch_reverse_pairs(h->b, bp_<int>(h, mld_gpu_handle::B_REV), h->st));
-  CK(launch_eval_gather<T>(h->b, h->bp, bp_<int>(h, mld_gpu_handle::B_REV), ev, E, F, S, h->st));
+  CK(launch_eval_gather<T>(h->b, h->bp, bp_<int>(h, mld_gpu_handle::B_REV), ev, max_atoms, E, F, S, h->st));
   nl(h, 3);
   return MLD_OK;
 }

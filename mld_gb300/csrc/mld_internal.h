@@ -458,6 +458,7 @@ struct DevEval {
   T* pair = nullptr;             // P x 3: the pair's force contribution
   double* Satom = nullptr;       // A x 6: sum over the atom's pairs of the stress products (xx yy zz yz xz xy)
   double* Eatom = nullptr;       // A: energy of each atom (written for the linear model)
+  double* part = nullptr;        // eval_part_doubles: sums over parts of large structures
 };
 
 // Descriptor kernel (bispectrum.cu): B (A x nch*K) and w_ch * dB (P x 3 x nch*K) of the batch.  Atoms are taken in `order` (null: index order) through `counter` (one int
@@ -477,8 +478,11 @@ template <typename T>
 cudaError_t launch_lin_rows(const DevBatch& b, const DevRows& rows, const BsoParams& p, int KK, const int* rev,
                             const T* B, const T* dB, T* Sp, T* X, cudaStream_t st);
 // E (S), F (3A) and S (6S) from the atoms' energies and stresses and the pairs' forces of evaluation.
+size_t eval_part_doubles(int A, int S);
+// max_atoms: atoms of the largest structure
 template <typename T>
-cudaError_t launch_eval_gather(const DevBatch& b, const BsoParams& p, const int* rev, const DevEval<T>& ev, double* E,
+cudaError_t launch_eval_gather(const DevBatch& b, const BsoParams& p, const int* rev, const DevEval<T>& ev,
+                               int max_atoms, double* E,
                                double* F, double* S, cudaStream_t st);
 // Atoms ordered by descending neighbour count (the descriptor kernel's queue); tmp holds
 // atom_order_tmp_ints(maxnn) ints.

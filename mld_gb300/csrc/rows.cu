@@ -130,41 +130,65 @@ __global__ void k_eval_forces(int A, const int* __restrict__ nbr_off, const int*
   F[t] = sum;
 }
 
-// Evaluation, one CTA per structure: E_s = sum_i Eatom_i, S_s = sign_stress*3/V * sum_i Satom_i;
-// per-thread sums over a fixed atom stride, then a fixed tree over the lanes and the warps.
-constexpr int kStructThreads = 1024;
+// Evaluation: E_s = sum_i Eatom_i, S_s = sign_stress*3/V * sum_i Satom_i.  Grid (S, chunks of kStructChunk
+// atoms of the largest structure); per-thread sums over a fixed atom stride, a fixed tree over the lanes,
+// the warps in order.  A structure of one chunk is finished here, the chunks of a larger one by
+// k_eval_struct_sum.  Bound: the FP64 pipe makes two sums a clock and SM, so large structures are spread
+// (20,000 atoms took 55 us in one CTA of 1024 threads: the step 2.53 -> 2.49 ms) and warps without atoms
+// add nothing.
+constexpr int kStructThreads = 256, kStructChunk = 1024;
+__device__ __forceinline__ void put_struct(int s, int c, double t, const double* volume, double sign_stress, double* E,
+                                           double* S) {
+  if (c == 0) E[s] = t;
+  else S[6 * (size_t)s + c - 1] = sign_stress * 3.0 / volume[s] * t;
+}
 __global__ void __launch_bounds__(kStructThreads) k_eval_struct(const int* __restrict__ atom_start,
                                                                 const double* __restrict__ Satom,
                                                                 const double* __restrict__ Eatom,
                                                                 const double* __restrict__ volume, double sign_stress,
-                                                                double* __restrict__ E, double* __restrict__ S) {
+                                                                double* __restrict__ part, double* __restrict__ E,
+                                                                double* __restrict__ S) {
   __shared__ double red[7][kStructThreads / 32];
-  const int s = blockIdx.x, tid = threadIdx.x;
+  const int s = blockIdx.x, tid = threadIdx.x, warp = tid >> 5;
+  const int start = atom_start[s], n = atom_start[s + 1] - start, c0 = blockIdx.y * kStructChunk;
+  if (c0 > 0 && c0 >= n) return;
   double v[7] = {0, 0, 0, 0, 0, 0, 0};
-  const int a1 = atom_start[s + 1];
-  for (int i = atom_start[s] + tid; i < a1; i += kStructThreads) {
+  const int a1 = start + min(n, c0 + kStructChunk), a0 = start + c0;
+#pragma unroll 4
+  for (int i = a0 + tid; i < a1; i += kStructThreads) {
     v[0] += Eatom[i];
 #pragma unroll
     for (int c = 0; c < 6; ++c) v[1 + c] += Satom[(size_t)i * 6 + c];
   }
-  // (warps without atoms add nothing: their sums are zero.  The FP64 pipe makes two sums a clock.)
-  const bool some = atom_start[s] + (tid & ~31) < a1;
+  const bool some = a0 + (tid & ~31) < a1;
 #pragma unroll
   for (int c = 0; c < 7; ++c) {
     if (some)
       for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
-    if ((tid & 31) == 0) red[c][tid >> 5] = v[c];
+    if ((tid & 31) == 0) red[c][warp] = v[c];
   }
   __syncthreads();
-  const int c = tid >> 5;
-  if (c < 7) {
-    double t = red[c][tid & 31];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if ((tid & 31) == 0) {
-      if (c == 0) E[s] = t;
-      else S[6 * (size_t)s + c - 1] = sign_stress * 3.0 / volume[s] * t;
-    }
-  }
+  if (tid >= 7) return;
+  double t = red[tid][0];
+#pragma unroll
+  for (int w = 1; w < kStructThreads / 32; ++w) t += red[tid][w];
+  if (n <= kStructChunk) put_struct(s, tid, t, volume, sign_stress, E, S);
+  else part[7 * ((size_t)(start / kStructChunk) + s + blockIdx.y) + tid] = t;
+}
+
+// a warp per sum, lane l adds the chunks l, l + 32, ... in turn, then a fixed xor tree
+__global__ void __launch_bounds__(7 * 32) k_eval_struct_sum(const int* __restrict__ atom_start,
+                                                            const double* __restrict__ part,
+                                                            const double* __restrict__ volume, double sign_stress,
+                                                            double* __restrict__ E, double* __restrict__ S) {
+  const int s = blockIdx.x, c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int start = atom_start[s], n = atom_start[s + 1] - start;
+  if (n <= kStructChunk) return;
+  const double* p = part + 7 * ((size_t)(start / kStructChunk) + s) + c;
+  double t = 0.0;
+  for (int k = lane; k < (n + kStructChunk - 1) / kStructChunk; k += 32) t += p[7 * (size_t)k];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) put_struct(s, c, t, volume, sign_stress, E, S);
 }
 
 // ---- longest-first atom order (counting sort on the neighbour count, descending) ----
@@ -245,23 +269,29 @@ cudaError_t launch_lin_rows(const DevBatch& b, const DevRows& rows, const BsoPar
   return cudaGetLastError();
 }
 
+size_t eval_part_doubles(int A, int S) { return 7 * ((size_t)A / kStructChunk + S + 1); }
+
 template <typename T>
-cudaError_t launch_eval_gather(const DevBatch& b, const BsoParams& p, const int* rev, const DevEval<T>& ev, double* E,
-                               double* F, double* S, cudaStream_t st) {
+cudaError_t launch_eval_gather(const DevBatch& b, const BsoParams& p, const int* rev, const DevEval<T>& ev, int max_atoms,
+                               double* E, double* F, double* S, cudaStream_t st) {
   if (b.A == 0) return cudaSuccess;
   const long long n = 3LL * b.A;
   // small blocks: a cell of some fifty atoms, whose sums take the FP64 pipe, spreads over several SMs
   k_eval_forces<T><<<(unsigned)((n + 63) / 64), 64, 0, st>>>(b.A, b.nbr_off, rev, ev.pair, F);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_eval_struct<<<b.S, kStructThreads, 0, st>>>(b.atom_start, ev.Satom, ev.Eatom, b.volume, p.sign_stress, E, S);
+  const unsigned chunks = (unsigned)std::max(1, (max_atoms + kStructChunk - 1) / kStructChunk);
+  k_eval_struct<<<dim3(b.S, chunks), kStructThreads, 0, st>>>(b.atom_start, ev.Satom, ev.Eatom, b.volume, p.sign_stress,
+                                                              ev.part, E, S);
+  if (chunks > 1)
+    k_eval_struct_sum<<<b.S, 7 * 32, 0, st>>>(b.atom_start, ev.part, b.volume, p.sign_stress, E, S);
   return cudaGetLastError();
 }
 
 template cudaError_t launch_eval_gather<double>(const DevBatch&, const BsoParams&, const int*, const DevEval<double>&,
-                                                double*, double*, double*, cudaStream_t);
+                                                int, double*, double*, double*, cudaStream_t);
 template cudaError_t launch_eval_gather<float>(const DevBatch&, const BsoParams&, const int*, const DevEval<float>&,
-                                               double*, double*, double*, cudaStream_t);
+                                               int, double*, double*, double*, cudaStream_t);
 template cudaError_t launch_lin_rows<double>(const DevBatch&, const DevRows&, const BsoParams&, int, const int*,
                                              const double*, const double*, double*, double*, cudaStream_t);
 template cudaError_t launch_lin_rows<float>(const DevBatch&, const DevRows&, const BsoParams&, int, const int*,
