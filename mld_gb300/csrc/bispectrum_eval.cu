@@ -156,12 +156,14 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4_eval(
     nquad += c;
   }
 
+  // two places for the queue position in turn: an atom without neighbours passes no other barrier, and
+  // thread 0 publishes the next position while other warps may still read this one
   int nxt = 0;
   if (tid == 0) nxt = atomicAdd(args.counter, 1);
-  for (;;) {
-    if (tid == 0) snext[0] = nxt;
+  for (int turn = 0;; turn ^= 1) {
+    if (tid == 0) snext[turn] = nxt;
     __syncthreads();  // also orders the table staging and the previous atom's last reads
-    const int qi = snext[0];
+    const int qi = snext[turn];
     if (qi >= A) break;
     if (tid == 0) nxt = atomicAdd(args.counter, 1);
     const int atom = args.order ? args.order[qi] : qi;

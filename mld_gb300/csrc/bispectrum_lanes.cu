@@ -403,12 +403,14 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_c_half(CAr
   cx<T>* chalf = reinterpret_cast<cx<T>*>(smem_raw + sp.c);
   cx<T>* Us = reinterpret_cast<cx<T>*>(smem_raw + sp.U);
   for (int e = tid; e < HU; e += nth) shd[e] = tb.half_diag[e];
+  // two places for the queue position in turn: an atom without neighbours passes no other barrier, and
+  // thread 0 publishes the next position while other warps may still read this one
   int nxt = 0;
   if (tid == 0) nxt = atomicAdd(args.counter, 1);
-  for (;;) {
-    if (tid == 0) snext[0] = nxt;
+  for (int turn = 0;; turn ^= 1) {
+    if (tid == 0) snext[turn] = nxt;
     __syncthreads();
-    const int qi = snext[0];
+    const int qi = snext[turn];
     if (qi >= A) break;
     if (tid == 0) nxt = atomicAdd(args.counter, 1);
     const int atom = args.order ? args.order[qi] : args.first + qi;
