@@ -366,12 +366,12 @@ bool deriv_route(const mld_gpu_handle* h) {
   return h->A > h->nsm && bso4_available(h->dt, h->nch, (int)sizeof(T)) && deriv_available(h->dt, h->nch, (int)sizeof(T));
 }
 
-// atoms of a pass of the derivative route: whole tiles within kZCap, passes of equal size
-template <typename T>
-int deriv_pass(const mld_gpu_handle* h, size_t* zbytes, size_t* ybytes) {
-  const int tile = lane_tile(h->dt, (int)sizeof(T)), A = std::max(1, h->A);
-  const size_t yper = (size_t)h->nch * h->dt.NYP * 2 * sizeof(T) * tile;
-  const size_t zper = (size_t)h->nch * h->dt.NZTP * 2 * sizeof(T) * tile;
+// atoms of a pass of the derivative route over `atoms` atoms: whole tiles within kZCap, passes of equal size
+int pass_of(const mld_gpu_handle* h, long long atoms, size_t* zbytes, size_t* ybytes) {
+  const int eb = h->mixed ? 4 : 8, tile = lane_tile(h->dt, eb);
+  const long long A = std::max<long long>(1, atoms);
+  const size_t yper = (size_t)h->nch * h->dt.NYP * 2 * eb * tile;
+  const size_t zper = (size_t)h->nch * h->dt.NZTP * 2 * eb * tile;
   const long long tiles = (A + tile - 1) / tile, most = std::max<long long>(1, (long long)(kZCap / (zper + yper)));
   const long long passes = (tiles + most - 1) / most, n = (tiles + passes - 1) / passes;
   *zbytes = (size_t)n * zper;
@@ -392,7 +392,7 @@ int launch_rows_descriptors(mld_gpu_handle* h, T* Bout, T* dB, const Bso4Launch&
     return MLD_OK;
   }
   size_t zb = 0, yb = 0;
-  const int pass = deriv_pass<T>(h, &zb, &yb);
+  const int pass = pass_of(h, h->A, &zb, &yb);
   void* c = bp_<void>(h, mld_gpu_handle::B_CHALF);
   void* z = bp_<void>(h, mld_gpu_handle::B_ZT);
   void* y = bp_<void>(h, mld_gpu_handle::B_YSCR);
@@ -463,7 +463,7 @@ template <typename T>
 int prepare_descriptors(mld_gpu_handle* h) {
   size_t zb = 0, yb = 0;
   if (deriv_route<T>(h)) {
-    const int pass = deriv_pass<T>(h, &zb, &yb);
+    const int pass = pass_of(h, h->A, &zb, &yb);
     CK(ensure(h, mld_gpu_handle::B_ZT, zb));
     CK(ensure(h, mld_gpu_handle::B_CHALF, sizeof(T) * 2 * (size_t)pass * h->nch * h->dt.HU));
   } else {
@@ -1784,7 +1784,7 @@ static int eval_run(mld_gpu_handle* h, double* out) {
     // the same terms, which are formed again where one pass (kZCap) does not hold them all
     const size_t na = (size_t)std::max(1, h->A);
     size_t zb = 0, yb = 0;
-    const int pass = deriv_pass<T>(h, &zb, &yb);
+    const int pass = pass_of(h, h->A, &zb, &yb);
     CK(ensure(h, mld_gpu_handle::B_EB, sizeof(T) * na * KK));
     CK(ensure(h, mld_gpu_handle::B_EBETA, sizeof(T) * na * h->nch * h->dt.NBLKP));
     CK(ensure(h, mld_gpu_handle::B_CHALF, sizeof(T) * 2 * na * h->nch * h->dt.HU));
@@ -1861,11 +1861,18 @@ int eval_launch(mld_gpu_handle* h, cudaEvent_t done, double** pinned_out) {
   return MLD_OK;
 }
 
-// bytes of an atom in the buffers between the evaluation's kernels
+// bytes of an atom in the buffers between the evaluation's kernels, but for the Z terms
 size_t eval_atom_bytes(const mld_gpu_handle* h) {
   const size_t eb = h->mixed ? 4 : 8, c = 2 * eb * h->nch * h->dt.HU;
   if (!h->quad) return 2 * c;  // c and y
-  return c + eb * (h->KK + (size_t)h->nch * h->dt.NBLKP + 2 * (size_t)h->nch * h->dt.NZTP);  // c, B, weights, Z terms
+  return c + eb * (h->KK + (size_t)h->nch * h->dt.NBLKP);  // c, B, weights
+}
+// bytes of the Z terms that the evaluation of a batch holds at a time
+size_t eval_z_bytes(const mld_gpu_handle* h, long long atoms) {
+  if (!h->quad || atoms <= 0) return 0;
+  size_t zb = 0, yb = 0;
+  pass_of(h, atoms, &zb, &yb);
+  return zb;
 }
 
 void eval_collect(const mld_gpu_handle* h, int s, double* E, double* F, double* Sout) {

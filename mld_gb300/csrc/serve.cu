@@ -33,6 +33,7 @@ void eval_collect(const mld_gpu_handle* h, int s, double* E, double* F, double* 
 int eval_weights_upload(mld_gpu_handle* h, const double* w_full);
 int handle_dims(const mld_gpu_handle* h, int* D, int* ldx, int* KK, int* nch);
 size_t eval_atom_bytes(const mld_gpu_handle* h);
+size_t eval_z_bytes(const mld_gpu_handle* h, long long atoms);
 void handle_release_buffers(mld_gpu_handle* h);
 }  // namespace mld
 
@@ -53,7 +54,7 @@ struct Request {
   double E = 0;
   std::vector<double> F;
   double S[6] = {0, 0, 0, 0, 0, 0};
-  double bytes = 0;
+  double bytes = 0;  // request_bytes
 };
 
 struct Slot {
@@ -90,7 +91,8 @@ int sfail(mld_gpu_server* s, int code, const std::string& msg) {
 }
 
 // device bytes of one structure's batch buffers: neighbour pairs (expected neighbours from the
-// number density within r_cut, 1.5x margin), per-atom buffers of the evaluation, the FP64 outputs
+// number density within r_cut, 1.5x margin), per-atom buffers of the evaluation, the FP64 outputs.  The
+// Z terms, of which a batch of any size holds only as many as a pass takes, are added by batch_bytes.
 double request_bytes(const mld_gpu_server* s, int nat, const double* cell) {
   const double* c = cell;
   const double vol = std::fabs(c[0] * (c[4] * c[8] - c[5] * c[7]) - c[1] * (c[3] * c[8] - c[5] * c[6]) +
@@ -102,6 +104,11 @@ double request_bytes(const mld_gpu_server* s, int nat, const double* cell) {
   // per pair: index, FP64 and FP32 displacement, reverse pair, the single-pass search row, the force;
   // per atom: position and outputs, energy and stress, and what the evaluation kernels hand on
   return pairs * (44.0 + 3.0 * eb) + nat * (24.0 + 64.0 + 56.0 + (double)mld::eval_atom_bytes(s->slots[0].h)) + 128.0;
+}
+
+// device bytes of a batch of `atoms` atoms whose structures' request_bytes add up to `sum`
+double batch_bytes(const mld_gpu_server* s, double sum, long long atoms) {
+  return sum + (double)mld::eval_z_bytes(s->slots[0].h, atoms);
 }
 
 void retire(mld_gpu_server* s, int idx) {
@@ -152,15 +159,16 @@ int launch(mld_gpu_server* s, int idx) {
     const long long id = s->queue.front();
     Request& r = s->reqs[id];
     const bool first = batch.empty();
-    if (!first && (used + r.bytes > share || atoms + r.nat > s->max_batch_atoms)) break;
-    if (first && r.bytes > s->budget) {
+    const double with = batch_bytes(s, used + r.bytes, atoms + r.nat);
+    if (!first && (with > share || atoms + r.nat > s->max_batch_atoms)) break;
+    if (first && with > s->budget) {
       s->queue.pop_front();
       r.state = 3;
       r.err = MLD_ERR_OOM;
       r.t_done = now_ms();
       continue;
     }
-    if (first && r.bytes > share) {
+    if (first && with > share) {
       // runs alone: hold it at the head (and launch nothing else) until every slot is idle
       if (bytes_in_flight(s) > 0) return MLD_OK;
       exclusive = true;
@@ -169,7 +177,7 @@ int launch(mld_gpu_server* s, int idx) {
     used += r.bytes;
     atoms += r.nat;
     s->queue.pop_front();
-    if (first && (r.bytes > share || r.nat > s->max_batch_atoms)) break;  // a large request runs alone
+    if (first && (with > share || r.nat > s->max_batch_atoms)) break;  // a large request runs alone
   }
   if (batch.empty()) return MLD_OK;
   std::vector<int> nat(batch.size());
@@ -202,10 +210,10 @@ int launch(mld_gpu_server* s, int idx) {
   }
   sl.batch = std::move(batch);
   sl.busy = true;
-  sl.bytes = used;
+  sl.bytes = batch_bytes(s, used, atoms);
   if (exclusive) s->exclusive_slot = idx;
   s->peak_in_flight = std::max(s->peak_in_flight, bytes_in_flight(s));
-  s->largest_request = std::max(s->largest_request, used);
+  s->largest_request = std::max(s->largest_request, sl.bytes);
   ++s->batches;
   return MLD_OK;
 }
