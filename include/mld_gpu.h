@@ -226,6 +226,12 @@ int mld_gpu_tuning(const mld_gpu_handle* h, int mode, int* shape, int* ncand, do
  * handle stays usable.  (0, 0) restores normal operation.  Process-wide; not for production use. */
 int mld_gpu_test_pipeline_timeout(int skip_loads, long long wait_limit_clocks);
 
+/* Test hook of the memory limits of one handle (no reference counterpart): pass_bytes bounds the
+ * Clebsch-Gordan terms and rows that a pass over the atoms of a batch holds (0: the default of 2 GB),
+ * and buffer_limit what the handle's device buffers may take together before an allocation fails as
+ * it does on a full device (0: no limit).  Passes shrink to what fits, with the same results. */
+int mld_gpu_test_memory(mld_gpu_handle* h, long long pass_bytes, long long buffer_limit);
+
 /* ---------------------------------------------------------------------------------------
  * Serving loop (evaluation with a fitted potential under continuous batching; the evaluation
  * side of mld.F90:1579-1867 as driven by mld_md_driver.F90:324-375,579-651).

@@ -31,7 +31,7 @@ EXPORTED = ["mld_gpu_config_defaults", "mld_gpu_create", "mld_gpu_destroy", "mld
             "mld_gpu_set_kernel_points", "mld_gpu_server_create", "mld_gpu_server_destroy",
             "mld_gpu_server_last_error", "mld_gpu_server_submit", "mld_gpu_server_progress",
             "mld_gpu_server_result", "mld_gpu_server_wait", "mld_gpu_server_stats", "mld_gpu_server_admission",
-            "mld_gpu_test_pipeline_timeout", "mld_gpu_tuning"]
+            "mld_gpu_test_pipeline_timeout", "mld_gpu_test_memory", "mld_gpu_tuning"]
 NPHASE = 6
 PHASES = ["neighbours", "rows", "descriptors", "gram", "solve", "predict"]
 
@@ -109,6 +109,7 @@ def load(path: str = LIB_PATH) -> ctypes.CDLL:
     L.mld_gpu_timer_stop.argtypes = [P, ctypes.POINTER(D)]
     L.mld_gpu_work_counts.argtypes = [P, P]
     L.mld_gpu_peak_flops.argtypes = [P, I, ctypes.POINTER(D)]
+    L.mld_gpu_test_memory.argtypes = [P, LL, LL]
     L.mld_gpu_descriptors_noalloc.argtypes = [ctypes.POINTER(MldGpuConfig), I, P, P, P, P, P, ctypes.c_char_p, I]
     for n in EXPORTED:
         if n not in ("mld_gpu_config_defaults", "mld_gpu_destroy", "mld_gpu_last_error"):

@@ -30,6 +30,8 @@ struct RowLayout {
   long long M = 0;
 };
 
+constexpr size_t kZCap = size_t(2) << 30;  // Z terms and Y rows held at a time
+
 }  // namespace
 
 struct mld_gpu_handle {
@@ -114,6 +116,9 @@ struct mld_gpu_handle {
   long long rows_graph_launches = 0;
   bool rows_graph_off = false;  // a capture failed once: run the stage directly from then on
 
+  size_t z_cap = kZCap;     // Z terms and Y rows of a pass: less once they did not fit (ensure_passes)
+  size_t buffer_limit = 0;  // test hook: bytes that the buffers may take together (0: what the device has)
+
   std::vector<void*> owned;  // table allocations
   Buf bufs[80];
   enum {
@@ -150,6 +155,32 @@ int cuda_fail(mld_gpu_handle* h, cudaError_t e, const char* where) {
     if (_e != cudaSuccess) return cuda_fail(h, _e, #call); \
   } while (0)
 
+cudaError_t grab(mld_gpu_handle* h, void** p, size_t bytes) {
+  if (h->buffer_limit) {
+    size_t held = 0;
+    for (const Buf& bf : h->bufs) held += bf.cap;
+    if (held + bytes > h->buffer_limit) return cudaErrorMemoryAllocation;
+  }
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) (void)cudaGetLastError();  // a failed allocation leaves no error for later launches
+  return e;
+}
+
+// Frees the Z terms and Y rows and halves what a later pass may take; false if there were none.
+bool shrink_passes(mld_gpu_handle* h) {
+  size_t held = 0;
+  for (int id : {mld_gpu_handle::B_ZT, mld_gpu_handle::B_YSCR}) {
+    Buf& bf = h->bufs[id];
+    if (bf.p) cudaFree(bf.p);
+    held += bf.cap;
+    bf = Buf{};
+  }
+  if (!held) return false;
+  ++h->buf_gen;
+  h->z_cap = std::min(h->z_cap, held / 2);
+  return true;
+}
+
 cudaError_t ensure(mld_gpu_handle* h, int id, size_t bytes) {
   Buf& bf = h->bufs[id];
   if (bytes <= bf.cap && bf.p) return cudaSuccess;
@@ -159,12 +190,15 @@ cudaError_t ensure(mld_gpu_handle* h, int id, size_t bytes) {
   bf.cap = 0;
   size_t want = std::max<size_t>(bytes, 256);
   want = want + want / 8;  // headroom for slowly growing batches
-  cudaError_t e = cudaMalloc(&bf.p, want);
+  cudaError_t e = grab(h, &bf.p, want);
   if (e == cudaErrorMemoryAllocation) {  // memory kept by mld_gpu_gram_rows may be what is missing
-    (void)cudaGetLastError();
     rows_pool_trim(h->device);
-    e = cudaMalloc(&bf.p, want);
+    e = grab(h, &bf.p, want);
   }
+  // passes can be smaller; so do without: the passes' own buffers (ensure_passes), optional workspaces
+  const bool own = id == mld_gpu_handle::B_ZT || id == mld_gpu_handle::B_YSCR;
+  const bool optional = id == mld_gpu_handle::B_NBRTMP || id == mld_gpu_handle::B_GP;
+  if (e == cudaErrorMemoryAllocation && !own && !optional && shrink_passes(h)) e = grab(h, &bf.p, want);
   if (e != cudaSuccess) return e;
   bf.cap = want;
   return cudaSuccess;
@@ -358,25 +392,42 @@ constexpr size_t kKrrTcWorkspaceCap = size_t(6) << 30;
 // Design rows of one Fe structure at j_max 4, one kernel / three: 100 atoms FP64 0.69 / 1.00 ms, FP32
 // 309 / 349 us; 250 atoms 1.33 / 1.28 ms, 426 / 418 us; 1000 atoms FP64 3.38 / 3.12 ms; 23,000 FP32
 // atoms in 60 structures at j_max 2, FP64: 5.2 / 3.2 ms.
-constexpr size_t kZCap = size_t(2) << 30;  // Z terms and Y rows held at a time
-
 template <typename T>
 bool deriv_route(const mld_gpu_handle* h) {
   // (a configuration is taken or refused whatever the batch)
   return h->A > h->nsm && bso4_available(h->dt, h->nch, (int)sizeof(T)) && deriv_available(h->dt, h->nch, (int)sizeof(T));
 }
 
-// atoms of a pass of the derivative route over `atoms` atoms: whole tiles within kZCap, passes of equal size
-int pass_of(const mld_gpu_handle* h, long long atoms, size_t* zbytes, size_t* ybytes) {
+// atoms of a pass over `atoms` atoms: whole tiles whose Z terms and Y rows fit in `cap`, passes of equal size
+int pass_of(const mld_gpu_handle* h, size_t cap, long long atoms, size_t* zbytes, size_t* ybytes) {
   const int eb = h->mixed ? 4 : 8, tile = lane_tile(h->dt, eb);
   const long long A = std::max<long long>(1, atoms);
   const size_t yper = (size_t)h->nch * h->dt.NYP * 2 * eb * tile;
   const size_t zper = (size_t)h->nch * h->dt.NZTP * 2 * eb * tile;
-  const long long tiles = (A + tile - 1) / tile, most = std::max<long long>(1, (long long)(kZCap / (zper + yper)));
+  const long long tiles = (A + tile - 1) / tile, most = std::max<long long>(1, (long long)(cap / (zper + yper)));
   const long long passes = (tiles + most - 1) / most, n = (tiles + passes - 1) / passes;
   *zbytes = (size_t)n * zper;
   *ybytes = (size_t)n * yper;
   return (int)std::min<long long>(n * tile, A);
+}
+
+// Buffers of the passes over Z terms (and, for rows, Y rows): where they do not fit, passes of half the
+// size, down to one tile of atoms.
+int ensure_passes(mld_gpu_handle* h, bool rows, int* pass) {
+  const size_t cxb = h->mixed ? 8 : 16;
+  for (;;) {
+    size_t zb = 0, yb = 0;
+    *pass = pass_of(h, h->z_cap, h->A, &zb, &yb);
+    if (rows) CK(ensure(h, mld_gpu_handle::B_CHALF, cxb * (size_t)*pass * h->nch * h->dt.HU));
+    cudaError_t e = ensure(h, mld_gpu_handle::B_ZT, zb);
+    if (e == cudaSuccess && rows) e = ensure(h, mld_gpu_handle::B_YSCR, yb);
+    if (e != cudaErrorMemoryAllocation || *pass <= lane_tile(h->dt, h->mixed ? 4 : 8)) {
+      CK(e);
+      return MLD_OK;
+    }
+    shrink_passes(h);
+    h->z_cap = (zb + yb) / 2;
+  }
 }
 
 // B of the staged batch into Bout and w_ch * dB into dB, with one launch shape
@@ -392,7 +443,7 @@ int launch_rows_descriptors(mld_gpu_handle* h, T* Bout, T* dB, const Bso4Launch&
     return MLD_OK;
   }
   size_t zb = 0, yb = 0;
-  const int pass = pass_of(h, h->A, &zb, &yb);
+  const int pass = pass_of(h, h->z_cap, h->A, &zb, &yb);  // as ensure_passes left it
   void* c = bp_<void>(h, mld_gpu_handle::B_CHALF);
   void* z = bp_<void>(h, mld_gpu_handle::B_ZT);
   void* y = bp_<void>(h, mld_gpu_handle::B_YSCR);
@@ -458,19 +509,16 @@ int tuned_launch(mld_gpu_handle* h, T* Bout, T* dB) {
   return MLD_OK;
 }
 
-// buffers of run_descriptors with derivatives
+// buffers of run_descriptors with derivatives; the passes take what the others leave
 template <typename T>
 int prepare_descriptors(mld_gpu_handle* h) {
-  size_t zb = 0, yb = 0;
-  if (deriv_route<T>(h)) {
-    const int pass = pass_of(h, h->A, &zb, &yb);
-    CK(ensure(h, mld_gpu_handle::B_ZT, zb));
-    CK(ensure(h, mld_gpu_handle::B_CHALF, sizeof(T) * 2 * (size_t)pass * h->nch * h->dt.HU));
-  } else {
-    yb = bso4_y_scratch_bytes(h->dt, h->nch, (int)sizeof(T), 2 * std::max(1, h->nsm));
-  }
-  if (yb) CK(ensure(h, mld_gpu_handle::B_YSCR, yb));
   CK(ensure(h, mld_gpu_handle::B_DBOUT, sizeof(T) * std::max<size_t>((size_t)h->b.P * 3 * h->KK, 1)));
+  if (deriv_route<T>(h)) {
+    int pass = 0;
+    return ensure_passes(h, true, &pass);
+  }
+  const size_t yb = bso4_y_scratch_bytes(h->dt, h->nch, (int)sizeof(T), 2 * std::max(1, h->nsm));
+  if (yb) CK(ensure(h, mld_gpu_handle::B_YSCR, yb));
   return MLD_OK;
 }
 
@@ -1781,14 +1829,14 @@ static int eval_run(mld_gpu_handle* h, double* out) {
   ev.w0 = h->ew0;
   if (h->quad) {
     // c and Z terms of every atom, B from them; its weights and energy; then the evaluation kernel on
-    // the same terms, which are formed again where one pass (kZCap) does not hold them all
+    // the same terms, which are formed again where one pass does not hold them all
     const size_t na = (size_t)std::max(1, h->A);
-    size_t zb = 0, yb = 0;
-    const int pass = pass_of(h, h->A, &zb, &yb);
     CK(ensure(h, mld_gpu_handle::B_EB, sizeof(T) * na * KK));
     CK(ensure(h, mld_gpu_handle::B_EBETA, sizeof(T) * na * h->nch * h->dt.NBLKP));
     CK(ensure(h, mld_gpu_handle::B_CHALF, sizeof(T) * 2 * na * h->nch * h->dt.HU));
-    CK(ensure(h, mld_gpu_handle::B_ZT, zb));
+    int pass = 0;
+    const int rcp = ensure_passes(h, false, &pass);
+    if (rcp) return rcp;
     T* B = bp_<T>(h, mld_gpu_handle::B_EB);
     T* gamma = bp_<T>(h, mld_gpu_handle::B_EBETA);
     T* c = bp_<T>(h, mld_gpu_handle::B_CHALF);
@@ -1871,7 +1919,7 @@ size_t eval_atom_bytes(const mld_gpu_handle* h) {
 size_t eval_z_bytes(const mld_gpu_handle* h, long long atoms) {
   if (!h->quad || atoms <= 0) return 0;
   size_t zb = 0, yb = 0;
-  pass_of(h, atoms, &zb, &yb);
+  pass_of(h, kZCap, atoms, &zb, &yb);
   return zb;
 }
 
@@ -1906,6 +1954,7 @@ void handle_release_buffers(mld_gpu_handle* h) {
     bf.p = nullptr;
     bf.cap = 0;
   }
+  h->z_cap = kZCap;
   h->has_batch = false;
   h->nbr_valid = false;
 }
@@ -2050,6 +2099,14 @@ extern "C" int mld_gpu_tuning(const mld_gpu_handle* h, int mode, int* shape, int
 extern "C" int mld_gpu_test_pipeline_timeout(int skip_loads, long long wait_limit_clocks) {
   if (skip_loads < 0 || wait_limit_clocks < 0) return MLD_ERR_INVALID;
   mld::gram_tc_test_timeout(skip_loads, wait_limit_clocks);
+  return MLD_OK;
+}
+
+extern "C" int mld_gpu_test_memory(mld_gpu_handle* h, long long pass_bytes, long long buffer_limit) {
+  if (!h || pass_bytes < 0 || buffer_limit < 0) return MLD_ERR_INVALID;
+  h->z_cap = pass_bytes ? (size_t)pass_bytes : kZCap;
+  h->buffer_limit = (size_t)buffer_limit;
+  ++h->buf_gen;
   return MLD_OK;
 }
 

@@ -50,7 +50,8 @@ module mld_gpu_mod
             mld_gpu_server_admission, &
             mld_gpu_descriptor_derivatives, mld_gpu_last_error, mld_gpu_server_last_error, &
             mld_gpu_set_profiling, mld_gpu_profile, mld_gpu_timer_start, mld_gpu_timer_stop, &
-            mld_gpu_work_counts, mld_gpu_peak_flops, mld_gpu_descriptors_noalloc, mld_gpu_test_pipeline_timeout, mld_gpu_tuning, &
+            mld_gpu_work_counts, mld_gpu_peak_flops, mld_gpu_descriptors_noalloc, mld_gpu_test_pipeline_timeout, &
+            mld_gpu_test_memory, mld_gpu_tuning, &
             mld_gpu_synchronize
 
   interface
@@ -286,6 +287,12 @@ module mld_gpu_mod
       import :: c_int, c_long_long
       integer(c_int), value :: skip_loads
       integer(c_long_long), value :: wait_limit_clocks
+    end function
+
+    integer(c_int) function mld_gpu_test_memory(h, pass_bytes, buffer_limit) bind(C, name="mld_gpu_test_memory")
+      import :: c_int, c_ptr, c_long_long
+      type(c_ptr), value :: h
+      integer(c_long_long), value :: pass_bytes, buffer_limit
     end function
 
     integer(c_int) function mld_gpu_server_admission(srv, peak_bytes_in_flight, share_bytes, largest_batch_bytes) &
