@@ -186,10 +186,9 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_bso4(Kerne
 
   // thread 0 takes the next queue position while the current atom runs; it publishes it at the
   // top of the loop, after at least one barrier that follows every thread's read of the last one
-  int nxt = 0;
-  if (tid == 0) nxt = atomicAdd(args.counter, 1);
+  int nxt = first_ticket();
   for (;;) {
-    if (tid == 0) snext[0] = nxt;
+    if (tid == 0) snext[0] = ticket_position(nxt);
     __syncthreads();  // also orders the table staging and the previous atom's last reads
     const int qi = snext[0];
     if (qi >= A) break;

@@ -46,6 +46,15 @@ __device__ __forceinline__ cx<double> fma2(cx<double> a, cx<double> b, cx<double
 constexpr int kNW = 8;  // warps per CTA (== kZWarps)
 static_assert(kNW == kZWarps, "phase-2 schedule is built for the CTA's warps");
 
+// ---- work queue --------------------------------------------------------------------------------
+// A persistent CTA starts with the position of its block index; the counter hands out those behind the
+// grid.  Taken from the counter too, the first positions went to the CTAs that started first, which ask
+// for their second atom at once: of as many CTAs as atoms some took two and others none (derivatives of
+// 16 / 54 / 152 Fe atoms in FP64 at j_max 4: 860 / 900 / 925 us in most calls, 460 / 500 / 530 now).  A
+// ticket becomes a position where it is used: an addition behind the counter's read would wait for it.
+__device__ __forceinline__ int first_ticket() { return (int)blockIdx.x - (int)gridDim.x; }
+__device__ __forceinline__ int ticket_position(int ticket) { return ticket + (int)gridDim.x; }
+
 // ---- neighbour geometry --------------------------------------------------------------------
 // Record of a neighbour (kGeo values, a multiple of 4 so that records stay 16-byte aligned); the first
 // kGeoDeriv are what the derivatives need:

@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kDW * 32, 1) k_deriv(DerivArgs<T> args) {
       t += two;
     }
     *sntile = n;
-    snext[0] = atomicAdd(args.counter, 1);
+    snext[0] = ticket_position(first_ticket());
   }
   __syncthreads();
   const int ntile = *sntile;
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(kDW * 32, 1) k_deriv(DerivArgs<T> args) {
         if (tid == 0) {
           *sjob = 0;
           if (k == 0) {
-            snext[0] = nxt;  // asked for one atom ahead
+            snext[0] = ticket_position(nxt);  // asked for one atom ahead
             nxt = atomicAdd(args.counter, 1);
           }
         }

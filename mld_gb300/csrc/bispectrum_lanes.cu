@@ -405,10 +405,9 @@ __global__ void __launch_bounds__(kNW * 32, sizeof(T) == 4 ? 2 : 1) k_c_half(CAr
   for (int e = tid; e < HU; e += nth) shd[e] = tb.half_diag[e];
   // two places for the queue position in turn: an atom without neighbours passes no other barrier, and
   // thread 0 publishes the next position while other warps may still read this one
-  int nxt = 0;
-  if (tid == 0) nxt = atomicAdd(args.counter, 1);
+  int nxt = first_ticket();
   for (int turn = 0;; turn ^= 1) {
-    if (tid == 0) snext[turn] = nxt;
+    if (tid == 0) snext[turn] = ticket_position(nxt);
     __syncthreads();
     const int qi = snext[turn];
     if (qi >= A) break;
