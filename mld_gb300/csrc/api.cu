@@ -1783,8 +1783,7 @@ int eval_weights_upload(mld_gpu_handle* h, const double* w_full) {
     for (int i = 0; i < KK; ++i)
       for (int j = 0; j < KK; ++j) hw[KK + (size_t)i * KK + j] = W[(size_t)i * KK + j] + W[(size_t)j * KK + i];
   }
-  const size_t eb = h->mixed ? sizeof(float) : sizeof(double);
-  const size_t next = h->quad ? (h->mixed ? sizeof(float2) * n2 : 0) : eb * h->nch * h->dt.NBLKP;
+  const size_t next = h->quad ? (h->mixed ? sizeof(float2) * n2 : 0) : sizeof(double) * h->nch * h->dt.NBLKP;
   CK(ensure(h, mld_gpu_handle::B_EW, sizeof(double) * hw.size() + next + 256));
   double* dw = bp_<double>(h, mld_gpu_handle::B_EW);
   CK(cudaMemcpyAsync(dw, hw.data(), sizeof(double) * hw.size(), cudaMemcpyHostToDevice, h->st));
@@ -1792,11 +1791,9 @@ int eval_weights_upload(mld_gpu_handle* h, const double* w_full) {
   if (h->quad) {
     if (h->mixed) CK(launch_split_pairs(dw + KK, static_cast<float2*>(ext), n2, h->st));
   } else if (h->mixed) {
-    CK(launch_eval_gamma<float>(h->dt, nullptr, 1, h->nch, dw, nullptr, nullptr, 0.0, static_cast<float*>(ext), nullptr,
-                                h->st));
+    CK(launch_block_weights<float>(h->dt, h->nch, dw, ext, h->st));
   } else {
-    CK(launch_eval_gamma<double>(h->dt, nullptr, 1, h->nch, dw, nullptr, nullptr, 0.0, static_cast<double*>(ext), nullptr,
-                                 h->st));
+    CK(launch_block_weights<double>(h->dt, h->nch, dw, ext, h->st));
   }
   CK(cudaStreamSynchronize(h->st));
   h->ew0 = w_full[0];
@@ -1871,7 +1868,7 @@ static int eval_run(mld_gpu_handle* h, double* out) {
     ev.c = bp_<void>(h, mld_gpu_handle::B_CHALF);
     ev.y = bp_<void>(h, mld_gpu_handle::B_EY);
     CK(launch_c_half<T>(h->dt, h->b, h->bp, 0, h->A, order, false, counter, bp_<void>(h, mld_gpu_handle::B_CHALF), h->st));
-    CK(launch_lane_y<T>(h->dt, h->b, h->bp, 0, h->A, ev.c, static_cast<const T*>(wext), bp_<void>(h, mld_gpu_handle::B_EY), h->st));
+    CK(launch_lane_y<T>(h->dt, h->b, h->bp, 0, h->A, ev.c, wext, bp_<void>(h, mld_gpu_handle::B_EY), h->st));
     CK(launch_bso4_eval<T>(h->dt, h->b, h->bp, ev, order, h->A, counter, h->st));
     nl(h, 3);
   }

@@ -76,8 +76,6 @@ __device__ __forceinline__ double vmul(double a, double b) { return a * b; }
 __device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ double vneg(double a) { return -a; }
 __device__ __forceinline__ double vadd(double a, double b) { return a + b; }
-__device__ __forceinline__ F2 vdup(float a, F2) { return pack(a, a); }
-__device__ __forceinline__ double vdup(double a, double) { return a; }
 
 // complex value of a lane's atoms (16 bytes)
 template <typename V>
@@ -85,6 +83,20 @@ struct alignas(16) vcx {
   V x, y;
 };
 
+// acc += weight * z.  In FP32 a weight is a double-FP32 pair: rounded to 32 bits, it would shift the energies
+// of all atoms alike.  The low part joins the product, whose rounding keeps it on average; next to the sum
+// it would be below the last bit.
+__device__ __forceinline__ void add_weighted(F2 weight, vcx<F2> z, vcx<F2>& acc) {
+  float g[2];
+  unpack(weight, g);
+  const F2 h = pack(g[0], g[0]), l = pack(g[1], g[1]);
+  acc.x = vadd(acc.x, vfma(h, z.x, vmul(l, z.x)));
+  acc.y = vadd(acc.y, vfma(h, z.y, vmul(l, z.y)));
+}
+__device__ __forceinline__ void add_weighted(double weight, vcx<double> z, vcx<double>& acc) {
+  acc.x = vfma(weight, z.x, acc.x);
+  acc.y = vfma(weight, z.y, acc.y);
+}
 
 // the atoms' values one after the other, (re, im) each
 __device__ __forceinline__ vcx<F2> interleave(vcx<F2> v) {
@@ -104,7 +116,7 @@ struct LaneArgs {
   const void* cg;       // FP32: every coefficient twice (for the packed instructions)
   const cx<T>* c;       // A x nch x HU
   const int* nbr_off;   // of the first atom
-  const T* gamma;       // y: nch * NBLKP
+  const void* gamma;    // y: nch * NBLKP weights (FP32: double-FP32 pairs)
   int A, nch;
   T* B;                 // A x nch*K
   cx<T>* y;             // A x nch x HU
@@ -222,21 +234,14 @@ __device__ __forceinline__ void lane_record(uint4 z0, uint4 z1, const vcx<V>* __
     const int off = z0.w >> 24;
     if (off == 0) {  // pairs that reach the highest layers: most of the work
 #pragma unroll
-      for (int o = 0; o < NJ; ++o) {
-        const V g = gam[out_of(z1, o)];
-        acc[o].x = vfma(g, zs[o].x, acc[o].x);
-        acc[o].y = vfma(g, zs[o].y, acc[o].y);
-      }
+      for (int o = 0; o < NJ; ++o) add_weighted(gam[out_of(z1, o)], zs[o], acc[o]);
     } else {
 #pragma unroll
       for (int o = 0; o < NJ; ++o) {
         const V g = gam[out_of(z1, o)];
 #pragma unroll
         for (int k = 1; k + o < kMaxZOut; ++k)
-          if (k == off) {
-            acc[k + o].x = vfma(g, zs[o].x, acc[k + o].x);
-            acc[k + o].y = vfma(g, zs[o].y, acc[k + o].y);
-          }
+          if (k == off) add_weighted(g, zs[o], acc[k + o]);
       }
     }
   } else {
@@ -284,7 +289,7 @@ __global__ void __launch_bounds__(LaneVec<T>::warps * 32, 1) k_lanes(LaneArgs<T>
     cg = scg;
   }
   if constexpr (kMode == kLaneY) {
-    for (int b = tid; b < tb.NBLKP; b += nth) sg[b] = vdup(args.gamma[ch * tb.NBLKP + b], V{});
+    for (int b = tid; b < tb.NBLKP; b += nth) sg[b] = static_cast<const V*>(args.gamma)[ch * tb.NBLKP + b];
   }
   __syncthreads();
   const int al = lane < lanes ? lane : lane - lanes;  // (16 lanes: both halves of the warp hold the same atoms)
@@ -637,7 +642,7 @@ cudaError_t launch_lane_descriptors(const DevTables& tb, const DevBatch& b, cons
 
 template <typename T>
 cudaError_t launch_lane_y(const DevTables& tb, const DevBatch& b, const BsoParams& p, int first, int count,
-                          const void* c, const T* gamma, void* y, cudaStream_t st) {
+                          const void* c, const void* gamma, void* y, cudaStream_t st) {
   LaneArgs<T> a = lane_args<T>(tb, b, p, first, count, c);
   a.recs = tb.yrecs;
   a.jobs = tb.yjobs;
@@ -709,8 +714,8 @@ template cudaError_t launch_lane_descriptors<double>(const DevTables&, const Dev
 template cudaError_t launch_lane_descriptors<float>(const DevTables&, const DevBatch&, const BsoParams&, int, int,
                                                     const void*, float*, cudaStream_t);
 template cudaError_t launch_lane_y<double>(const DevTables&, const DevBatch&, const BsoParams&, int, int, const void*,
-                                           const double*, void*, cudaStream_t);
+                                           const void*, void*, cudaStream_t);
 template cudaError_t launch_lane_y<float>(const DevTables&, const DevBatch&, const BsoParams&, int, int, const void*,
-                                          const float*, void*, cudaStream_t);
+                                          const void*, void*, cudaStream_t);
 
 }  // namespace mld

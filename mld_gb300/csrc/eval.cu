@@ -9,6 +9,8 @@
 // that use block b: the evaluation kernel takes gamma instead of beta.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "ds.cuh"
 #include "mld_internal.h"
 
@@ -31,15 +33,23 @@ __global__ void k_split_pairs(const double* __restrict__ in, float2* __restrict_
 // read consecutive k), the atom's energy w0 + B . (beta + w_lin) / 2 and gamma of every channel and
 // block.  The sums over j run in double-FP32 for FP32 descriptors (2^-44 relative; FP64 issues at 1/64
 // of the FP32 rate and took 182 us of a 4,001-atom step with K = 110, 2 channels), in FP64 for FP64
-// ones.  B null: beta = w_lin, no energy.
-template <typename T>
+// ones.  B null: beta = w_lin, no energy, and G holds every weight in full (a pair for T = float).
+__device__ __forceinline__ void put_weight(float* g, double v) { *g = (float)v; }
+__device__ __forceinline__ void put_weight(double* g, double v) { *g = v; }
+__device__ __forceinline__ void put_weight(float2* g, double v) {
+  float h, l;
+  ds_split(v, h, l);
+  *g = make_float2(h, l);
+}
+
+template <typename T, typename G>
 __global__ void __launch_bounds__(kGammaThreads) k_eval_gamma(const int* __restrict__ gam_off,
                                                               const GammaItem* __restrict__ gam, int nblk, int nch,
                                                               int K, int A, const T* __restrict__ B,
                                                               const double* __restrict__ wlin,
                                                               const double* __restrict__ wsym,
                                                               const float2* __restrict__ wsym32, double w0,
-                                                              T* __restrict__ gamma, double* __restrict__ Eatom) {
+                                                              G* __restrict__ gamma, double* __restrict__ Eatom) {
   extern __shared__ double beta[];  // [kGammaAtoms][nchK], then B as T
   __shared__ double red[kGammaAtoms][kGammaThreads / 32];
   const int tid = threadIdx.x, nchK = nch * K, a0 = blockIdx.x * kGammaAtoms;
@@ -81,7 +91,7 @@ __global__ void __launch_bounds__(kGammaThreads) k_eval_gamma(const int* __restr
       for (int a = 0; a < kGammaAtoms; ++a) e[a] = fma(0.5 * (double)bsh[a * nchK + k], v[a] + wlin[k], e[a]);
     }
 #pragma unroll
-    for (int a = 0; a < kGammaAtoms; ++a) beta[a * nchK + k] = (double)(T)v[a];  // in the method's precision
+    for (int a = 0; a < kGammaAtoms; ++a) beta[a * nchK + k] = B ? (double)(T)v[a] : v[a];  // B: in the method's precision
   }
   __syncthreads();
   for (int b = tid; b < nch * nblk; b += kGammaThreads) {
@@ -98,7 +108,7 @@ __global__ void __launch_bounds__(kGammaThreads) k_eval_gamma(const int* __restr
     }
 #pragma unroll
     for (int a = 0; a < kGammaAtoms; ++a)
-      if (a < na) gamma[(size_t)(a0 + a) * nch * nblk + b] = (T)g[a];
+      if (a < na) put_weight(gamma + (size_t)(a0 + a) * nch * nblk + b, g[a]);
   }
   if (!B) return;
 #pragma unroll
@@ -123,14 +133,22 @@ cudaError_t launch_eval_gamma(const DevTables& tb, const T* B, int A, int nch, c
                               const float2* wsym32, double w0, T* gamma, double* Eatom, cudaStream_t st) {
   if (A <= 0) return cudaSuccess;
   const size_t smem = (sizeof(double) + sizeof(T)) * kGammaAtoms * nch * tb.K;
-  if (B)
-    k_eval_gamma<T><<<(A + kGammaAtoms - 1) / kGammaAtoms, kGammaThreads, smem, st>>>(
-        tb.gamp_off, tb.gamp, tb.NBLKP, nch, tb.K, A, B, wlin, wsym, wsym32, w0, gamma, Eatom);
-  else
-    k_eval_gamma<T><<<1, kGammaThreads, smem, st>>>(tb.gamp_off, tb.gamp, tb.NBLKP, nch, tb.K, 1, nullptr, wlin, nullptr,
-                                                    nullptr, w0, gamma, nullptr);
+  k_eval_gamma<T, T><<<(A + kGammaAtoms - 1) / kGammaAtoms, kGammaThreads, smem, st>>>(
+      tb.gamp_off, tb.gamp, tb.NBLKP, nch, tb.K, A, B, wlin, wsym, wsym32, w0, gamma, Eatom);
   return cudaGetLastError();
 }
+
+template <typename T>
+cudaError_t launch_block_weights(const DevTables& tb, int nch, const double* wlin, void* gamma, cudaStream_t st) {
+  using G = typename std::conditional<sizeof(T) == 4, float2, double>::type;
+  const size_t smem = (sizeof(double) + sizeof(T)) * kGammaAtoms * nch * tb.K;
+  k_eval_gamma<T, G><<<1, kGammaThreads, smem, st>>>(tb.gamp_off, tb.gamp, tb.NBLKP, nch, tb.K, 1, nullptr, wlin,
+                                                     nullptr, nullptr, 0.0, static_cast<G*>(gamma), nullptr);
+  return cudaGetLastError();
+}
+
+template cudaError_t launch_block_weights<double>(const DevTables&, int, const double*, void*, cudaStream_t);
+template cudaError_t launch_block_weights<float>(const DevTables&, int, const double*, void*, cudaStream_t);
 
 template cudaError_t launch_eval_gamma<double>(const DevTables&, const double*, int, int, const double*, const double*,
                                                const float2*, double, double*, double*, cudaStream_t);

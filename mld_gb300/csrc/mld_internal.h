@@ -420,10 +420,11 @@ cudaError_t launch_c_half(const DevTables& tb, const DevBatch& b, const BsoParam
 template <typename T>
 cudaError_t launch_lane_descriptors(const DevTables& tb, const DevBatch& b, const BsoParams& p, int first, int count,
                                     const void* c, T* B, cudaStream_t st);
-// y = dE/dc (as c) of the same atoms with the pair-block weights gamma (nch * NBLKP).
+// y = dE/dc (as c) of the same atoms with the pair-block weights gamma (nch * NBLKP, from
+// launch_block_weights).
 template <typename T>
 cudaError_t launch_lane_y(const DevTables& tb, const DevBatch& b, const BsoParams& p, int first, int count,
-                          const void* c, const T* gamma, void* y, cudaStream_t st);
+                          const void* c, const void* gamma, void* y, cudaStream_t st);
 
 // Y rows of `count` rows of Z terms, [position][nch][NYP], and from them and c (by position) B and
 // w_ch * dB (whole-batch arrays) of atoms first .. first + count - 1, or of order[0 .. count - 1]
@@ -489,11 +490,14 @@ cudaError_t launch_eval_gather(const DevBatch& b, const BsoParams& p, const int*
 size_t atom_order_tmp_ints(int maxnn);
 cudaError_t launch_atom_order(const int* nn, int A, int maxnn, int* order, int* tmp, cudaStream_t st);
 // The pair-block weights gamma (nch * NBLKP per atom) of beta_a = w_lin + Wsym B_a and the energies
-// Eatom_a = w0 + B_a . (beta_a + w_lin) / 2; with B null the pair-block weights (nch * NBLKP) of
-// beta = w_lin, once (eval.cu).  wsym32: Wsym as double-FP32 pairs (launch_split_pairs), for T = float.
+// Eatom_a = w0 + B_a . (beta_a + w_lin) / 2 (eval.cu).  wsym32: Wsym as double-FP32 pairs
+// (launch_split_pairs), for T = float.
 template <typename T>
 cudaError_t launch_eval_gamma(const DevTables& tb, const T* B, int A, int nch, const double* wlin, const double* wsym,
                               const float2* wsym32, double w0, T* gamma, double* Eatom, cudaStream_t st);
+// The pair-block weights (nch * NBLKP) of beta = w_lin: FP64, or double-FP32 pairs for T = float.
+template <typename T>
+cudaError_t launch_block_weights(const DevTables& tb, int nch, const double* wlin, void* gamma, cudaStream_t st);
 cudaError_t launch_split_pairs(const double* in, float2* out, size_t n, cudaStream_t st);
 
 // FP64 Gram and rhs on the CUDA cores; with ws (gram_workspace_doubles(M, D) doubles) the
