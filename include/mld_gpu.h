@@ -122,8 +122,8 @@ int mld_gpu_set_labels(mld_gpu_handle* h, const double* energy, const double* fo
 int mld_gpu_descriptors(mld_gpu_handle* h, double* B_out, int* n_neigh_out);
 
 /* Per-pair derivatives dB/du of the structures of the last mld_gpu_descriptors call (computed
- * here, when dB_out is given: a caller that wants only the descriptors does not pay for them), in
- * neighbour-list order:
+ * here, when dB_out is given for the first time: a caller that wants only the descriptors does not pay
+ * for them; further calls copy them until another call forms the lists again), in neighbour-list order:
  * nbr_out[P] (global atom index of each neighbour, per centre atom in order), u_out[3*P]
  * (x_neighbour - x_centre), dB_out[3*dim_desc*P] (derivative with the sign of
  * descriptors.F90:298-302).  *P_inout: capacity in pairs on input, pairs on output. */

@@ -58,6 +58,7 @@ struct mld_gpu_handle {
   DevBatch b;
   bool has_batch = false;
   bool nbr_valid = false;
+  bool dB_valid = false;  // B_DBOUT holds the derivatives of the lists (mld_gpu_descriptor_derivatives)
   int max_nn = 0;
   // neighbours per atom that the single-pass search reserves: 1.5 x the densest structure's
   // mean count within r_cut, + 8 (at most imm_neigh); an atom above it reruns the two passes
@@ -310,6 +311,7 @@ inline void nl(mld_gpu_handle* h, long long n) { h->cur_launches += n; }
 int build_neighbours(mld_gpu_handle* h) {
   if (!h->has_batch) return fail(h, MLD_ERR_STATE, "no structures staged");
   DevBatch& b = h->b;
+  h->dB_valid = false;
   CK(ensure(h, mld_gpu_handle::B_NN, sizeof(int) * std::max(1, h->A)));
   CK(ensure(h, mld_gpu_handle::B_NBR_OFF, sizeof(int) * (h->A + 1)));
   CK(ensure(h, mld_gpu_handle::B_SCAN_TMP, sizeof(int) * ((h->A + 1023) / 1024 + 2)));
@@ -1501,12 +1503,15 @@ int mld_gpu_descriptor_derivatives(mld_gpu_handle* h, long long* P_inout, int* n
   if (u_out) CK(cudaMemcpyAsync(u_out, h->b.nbr_u, sizeof(double) * 3 * P, cudaMemcpyDeviceToHost, h->st));
   const size_t nd = (size_t)P * 3 * h->KK;
   if (dB_out) {
-    // the derivatives of the staged batch; its B come along
-    const size_t nB = std::max<size_t>((size_t)h->A * h->KK, 1);
-    CK(ensure(h, mld_gpu_handle::B_BOUT, (h->mixed ? sizeof(float) : sizeof(double)) * nB));
-    const int rc = h->mixed ? run_descriptors<float>(h, true, bp_<float>(h, mld_gpu_handle::B_BOUT))
-                            : run_descriptors<double>(h, true, bp_<double>(h, mld_gpu_handle::B_BOUT));
-    if (rc) return rc;
+    // the derivatives of the staged batch, unless a call like this one has left them; its B come along
+    if (!h->dB_valid) {
+      const size_t nB = std::max<size_t>((size_t)h->A * h->KK, 1);
+      CK(ensure(h, mld_gpu_handle::B_BOUT, (h->mixed ? sizeof(float) : sizeof(double)) * nB));
+      const int rc = h->mixed ? run_descriptors<float>(h, true, bp_<float>(h, mld_gpu_handle::B_BOUT))
+                              : run_descriptors<double>(h, true, bp_<double>(h, mld_gpu_handle::B_BOUT));
+      if (rc) return rc;
+      h->dB_valid = true;
+    }
     if (h->mixed) {
       std::vector<float> tmp(nd);
       CK(cudaMemcpyAsync(tmp.data(), bp_<float>(h, mld_gpu_handle::B_DBOUT), sizeof(float) * nd,
