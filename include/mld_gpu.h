@@ -209,12 +209,13 @@ int mld_gpu_solve_info(const mld_gpu_handle* h, int* pcg_iterations /*[2]*/, dou
 
 /* Launch shape of the descriptor kernels chosen by the handle's autotuner for one output mode
  * (0: design rows, i.e. B and dB; 1: evaluation with fitted weights; 2: descriptors only).  Only
- * mode 0 is tuned (modes 1 and 2 run other kernels and report the default shape).  The tuner times every candidate once on the first batch with
- * enough atoms (64 per SM) and keeps the fastest;
- * all candidates give bitwise the same results.  shape[4] = {column tile (4 or 2), persistent
- * CTAs per SM (0 = as many as fit), longest-first queue (1) or index order (0), tuned (1/0)};
- * *ncand: capacity of ms on input, candidates timed on output; ms[i] the time [ms] of candidate
- * i in the order (column tile 4, 2) x (CTAs per SM max, 1) x (queue sorted, index).
+ * mode 0 is tuned (modes 1 and 2 run other kernels and report the default shape).  The tuner times
+ * every candidate once on the first batch with enough atoms (64 per SM) and keeps the fastest; all
+ * candidates give bitwise the same results.  shape[4] = {column tile (4 or 2), persistent CTAs per SM
+ * (0 = as many as fit, always), longest-first queue (1) or index order (0), tuned (1/0)}; *ncand:
+ * capacity of ms on input, candidates on output; ms[i] the time [ms] of candidate i in the order
+ * (column tile 4, 2) x (CTAs per SM max, 1) x (queue sorted, index).  The tuned kernel runs one CTA per
+ * SM whatever is asked, so the two candidates that differ in that are one run and have one time.
  * (No reference counterpart.) */
 int mld_gpu_tuning(const mld_gpu_handle* h, int mode, int* shape, int* ncand, double* ms);
 

@@ -105,7 +105,6 @@ struct mld_gpu_handle {
   struct Tune {
     bool done = false;
     Bso4Launch best;
-    std::vector<Bso4Launch> cand;
     std::vector<float> ms;
   } tune[3];
 
@@ -463,11 +462,12 @@ int launch_rows_descriptors(mld_gpu_handle* h, T* Bout, T* dB, const Bso4Launch&
   return MLD_OK;
 }
 
-// Autotuner of the descriptor kernel's launch shape for the design rows of a fit: on the first
-// batch large enough (at least kTuneMinAtoms atoms per SM) each candidate shape (column tile 4 or 2, as many persistent CTAs
-// per SM as fit or one, longest-first or index-order queue) runs once on the real batch, timed
-// with CUDA events on the handle's stream, and the fastest is kept for the handle.  Every shape
-// computes bitwise the same outputs, so the last candidate's run is the result.
+// Autotuner of the launch shape of the design rows of a fit: on the first batch large enough (at least
+// kTuneMinAtoms atoms per SM) each candidate shape (column tile of k_deriv 4 or 2, longest-first or
+// index-order queue) runs once on the real batch, timed with CUDA events on the handle's stream, and
+// the fastest is kept for the handle.  Every shape computes bitwise the same outputs, so the last
+// candidate's run is the result.  The report (mld_gpu_tuning) has a place for the CTAs per SM between
+// the two, of which k_deriv runs one whatever is asked: both of its entries are the one run.
 constexpr int kTuneMinAtoms = 64;
 
 template <typename T>
@@ -481,29 +481,28 @@ int tuned_launch(mld_gpu_handle* h, T* Bout, T* dB) {
     nl(h, launches);
     return rc;
   }
-  tn.cand.clear();
   tn.ms.clear();
-  for (int ct : {4, 2})
-    for (int cps : {0, 1})
-      for (int sorted : {1, 0}) tn.cand.push_back(Bso4Launch{ct, cps, sorted});
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   CK(cudaEventCreate(&ev0));
   CK(cudaEventCreate(&ev1));
   float best = 0.f;
-  for (const Bso4Launch& c : tn.cand) {
-    CK(cudaEventRecord(ev0, h->st));
-    const int rc = launch_rows_descriptors<T>(h, Bout, dB, c, &launches);
-    nl(h, launches);
-    if (rc) return rc;
-    CK(cudaEventRecord(ev1, h->st));
-    CK(cudaEventSynchronize(ev1));
-    float ms = 0.f;
-    CK(cudaEventElapsedTime(&ms, ev0, ev1));
-    tn.ms.push_back(ms);
-    if (tn.ms.size() == 1 || ms < best) {
-      best = ms;
-      tn.best = c;
+  for (int ct : {4, 2}) {
+    float ms[2] = {0.f, 0.f};
+    for (int index_order : {0, 1}) {
+      const Bso4Launch c{ct, 1 - index_order};
+      CK(cudaEventRecord(ev0, h->st));
+      const int rc = launch_rows_descriptors<T>(h, Bout, dB, c, &launches);
+      nl(h, launches);
+      if (rc) return rc;
+      CK(cudaEventRecord(ev1, h->st));
+      CK(cudaEventSynchronize(ev1));
+      CK(cudaEventElapsedTime(&ms[index_order], ev0, ev1));
+      if ((ct == 4 && !index_order) || ms[index_order] < best) {
+        best = ms[index_order];
+        tn.best = c;
+      }
     }
+    tn.ms.insert(tn.ms.end(), {ms[0], ms[1], ms[0], ms[1]});
   }
   cudaEventDestroy(ev0);
   cudaEventDestroy(ev1);
@@ -2087,7 +2086,7 @@ extern "C" int mld_gpu_tuning(const mld_gpu_handle* h, int mode, int* shape, int
   if (!h || mode < 0 || mode > 2 || !shape || !ncand) return MLD_ERR_INVALID;
   const auto& tn = h->tune[mode];
   shape[0] = tn.best.col_tile;
-  shape[1] = tn.best.ctas_per_sm;
+  shape[1] = 0;  // as many as fit
   shape[2] = tn.best.sorted_queue;
   shape[3] = tn.done ? 1 : 0;
   const int n = std::min<int>(*ncand, (int)tn.ms.size());

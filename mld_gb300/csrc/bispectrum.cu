@@ -533,7 +533,6 @@ cudaError_t launch_bso4(const DevTables& tb, const DevBatch& b, const BsoParams&
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kNW * 32, smem);
   if (e != cudaSuccess) return e;
   if (occ < 1) return cudaErrorInvalidConfiguration;
-  if (sh.ctas_per_sm > 0) occ = std::min(occ, sh.ctas_per_sm);
   long long grid = std::min<long long>((long long)b.A, (long long)nsm * occ);
   if (!y_in_smem) {
     // one Y slice per persistent CTA

@@ -407,7 +407,6 @@ bool bso4_available(const DevTables& tb, int nch, int eb);
 struct Bso4Launch {
   int col_tile = 2;      // columns per register tile of k_deriv's contraction: 2 or 4 (492,000 Fe atoms: 58
                          // against 62 ms; wider tiles leave long jobs to few warps at the end of a phase)
-  int ctas_per_sm = 0;   // persistent CTAs per SM (0: as many as fit)
   int sorted_queue = 1;  // atoms longest first (1) or in index order (0)
 };
 // c (count x nch x HU complex of T) of atoms first .. first + count - 1, or of order[0 .. count - 1]
