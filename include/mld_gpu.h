@@ -95,6 +95,7 @@ void mld_gpu_config_defaults(mld_gpu_config* cfg);
 
 /* Create a handle on the current CUDA device (init_descriptors, descriptors.F90:658-671). */
 int mld_gpu_create(const mld_gpu_config* cfg, mld_gpu_handle** out);
+/* NULL: gives back the workspace that mld_gpu_gram_rows keeps on the current device */
 void mld_gpu_destroy(mld_gpu_handle* h);
 const char* mld_gpu_last_error(const mld_gpu_handle* h);
 
@@ -273,8 +274,12 @@ int mld_gpu_server_admission(const mld_gpu_server* s, double* peak_bytes_in_flig
  * X holds M rows of D values with a row stride of ldx elements, FP64 (x_is_fp32 = 0) or FP32.
  * method MLD_PRECISION_PLAIN_FP64: FP64 accumulation on the CUDA cores; MLD_PRECISION_MIXED:
  * tensor cores in BF16 split precision (x = hi + lo, hi*hi + hi*lo + lo*hi) with FP32
- * accumulation per row split and FP64 accumulation across splits.  Allocates and frees its own
- * workspace; `stream` may be NULL; returns after the stream has synchronised. */
+ * accumulation per row split and FP64 accumulation across splits.  `stream` may be NULL; returns after
+ * the stream has synchronised.  The workspace comes from a memory pool of the library's own, of which at
+ * most 512 MiB per device stay mapped for later calls of any thread and stream; larger workspaces are
+ * unmapped before the call returns.  mld_gpu_destroy gives the kept memory of the device back: of any
+ * handle on it, or mld_gpu_destroy(NULL) for the current device.  A handle that runs out of memory takes
+ * it first.  (cudaDeviceReset ends the pool as it ends handles: neither may be used after it.) */
 int mld_gpu_gram_rows(int method, const void* X, int x_is_fp32, long long M, int D, int ldx, const double* w,
                       const double* y, double* G, double* rhs, void* stream, char* err, int err_len);
 
