@@ -5,8 +5,8 @@ with 0-3 extra vacancies, sigma = 0.08 A noise, +-2 % strain, Morse labels; bisp
 (55 components), r_cut = 4.7 A, linear model (1 + 55 columns), energy + 3N force + 6 stress
 rows per structure, ridge lambda = 1e-8, min-norm solve.  Seeded synthetic data (no dataset).
 
-One step = one full fit of the whole set on the GPU: neighbour lists, fused descriptor +
-design-row kernel, weighted Gram, ridge solve, train predictions/RMSE.
+One step = one full fit of the whole set on the GPU: neighbour lists, descriptors, their derivatives
+and the design rows, weighted Gram, ridge solve, train predictions/RMSE.
 
   value   design rows / s of the mixed method (FP32 descriptors and rows, FP64 Gram and solve),
           inputs resident in HBM, device time from CUDA events on the library's stream;
@@ -139,20 +139,57 @@ def make_dataset(n_struct):
     return synth.fe_bcc_batched(n_struct=n_struct, rcut=RCUT, workers=min(16, os.cpu_count() or 1))
 
 
-def flops_model(wc, n_pairs, n_atoms):
-    """Algorithmic FLOPs of one launch of the fused descriptor kernel (per atom and per pair).
+def contraction_counts(J):
+    """Sizes of the contractions of one channel at doubled angular momentum J, on half layers: products
+    of c (a pair of operand layers at an output position, once for all its output layers), the sums of
+    them into Z terms (complex by real), entries of the Y rows (triple, layer) and terms in them."""
+    triples = [(a, b, c) for a in range(J + 1) for b in range(a + 1) for c in range(a - b, min(J, a + b) + 1)
+               if (a + b + c) % 2 == 0 and c >= a]
+    half = [((j + 1) ** 2 + 1) // 2 for j in range(J + 1)]
+    outs = {}
+    for l1, l2, l in triples:  # the blocks (operands, output) that a triple needs
+        for a, b, o in ((l1, l2, l), (l, l2, l1), (l1, l, l2)):
+            outs.setdefault((max(a, b), min(a, b)), set()).add(o)
+    n = {"products": 0, "sums": 0, "row_entries": sum(half[j] for t in triples for j in set(t)),
+         "row_terms": sum(half[j] for t in triples for j in t), "triples": len(triples), "half": sum(half),
+         "rows": sum(len(set(t)) for t in triples)}
+    for (a, b), layers in outs.items():
+        top = max(layers)
+        places = [(m1, m2) for m1 in range(-top, top + 1, 2) for m2 in range(-top, top + 1, 2)][:half[top]]
+        for m1, m2 in places:
+            na, nb = ((min(a, m + b) - max(-a, m - b)) // 2 + 1 for m in (m1, m2))
+            n["products"] += na * nb
+            n["sums"] += sum(o >= max(abs(m1), abs(m2)) for o in layers) * (na * nb + na)
+    return n
 
-    Per neighbour pair: U recursion (8 flops for a one-term entry, 18 for a two-term entry),
-    f_c*w*U accumulation (4 per entry per channel), U+dU recursion (U as above plus 54 per source
-    term), vecall (12 per entry), dB contraction (3 components x 4 flops per merged Y slot per
-    channel) and the row scatter (3*K adds per channel).  Per atom: the Z contraction (8 flops per
-    CG term + 2 per row extent + 4 per output for the scale) and B (4 flops per ZA slot), per
-    channel."""
-    nch, NU, one, two = wc["nch"], wc["NU"], wc["u_one_term"], wc["u_two_term"]
-    u_flops = 8 * one + 18 * two
-    per_pair = (u_flops + 4 * NU * nch) + (u_flops + 54 * (one + 2 * two) + 12 * NU) + \
-        nch * (12 * wc["y_slots"] + 3 * wc["K"])
-    per_atom = nch * (8 * wc["cg_terms"] + 2 * wc["z_row_extents"] + 4 * wc["z_outputs"] + 4 * wc["y_slots_za"])
+
+def chain_flops(J):
+    """U of a neighbour by column chains: column 0 of layer d from powers, then one column per layer."""
+    n = 0
+    for d in range(1, J + 1):
+        n += 6 * (d - 1) + 14 * (d - 1)
+        for s in range(d + 1):
+            if d + s > J:
+                break
+            n += 2 * (d + 1 if s == d else d + s + 1)      # normalised and stored
+            if s < d and d + s < J:
+                n += 12 + 14 * (d + s)                     # the next column
+    return n
+
+
+def flops_model(wc, n_pairs, n_atoms):
+    """FLOPs that the descriptor kernels (k_c_half, k_lanes, k_y_rows, k_deriv) cannot do without: every
+    quantity once, though U is formed by two of them.
+
+    Per neighbour pair: U by column chains, its sum into c (4 per half entry and channel), the three
+    generator products (27 per half entry), their contraction with the Y rows (3 x 4 per row entry and
+    channel), the ranks' sums and the three components (18 per triple and channel).  Per atom and channel:
+    the products of c (6 each), their sums into Z terms (4 each), the Y rows (4 per term, 2 per entry) and
+    B = Y.c / 3 (4 per row entry)."""
+    nch, n = wc["nch"], contraction_counts(int(round(2 * J_MAX)))
+    per_pair = chain_flops(int(round(2 * J_MAX))) + n["half"] * (4 * nch + 27) + \
+        nch * (12 * n["row_entries"] + 3 * (n["rows"] - n["triples"]) + 18 * n["triples"])
+    per_atom = nch * (6 * n["products"] + 4 * n["sums"] + 4 * n["row_terms"] + 6 * n["row_entries"] + n["triples"])
     return per_pair * n_pairs + per_atom * n_atoms, per_pair, per_atom
 
 
