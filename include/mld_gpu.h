@@ -93,7 +93,11 @@ typedef struct mld_gpu_handle mld_gpu_handle;
 /* Fill *cfg with the reference's namelist defaults (read_ml_file.F90:307-611). */
 void mld_gpu_config_defaults(mld_gpu_config* cfg);
 
-/* Create a handle on the current CUDA device (init_descriptors, descriptors.F90:658-671). */
+/* Create a handle on the current CUDA device (init_descriptors, descriptors.F90:658-671).
+ * j_max up to 5, every channel count.  In FP64 at j_max 5, and at 4.5 with two or three channels, the
+ * descriptors (mld_gpu_descriptors, mld_gpu_descriptors_noalloc) and the evaluation (mld_gpu_evaluate, the
+ * server) work; the derivatives and what is built on design rows (design matrix, gram, fit, predict)
+ * return MLD_ERR_CUDA (no launch shape). */
 int mld_gpu_create(const mld_gpu_config* cfg, mld_gpu_handle** out);
 /* NULL: gives back the workspace that mld_gpu_gram_rows keeps on the current device */
 void mld_gpu_destroy(mld_gpu_handle* h);
@@ -135,6 +139,9 @@ int mld_gpu_descriptor_derivatives(mld_gpu_handle* h, long long* P_inout, int* n
  * as the has_efs flags and desc_forces select). */
 int mld_gpu_num_rows(mld_gpu_handle* h, long long* M);
 
+/* Repeated calls on one batch give bitwise the same rows (and derivatives).  Another batch may give a
+ * structure's rows other last bits: batches of up to an atom per SM take another kernel than larger ones.
+ * The evaluation of a structure does not depend on its batch. */
 /* Build and return the design matrix A[M*dim_design_line], labels y[M] and row weights w[M]
  * (any may be NULL). */
 int mld_gpu_design_matrix(mld_gpu_handle* h, double* A, double* y, double* w);

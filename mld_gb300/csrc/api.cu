@@ -390,9 +390,12 @@ constexpr size_t kKrrTcWorkspaceCap = size_t(6) << 30;
 // Route of B with dB.  More atoms than SMs: Z terms with atoms on lanes, Y rows, derivatives
 // (bispectrum_deriv.cu).  Up to an atom per SM, and for tables too large for it, the one kernel that
 // forms Z itself, a CTA per atom (bispectrum.cu): the tiles of lanes are then few and three launches go.
-// Design rows of one Fe structure at j_max 4, one kernel / three: 100 atoms FP64 0.69 / 1.00 ms, FP32
-// 309 / 349 us; 250 atoms 1.33 / 1.28 ms, 426 / 418 us; 1000 atoms FP64 3.38 / 3.12 ms; 23,000 FP32
-// atoms in 60 structures at j_max 2, FP64: 5.2 / 3.2 ms.
+// Predictions of one Fe structure at j_max 4, one kernel / four: 100 atoms FP64 570 / 598 us, FP32 187 /
+// 212; 152 atoms (one per SM) 642 / 696, 228 / 258; 160 atoms FP64 946 / 896; 300 atoms 1115 / 1062,
+// 258 / 294; 1000 atoms 3.04 / 2.53 ms, 398 / 398 us.  60 structures, j_max 2, FP64: 5.2 / 3.2 ms.  In FP32
+// the one kernel is ahead up to some 1000 atoms, by the 30 us of the launches; the line is FP64's.
+// The routes sum in different orders, so a structure's rows may differ in their last bits between
+// batches on either side of the line (one route for all would cost small batches the difference above).
 template <typename T>
 bool deriv_route(const mld_gpu_handle* h) {
   // (a configuration is taken or refused whatever the batch)

@@ -19,7 +19,8 @@
 // land in a term buffer from which the Y rows and B are summed, and the dB contraction writes
 // each layer row into the buffer of its rank (a triple's distinct layers in ascending order),
 // where every triple has at most one row, so dB = (rank 0 + rank 1) + rank 2.  Results are
-// therefore bitwise reproducible and do not depend on which CTA takes which atom.
+// therefore bitwise reproducible and do not depend on which CTA takes which atom.  (Batches of more
+// atoms take other kernels, whose sums run in another order.)
 //
 // CTAs are persistent: they stage the small tables in shared memory once, then pull atoms from a
 // queue (ordered by descending neighbour count, or in index order, whichever the launch-shape
@@ -514,8 +515,8 @@ cudaError_t launch_bso4(const DevTables& tb, const DevBatch& b, const BsoParams&
   size_t smem = smem_plan(tb, p.nch, sizeof(T), y_in_smem, a.g1).total;
   if (smem > (size_t)max_optin_smem()) return cudaErrorInvalidConfiguration;
   // geometry records for the first geo_cap neighbours of an atom (at most 128), as many as keep
-  // the resident CTAs per SM as they are.  The count depends on the configuration only, not on
-  // the batch, so that an atom's results do not depend on the batch it is evaluated in.
+  // the resident CTAs per SM as they are.  The count depends on the configuration only, so an atom's
+  // results are the same in every batch that takes this kernel (larger ones round differently).
   a.geo_cap = 0;
   for (int cap = 128; cap > 0; cap -= 8) {
     const size_t sc = smem_plan(tb, p.nch, sizeof(T), y_in_smem, a.g1, cap).total;

@@ -6,7 +6,8 @@
 //   k_deriv   dB_k/du_a = w_ch(type_n) sum_b xi[a][b] Re sum Y_k V_b, V_b = f_c U rho(T_b) + kappa_b U
 //             (bispectrum.cuh); B = dB/dc . c / 3, since B is a cubic form of c
 //
-// Every sum has a fixed order that depends neither on the batch nor on the launch shape.
+// Every sum has a fixed order that depends neither on the batch, among those that take these kernels
+// (deriv_route, api.cu), nor on the launch shape.
 #include <cuda_runtime.h>
 
 #include <algorithm>

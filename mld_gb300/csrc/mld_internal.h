@@ -62,28 +62,21 @@ static_assert(offsetof(ZItem, i2) == 2 && offsetof(ZItem, cg1) == 4 && offsetof(
               "ZItem layout");
 constexpr uint16_t kNoTerm = 0xFFFF;
 
-// One folded Y slot for the kernel (16 bytes): Y[ypos] = wgt * sum_t (snum_t / sden_t) Z[term_t].
+// One folded Y slot with its distinct terms (host only; the kernels take the rows' sources instead, whose
+// order tests compare with it): Y[ypos] = wgt * sum_t (snum_t / sden_t) Z[term_t].
 struct SlotEntry {
   uint16_t term[3];
   uint16_t ypos;
   uint8_t nterm, wgt;
   uint8_t snum[3], sden[3];
 };
-static_assert(sizeof(SlotEntry) == 16, "slot entries are 16 bytes");
-static_assert(offsetof(SlotEntry, ypos) == 6 && offsetof(SlotEntry, nterm) == 8 && offsetof(SlotEntry, wgt) == 9 &&
-                  offsetof(SlotEntry, snum) == 10 && offsetof(SlotEntry, sden) == 13,
-              "SlotEntry layout (decoded from its words by the descriptor kernel)");
-// snum and sden are doubled angular momenta + 1 <= kMaxJ + 1; the descriptor kernel looks
-// snum / sden up in a 16 x 16 table
-static_assert(kMaxJ + 1 < 16, "slot scales index a 16 x 16 table");
 
-// One ZA half entry of a triple: B_k = sum over its entries of wgt * Re(conj(c[ufull]) Z[term]).
+// One ZA half entry of a triple (host only, as SlotEntry): B_k = sum over its entries of
+// wgt * Re(conj(c[ufull]) Z[term]).
 struct BkItem {
   uint16_t term, ufull;
   uint8_t wgt, pad[3];
 };
-static_assert(sizeof(BkItem) == 8, "B items are 8 bytes");
-static_assert(offsetof(BkItem, ufull) == 2 && offsetof(BkItem, wgt) == 4, "BkItem layout (decoded by the descriptor kernel)");
 
 // A record of the atoms-on-lanes sums (bispectrum_lanes.cu; 32 bytes): for an operand pair jA >= jB and
 // an output position (m1, m2), the Z terms of nj of the pair's output layers in descending jO,
@@ -157,7 +150,8 @@ struct Bso4Tables {
   std::vector<int> tiles;       // row tiles (j << 8 | rt), heaviest layers first
   int nrank[kRounds] = {0};     // triples with a row of rank r (rank 0: all K)
   std::vector<int16_t> rank_slot;  // K x (kRounds - 1): slot of triple k in the rank-1 / rank-2 buffers, -1 none
-  // recursion on half layers: U = tz*Zsel*U[src_z] + tx*(-i)*Xsel*U[src_x]
+  // recursion on half layers, U = tz*Zsel*U[src_z] + tx*(-i)*Xsel*U[src_x] (host only: the kernels run
+  // column chains)
   std::vector<double> rec_tz, rec_tx;
   std::vector<int16_t> rec_sz, rec_sx;
   std::vector<int8_t> rec_qneg;
