@@ -233,6 +233,7 @@ struct TablePack {
   cudaError_t upload(mld_gpu_handle* h) {
     unsigned char* base = nullptr;
     cudaError_t e = cudaMalloc((void**)&base, bytes.size());
+    if (e != cudaSuccess) (void)cudaGetLastError();  // as in grab
     if (e != cudaSuccess) return e;
     h->owned.push_back(base);
     for (const auto& s : slots) {
@@ -2181,7 +2182,9 @@ struct RowsWorkspace {
     cudaMemPool_t pool = nullptr;
     cudaError_t e = rows_pool(dev, &pool);
     st = stream;
-    return e == cudaSuccess ? cudaMallocFromPoolAsync(&p, bytes, pool, st) : e;
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&p, bytes, pool, st);
+    if (e != cudaSuccess) (void)cudaGetLastError();  // as in grab
+    return e;
   }
   // after the last launch that uses it and before the stream is waited for: what exceeds
   // kRowsPoolKeep is unmapped by that wait
