@@ -116,7 +116,8 @@ struct mld_gpu_handle {
   long long rows_graph_launches = 0;
   bool rows_graph_off = false;  // a capture failed once: run the stage directly from then on
 
-  size_t z_cap = kZCap;     // Z terms and Y rows of a pass: less once they did not fit (ensure_passes)
+  size_t z_limit = kZCap;   // Z terms and Y rows of a pass at most (test hook)
+  size_t z_cap = kZCap;     // and for the staged batch: less where they did not fit (ensure_passes)
   size_t buffer_limit = 0;  // test hook: bytes that the buffers may take together (0: what the device has)
 
   std::vector<void*> owned;  // table allocations
@@ -166,19 +167,18 @@ cudaError_t grab(mld_gpu_handle* h, void** p, size_t bytes) {
   return e;
 }
 
-// Frees the Z terms and Y rows and halves what a later pass may take; false if there were none.
-bool shrink_passes(mld_gpu_handle* h) {
-  size_t held = 0;
+// Frees the Z terms and Y rows, which the next call takes again in passes of what is then left; false if
+// there were none.
+bool free_passes(mld_gpu_handle* h) {
+  bool any = false;
   for (int id : {mld_gpu_handle::B_ZT, mld_gpu_handle::B_YSCR}) {
     Buf& bf = h->bufs[id];
     if (bf.p) cudaFree(bf.p);
-    held += bf.cap;
+    any |= bf.p != nullptr;
     bf = Buf{};
   }
-  if (!held) return false;
-  ++h->buf_gen;
-  h->z_cap = std::min(h->z_cap, held / 2);
-  return true;
+  if (any) ++h->buf_gen;
+  return any;
 }
 
 cudaError_t ensure(mld_gpu_handle* h, int id, size_t bytes) {
@@ -198,7 +198,7 @@ cudaError_t ensure(mld_gpu_handle* h, int id, size_t bytes) {
   // passes can be smaller; so do without: the passes' own buffers (ensure_passes), optional workspaces
   const bool own = id == mld_gpu_handle::B_ZT || id == mld_gpu_handle::B_YSCR;
   const bool optional = id == mld_gpu_handle::B_NBRTMP || id == mld_gpu_handle::B_GP;
-  if (e == cudaErrorMemoryAllocation && !own && !optional && shrink_passes(h)) e = grab(h, &bf.p, want);
+  if (e == cudaErrorMemoryAllocation && !own && !optional && free_passes(h)) e = grab(h, &bf.p, want);
   if (e != cudaSuccess) return e;
   bf.cap = want;
   return cudaSuccess;
@@ -430,7 +430,7 @@ int ensure_passes(mld_gpu_handle* h, bool rows, int* pass) {
       CK(e);
       return MLD_OK;
     }
-    shrink_passes(h);
+    free_passes(h);
     h->z_cap = (zb + yb) / 2;
   }
 }
@@ -1433,6 +1433,8 @@ int mld_gpu_set_structures(mld_gpu_handle* h, int nstruct, const int* nat, const
   h->has_batch = true;
   h->nbr_valid = false;
   h->has_labels = false;
+  if (h->z_cap != h->z_limit) ++h->buf_gen;  // (a graph of the rows is that of its passes)
+  h->z_cap = h->z_limit;
   return MLD_OK;
 }
 
@@ -1963,7 +1965,7 @@ void handle_release_buffers(mld_gpu_handle* h) {
     bf.p = nullptr;
     bf.cap = 0;
   }
-  h->z_cap = kZCap;
+  h->z_cap = h->z_limit;
   h->has_batch = false;
   h->nbr_valid = false;
 }
@@ -2113,7 +2115,7 @@ extern "C" int mld_gpu_test_pipeline_timeout(int skip_loads, long long wait_limi
 
 extern "C" int mld_gpu_test_memory(mld_gpu_handle* h, long long pass_bytes, long long buffer_limit) {
   if (!h || pass_bytes < 0 || buffer_limit < 0) return MLD_ERR_INVALID;
-  h->z_cap = pass_bytes ? (size_t)pass_bytes : kZCap;
+  h->z_limit = h->z_cap = pass_bytes ? (size_t)pass_bytes : kZCap;
   h->buffer_limit = (size_t)buffer_limit;
   ++h->buf_gen;
   return MLD_OK;

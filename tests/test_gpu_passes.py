@@ -68,3 +68,24 @@ def test_passes_shrink_to_the_memory(lib, precision, limit):
         assert lib.mld_gpu_test_memory(h._h, 0, 0) == 0
         for a, b in zip(_all(h, structs, w), want):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_a_fit_replays_its_rows_after_smaller_passes(lib, precision):
+    """Rows of a batch in whole passes, in smaller ones and in whole ones again, through one handle whose
+    later calls replay a captured graph of them."""
+    from mld_gb300 import _lib, synth
+    ds = synth.fe_bcc_batched(n_struct=70, nmin=100, nmax=300, seed=51)
+    nat, pos, cell, types = ds.arrays()
+    E, F, S, has = ds.labels()
+    c = _lib.default_config()
+    c.j_max, c.r_cut, c.lambda_krr, c.precision = 2.0, 4.7, 1e-8, precision
+    with _lib.Handle(c) as h:
+        got = []
+        for pass_bytes in (0, 1 << 20, 0):
+            assert lib.mld_gpu_test_memory(h._h, pass_bytes, 0) == 0
+            h.set_structures(nat, pos, cell, types)
+            h.set_labels(E, F, S, has, np.ones((len(nat), 3)))
+            got += [h.design_matrix()[0] for _ in range(3)]  # tuned, captured, replayed
+    for a in got[1:]:
+        assert np.array_equal(a, got[0])
